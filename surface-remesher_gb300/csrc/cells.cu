@@ -44,8 +44,15 @@
 //
 // Work split.  k_cell runs one warp per block, as many blocks as fit on the
 // GPU; each warp takes the next group of 32 listed sites from a ticket, one
-// site per lane.  A lane keeps its site's candidates as 8-byte records and
-// bounds two rows per pass over them.  The energy is reduced in a fixed order
+// site per lane.  A lane keeps its site's candidates as two bytes each, bounds
+// eight rows per pass over them in floats (cell_float: exact where float_walk
+// says so, else cell_general's integer division), lists the rows and sums
+// their pixels two rows at a time in packed FP32.  What bounds it: issue slots
+// and the latency of L1 misses, not bandwidth (60 MB an iteration).  Against
+// integer bounds row pair by row pair and scalar sums: 118 -> 81 us an
+// iteration at 4096^2 / 262,144 sites (75.5 -> 46.2 M warp instructions), 0.42
+// -> 0.28 ms at 8192^2.  Records of 8 bytes in shared memory (4 KB a warp) took
+// 120 us: they leave the density rows too little L1.  The energy is reduced in a fixed order
 // whatever warp takes which group: the sites of a group by a butterfly, 64
 // groups by the warp finishing the last of them, the 64-group totals by the
 // warp finishing the last 64-group; that warp also runs the schedule.  Sites move by atomicOr into the next bitmap;
@@ -79,6 +86,62 @@ __device__ __forceinline__ void dfa_scaled(float &ah, float &al, float k, float 
   const float ph = __fmul_rn(k, bh);
   const float pl = __fmaf_rn(k, bh, -ph) + k * bl;
   dfa(ah, al, ph, pl);
+}
+
+// Two floats in one 64-bit register: the packed FP32 instructions of sm_100+
+// do both halves in one issue slot, each half rounded as the scalar
+// instruction rounds it.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float f2_lo(F2 a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+  return x;
+}
+__device__ __forceinline__ float f2_hi(F2 a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+  return y;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+// a - b: the product b * -1 is exact, so the sum is rounded once
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, f2(-1.f, -1.f), a); }
+
+// dfa on both halves: (ah, al) += (bh, bl).
+__device__ __forceinline__ void dfa2(F2 &ah, F2 &al, F2 bh, F2 bl) {
+  const F2 s = add2(ah, bh), bp = sub2(s, ah), ap = sub2(s, bp);
+  F2 e = add2(sub2(ah, ap), sub2(bh, bp));
+  e = add2(e, add2(al, bl));
+  ah = add2(s, e);
+  al = sub2(e, sub2(ah, s));
+}
+// the same with bl = 0
+__device__ __forceinline__ void dfa2_0(F2 &ah, F2 &al, F2 bh) {
+  const F2 s = add2(ah, bh), bp = sub2(s, ah), ap = sub2(s, bp);
+  F2 e = add2(sub2(ah, ap), sub2(bh, bp));
+  e = add2(e, al);
+  ah = add2(s, e);
+  al = sub2(e, sub2(ah, s));
 }
 
 // floor(sqrt(v)) and ceil(sqrt(v)) for 0 <= v < 2^30, exact.
@@ -241,9 +304,9 @@ __device__ __forceinline__ void row_sums(const float *__restrict__ row, int da, 
 
 // The pixels [da, db] of row v the cell with bounds [lo, hi] sums: clipped to
 // the density support and the covering disc; false when none.
-__device__ __forceinline__ bool row_span(const LevelBufs &a, int sx, int sy, int rb2, int v,
-                                         int lo, int hi, int &da, int &db) {
-  const int2 s = a.support[sy + v];
+__device__ __forceinline__ bool row_span(const int2 *__restrict__ support, int sx, int sy, int rb2,
+                                         int v, int lo, int hi, int &da, int &db) {
+  const int2 s = __ldg(support + sy + v);
   da = max(lo, s.x - sx), db = min(hi, s.y - 1 - sx);
   if (da > db) return false;
   if (max(da * da, db * db) + v * v > rb2) {  // clip to the covering disc
@@ -256,12 +319,13 @@ __device__ __forceinline__ bool row_span(const LevelBufs &a, int sx, int sy, int
 }
 
 // Row v of the cell with bounds [lo, hi]: its span, R2, its sums.
-__device__ __forceinline__ void take_row(const LevelBufs &a, int n, int sx, int sy, int rb2, int v,
-                                         int lo, int hi, int &R2, CellSums &c) {
+__device__ __forceinline__ void take_row(const float *__restrict__ density,
+                                         const int2 *__restrict__ support, int n, int sx, int sy,
+                                         int rb2, int v, int lo, int hi, int &R2, CellSums &c) {
   int da, db;
-  if (!row_span(a, sx, sy, rb2, v, lo, hi, da, db)) return;
+  if (!row_span(support, sx, sy, rb2, v, lo, hi, da, db)) return;
   R2 = max(R2, max(da * da, db * db) + v * v);
-  row_sums(a.density + (size_t)(sy + v) * n + sx, da, db, v, c);
+  row_sums(density + (size_t)(sy + v) * n + sx, da, db, v, c);
 }
 
 // A site in s's own column at row offset B != 0: s keeps the rows strictly on
@@ -309,74 +373,402 @@ __device__ __forceinline__ void gather_word(uint64_t w, int A, int B0, int sy, l
   }
 }
 
+// The float accumulators of a cell, packed: (W, SX) and (SY, E), two-float.
+struct CellAcc {
+  F2 wxh, wxl, yeh, yel;
+};
+
+// fold_chunk on the packed accumulators: the same operations in the same
+// order, two of the four sums per instruction (34 instructions instead of 56).
+__device__ __forceinline__ void fold_chunk2(CellAcc &c, float rw, float rx, float rq, float fv,
+                                            float fv2) {
+  dfa2_0(c.wxh, c.wxl, f2(rw, rx));
+  const F2 rr = f2(rw, rw), k = f2(fv, fv2);
+  const F2 nph = mul2(f2(-fv, -fv2), rr);  // -(v rw, v^2 rw)
+  const F2 pl = fma2(k, rr, nph);
+  const float ph = -f2_hi(nph);
+  float s, e;  // (rq, 0) += (ph, pl)
+  tsum_c(rq, ph, s, e);
+  e = __fadd_rn(e, f2_hi(pl));
+  const float qh = __fadd_rn(s, e);
+  const float ql = __fsub_rn(e, __fsub_rn(qh, s));
+  dfa2(c.yeh, c.yel, f2(-f2_lo(nph), qh), f2(f2_lo(pl), ql));
+}
+
+// The pixels of a row span as bits from its first aligned column, and that
+// column; an empty span has no bits.
+struct RowPix {
+  const float *p;  // the density at the first aligned column
+  unsigned m;
+  float dx;        // that column relative to the site
+};
+
+// chunk_sums of two rows at once (at most 16 pixels each): aligned 16-byte
+// loads, the first eight columns of both rows in flight together, the two rows
+// in the two halves of the packed instructions.  Pixels outside a span add
+// +-0, which changes no sum.
+__device__ __forceinline__ void pair_sums(const RowPix &a, const RowPix &b, F2 &rw, F2 &rx,
+                                          F2 &rq) {
+  const F2 one = f2(1.f, 1.f);
+  F2 dx = f2(a.dx, b.dx);
+  rw = rx = rq = f2(0.f, 0.f);
+  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 *pa = reinterpret_cast<const float4 *>(a.p);
+  const float4 *pb = reinterpret_cast<const float4 *>(b.p);
+  unsigned ma = a.m, mb = b.m;
+  float4 qa = ma ? __ldg(pa) : z, qb = mb ? __ldg(pb) : z;
+  float4 na = ma >> 4 ? __ldg(pa + 1) : z, nb = mb >> 4 ? __ldg(pb + 1) : z;
+  for (int k = 2;; ++k) {
+    const float va[4] = {qa.x, qa.y, qa.z, qa.w}, vb[4] = {qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const F2 p = f2((ma >> j) & 1u ? va[j] : 0.f, (mb >> j) & 1u ? vb[j] : 0.f);
+      const F2 t = mul2(dx, p);
+      rw = add2(rw, p);
+      rx = add2(rx, t);
+      rq = fma2(t, dx, rq);
+      dx = add2(dx, one);
+    }
+    ma >>= 4;
+    mb >>= 4;
+    if (!(ma | mb)) break;
+    qa = na;
+    qb = nb;
+    na = ma >> 4 ? __ldg(pa + k) : z;
+    nb = mb >> 4 ? __ldg(pb + k) : z;
+  }
+}
+
+// One attempt at the cell with the window radius W, general form: candidates
+// as integer records (or straight from the bitmap when they do not fit),
+// bounds by exact integer division.  Returns the cell's sums; c.r2 = max
+// |p - s|^2.
+__device__ __noinline__ CellSums cell_general(const float *__restrict__ density,
+                                              const int2 *__restrict__ support,
+                                              const uint64_t *__restrict__ bits, int n, int sx,
+                                              int sy, int W, int rb, int vmin, int vmax) {
+  int2 rec[kMaxCand];  // {K, S | D << 16} of the window's candidates
+  const int rb2 = rb * rb;
+  const int x0 = max(0, sx - W), x1 = min(n - 1, sx + W);
+  const int y0 = max(0, sy - W), y1 = min(n - 1, sy + W);
+  const bool whole = x0 == 0 && y0 == 0 && x1 == n - 1 && y1 == n - 1;
+  const int b0 = y0 >> 6, b1 = y1 >> 6;
+  const long long W2 = (long long)W * W;
+  // candidates: the disc of radius W, or every site when the window holds
+  // the grid (no certificate needed then)
+  const long long Wc = whole ? (1ll << 62) : W2;
+  int cnt = 0;
+  bool ovf = false;
+  for (int x = x0; x <= x1; ++x)
+    for (int b = b0; b <= b1; ++b)
+      gather_word(__ldg(bits + (size_t)b * n + x) &
+                      row_mask(max(y0 - 64 * b, 0), min(y1 - 64 * b, 63)),
+                  x - sx, 64 * b - sy, sy, Wc, rec, cnt, ovf, vmin, vmax);
+  // |K - S v| <= 2 W^2 + 2 W rb: below 2^23 the reciprocal estimate is safe
+  const bool fast = 2 * W2 + 2 * (long long)W * rb < (1ll << 23);
+  CellSums c{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
+  int R2 = 0;
+  // rows outward from s, two per pass over the records: up from v = 0, down
+  // from v = -1, inside the row limits
+  for (int dir = 1; dir >= -1; dir -= 2) {
+    const int vend = dir > 0 ? vmax : vmin;
+    for (int v = dir > 0 ? max(0, vmin) : min(-1, vmax); dir > 0 ? v <= vend : v >= vend;
+         v += 2 * dir) {
+      const RowPair p =
+          row_bounds2(rec, cnt, ovf, fast, bits, n, sx, sy, x0, x1, b0, b1, y0, y1, Wc, v, dir);
+      if (p.lo0 > p.hi0 + 1) break;  // the cell has ended in this direction
+      if (p.lo0 <= p.hi0) take_row(density, support, n, sx, sy, rb2, v, p.lo0, p.hi0, R2, c);
+      const int v1 = v + dir;
+      if ((dir > 0 ? v1 > vend : v1 < vend) || p.lo1 > p.hi1 + 1) break;
+      if (p.lo1 <= p.hi1) take_row(density, support, n, sx, sy, rb2, v1, p.lo1, p.hi1, R2, c);
+    }
+  }
+  c.r2 = R2;
+  return c;
+}
+
+// Where the float walk below is exact: W^2 (W + 2 rb) < 1.25 2^20.  A candidate
+// (A, B) bounds row v by floor(t) (+ 1 for a lower bound), t = (K - 2 B v) / 2A,
+// computed as k + s v with k = K / 2A and s = -B / A rounded (r ~ 1/A within an
+// ulp scales both alike).  Its error, the row steps and the final sum included,
+// is below 6 2^-24 (|k| + |s v|) <= 6 2^-24 (W^2 / 2 + W rb) < 1 / 4W there, and t
+// is a multiple of 1 / 2|A| >= 1 / 2W, so floor(t) = floor(t~ + 1 / 4W) -- for
+// every record alike, so the smallest (largest) t~ of a row gives its bound
+// with one floor.  (W <= 109 follows; rb <= 511 lets a row fit one word.)
+__device__ __forceinline__ bool float_walk(int W, int rb) {
+  return W <= 127 && rb <= 511 && W * W * (W + 2 * rb) < (5 << 18);
+}
+
+constexpr int kRowsPass = 8;   // rows bounded per pass over the records
+constexpr int kRowList = 24;   // rows listed before their pixels are summed
+
+// The float 128 + a byte minus 128 (no conversion instruction).
+__device__ __forceinline__ float byte_val(uint32_t w, unsigned sel) {
+  return __uint_as_float(__byte_perm(w, 0x4b000000u, sel)) - 8388736.0f;
+}
+
+// Record i (0 or 1) of a record word: bound k + s v.
+__device__ __forceinline__ void rec_line(uint32_t w, int i, float &k, float &s) {
+  const float A = byte_val(w, i ? 0x7442u : 0x7440u), B = byte_val(w, i ? 0x7443u : 0x7441u);
+  const float r = rcp_approx(A);
+  s = -B * r;
+  k = __fmaf_rn(A, A, B * B) * (0.5f * r);
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// A listed row: v, first column da and last column db relative to the site.
+__device__ __forceinline__ uint32_t pack_row(int v, int da, int db) {
+  return (uint32_t)(v & 0x3ff) | ((uint32_t)(da & 0x7ff) << 10) | ((uint32_t)(db - da) << 21);
+}
+
+// One attempt at the cell with the window radius W where float_walk holds.
+// False when the candidates do not fit (the caller takes cell_general).
+// What lives per lane decides the speed: 32 warps share an SM's L1, which also
+// holds the density rows, so a candidate is two bytes (A + 128, B + 128; its line is
+// recomputed per pass) and a row one word.
+__device__ __forceinline__ bool cell_float(const float *__restrict__ density,
+                                           const int2 *__restrict__ support,
+                                           const uint64_t *__restrict__ bits, int n, int sx, int sy,
+                                           int W, int rb, int vmin, int vmax, CellSums &out) {
+  uint32_t rec[kMaxCand / 2];  // two candidates a word: those left of s, then those right of it
+  uint32_t rows[kRowList + kRowsPass];
+  unsigned short *rec16 = reinterpret_cast<unsigned short *>(rec);
+  const int rb2 = rb * rb, W2 = W * W;
+  const int x0 = max(0, sx - W), x1 = min(n - 1, sx + W);
+  const int y0 = max(0, sy - W), y1 = min(n - 1, sy + W);
+  int cnt = 0, nl = 0;
+  auto put = [&](int A, int B) {
+    if (A * A + B * B > W2) return;
+    if (cnt < kMaxCand) rec16[cnt] = (unsigned short)((A + 128) | ((B + 128) << 8));
+    ++cnt;
+  };
+  auto even = [&]() {  // an odd list repeats its last record
+    if ((cnt & 1) && cnt < kMaxCand) rec16[cnt] = rec16[cnt - 1];
+    cnt += cnt & 1;
+  };
+  if (W <= 31) {
+    // a column's window rows as one word of up to 63 bits, bit i = row y0 + i,
+    // from two or three 32-row halves of the bitmap words
+    const uint32_t *hw = reinterpret_cast<const uint32_t *>(bits);
+    const int h0 = y0 >> 5, sh = y0 & 31, nr = y1 - y0 + 1;
+    const int h1 = h0 + (sh + nr > 32), h2 = h1 + (sh + nr > 64);
+    const uint32_t *p0 = hw + 2 * (size_t)(h0 >> 1) * n + (h0 & 1);
+    const uint32_t *p1 = hw + 2 * (size_t)(h1 >> 1) * n + (h1 & 1);
+    const uint32_t *p2 = hw + 2 * (size_t)(h2 >> 1) * n + (h2 & 1);
+    const bool tall = nr > 32;
+    const uint32_t mlo = nr >= 32 ? ~0u : (1u << nr) - 1u;
+    const uint32_t mhi = tall ? (1u << (nr - 32)) - 1u : 0u;
+    const int o = sy - y0;  // s's own bit
+    uint32_t w0 = __ldg(p0 + 2 * x0), w1 = __ldg(p1 + 2 * x0), w2 = tall ? __ldg(p2 + 2 * x0) : 0u;
+    for (int x = x0; x <= x1; ++x) {
+      uint32_t lo = __funnelshift_r(w0, w1, sh) & mlo;
+      uint32_t hi = tall ? __funnelshift_r(w1, w2, sh) & mhi : 0u;
+      if (x < x1) {  // the next column's words in flight
+        w0 = __ldg(p0 + 2 * x + 2);
+        w1 = __ldg(p1 + 2 * x + 2);
+        if (tall) w2 = __ldg(p2 + 2 * x + 2);
+      }
+      const int A = x - sx;
+      if (A == 0) {
+        // s's own column: the nearest site on each side limits the rows
+        even();
+        nl = cnt;
+        const uint64_t col = (uint64_t)lo | ((uint64_t)hi << 32);
+        const uint64_t up = (col >> o) >> 1, dn = col & ((1ull << o) - 1ull);
+        if (up) same_column_limit(__ffsll((long long)up), sy, vmin, vmax);
+        if (dn) same_column_limit(63 - __clzll((long long)dn) - o, sy, vmin, vmax);
+        continue;
+      }
+      while (lo) {
+        const int i = __ffs(lo) - 1;
+        lo &= lo - 1u;
+        put(A, i - o);
+      }
+      while (hi) {
+        const int i = __ffs(hi) + 31;
+        hi &= hi - 1u;
+        put(A, i - o);
+      }
+    }
+  } else {
+    const int b0 = y0 >> 6, b1 = y1 >> 6;
+    for (int x = x0; x <= x1; ++x) {
+      const int A = x - sx;
+      if (A == 0) {
+        even();
+        nl = cnt;
+      }
+      for (int b = b0; b <= b1; ++b) {
+        uint64_t w = __ldg(bits + (size_t)b * n + x) &
+                     row_mask(max(y0 - 64 * b, 0), min(y1 - 64 * b, 63));
+        while (w) {
+          const int i = __ffsll((long long)w) - 1;
+          w &= w - 1ull;
+          const int B = 64 * b + i - sy;
+          if (A) put(A, B);
+          else if (B) same_column_limit(B, sy, vmin, vmax);
+        }
+      }
+    }
+  }
+  even();
+  if (cnt > kMaxCand) return false;
+  nl >>= 1;
+  cnt >>= 1;
+  const float eps = 0.25f / (float)W;
+  const F2 z = f2(0.f, 0.f);
+  CellAcc acc{z, z, z, z};
+  int R2 = 0;
+  // rows outward from s: up from v = 0, then down from v = -1, inside the row
+  // limits, kRowsPass per pass over the records.  One loop for both
+  // directions, and the rows are listed before they are summed: a lane whose
+  // cell has ended upwards goes on downwards while its neighbours are still
+  // going up.
+  int dir = 1, v = max(0, vmin);
+  bool done = false;
+  do {
+    int m = 0;
+    do {
+      if (dir > 0 && v > vmax) {
+        dir = -1;
+        v = min(-1, vmax);
+      }
+      if (dir < 0 && v < vmin) {
+        done = true;
+        break;
+      }
+      float lo[kRowsPass], hi[kRowsPass];
+#pragma unroll
+      for (int j = 0; j < kRowsPass; ++j) {
+        lo[j] = (float)(-sx - 1);
+        hi[j] = (float)(n - 1 - sx);
+      }
+      const float fv = (float)v, fd = (float)dir;
+      for (int k = 0; k < nl; ++k) {
+        const uint32_t w = rec[k];
+        float k0, s0, k1, s1;
+        rec_line(w, 0, k0, s0);
+        rec_line(w, 1, k1, s1);
+        k0 = __fmaf_rn(s0, fv, k0), k1 = __fmaf_rn(s1, fv, k1);
+        s0 *= fd, s1 *= fd;
+#pragma unroll
+        for (int j = 0; j < kRowsPass; ++j)
+          lo[j] = max3(lo[j], __fmaf_rn(s0, (float)j, k0), __fmaf_rn(s1, (float)j, k1));
+      }
+      for (int k = nl; k < cnt; ++k) {
+        const uint32_t w = rec[k];
+        float k0, s0, k1, s1;
+        rec_line(w, 0, k0, s0);
+        rec_line(w, 1, k1, s1);
+        k0 = __fmaf_rn(s0, fv, k0), k1 = __fmaf_rn(s1, fv, k1);
+        s0 *= fd, s1 *= fd;
+#pragma unroll
+        for (int j = 0; j < kRowsPass; ++j)
+          hi[j] = min3(hi[j], __fmaf_rn(s0, (float)j, k0), __fmaf_rn(s1, (float)j, k1));
+      }
+      // the rows' spans until the row limit, or until the cell has ended in
+      // this direction
+      bool ended = false;
+#pragma unroll
+      for (int j = 0; j < kRowsPass; ++j) {
+        const int vv = v + j * dir;
+        const int2 sup = __ldg(support + min(max(sy + vv, 0), n - 1));
+        const int l = __float2int_rd(lo[j] + eps) + 1, h = __float2int_rd(hi[j] + eps);
+        ended = ended || l > h + 1 || (dir > 0 ? vv > vmax : vv < vmin);
+        int da = max(l, sup.x - sx), db = min(h, sup.y - 1 - sx);
+        if (!ended && da <= db) {
+          int d2 = max(da * da, db * db) + vv * vv;
+          if (d2 > rb2) {  // clip to the covering disc
+            const int hx = isqrt_floor(rb2 - vv * vv);
+            da = max(da, -hx);
+            db = min(db, hx);
+            d2 = max(da * da, db * db) + vv * vv;
+          }
+          if (da <= db) {
+            R2 = max(R2, d2);
+            rows[m++] = pack_row(vv, da, db);
+          }
+        }
+      }
+      if (ended) {
+        done = dir < 0;
+        dir = -1;
+        v = min(-1, vmax);
+      } else {
+        v += kRowsPass * dir;
+      }
+    } while (!done && m <= kRowList);
+    // the listed rows' pixels, two rows at a time
+    for (int i = 0; i < m; i += 2) {
+      const uint32_t wa = rows[i], wb = i + 1 < m ? rows[i + 1] : 0u;
+      const int va = (int)(wa << 22) >> 22, vb = (int)(wb << 22) >> 22;
+      const int da = sx + ((int)(wa << 11) >> 21), db = sx + ((int)(wb << 11) >> 21);
+      const int la = (int)(wa >> 21), lb = (int)(wb >> 21);
+      const float *ra = density + (size_t)(sy + va) * n, *rb_ = density + (size_t)(sy + vb) * n;
+      const float fa = (float)va, fb = (float)vb;
+      if (max(la, lb) < 16) {
+        RowPix pa, pb;
+        const int qa = da & ~3, qb = db & ~3;
+        pa.p = ra + qa;
+        pb.p = rb_ + qb;
+        pa.dx = (float)(qa - sx);
+        pb.dx = (float)(qb - sx);
+        pa.m = ((2u << la) - 1u) << (da - qa);
+        pb.m = i + 1 < m ? ((2u << lb) - 1u) << (db - qb) : 0u;
+        F2 rw, rx, rq;
+        pair_sums(pa, pb, rw, rx, rq);
+        // (an empty row folds as zeros: the accumulators are normalised)
+        fold_chunk2(acc, f2_lo(rw), f2_lo(rx), f2_lo(rq), fa, fa * fa);
+        fold_chunk2(acc, f2_hi(rw), f2_hi(rx), f2_hi(rq), fb, fb * fb);
+      } else {
+#pragma unroll 1
+        for (int k = 0; k < 2 && i + k < m; ++k) {
+          const int u1 = (k ? db + lb : da + la) - sx;
+          for (int u0 = (k ? db : da) - sx; u0 <= u1; u0 += 16) {
+            float rw, rx, rq;
+            chunk_sums((k ? rb_ : ra) + sx, u0, min(u1, u0 + 15), rw, rx, rq);
+            fold_chunk2(acc, rw, rx, rq, k ? fb : fa, k ? fb * fb : fa * fa);
+          }
+        }
+      }
+    }
+  } while (!done);
+  out.wh = f2_lo(acc.wxh), out.wl = f2_lo(acc.wxl);
+  out.xh = f2_hi(acc.wxh), out.xl = f2_hi(acc.wxl);
+  out.yh = f2_lo(acc.yeh), out.yl = f2_lo(acc.yel);
+  out.eh = f2_hi(acc.yeh), out.el = f2_hi(acc.yel);
+  out.r2 = R2;
+  return true;
+}
+
 // Exact cell of site (sx, sy) and its sums.  bits: current site bitmap;
 // W: initial window radius; rb: the covering bound.
 __device__ CellSums cell_sums(const LevelBufs &a, const uint64_t *__restrict__ bits, int n, int sx,
                               int sy, int W, int rb) {
-  int2 rec[kMaxCand];  // {K, S | D << 16} of the window's candidates
+  const float *density = a.density;
+  const int2 *support = a.support;
   const int2 yr = *a.sup_range;  // rows [yr.x, yr.y) hold every nonzero density
-  const int vlo_sup = max(yr.x, sy - rb) - sy, vhi_sup = min(yr.y - 1, sy + rb) - sy;
-  const int rb2 = rb * rb;
+  const int vlo = max(yr.x, sy - rb) - sy, vhi = min(yr.y - 1, sy + rb) - sy;
   W = max(1, min(W, 2 * rb));
   CellSums c;
   for (;;) {
-    const int x0 = max(0, sx - W), x1 = min(n - 1, sx + W);
-    const int y0 = max(0, sy - W), y1 = min(n - 1, sy + W);
-    const bool whole = x0 == 0 && y0 == 0 && x1 == n - 1 && y1 == n - 1;
-    const int b0 = y0 >> 6, b1 = y1 >> 6;
-    const long long W2 = (long long)W * W;
-    // candidates: the disc of radius W, or every site when the window holds
-    // the grid (no certificate needed then)
-    const long long Wc = whole ? (1ll << 62) : W2;
-    int cnt = 0;
-    bool ovf = false;
-    int vmin = vlo_sup, vmax = vhi_sup;  // row limits, same-column sites folded in
-    if (b1 - b0 <= 1) {  // one or two bands: load the next column ahead
-      const uint64_t *p0 = bits + (size_t)b0 * n, *p1 = bits + (size_t)b1 * n;
-      const uint64_t m0 = row_mask(y0 - 64 * b0, min(y1 - 64 * b0, 63));
-      const uint64_t m1 = b1 > b0 ? row_mask(0, y1 - 64 * b1) : 0ull;
-      uint64_t c0 = __ldg(p0 + x0) & m0, c1 = m1 ? __ldg(p1 + x0) & m1 : 0ull;
-      for (int x = x0; x <= x1; ++x) {
-        uint64_t n0 = 0ull, n1 = 0ull;
-        if (x < x1) {
-          n0 = __ldg(p0 + x + 1) & m0;
-          if (m1) n1 = __ldg(p1 + x + 1) & m1;
-        }
-        gather_word(c0, x - sx, 64 * b0 - sy, sy, Wc, rec, cnt, ovf, vmin, vmax);
-        gather_word(c1, x - sx, 64 * b1 - sy, sy, Wc, rec, cnt, ovf, vmin, vmax);
-        c0 = n0;
-        c1 = n1;
-      }
-    } else {
-      for (int x = x0; x <= x1; ++x)
-        for (int b = b0; b <= b1; ++b)
-          gather_word(__ldg(bits + (size_t)b * n + x) &
-                          row_mask(max(y0 - 64 * b, 0), min(y1 - 64 * b, 63)),
-                      x - sx, 64 * b - sy, sy, Wc, rec, cnt, ovf, vmin, vmax);
-    }
-    // |K - S v| <= 2 W^2 + 2 W rb: below 2^23 the reciprocal estimate is safe
-    const bool fast = 2 * W2 + 2 * (long long)W * rb < (1ll << 23);
-    c = CellSums{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
-    int R2 = 0;
-    // rows outward from s, two per pass over the records: up from v = 0, down
-    // from v = -1, inside the row limits
-    for (int dir = 1; dir >= -1; dir -= 2) {
-      const int vend = dir > 0 ? vmax : vmin;
-      for (int v = dir > 0 ? max(0, vmin) : min(-1, vmax); dir > 0 ? v <= vend : v >= vend;
-           v += 2 * dir) {
-        const RowPair p =
-            row_bounds2(rec, cnt, ovf, fast, bits, n, sx, sy, x0, x1, b0, b1, y0, y1, Wc, v, dir);
-        if (p.lo0 > p.hi0 + 1) break;  // the cell has ended in this direction
-        if (p.lo0 <= p.hi0) take_row(a, n, sx, sy, rb2, v, p.lo0, p.hi0, R2, c);
-        const int v1 = v + dir;
-        if ((dir > 0 ? v1 > vend : v1 < vend) || p.lo1 > p.hi1 + 1) break;
-        if (p.lo1 <= p.hi1) take_row(a, n, sx, sy, rb2, v1, p.lo1, p.hi1, R2, c);
-      }
-    }
-    c.r2 = R2;
+    if (!float_walk(W, rb) ||
+        !cell_float(density, support, bits, n, sx, sy, W, rb, vlo, vhi, c))
+      c = cell_general(density, support, bits, n, sx, sy, W, rb, vlo, vhi);
+    const bool whole = W >= sx && W >= sy && W >= n - 1 - sx && W >= n - 1 - sy;
     // R2 <= rb^2, so a window of 2 rb always passes
-    if (whole || 4 * (long long)R2 <= W2) return c;
-    W = min(min(2 * isqrt_ceil(R2) + 1, 2 * W), 2 * rb);
+    if (whole || 4ll * c.r2 <= (long long)W * W) return c;
+    W = min(min(2 * isqrt_ceil(c.r2) + 1, 2 * W), 2 * rb);
   }
 }
 
@@ -824,7 +1216,7 @@ __device__ CellSums cell_sums_warp(const LevelBufs &a, const uint64_t *__restric
         const unsigned sb = __ballot_sync(kFull, !inr || lo > hi + 1);
         const int f = sb ? __ffs(sb) - 1 : 32;  // rows 0 .. f-1 of this step are walked
         int da = 1, db = 0;
-        if (lane < f && lo <= hi && row_span(a, sx, sy, rb2, vr, lo, hi, da, db)) {
+        if (lane < f && lo <= hi && row_span(a.support, sx, sy, rb2, vr, lo, hi, da, db)) {
           R2 = max(R2, max(da * da, db * db) + vr * vr);
           const float *row = a.density + (size_t)(sy + vr) * n + sx;
           int k = 0;
@@ -1253,7 +1645,7 @@ cudaError_t cells_configure() {
   int sms = 0, per0 = 0, per1 = 0;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return e;
-  // the candidate records live in local memory: shared memory only for the
+  // candidates and rows live in local memory: shared memory only for the
   // 1 KB the runtime reserves per block (32 blocks per SM), the rest as L1
   const int carve = 15;
   if ((e = cudaFuncSetAttribute(k_cell<0>, cudaFuncAttributePreferredSharedMemoryCarveout,

@@ -1,0 +1,65 @@
+"""The Lloyd kernel's float row bounds at the edges of their dispatch: crowded
+windows (more candidates than a lane's list holds), cells of more rows than the
+row list and wider than a 16-pixel chunk, windows above and below one 32-row
+word and two, covering bounds beyond the float range, sites in one column or
+row, sites at the grid's border.  Moments against the FP64 oracle (1e-5
+relative, the engine's contract: FP32 chunks of 16 pixels, two-float sums), and
+the lane-per-site and warp-per-site kernels against each other, bit for bit
+(they do the same sums in the same order)."""
+import numpy as np
+import pytest
+
+from workloads import gaussian_density
+
+pytestmark = pytest.mark.gpu
+
+
+def points(kind, n, rng):
+    """Distinct (x, y) of a site set."""
+    if kind == "crowd":    # a packed block (windows of hundreds of sites) and a few far ones
+        b = np.stack(np.meshgrid(np.arange(24), np.arange(24)), -1).reshape(-1, 2) + n // 2
+        return np.concatenate([b, rng.integers(0, n, (30, 2))])
+    if kind == "one":      # a single cell: the whole support
+        return np.array([[n // 2, n // 3]])
+    if kind == "column":   # horizontal slabs, same-column limits on both sides
+        return np.stack([np.full(n // 16, n // 2), np.arange(n // 16) * 16 + 3], 1)
+    if kind == "row":      # vertical slabs: one row bound per side, tall cells
+        return np.stack([np.arange(n // 16) * 16 + 5, np.full(n // 16, n // 2)], 1)
+    if kind == "border":   # along the grid's edges
+        t = np.arange(0, n, 7)
+        return np.concatenate([np.stack([t, 0 * t], 1), np.stack([0 * t + n - 1, t], 1),
+                               rng.integers(0, n, (40, 2))])
+    return rng.integers(0, n, (int(kind), 2))  # that many at random
+
+
+@pytest.mark.parametrize("n,kind", [(256, "crowd"), (512, "crowd"), (256, "one"), (1024, "one"),
+                                    (512, "column"), (512, "row"), (768, "border"), (512, 12),
+                                    (1024, 60), (512, 250), (512, 1200), (512, 6000),
+                                    (768, 20000)])
+def test_cells_match_fp64_and_each_other(gcvt_lib, oracle, cuda_device, n, kind):
+    rng = np.random.default_rng(n)
+    q = np.unique(points(kind, n, rng), axis=0)
+    sites = gcvt_lib.sites_from_points(n, q[:, 0], q[:, 1])
+    rho = gaussian_density(n, 6, 4.0, 0.05, 0.2, 3)
+    if kind == "border":
+        rho = np.maximum(rho, np.float32(0.25))  # density up to the grid's edge
+    mask = np.zeros((n, n), np.uint8)
+    _, mom, energy, _ = oracle.lloyd_step(sites, rho, mask, 2.0)
+    ctx = gcvt_lib.Context(n)
+    ctx.load(sites, rho, mask)
+    got = ctx.moments()
+    ys, xs = np.nonzero(sites[..., 0] != -32768)
+    for k in range(3):
+        want, have = mom[k][ys, xs], got[k][ys, xs]
+        assert (np.abs(have - want) <= 1e-5 * np.abs(want)).all()
+    e = got[3][ys, xs].sum() / (n * n)
+    assert abs(e - energy) <= 1e-5 * energy
+    runs = []
+    for mode in (1, 2):
+        ctx.set_tuning(cell_mode=mode)
+        ctx.load(sites, rho, mask)
+        ctx.iterate(4)
+        runs.append((ctx.sites(), ctx.info()))
+    assert np.array_equal(runs[0][0], runs[1][0])
+    assert runs[0][1] == runs[1][1]
+    ctx.close()
