@@ -59,9 +59,9 @@ typedef struct {
                                0, the default: every step its own launch) */
     float lloyd_ms;         /* autotune: best time of one Lloyd iteration (ms)           */
     float jfa_ms;           /* autotune: best time of one jump-flooding labelling (ms)   */
-    int cell_mode;          /* Lloyd cells: 0 = one site per warp up to 8192 sites, else
-                               one per lane; 1 = one per lane; 2 = one per warp (up to
-                               8192 sites; a learned step's two passes run one per lane) */
+    int cell_mode;          /* Lloyd cells: 0 = one site per warp for few sites (up to 8192,
+                               up to 32,768 when their cells are large), else one per lane;
+                               1 = one per lane; 2 = one per warp (up to 32,768 sites) */
 } gcvt_tuning;
 
 /* Human-readable text of a status code. */

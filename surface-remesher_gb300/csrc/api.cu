@@ -28,6 +28,7 @@ struct gcvt_ctx {
   int input_err = 0;    // the loaded grid is malformed at full resolution
   int cur_n = 0;        // size of the level currently held in the bitmaps
   int sites = 0;        // sites in the grid the bitmaps were built from
+  double per_site = 0;  // density pixels per site of the level last started
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
   float *density[8] = {};      // pyramid, [0] = full resolution
@@ -77,6 +78,7 @@ struct gcvt_ctx {
   cudaGraphExec_t chunk_exec = nullptr;  // kChunk iterations of one level
   int chunk_n = 0;
   int chunk_level = -1;
+  bool chunk_warp = false;  // captured one site per warp
 };
 
 namespace {
@@ -92,6 +94,16 @@ constexpr int kChunk = 10;  // iterations per graph; the schedule acts every 10
 bool valid_n(int n) { return n >= kMinN && n <= kMaxN && n % 256 == 0; }
 bool pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 size_t bits_words(int n) { return (size_t)(n / kBand) * n; }
+
+// One site per warp when the sites are too few to fill the GPU one per lane.
+// Measured (us an iteration, lane / warp): 8192 sites of 93 pixels 34 / 28, 12,000
+// of 63 31 / 34, of 253 74 / 39, 16,384 of 46 30 / 42, of 185 62 / 45, 24,000 of 126
+// 46 / 57: a lane's time grows with the cell (20 + 0.22 per pixel: one group's
+// latency), the warps' with the sites (8 + 0.0023 per site).
+bool warp_cells(const gcvt_ctx *c) {
+  if (c->cell_mode) return c->cell_mode == 2;
+  return c->sites <= 8192 || (c->sites <= kWarpSites && c->per_site > c->sites / 96.0 - 55.0);
+}
 
 LevelBufs level_bufs(gcvt_ctx *c, int n, int level) {
   LevelBufs b = {};
@@ -111,8 +123,7 @@ LevelBufs level_bufs(gcvt_ctx *c, int n, int level) {
   b.gslot = c->gslot;
   b.sslot = c->sslot;
   b.scnt = c->scnt;
-  // one site per warp when the sites are too few to fill the GPU one per lane
-  if (c->cell_mode == 2 || (c->cell_mode == 0 && c->sites <= kWarpSites)) {
+  if (warp_cells(c)) {
     b.sitev = c->sitev;
     b.gcnt = c->gcnt;
   }
@@ -144,7 +155,8 @@ int push_state(gcvt_ctx *c) {
 // (size, level); a stream that cannot be captured (the legacy default stream)
 // gets plain launches.
 int enqueue_chunk(gcvt_ctx *c, int n, int level) {
-  if (c->chunk_exec && (c->chunk_n != n || c->chunk_level != level)) {
+  if (c->chunk_exec &&
+      (c->chunk_n != n || c->chunk_level != level || c->chunk_warp != warp_cells(c))) {
     cudaGraphExecDestroy(c->chunk_exec);
     c->chunk_exec = nullptr;
   }
@@ -177,6 +189,7 @@ int enqueue_chunk(gcvt_ctx *c, int n, int level) {
     }
     c->chunk_n = n;
     c->chunk_level = level;
+    c->chunk_warp = warp_cells(c);
   }
   CK(cudaGraphLaunch(c->chunk_exec, c->stream));
   return GCVT_OK;
@@ -235,6 +248,7 @@ int initial_window(gcvt_ctx *c, int level, int *w, float *radius = nullptr) {
                      c->stream));
   CK(cudaStreamSynchronize(c->stream));
   const double per_site = c->sites > 0 ? (double)pix / c->sites : 64.0;
+  c->per_site = per_site;
   const int v = (int)std::ceil(2.5 * std::sqrt(per_site / 3.14159265358979));
   *w = v < 2 ? 2 : (v > 1024 ? 1024 : v);
   if (radius) {  // mean cell radius

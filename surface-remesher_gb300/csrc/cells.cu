@@ -100,13 +100,13 @@ __device__ __forceinline__ F2 f2(float a, float b) {
   return r;
 }
 __device__ __forceinline__ float f2_lo(F2 a) {
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+  float x;
+  asm("mov.b64 {%0, _}, %1;" : "=f"(x) : "l"(a.v));
   return x;
 }
 __device__ __forceinline__ float f2_hi(F2 a) {
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+  float y;
+  asm("mov.b64 {_, %0}, %1;" : "=f"(y) : "l"(a.v));
   return y;
 }
 __device__ __forceinline__ F2 add2(F2 a, F2 b) {
@@ -783,13 +783,16 @@ __device__ __forceinline__ float cell_centroid(int base, float Sh, float Sl, flo
   return __fadd_rn(s, __fadd_rn(e, q2));
 }
 
-// Add one to *counter after every earlier write of this thread is visible
+// Add to *counter after every earlier write of this thread is visible
 // (an atomic with release semantics): the writer's half of a counter
 // handoff, where whoever brings the counter to its target fences and reads
 // the others' results.  Cheaper than a full fence before a plain atomic.
-__device__ __forceinline__ unsigned add_release(unsigned *counter) {
+__device__ __forceinline__ unsigned add_release(unsigned *counter, unsigned by = 1u) {
   unsigned prev;
-  asm volatile("atom.add.release.gpu.u32 %0, [%1], 1;" : "=r"(prev) : "l"(counter) : "memory");
+  asm volatile("atom.add.release.gpu.u32 %0, [%1], %2;"
+               : "=r"(prev)
+               : "l"(counter), "r"(by)
+               : "memory");
   return prev;
 }
 
@@ -1095,225 +1098,484 @@ __device__ void cell_group(const LevelBufs &a, const IterView &v, unsigned g, in
 }
 
 // ---------------------------------------------------------------------------
-// One site per warp, for problems with fewer sites than the GPU holds warps
-// (a lane-per-site group then runs one site's whole cell serially, and only
-// a few groups exist).  The same cell and the same sums, bit for bit: the
-// candidates are gathered by the lanes into shared memory, the rows of the
-// walk are bounded and summed one per lane, 32 at a time, and lane 0 folds
-// the rows' chunk sums into the cell sums in the lane-per-site order.  The
-// energy reduction keeps its groups: each site's contribution waits in
-// LevelBufs::sitev, and the warp finishing a group's last site reduces it.
+// One site per warp, for problems with few sites (a lane-per-site group runs
+// one site's whole cell serially, and only a few groups exist).  The same cell
+// and the same sums, bit for bit: a warp gathers its site's candidates, bounds
+// the rows one per lane and sums their 16-pixel chunks one per lane; the chunks
+// are then folded into the cell sums in the lane-per-site order.  The energy
+// reduction keeps its groups: each site's contribution waits in
+// LevelBufs::sitev, and the warp finishing a group's last sites reduces it.
 // ---------------------------------------------------------------------------
 
-constexpr int kWarpChunks = 4;  // chunk sums per row kept in shared memory
+constexpr int kWarpEnts = 96;  // chunk sums of a site kept in shared memory
+
+constexpr int kWarpRec = 128;  // candidates of a site kept in shared memory
+constexpr int kBlockSites = 8;  // sites (warps) per block
 
 struct WarpScratch {
-  int2 rec[kMaxCand];
-  float part[32][kWarpChunks][3];  // per row (lane): chunk sums rw, rx, rq
-  int2 span[32];                   // per row: summed pixels [da, db]
+  int2 rec[kWarpRec];  // left of s first: float lines {k, s}, or make_rec's records
+  // per 16-pixel chunk of the rows, in fold order: the terms of (W, SX, SY, E),
+  // high then low parts (the padding spreads the block's sites over the banks)
+  float ent[kWarpEnts][8];
+  float sum[8];   // folded already: (W, SX, SY, E) high, then low
+  int m;          // chunks left to fold; -1: sum holds the result
+  int r2;
+  int pad[26];
 };
+static_assert(sizeof(WarpScratch) % 128 == 16, "sites 4 banks apart (fold: lane 4 s + q)");
 
-__device__ CellSums cell_sums_warp(const LevelBufs &a, const uint64_t *__restrict__ bits, int n,
-                                   int sx, int sy, int W, int rb, int lane, WarpScratch &ws) {
-  constexpr unsigned kFull = 0xffffffffu;
-  const int2 yr = *a.sup_range;
-  const int vlo_sup = max(yr.x, sy - rb) - sy, vhi_sup = min(yr.y - 1, sy + rb) - sy;
-  const int rb2 = rb * rb;
-  W = max(1, min(W, 2 * rb));
-  CellSums c;
-  for (;;) {
-    const int x0 = max(0, sx - W), x1 = min(n - 1, sx + W);
-    const int y0 = max(0, sy - W), y1 = min(n - 1, sy + W);
-    const bool whole = x0 == 0 && y0 == 0 && x1 == n - 1 && y1 == n - 1;
-    const int b0 = y0 >> 6, b1 = y1 >> 6, nb = b1 - b0 + 1, ncol = x1 - x0 + 1;
-    const long long W2 = (long long)W * W;
-    const long long Wc = whole ? (1ll << 62) : W2;
-    // candidates: lanes over the window's (column, band) words, records
-    // compacted into shared memory in word order
-    int cnt = 0;
-    int vmin = vlo_sup, vmax = vhi_sup;
-    for (int t0 = 0; t0 < ncol * nb; t0 += 32) {
-      const int t = t0 + lane;
-      uint64_t w = 0ull;
-      int A = 0, B0 = 0;
-      if (t < ncol * nb) {
-        const int x = x0 + t / nb, b = b0 + t % nb;
-        w = __ldg(bits + (size_t)b * n + x) & row_mask(max(y0 - 64 * b, 0), min(y1 - 64 * b, 63));
-        A = x - sx;
-        B0 = 64 * b - sy;
-      }
-      int mine = 0;
-      for (uint64_t q = w; q; q &= q - 1ull) {
-        const int B = B0 + __ffsll((long long)q) - 1;
-        const int K = A * A + B * B;
-        if (K == 0 || (long long)K > Wc) continue;
-        if (A == 0) same_column_limit(B, sy, vmin, vmax);
-        else ++mine;
-      }
-      int incl = mine;
+// Sums of the pixels [u0, u1] (at most 16, relative to the site) of a row, all
+// its aligned 16-byte loads in flight together.
+__device__ __forceinline__ void chunk_quads(const float *__restrict__ row, int u0, int u1, int sx,
+                                            float &rw, float &rx, float &rq) {
+  const int q0 = (sx + u0) & ~3, last = (sx + u1 - q0) >> 2;
+  const float4 *p = reinterpret_cast<const float4 *>(row + q0);
+  const unsigned m = ((2u << (u1 - u0)) - 1u) << (sx + u0 - q0);
+  float4 q[5];
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += u;
-      }
-      int pos = cnt + incl - mine;
-      if (mine) {
-        for (uint64_t q = w; q; q &= q - 1ull) {
-          const int B = B0 + __ffsll((long long)q) - 1;
-          const int K = A * A + B * B;
-          if (K == 0 || (long long)K > Wc || A == 0) continue;
-          if (pos < kMaxCand) ws.rec[pos] = make_rec(A, B, K);
-          ++pos;
-        }
-      }
-      cnt += __shfl_sync(kFull, incl, 31);
+  for (int k = 0; k < 5; ++k)
+    q[k] = k <= last ? __ldg(p + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  rw = 0.f, rx = 0.f, rq = 0.f;
+  float dx = (float)(q0 - sx);
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    if (k > last) break;
+    const float v[4] = {q[k].x, q[k].y, q[k].z, q[k].w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float rho = (m >> (4 * k + j)) & 1u ? v[j] : 0.f;
+      const float t = __fmul_rn(dx, rho);
+      rw = __fadd_rn(rw, rho);
+      rx = __fadd_rn(rx, t);
+      rq = __fmaf_rn(t, dx, rq);
+      dx = __fadd_rn(dx, 1.0f);
     }
-    vmin = __reduce_max_sync(kFull, vmin);
-    vmax = __reduce_min_sync(kFull, vmax);
-    const bool ovf = cnt > kMaxCand;
-    __syncwarp();
-    const bool fast = 2 * W2 + 2 * (long long)W * rb < (1ll << 23);
-    c = CellSums{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};  // lane 0 accumulates
-    int R2 = 0;
-    // rows outward from s, up from v = 0 then down from v = -1, 32 per step
-    // (one per lane); the walk ends at its first row with lo > hi + 1
-    for (int dir = 1; dir >= -1; dir -= 2) {
-      const int vend = dir > 0 ? vmax : vmin;
-      const int vstart = dir > 0 ? max(0, vmin) : min(-1, vmax);
-      for (int base = vstart; dir > 0 ? base <= vend : base >= vend; base += 32 * dir) {
-        const int vr = base + dir * lane;
-        const bool inr = dir > 0 ? vr <= vend : vr >= vend;
-        int lo = -sx, hi = n - 1 - sx;
-        if (inr) {
-          if (!ovf) {
-            for (int k = 0; k < cnt; ++k) {
-              const int2 r = ws.rec[k];
-              const int S = (int)(int16_t)((unsigned)r.y & 0xffffu);
-              const int D = (int)(int16_t)((unsigned)r.y >> 16);
-              const int aD = abs(D);
-              const int N = r.x - S * vr;
-              const int q = fast ? floordiv_r(N, aD, rcp_approx((float)aD))
-                                 : floordiv_est(N, aD, 0.f, false);
-              if (D > 0) hi = min(hi, q);
-              else lo = max(lo, q + 1);
-            }
-          } else {
-            for (int x = x0; x <= x1; ++x)
-              for (int b = b0; b <= b1; ++b) {
-                uint64_t w = __ldg(bits + (size_t)b * n + x) &
-                             row_mask(max(y0 - 64 * b, 0), min(y1 - 64 * b, 63));
-                while (w) {
-                  const int i = __ffsll((long long)w) - 1;
-                  w &= w - 1ull;
-                  const int A = x - sx, B = 64 * b + i - sy;
-                  const int K = A * A + B * B;
-                  if (K == 0 || (long long)K > Wc) continue;
-                  constrain_rel(A, B, vr, lo, hi);
-                }
-              }
-          }
-        }
-        const unsigned sb = __ballot_sync(kFull, !inr || lo > hi + 1);
-        const int f = sb ? __ffs(sb) - 1 : 32;  // rows 0 .. f-1 of this step are walked
-        int da = 1, db = 0;
-        if (lane < f && lo <= hi && row_span(a.support, sx, sy, rb2, vr, lo, hi, da, db)) {
-          R2 = max(R2, max(da * da, db * db) + vr * vr);
-          const float *row = a.density + (size_t)(sy + vr) * n + sx;
-          int k = 0;
-          for (int u0 = da; u0 <= db && k < kWarpChunks; u0 += 16, ++k)
-            chunk_sums(row, u0, min(db, u0 + 15), ws.part[lane][k][0], ws.part[lane][k][1],
-                       ws.part[lane][k][2]);
-        }
-        ws.span[lane] = make_int2(da, db);
-        __syncwarp();
-        if (lane == 0) {
-          for (int r = 0; r < f; ++r) {
-            const int2 sp = ws.span[r];
-            if (sp.x > sp.y) continue;
-            const int vv = base + dir * r;
-            const float fv = (float)vv, fv2 = (float)(vv * vv);
-            const float *row = a.density + (size_t)(sy + vv) * n + sx;
-            int k = 0;
-            for (int u0 = sp.x; u0 <= sp.y; u0 += 16, ++k) {
-              float rw, rx, rq;
-              if (k < kWarpChunks) {
-                rw = ws.part[r][k][0];
-                rx = ws.part[r][k][1];
-                rq = ws.part[r][k][2];
-              } else {
-                chunk_sums(row, u0, min(sp.y, u0 + 15), rw, rx, rq);
-              }
-              fold_chunk(c, rw, rx, rq, fv, fv2);
-            }
-          }
-        }
-        __syncwarp();
-        if (f < 32) break;
-      }
-    }
-    R2 = __reduce_max_sync(kFull, R2);
-    if (lane == 0) c.r2 = R2;
-    if (whole || 4 * (long long)R2 <= W2) return c;
-    W = min(min(2 * isqrt_ceil(R2) + 1, 2 * W), 2 * rb);
   }
 }
 
-// One Lloyd iteration, one listed site per warp from a site ticket.  MODE
-// 0, 4 and 5 as in k_cell (MODE 4 also writes the learned step's features,
-// MODE 5 judges a jump and does not clear ahead).
+// Row v's summed pixels [da, db] of a cell from its records; false when the
+// cell has ended there (or v is past the row limits).
+template <bool FLT>
+__device__ __forceinline__ bool warp_row(const int2 *__restrict__ support, const WarpScratch &ws,
+                                         int n, int sx, int sy, int rb2, int nl, int cnt, float eps,
+                                         bool fast, int v, int vmin, int vmax, int &da, int &db) {
+  const int2 sup = __ldg(support + min(max(sy + v, 0), n - 1));
+  int l = -sx, h = n - 1 - sx;
+  if (FLT) {
+    float lo = (float)(-sx - 1), hi = (float)(n - 1 - sx);
+    const float fv = (float)v;
+    const float2 *rec = reinterpret_cast<const float2 *>(ws.rec);
+    for (int k = 0; k < nl; ++k) lo = fmaxf(lo, __fmaf_rn(rec[k].y, fv, rec[k].x));
+    for (int k = nl; k < cnt; ++k) hi = fminf(hi, __fmaf_rn(rec[k].y, fv, rec[k].x));
+    l = __float2int_rd(lo + eps) + 1, h = __float2int_rd(hi + eps);
+  } else {
+    for (int k = 0; k < cnt; ++k) {
+      const int2 r = ws.rec[k];
+      const int S = (int)(int16_t)((unsigned)r.y & 0xffffu);
+      const int D = (int)(int16_t)((unsigned)r.y >> 16);
+      const int aD = abs(D), N = r.x - S * v;
+      const int q = fast ? floordiv_r(N, aD, rcp_approx((float)aD))
+                         : floordiv_est(N, aD, 0.f, false);
+      if (D > 0) h = min(h, q);
+      else l = max(l, q + 1);
+    }
+  }
+  da = max(l, sup.x - sx), db = min(h, sup.y - 1 - sx);
+  if (l > h + 1 || v < vmin || v > vmax) return false;
+  if (da <= db && max(da * da, db * db) + v * v > rb2) {  // clip to the covering disc
+    const int hx = isqrt_floor(rb2 - v * v);
+    da = max(da, -hx);
+    db = min(db, hx);
+  }
+  return true;
+}
+
+// The candidates of a column as bits from row y0 of the window (W <= 31): the
+// rows of the disc of radius W2^(1/2) around the site, its own column and bit
+// excepted.
+__device__ __forceinline__ uint64_t disc_rows(uint64_t col, int A, int W2, int o) {
+  const int h2 = W2 - A * A;
+  int h = (int)sqrtf((float)h2);  // floor(sqrt(h2)), at most one off
+  h += ((h + 1) * (h + 1) <= h2) - (h * h > h2);
+  const int lo = max(o - h, 0), hi = o + h;  // hi <= 62
+  return col & (((2ull << hi) - 1ull) & ~((1ull << lo) - 1ull));
+}
+
+// The cell of a site by a warp with the window radius W (FLT: float_walk
+// holds): its rows' chunk sums into ws.ent, or, when they are too many for
+// it or the cell is tall, folded into ws.sum.  False when the candidates do not
+// fit.  What bounds it is latency and issue slots, so every step is spread
+// over the lanes: a lane per window column, per row, per 16-pixel chunk.
+template <bool FLT>
+__device__ __forceinline__ bool warp_cell(const float *__restrict__ density,
+                                          const int2 *__restrict__ support,
+                                          const uint64_t *__restrict__ bits, int n, int sx, int sy,
+                                          int W, int rb, int vmin, int vmax, int lane,
+                                          WarpScratch &ws, int &r2) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int rb2 = rb * rb;
+  const int x0 = max(0, sx - W), x1 = min(n - 1, sx + W);
+  const int y0 = max(0, sy - W), y1 = min(n - 1, sy + W);
+  // candidates: a lane per column, compacted into shared memory in column order
+  int cnt = 0, nl = 0;
+  const int b0 = y0 >> 6, b1 = y1 >> 6;
+  if (FLT && W <= 31) {  // at most 63 columns of at most 63 rows: one word a column
+    const int sh = y0 & 63, W2 = W * W, o = sy - y0;
+    const uint64_t rm = row_mask(0, y1 - y0);
+    const uint64_t *p0 = bits + (size_t)b0 * n, *p1 = bits + (size_t)b1 * n;
+    uint64_t w[2][2];  // two columns a lane, all words in flight together
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int x = x0 + 32 * k + lane;
+      w[k][0] = x <= x1 ? __ldg(p0 + x) : 0ull;
+      w[k][1] = x <= x1 && b1 > b0 ? __ldg(p1 + x) : 0ull;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (x0 + 32 * k > x1) break;
+      const int x = x0 + 32 * k + lane, A = x - sx;
+      uint64_t col = w[k][0] >> sh;
+      if (sh) col |= w[k][1] << (64 - sh);
+      col &= rm;
+      if (A == 0) {  // s's own column: the nearest site on each side limits the rows
+        const uint64_t up = (col >> o) >> 1, dn = col & ((1ull << o) - 1ull);
+        if (up) same_column_limit(__ffsll((long long)up), sy, vmin, vmax);
+        if (dn) same_column_limit(63 - __clzll((long long)dn) - o, sy, vmin, vmax);
+        col = 0ull;
+      } else if (x <= x1) {
+        col = disc_rows(col, A, W2, o);
+      }
+      const int mine = __popcll(col);
+      int incl = mine;
+#pragma unroll
+      for (int i = 1; i < 32; i <<= 1) {
+        const int u = __shfl_up_sync(kFull, incl, i);
+        if (lane >= i) incl += u;
+      }
+      nl += __reduce_add_sync(kFull, A < 0 ? mine : 0);
+      int pos = cnt + incl - mine;
+      const float r = rcp_approx((float)A);
+      while (col) {
+        const int B = __ffsll((long long)col) - 1 - o;
+        col &= col - 1ull;
+        if (pos < kWarpRec)
+          ws.rec[pos] = make_int2(__float_as_int(0.5f * (float)(A * A + B * B) * r),
+                                  __float_as_int(-(float)B * r));
+        ++pos;
+      }
+      cnt += __shfl_sync(kFull, incl, 31);
+    }
+  } else {
+    const bool whole = x0 == 0 && y0 == 0 && x1 == n - 1 && y1 == n - 1;
+    // every site when the window holds the grid (no certificate needed then)
+    const int Wc = whole ? 0x7fffffff : (int)min((long long)W * W, 0x7fffffffll);
+    for (int c0 = x0; c0 <= x1; c0 += 32) {
+      const int x = c0 + lane, A = x - sx;
+      int mine = 0;
+      auto each = [&](auto &&f) {  // f(B, K) of the column's candidates
+        if (x > x1) return;
+        for (int b = b0; b <= b1; ++b) {
+          uint64_t w = __ldg(bits + (size_t)b * n + x) &
+                       row_mask(max(y0 - 64 * b, 0), min(y1 - 64 * b, 63));
+          while (w) {
+            const int B = 64 * b + __ffsll((long long)w) - 1 - sy;
+            w &= w - 1ull;
+            const int K = A * A + B * B;
+            if (K && K <= Wc) f(B, K);
+          }
+        }
+      };
+      each([&](int B, int) {
+        if (A == 0) same_column_limit(B, sy, vmin, vmax);
+        else ++mine;
+      });
+      int incl = mine;
+#pragma unroll
+      for (int i = 1; i < 32; i <<= 1) {
+        const int u = __shfl_up_sync(kFull, incl, i);
+        if (lane >= i) incl += u;
+      }
+      nl += __reduce_add_sync(kFull, A < 0 ? mine : 0);
+      if (mine) {
+        int pos = cnt + incl - mine;
+        const float r = rcp_approx((float)A);
+        each([&](int B, int K) {
+          if (pos < kWarpRec)
+            ws.rec[pos] = FLT ? make_int2(__float_as_int(0.5f * (float)K * r),
+                                          __float_as_int(-(float)B * r))
+                              : make_rec(A, B, K);
+          ++pos;
+        });
+      }
+      cnt += __shfl_sync(kFull, incl, 31);
+    }
+  }
+  vmin = __reduce_max_sync(kFull, vmin);
+  vmax = __reduce_min_sync(kFull, vmax);
+  if (cnt > kWarpRec) return false;
+  __syncwarp();
+  const float eps = 0.25f / (float)W;
+  // |K - S v| <= 2 W^2 + 2 W rb: below 2^23 the reciprocal estimate is safe
+  const bool fast = 2ll * W * W + 2ll * W * rb < (1ll << 23);
+  int R2 = 0;
+  // rows outward from s, one per lane: first sixteen up and sixteen down at
+  // once; a cell that has not ended there on both sides is walked again 32
+  // rows at a time, up and then down
+  float ah = 0.f, al = 0.f;  // folded here: lane q < 4 holds sum q of (W, SX, SY, E)
+  int pass = 0, dir = 1, base = 0, left = -1;
+  for (;;) {
+    const int v = pass == 0 ? (lane < 16 ? lane : 15 - lane) : base + dir * lane;
+    int da = 1, db = 0;
+    const bool in = warp_row<FLT>(support, ws, n, sx, sy, rb2, nl, cnt, eps, fast, v, vmin, vmax,
+                                  da, db);
+    // (a row before the limits' near end is skipped, one past their far end
+    // ends the walk)
+    const bool skip = v >= 0 ? v < vmin : v > vmax;
+    const unsigned stop = __ballot_sync(kFull, !in && !skip);
+    unsigned live;  // the lanes whose rows are walked
+    if (pass == 0) {
+      const unsigned su = stop & 0xffffu, sd = stop >> 16;
+      if (!su || !sd) {
+        pass = 1;
+        continue;
+      }
+      live = ((1u << (__ffs(su) - 1)) - 1u) | (((1u << (__ffs(sd) - 1)) - 1u) << 16);
+    } else {
+      live = stop ? (1u << (__ffs(stop) - 1)) - 1u : kFull;
+    }
+    const bool has = ((live >> lane) & 1u) && in && da <= db;
+    if (has) R2 = max(R2, max(da * da, db * db) + v * v);
+    // the rows' 16-pixel chunks in fold order (row after row), one per lane
+    const int nch = has ? (db - da + 16) >> 4 : 0;
+    int incl = nch;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += u;
+    }
+    const int total = __shfl_sync(kFull, incl, 31);
+    const bool defer = pass == 0 && total <= kWarpEnts;
+    for (int e0 = 0; e0 < total; e0 += kWarpEnts) {
+      const int m = min(total - e0, kWarpEnts);
+      for (int k = lane; k - lane < m; k += 32) {
+        const int e = e0 + k;
+        int r = 0;  // the row of chunk e: the rows whose chunks all come before it
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          if (__shfl_sync(kFull, incl, r + o - 1) <= e) r += o;
+        const int ra = __shfl_sync(kFull, da, r), rb_ = __shfl_sync(kFull, db, r);
+        const int rv = __shfl_sync(kFull, v, r), ri = __shfl_sync(kFull, incl - nch, r);
+        if (k < m) {
+          const int u0 = ra + 16 * (e - ri);
+          float rw, rx, rq;
+          chunk_quads(density + (size_t)(sy + rv) * n, u0, min(rb_, u0 + 15), sx, rw, rx, rq);
+          // fold_chunk's terms of SY and E
+          const float fv = (float)rv, fv2 = (float)(rv * rv);
+          const float yh = __fmul_rn(fv, rw), yl = __fmaf_rn(fv, rw, -yh);
+          float qh = rq, ql = 0.f;
+          dfa_scaled(qh, ql, fv2, rw, 0.f);
+          float4 *o = reinterpret_cast<float4 *>(ws.ent[k]);
+          o[0] = make_float4(rw, rx, yh, qh);
+          o[1] = make_float4(0.f, 0.f, yl, ql);
+        }
+      }
+      __syncwarp();
+      if (defer) continue;
+      if (lane < 4) {  // the four sums side by side, chunk after chunk
+#pragma unroll 4
+        for (int k = 0; k < m; ++k) dfa(ah, al, ws.ent[k][lane], ws.ent[k][4 + lane]);
+      }
+      __syncwarp();
+    }
+    if (pass == 0) {
+      if (defer) left = total;
+      break;
+    }
+    if (stop) {
+      if (dir < 0) break;
+      dir = -1;
+      base = -1;
+    } else {
+      base += 32 * dir;
+    }
+  }
+  if (left < 0 && lane < 4) {
+    ws.sum[lane] = ah;
+    ws.sum[4 + lane] = al;
+  }
+  if (lane == 0) ws.m = left;
+  r2 = __reduce_max_sync(kFull, R2);
+  return true;
+}
+
+// The cell of a site by a warp, left in ws (chunks to fold, or the sums).
+__device__ void cell_sums_warp(const LevelBufs &a, const uint64_t *__restrict__ bits, int n, int sx,
+                               int sy, int W, int rb, int lane, WarpScratch &ws) {
+  const float *density = a.density;
+  const int2 *support = a.support;
+  const int2 yr = *a.sup_range;
+  const int vlo = max(yr.x, sy - rb) - sy, vhi = min(yr.y - 1, sy + rb) - sy;
+  W = max(1, min(W, 2 * rb));
+  int r2 = 0;
+  for (;;) {
+    const bool fits =
+        float_walk(W, rb)
+            ? warp_cell<true>(density, support, bits, n, sx, sy, W, rb, vlo, vhi, lane, ws, r2)
+            : warp_cell<false>(density, support, bits, n, sx, sy, W, rb, vlo, vhi, lane, ws, r2);
+    if (!fits) {
+      // rare, a window of more than kWarpRec candidates: every lane does it all
+      const CellSums c = cell_general(density, support, bits, n, sx, sy, W, rb, vlo, vhi);
+      r2 = c.r2;
+      if (lane == 0) {
+        ws.sum[0] = c.wh, ws.sum[1] = c.xh, ws.sum[2] = c.yh, ws.sum[3] = c.eh;
+        ws.sum[4] = c.wl, ws.sum[5] = c.xl, ws.sum[6] = c.yl, ws.sum[7] = c.el;
+        ws.m = -1;
+      }
+    }
+    const bool whole = W >= sx && W >= sy && W >= n - 1 - sx && W >= n - 1 - sy;
+    if (whole || 4ll * r2 <= (long long)W * W) break;
+    W = min(min(2 * isqrt_ceil(r2) + 1, 2 * W), 2 * rb);
+    __syncwarp();
+  }
+  if (lane == 0) ws.r2 = r2;
+}
+
+// The energy reduction after group g of the block kernel below: group_tail's
+// sums in the same order, but with one counter (the groups are few), so the
+// warp finishing the last group reduces every slot.
 template <int MODE>
-__global__ void __launch_bounds__(32, 32) k_cell_warp(LevelBufs a) {
-  __shared__ WarpScratch ws;
+__device__ __forceinline__ void few_groups_tail(const LevelBufs &a, const IterView &v, unsigned g,
+                                                int lane, float eh, float el, unsigned r2,
+                                                unsigned mv) {
+  DevState *st = a.st;
+  warp_reduce(eh, el, r2, mv);
+  int last = 0;
+  if (lane == 0) {
+    a.gslot[g] = make_float4(eh, el, __uint_as_float(r2), __uint_as_float(mv));
+    last = add_release(&st->done_blocks) == v.ngroups - 1;
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  __threadfence();
+  float th = 0.f, tl = 0.f;  // lane k: slot k's total
+  unsigned tr2 = 0, tmv = 0;
+  for (unsigned sb = 0, k = 0; sb < v.ngroups; sb += kGroupsPerSlot, ++k) {
+    eh = el = 0.f;
+    r2 = mv = 0;
+    for (unsigned i = lane; i < min((unsigned)kGroupsPerSlot, v.ngroups - sb); i += 32) {
+      const float4 q = __ldcg(a.gslot + sb + i);
+      dfa(eh, el, q.x, q.y);
+      r2 = max(r2, __float_as_uint(q.z));
+      mv = max(mv, __float_as_uint(q.w));
+    }
+    warp_reduce(eh, el, r2, mv);
+    tr2 = max(tr2, r2), tmv = max(tmv, mv);
+    if (lane == (int)k) dfa(th, tl, eh, el);
+  }
+  warp_reduce(th, tl, tr2, tmv);
+  if (lane == 0) {
+    const double E = ((double)th + (double)tl) * st->energy_scale;
+    pass_done<MODE>(st, E, tr2, tmv, a.n, v.cur);
+  }
+}
+
+// One Lloyd iteration, one listed site per warp, kBlockSites sites per block.
+// Each warp leaves its site's chunk sums in shared memory; then one warp folds
+// and moves the block's sites, four lanes a site (a fold is one long chain of
+// dependent additions, and most of a site's instructions when a warp runs it
+// alone).  1024^2 / 4096 sites, list included: 43 -> 19 us an iteration (38.8 -> 25 us
+// for the cell kernel with each warp folding its own site).  MODE 0, 4 and 5 as
+// in k_cell (MODE 4 also writes the learned step's features, MODE 5 judges a
+// jump and does not clear ahead).
+template <int MODE>
+__global__ void __launch_bounds__(32 * kBlockSites, 4) k_cell_warp(LevelBufs a) {
+  __shared__ WarpScratch scratch[kBlockSites];
+  __shared__ unsigned s_item;
+  static_assert(kBlockSites == 8 && kWarpSites / 32 <= 32 * kGroupsPerSlot, "lane 4 s + q; slots");
   DevState *st = a.st;
   if (st->snap_stopped) return;
-  const int lane = threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const IterView v = iter_view(a);
   if (MODE != 5 || !st->gate_active)
-    clear_ahead(a, v.cur, (size_t)blockIdx.x * 32 + lane, (size_t)gridDim.x * 32);
+    clear_ahead(a, v.cur, (size_t)blockIdx.x * blockDim.x + threadIdx.x,
+                (size_t)gridDim.x * blockDim.x);
   if (v.ngroups == 0) {  // no sites: the schedule still advances
-    if (blockIdx.x == 0 && lane == 0) pass_done<MODE>(st, 0.0, 0u, 0u, a.n, v.cur);
+    if (blockIdx.x == 0 && threadIdx.x == 0) pass_done<MODE>(st, 0.0, 0u, 0u, a.n, v.cur);
     return;
   }
-  if (v.nsites > kWarpSites) {  // more sites than LevelBufs::sitev holds: per lane
-    for (bool first = true;; first = false) {
-      const unsigned g = next_item(&st->ticket, first, lane);
-      if (g >= v.ngroups) return;
-      cell_group<MODE>(a, v, g, lane, nullptr);
-    }
-  }
   const int n = a.n;
-  for (bool first = true;; first = false) {
-    const unsigned idx = next_item(&st->ticket, first, lane);
-    if (idx >= (unsigned)v.nsites) break;
-    const uint32_t e = a.list[idx];
-    const int sx = (int)(e & 0x7fffu), sy = (int)(e >> 16);
-    const int h = a.hint[(size_t)sy * n + sx];
-    const CellSums cs = cell_sums_warp(a, v.bits, n, sx, sy, h ? h : v.W0, v.rb, lane, ws);
-    const unsigned g = idx / 32;
-    int last = 0;
-    if (lane == 0) {
-      float eh = 0.f, el = 0.f;
-      dfa(eh, el, cs.eh, cs.el);
-      if (MODE == 4) {
-        site_features(a, v, (int)idx, sx, sy, cs);
-        a.jaux[idx] = (uint32_t)min(2 * isqrt_ceil(cs.r2) + v.slack, 255);
+  if (v.nsites > kWarpSites) {  // more sites than LevelBufs::sitev holds: per lane
+    unsigned g = blockIdx.x * kBlockSites + warp;
+    while (g < v.ngroups) {
+      cell_group<MODE>(a, v, g, lane, nullptr);
+      if (lane == 0) g = gridDim.x * kBlockSites + atomicAdd(&st->ticket, 1u);
+      g = __shfl_sync(0xffffffffu, g, 0);
+    }
+    return;
+  }
+  for (unsigned item = blockIdx.x; item * kBlockSites < (unsigned)v.nsites;) {
+    const unsigned idx0 = item * kBlockSites, idx = idx0 + warp;
+    const int count = min(kBlockSites, v.nsites - (int)idx0);
+    if ((int)warp < count) {
+      const uint32_t e = a.list[idx];
+      const int sx = (int)(e & 0x7fffu), sy = (int)(e >> 16);
+      const int h = a.hint[(size_t)sy * n + sx];
+      cell_sums_warp(a, v.bits, n, sx, sy, h ? h : v.W0, v.rb, lane, scratch[warp]);
+    }
+    if (threadIdx.x == 0) s_item = gridDim.x + atomicAdd(&st->ticket, 1u);
+    __syncthreads();
+    item = s_item;
+    if (warp == 0) {
+      // fold: lane 4 s + q takes sum q of site s
+      const int s = lane >> 2, q = lane & 3;
+      float ah = 0.f, al = 0.f;
+      if (s < count) {
+        const WarpScratch &ws = scratch[s];
+        const int m = ws.m;
+        if (m < 0) ah = ws.sum[q], al = ws.sum[4 + q];
+#pragma unroll 4
+        for (int k = 0; k < m; ++k) dfa(ah, al, ws.ent[k][q], ws.ent[k][4 + q]);
       }
-      const unsigned mv = move_site(a, v, e, sx, sy, cs);
-      a.sitev[idx] = make_float4(eh, el, __uint_as_float((unsigned)cs.r2), __uint_as_float(mv));
+      CellSums cs;
+      const int src = (lane & 7) * 4;
+      constexpr unsigned kFull = 0xffffffffu;
+      cs.wh = __shfl_sync(kFull, ah, src), cs.wl = __shfl_sync(kFull, al, src);
+      cs.xh = __shfl_sync(kFull, ah, src + 1), cs.xl = __shfl_sync(kFull, al, src + 1);
+      cs.yh = __shfl_sync(kFull, ah, src + 2), cs.yl = __shfl_sync(kFull, al, src + 2);
+      cs.eh = __shfl_sync(kFull, ah, src + 3), cs.el = __shfl_sync(kFull, al, src + 3);
+      const unsigned g = idx0 / 32;  // the block's sites lie in one group
+      if (lane < count) {
+        cs.r2 = scratch[lane].r2;
+        const uint32_t e = a.list[idx0 + lane];
+        const int sx = (int)(e & 0x7fffu), sy = (int)(e >> 16);
+        float eh = 0.f, el = 0.f;
+        dfa(eh, el, cs.eh, cs.el);
+        if (MODE == 4) {
+          site_features(a, v, (int)idx0 + lane, sx, sy, cs);
+          a.jaux[idx0 + lane] = (uint32_t)min(2 * isqrt_ceil(cs.r2) + v.slack, 255);
+        }
+        const unsigned mv = move_site(a, v, e, sx, sy, cs);
+        a.sitev[idx0 + lane] =
+            make_float4(eh, el, __uint_as_float((unsigned)cs.r2), __uint_as_float(mv));
+      }
+      __syncwarp();
+      // the group's last sites: its values in lane order, then the tail
       const unsigned gsize = min(32u, (unsigned)v.nsites - g * 32);
-      last = add_release(a.gcnt + g) == gsize - 1;
+      int last = 0;
+      if (lane == 0)
+        last = add_release(a.gcnt + g, (unsigned)count) == gsize - (unsigned)count;
+      if (__shfl_sync(0xffffffffu, last, 0)) {
+        __threadfence();
+        float eh = 0.f, el = 0.f;
+        unsigned r2 = 0, mv = 0;
+        if ((unsigned)lane < gsize) {
+          const float4 t = __ldcg(a.sitev + g * 32 + lane);
+          eh = t.x, el = t.y, r2 = __float_as_uint(t.z), mv = __float_as_uint(t.w);
+        }
+        if (lane == 0) a.gcnt[g] = 0u;
+        few_groups_tail<MODE>(a, v, g, lane, eh, el, r2, mv);
+      }
     }
-    if (!__shfl_sync(0xffffffffu, last, 0)) continue;
-    // the group's last site: its values in lane order, then the usual tail
-    __threadfence();
-    float eh = 0.f, el = 0.f;
-    unsigned r2 = 0, mv = 0;
-    if (g * 32 + lane < (unsigned)v.nsites) {
-      const float4 q = __ldcg(a.sitev + g * 32 + lane);
-      eh = q.x, el = q.y, r2 = __float_as_uint(q.z), mv = __float_as_uint(q.w);
-    }
-    if (lane == 0) a.gcnt[g] = 0u;
-    group_tail<MODE>(a, v, g, lane, eh, el, r2, mv);
+    __syncthreads();  // the scratch and s_item are free again
   }
 }
 
@@ -1670,15 +1932,15 @@ cudaError_t cells_configure() {
     if ((e = fit(fn)) != cudaSuccess) return e;
   for (auto fn : {k_cell<2>, k_cell<4>, k_cell<5>})
     if ((e = fit(fn)) != cudaSuccess) return e;
-  // one site per warp: its shared scratch (candidates, chunk sums) needs about
-  // 3.3 KB per block with the reserved 1 KB
+  // one site per warp: a block's shared scratch (candidates, chunk sums) is 34 KB
   int perw = 0;
   for (auto fn : {k_cell_warp<0>, k_cell_warp<4>, k_cell_warp<5>}) {
     int per = 0;
-    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 50)) !=
+    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 64)) !=
         cudaSuccess)
       return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 32, 0)) != cudaSuccess)
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 32 * kBlockSites, 0)) !=
+        cudaSuccess)
       return e;
     perw = perw ? min(perw, per) : per;
   }
@@ -1724,10 +1986,11 @@ cudaError_t launch_cells(const LevelBufs &b, int moments_only, double *out4, cud
   if (dev < 0 || dev >= 64 || !g_cell_grid[dev]) return cudaErrorNotReady;
   if (grid <= 0 || grid > g_cell_grid[dev]) grid = g_cell_grid[dev];
   if ((moments_only == 0 || moments_only == 4 || moments_only == 5) && b.sitev && b.gcnt) {
-    const int wg = min(grid, g_warp_grid[dev]);
-    if (moments_only == 4) k_cell_warp<4><<<wg, 32, 0, s>>>(b);
-    else if (moments_only == 5) k_cell_warp<5><<<wg, 32, 0, s>>>(b);
-    else k_cell_warp<0><<<wg, 32, 0, s>>>(b);
+    // (grid counts warps)
+    const int wg = max(1, min(grid / kBlockSites, g_warp_grid[dev])), wt = 32 * kBlockSites;
+    if (moments_only == 4) k_cell_warp<4><<<wg, wt, 0, s>>>(b);
+    else if (moments_only == 5) k_cell_warp<5><<<wg, wt, 0, s>>>(b);
+    else k_cell_warp<0><<<wg, wt, 0, s>>>(b);
     return cudaGetLastError();
   }
   switch (moments_only) {

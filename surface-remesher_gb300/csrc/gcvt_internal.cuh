@@ -20,7 +20,7 @@ constexpr int kNoneAbove = -32768;  // "no site above" in the column summaries
 constexpr int kNoneBelow = 32767;   // "no site below"
 constexpr int kBand = 64;           // PBA+ phase-1 band height: n / m1 == 64 for
                                     // every entry of gcvt.cu:842-847
-constexpr int kWarpSites = 8192;    // one site per warp up to this many sites
+constexpr int kWarpSites = 32768;  // one site per warp at most for this many sites
 constexpr int kListWords = 512;    // bitmap words per site-list block
 constexpr int kMinN = 256;   // n must be a multiple of 256 (S = n/32 >= 8)
 constexpr int kMaxN = 8192;  // largest grid (the row pass's whole-row buffer: 32 KB)
