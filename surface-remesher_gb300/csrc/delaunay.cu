@@ -132,6 +132,22 @@ __device__ bool disc_in_window(int ux, int uy, int wx, int wy, int sx, int sy, i
          clear_of(Nx, Ny, D, wx0, wx1, wy1 + 1, gy1);
 }
 
+// disc_in_window decided in floats where that is safe (false: not decided).
+// The centre's error is below e (its products' roundings over |D|), the
+// radius's below twice that; a grid point outside the window is at least a
+// pixel past its edge.
+__device__ __forceinline__ bool disc_surely_in(int ux, int uy, int wx, int wy, int sx, int sy,
+                                               int x0, int x1, int y0, int y1, int n) {
+  const float fux = (float)ux, fuy = (float)uy, fwx = (float)wx, fwy = (float)wy;
+  const float u2 = fux * fux + fuy * fuy, w2 = fwx * fwx + fwy * fwy;
+  const float iD = 0.5f / (float)(ux * wy - uy * wx);
+  const float cx = (fwy * u2 - fuy * w2) * iD, cy = (fux * w2 - fwx * u2) * iD;
+  const float e = (fabsf(fwy) + fabsf(fwx)) * u2 + (fabsf(fuy) + fabsf(fux)) * w2;
+  const float r = sqrtf(cx * cx + cy * cy) + 4.f * e * iD * 0x1p-21f + 0.01f;
+  return (x1 == n - 1 || cx + r < (float)(x1 + 1 - sx)) && (x0 == 0 || cx - r > (float)(x0 - 1 - sx)) &&
+         (y1 == n - 1 || cy + r < (float)(y1 + 1 - sy)) && (y0 == 0 || cy - r > (float)(y0 - 1 - sy));
+}
+
 // Site occupancy of 16 x 16 pixel tiles and its pyramid (level l: tiles of
 // 16 << l pixels, a byte each, nonzero when the tile holds a site).
 constexpr int kTile = 16;  // 1 << 4
@@ -285,6 +301,157 @@ __device__ __forceinline__ uint64_t band_rows(int b, int lo, int hi) {
   if (lo > hi) return 0ull;
   const uint64_t up = hi >= 63 ? ~0ull : ((2ull << hi) - 1ull);
   return up & ~((1ull << lo) - 1ull);
+}
+
+// The star of site (sx, sy) among the free sites of the window [x0, x1] x
+// [y0, y1] by gift wrapping, when they are at most 64 (else false, st unchanged).  The
+// candidates lie two per lane; from the nearest one (always a neighbour), the
+// next neighbour counter-clockwise of u is the candidate left of u that sees
+// (site, u) under the largest angle: a float cotangent (exact integer
+// numerator and denominator, one division) and one warp minimum decide, and
+// candidates within its error of the minimum -- co-circular ones above all -- are
+// compared with the exact perturbed predicate.  An open gap (no candidate to
+// the left) ends the walk; the rest is walked clockwise.  Inserting the same
+// candidates one by one (winsert) gives the same star in about ten times the
+// instructions: every insertion is a chain of decisions the lanes cannot share.
+__device__ bool wwrap(WStar &st, const uint64_t *bits, const uint64_t *fixed, int n, int sx, int sy,
+                      int x0, int x1, int y0, int y1, int *buf) {
+  const int lane = lane_id();
+  int cnt = 0;
+  for (int cx = x0; cx <= x1; cx += 32) {
+    const int x = cx + lane;
+    for (int b = y0 / kBand; b <= y1 / kBand; ++b) {
+      uint64_t w = 0;
+      if (x <= x1) w = free_word(bits, fixed, (size_t)b * n + x) & band_rows(b, y0, y1);
+      if (x == sx && sy / kBand == b) w &= ~(1ull << (sy % kBand));
+      const int mine = __popcll(w);
+      int incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int total = __shfl_sync(kFull, incl, 31);
+      if (cnt + total > 64) return false;
+      int pos = cnt + incl - mine;
+      while (w) {
+        const int i = __ffsll((long long)w) - 1;
+        w &= w - 1ull;
+        buf[pos++] = pk(x - sx, b * kBand + i - sy);
+      }
+      cnt += total;
+    }
+  }
+  __syncwarp();
+  const bool two = cnt > 32;
+  const int qa = lane < cnt ? buf[lane] : 0, qb = lane + 32 < cnt ? buf[lane + 32] : 0;
+  const int ax = pdx(qa), ay = pdy(qa), bx = pdx(qb), by = pdy(qb);
+  const int a2 = ax * ax + ay * ay, b2 = bx * bx + by * by;
+  __syncwarp();
+  st.a = st.b = 0;
+  st.m = 0;
+  if (cnt == 0) return true;
+  const long long hp = hkey(n, sx, sy);
+  // the neighbour after u in direction dir (1 counter-clockwise), 0: none
+  auto next = [&](int u, int dir) -> int {
+    const int ux = pdx(u), uy = pdy(u);
+    auto key = [&](int q, int qx, int qy, int q2) -> int {
+      const int c = dir * (ux * qy - uy * qx);
+      const float k = __fdividef((float)(q2 - ux * qx - uy * qy), (float)c);
+      const int i = __float_as_int(k);
+      return q != 0 && c > 0 ? i ^ ((i >> 31) & 0x7fffffff) : INT_MAX;
+    };
+    const int ka = key(qa, ax, ay, a2), kb = two ? key(qb, bx, by, b2) : INT_MAX;
+    const int k = __reduce_min_sync(kFull, min(ka, kb));
+    if (k == INT_MAX) return 0;
+    // integers below 2^28 to float and the division: 2^-20 relative in all
+    const float f = __int_as_float(k ^ ((k >> 31) & 0x7fffffff));
+    const float t = f + fabsf(f) * 0x1p-17f;
+    const int ti = __float_as_int(t), tk = ti ^ ((ti >> 31) & 0x7fffffff);
+    unsigned ma = __ballot_sync(kFull, ka <= tk), mb = two ? __ballot_sync(kFull, kb <= tk) : 0u;
+    int best = 0;
+    while (ma | mb) {
+      int c;
+      if (ma) {
+        c = __shfl_sync(kFull, qa, __ffs(ma) - 1);
+        ma &= ma - 1u;
+      } else {
+        c = __shfl_sync(kFull, qb, __ffs(mb) - 1);
+        mb &= mb - 1u;
+      }
+      if (best) {
+        const int px = pdx(best), py = pdy(best), cx = pdx(c), cy = pdy(c);
+        const long long hu = hkey(n, sx + ux, sy + uy), hb = hkey(n, sx + px, sy + py),
+                        hc = hkey(n, sx + cx, sy + cy);
+        const bool inside = dir > 0 ? in_circle(ux, uy, px, py, cx, cy, hp, hu, hb, hc)
+                                    : in_circle(px, py, ux, uy, cx, cy, hp, hb, hu, hc);
+        if (!inside) continue;
+      }
+      best = c;
+    }
+    return best;
+  };
+  // the nearest candidate
+  const unsigned da = lane < cnt ? (unsigned)a2 : 0xffffffffu,
+                 db = lane + 32 < cnt ? (unsigned)b2 : 0xffffffffu;
+  const unsigned dm = __reduce_min_sync(kFull, min(da, db));
+  const unsigned na = __ballot_sync(kFull, da == dm), nb = __ballot_sync(kFull, db == dm);
+  const int u0 = na ? __shfl_sync(kFull, qa, __ffs(na) - 1) : __shfl_sync(kFull, qb, __ffs(nb) - 1);
+  int m = 1, u = u0;
+  wset(st, 0, u0);
+  bool open = false;
+  for (;;) {
+    u = next(u, 1);
+    if (u == u0) break;
+    if (u == 0) {
+      open = true;
+      break;
+    }
+    if (m >= kStar) {  // (cannot happen with at most 64 candidates)
+      st.overflow = true;
+      return true;
+    }
+    wset(st, m++, u);
+  }
+  st.m = m;
+  if (open) {
+    for (u = u0;;) {
+      u = next(u, -1);
+      if (u == 0) break;
+      if (st.m >= kStar) {
+        st.overflow = true;
+        return true;
+      }
+      wins(st, 0, u);
+    }
+  }
+  // the list starts with the smallest angle from the +x axis
+  m = st.m;
+  auto before = [](int p, int q) {
+    const int px = pdx(p), py = pdy(p), qx = pdx(q), qy = pdy(q);
+    const int hp_ = half_of(px, py), hq_ = half_of(qx, qy);
+    return hp_ < hq_ || (hp_ == hq_ && px * qy - py * qx > 0);
+  };
+  const int last = wget(st, m - 1);
+  int pa = __shfl_up_sync(kFull, st.a, 1), pb = __shfl_up_sync(kFull, st.b, 1);
+  const int a31 = __shfl_sync(kFull, st.a, 31);
+  if (lane == 0) {
+    pa = last;
+    pb = a31;
+  }
+  const unsigned ra = __ballot_sync(kFull, lane < m && before(st.a, pa));
+  const unsigned rb = __ballot_sync(kFull, lane + 32 < m && before(st.b, pb));
+  const int rot = ra ? __ffs(ra) - 1 : (rb ? 31 + __ffs(rb) : 0);
+  auto at = [&](int k) {  // entry (k + rot) mod m
+    k += rot;
+    if (k >= m) k -= m;
+    const int va = __shfl_sync(kFull, st.a, k & 31), vb = __shfl_sync(kFull, st.b, k & 31);
+    return k < 32 ? va : vb;
+  };
+  const int ea = at(lane), eb = at(lane + 32);
+  st.a = ea;
+  st.b = eb;
+  return true;
 }
 
 // Insert the free sites of the window [nx0, nx1] x [ny0, ny1] that are not
@@ -589,8 +756,17 @@ __device__ __forceinline__ int wnext(const WStar &s, int k) {
 // ring).  kWindow and kWiden are the fastest of a sweep on converged CVT
 // sites and on uniform random ones at 4096^2 and 8192^2.  Returns false
 // when the star overflowed.
-constexpr float kWindow = 1.4f;
-constexpr int kWiden = 1;
+#ifndef KWIN
+#define KWIN 2.0f
+#endif
+#ifndef KWID
+#define KWID 1
+#endif
+#ifndef KGROW
+#define KGROW 1.7f
+#endif
+constexpr float kWindow = KWIN;
+constexpr int kWiden = KWID;
 constexpr int kBoxCols = 96, kBoxBands = 3;  // largest disc box scanned directly
 __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixed, int n, int sx,
                            int sy, const Pyr &py, const unsigned *tilecnt, unsigned *stk) {
@@ -598,20 +774,21 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
   st.m = 0;
   st.overflow = false;
   const int tx = sx / kTile, ty = sy / kTile, nt0 = py.nt[0], lane = lane_id();
-  unsigned cnt = 0, tiles = 0;
-  for (int j = max(ty - 1, 0); j <= min(ty + 1, nt0 - 1); ++j)
-    for (int i = max(tx - 1, 0); i <= min(tx + 1, nt0 - 1); ++i) {
-      cnt += tilecnt[brick_of(i, j, nt0)];
-      ++tiles;
-    }
+  // (a lane per tile)
+  const int ti = tx - 1 + lane % 3, tj = ty - 1 + lane / 3;
+  const bool tile = lane < 9 && ti >= 0 && ti < nt0 && tj >= 0 && tj < nt0;
+  const unsigned cnt = __reduce_add_sync(kFull, tile ? tilecnt[brick_of(ti, tj, nt0)] : 0u);
+  const int tiles = __popc(__ballot_sync(kFull, tile));
   int W = (int)ceilf(kWindow * sqrtf((float)(tiles * kTile * kTile) / (float)max(cnt, 1u)));
   W = min(max(W, 4), 2 * n);
   int x0 = sx, x1 = sx, y0 = sy, y1 = sy;  // the window so far: the site
-  bool first = true;
+  bool first = true, wrap = true;
   for (;;) {
     const int nx0 = max(0, sx - W), nx1 = min(n - 1, sx + W);
     const int ny0 = max(0, sy - W), ny1 = min(n - 1, sy + W);
-    wwindow(st, bits, fixed, n, sx, sy, nx0, nx1, ny0, ny1, x0, x1, y0, y1);
+    // wrapped while the candidates are few, then ring by ring
+    wrap = wrap && wwrap(st, bits, fixed, n, sx, sy, nx0, nx1, ny0, ny1, reinterpret_cast<int *>(stk));
+    if (!wrap) wwindow(st, bits, fixed, n, sx, sy, nx0, nx1, ny0, ny1, x0, x1, y0, y1);
     x0 = nx0;
     x1 = nx1;
     y0 = ny0;
@@ -644,12 +821,14 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
         if (lane < m) {
           const int ux = pdx(st.a), uy = pdy(st.a), wx = pdx(wa), wy = pdy(wa);
           need_a = open_gap(ux, uy, wx, wy) ||
-                   !disc_in_window(ux, uy, wx, wy, sx, sy, x0, x1, y0, y1, n);
+                   (!disc_surely_in(ux, uy, wx, wy, sx, sy, x0, x1, y0, y1, n) &&
+                    !disc_in_window(ux, uy, wx, wy, sx, sy, x0, x1, y0, y1, n));
         }
         if (lane + 32 < m) {
           const int ux = pdx(st.b), uy = pdy(st.b), wx = pdx(wb), wy = pdy(wb);
           need_b = open_gap(ux, uy, wx, wy) ||
-                   !disc_in_window(ux, uy, wx, wy, sx, sy, x0, x1, y0, y1, n);
+                   (!disc_surely_in(ux, uy, wx, wy, sx, sy, x0, x1, y0, y1, n) &&
+                    !disc_in_window(ux, uy, wx, wy, sx, sy, x0, x1, y0, y1, n));
         }
       }
       unsigned pa = __ballot_sync(kFull, need_a), pb = __ballot_sync(kFull, need_b);
@@ -706,8 +885,8 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
       }
     } while (changed);
     if (ok) return true;
+    W = first ? min((int)ceilf(KGROW * W), 2 * n) : min(2 * W, 2 * n);
     first = false;
-    W = min(2 * W, 2 * n);
   }
 }
 
@@ -814,50 +993,266 @@ __device__ __forceinline__ int site_index(const uint64_t *bits, const uint64_t *
   return (int)(coloff[x] + colpre[(size_t)b * n + x] + (unsigned)__popcll(below));
 }
 
-// The star of the t-th site in tile order (one warp per site), stored
-// under its index in delaunayInput's order with the number of triangles it
-// writes.
-__global__ void __launch_bounds__(32 * kWarpsPerBlock)
-    k_dt_star(const uint64_t *__restrict__ bits, const uint64_t *__restrict__ fixed, int n,
-              const int *__restrict__ order, int nsites, Pyr py,
-              const unsigned *__restrict__ coloff, const unsigned *__restrict__ colpre,
-              const unsigned *__restrict__ tilecnt, int *sitepos, int *stars, int *degree,
-              unsigned *tcount, int *err) {
-  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (t >= nsites) return;  // the whole warp
+#ifndef MB
+#define MB 6
+#endif
+// What a star kernel writes per site (under its index in delaunayInput's
+// order): its pixel, its star, the star's size and the triangles it writes --
+// the ones it comes first in, in (x, y) order.
+struct StarOut {
+  const unsigned *coloff, *colpre;
+  int *sitepos, *stars, *degree;
+  unsigned *tcount;
+  int *err;
+};
+
+__device__ __forceinline__ bool owns_tri(int sx, int sy, int u, int w) {
+  const int ux = sx + pdx(u), uy = sy + pdy(u), wx = sx + pdx(w), wy = sy + pdy(w);
+  return (sx < ux || (sx == ux && sy < uy)) && (sx < wx || (sx == wx && sy < wy));
+}
+
+// One site by the whole warp, any case.
+__device__ __noinline__ void full_site(const uint64_t *bits, const uint64_t *fixed, int n, int pos,
+                                       const Pyr &py, const unsigned *tilecnt, unsigned *stk,
+                                       const StarOut &out) {
   const int lane = lane_id();
-  const int sx = pdx(order[t]) & 0xffff, sy = pdy(order[t]);
-  const int xm = site_index(bits, fixed, n, coloff, colpre, sx, sy);
-  __shared__ unsigned s_front[kWarpsPerBlock][kFrontier];
+  const int sx = pdx(pos) & 0xffff, sy = pdy(pos);
+  const int xm = site_index(bits, fixed, n, out.coloff, out.colpre, sx, sy);
   WStar st;
-  if (!wsite_star(st, bits, fixed, n, sx, sy, py, tilecnt, s_front[threadIdx.x >> 5])) {
+  if (!wsite_star(st, bits, fixed, n, sx, sy, py, tilecnt, stk)) {
     if (lane == 0) {
-      atomicOr(err, 1);
-      sitepos[xm] = order[t];
-      degree[xm] = 0;
-      tcount[xm] = 0;
+      atomicOr(out.err, 1);
+      out.sitepos[xm] = pos;
+      out.degree[xm] = 0;
+      out.tcount[xm] = 0;
     }
     return;
   }
   const int m = st.m;
-  int *row = stars + (size_t)xm * kStar;
+  int *row = out.stars + (size_t)xm * kStar;
   if (lane < m) row[lane] = st.a;
   if (lane + 32 < m) row[lane + 32] = st.b;
-  // triangles (k, k + 1) this site writes: the one of its vertices first in
-  // (x, y) order
   auto owns = [&](int u, int w) {
-    if (m < 2 || open_gap(pdx(u), pdy(u), pdx(w), pdy(w))) return false;
-    const int ux = sx + pdx(u), uy = sy + pdy(u), wx = sx + pdx(w), wy = sy + pdy(w);
-    return (sx < ux || (sx == ux && sy < uy)) && (sx < wx || (sx == wx && sy < wy));
+    return m >= 2 && !open_gap(pdx(u), pdy(u), pdx(w), pdy(w)) && owns_tri(sx, sy, u, w);
   };
   const int wa = wnext(st, lane), wb = wnext(st, lane + 32);
   const bool oa = lane < m && owns(st.a, wa), ob = lane + 32 < m && owns(st.b, wb);
   const int own = __popc(__ballot_sync(kFull, oa)) + __popc(__ballot_sync(kFull, ob));
   if (lane == 0) {
-    sitepos[xm] = order[t];
-    degree[xm] = m;
-    tcount[xm] = own;
+    out.sitepos[xm] = pos;
+    out.degree[xm] = m;
+    out.tcount[xm] = own;
   }
+}
+
+// Four sites of a warp, eight lanes each, for the common case: at most 32
+// candidates in a window of kQuadWindow spacings (radius <= 31 pixels), a closed star
+// of at most 16 neighbours, every triangle's circle surely inside the window.
+// The same gift wrapping as wwrap; the four walks go in step, so a step's
+// instructions serve four sites.  Offsets up to 31 pixels keep every cotangent's
+// numerator and denominator exact in floats.  Returns the groups it leaves to
+// full_site.  4096^2, 262,144 CVT sites: a warp per site by wwrap alone took
+// 1,449 instructions a site.
+constexpr float kQuadWindow = 1.8f;
+constexpr int kQuadCand = 32, kQuadStar = 16;
+struct QuadScratch {
+  int cand[4][kQuadCand];
+  int star[4][kQuadStar];
+};
+
+__device__ __forceinline__ unsigned quad_stars(const uint64_t *bits, const uint64_t *fixed, int n,
+                                               const int *order, int t0, int nsites, const Pyr &py,
+                                               const unsigned *tilecnt, QuadScratch &sc,
+                                               const StarOut &out) {
+  const int lane = lane_id(), g = lane >> 3, l = lane & 7;
+  const bool on = t0 + g < nsites;
+  const int epos = order[min(t0 + g, nsites - 1)];
+  const int sx = pdx(epos) & 0xffff, sy = pdy(epos);
+  // the window from the 3 x 3 tiles' site counts
+  const int tx = sx / kTile, ty = sy / kTile, nt0 = py.nt[0];
+  unsigned near = 0;
+  for (int k = l; k < 9; k += 8) {
+    const int i = tx - 1 + k % 3, j = ty - 1 + k / 3;
+    if (i >= 0 && i < nt0 && j >= 0 && j < nt0) near += tilecnt[brick_of(i, j, nt0)];
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) near += __shfl_xor_sync(kFull, near, o);
+  const int tiles = (min(tx + 1, nt0 - 1) - max(tx - 1, 0) + 1) *
+                    (min(ty + 1, nt0 - 1) - max(ty - 1, 0) + 1);
+  int W = (int)ceilf(kQuadWindow * sqrtf((float)(tiles * kTile * kTile) / (float)max(near, 1u)));
+  W = max(W, 4);
+  bool ok = on && W <= 31;
+  W = min(W, 31);
+  const int x0 = max(0, sx - W), x1 = min(n - 1, sx + W);
+  const int y0 = max(0, sy - W), y1 = min(n - 1, sy + W), o = sy - y0;
+  // candidates: a lane per column, a column's rows as one word from row y0 on
+  int cnt = 0;
+  {
+    const int b0 = y0 / kBand, b1 = y1 / kBand, sh = y0 % kBand;
+    const uint64_t rm = (2ull << (y1 - y0)) - 1ull;
+    const int ncol = __reduce_max_sync(kFull, x1 - x0 + 1);
+    for (int c = 0; c < ncol; c += 8) {
+      const int x = x0 + c + l;
+      uint64_t w = 0;
+      if (ok && x <= x1) {
+        w = free_word(bits, fixed, (size_t)b0 * n + x) >> sh;
+        if (b1 > b0) w |= free_word(bits, fixed, (size_t)b1 * n + x) << (kBand - sh);
+        w &= rm;
+        if (x == sx) w &= ~(1ull << o);
+      }
+      const int mine = __popcll(w);
+      int incl = mine;
+#pragma unroll
+      for (int i = 1; i < 8; i <<= 1) {
+        const int v = __shfl_up_sync(kFull, incl, i, 8);
+        if (l >= i) incl += v;
+      }
+      int p = cnt + incl - mine;
+      cnt += __shfl_sync(kFull, incl, 7, 8);
+      while (w) {
+        const int i = __ffsll((long long)w) - 1;
+        w &= w - 1ull;
+        if (p < kQuadCand) sc.cand[g][p] = pk(x - sx, i - o);
+        ++p;
+      }
+    }
+  }
+  ok = ok && cnt >= 3 && cnt <= kQuadCand;
+  __syncwarp();
+  constexpr int kPer = kQuadCand / 8;
+  const int nj = (__reduce_max_sync(kFull, ok ? cnt : 0) + 7) / 8;  // candidates per lane used
+  float qx[kPer], qy[kPer], q2[kPer];
+  unsigned near_q = 0xffffffffu;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int k = l + 8 * j;
+    const int q = ok && k < cnt ? sc.cand[g][k] : 0;
+    qx[j] = (float)pdx(q), qy[j] = (float)pdy(q);
+    q2[j] = qx[j] * qx[j] + qy[j] * qy[j];
+    if (q) near_q = min(near_q, ((unsigned)q2[j] << 5) | (unsigned)k);
+  }
+#pragma unroll
+  for (int i = 4; i > 0; i >>= 1) near_q = min(near_q, __shfl_xor_sync(kFull, near_q, i));
+  const int u0 = ok ? sc.cand[g][near_q & 31u] : 0;  // the nearest: a neighbour
+  int u = u0, m = 1;
+  if (l == 0) sc.star[g][0] = u0;
+  bool act = ok;
+  const long long hp = hkey(n, sx, sy);
+  while (__any_sync(kFull, act)) {
+    const float ux = (float)pdx(u), uy = (float)pdy(u);
+    float k[kPer], kmin = INFINITY;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      k[j] = INFINITY;
+      if (j < nj) {
+        const float c = ux * qy[j] - uy * qx[j];
+        const float d = q2[j] - (ux * qx[j] + uy * qy[j]);
+        if (c > 0.f) k[j] = __fdividef(d, c);
+        kmin = fminf(kmin, k[j]);
+      }
+    }
+#pragma unroll
+    for (int i = 4; i > 0; i >>= 1) kmin = fminf(kmin, __shfl_xor_sync(kFull, kmin, i));
+    const float t = kmin + fabsf(kmin) * 0x1p-17f;
+    unsigned cand = 0;  // bit 8 j + lane: candidates within the error of the smallest
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+      if (j < nj) cand |= ((__ballot_sync(kFull, k[j] <= t) >> (8 * g)) & 0xffu) << (8 * j);
+    if (!(kmin < INFINITY)) {  // an open gap
+      if (act) ok = false;
+      act = false;
+    }
+    if (act) {
+      const int first = __ffs(cand) - 1;
+      cand &= cand - 1u;
+      int best = sc.cand[g][first];
+      while (cand) {  // co-circular, or nearly
+        const int c = sc.cand[g][__ffs(cand) - 1];
+        cand &= cand - 1u;
+        if (in_circle(pdx(u), pdy(u), pdx(best), pdy(best), pdx(c), pdy(c), hp,
+                      hkey(n, sx + pdx(u), sy + pdy(u)), hkey(n, sx + pdx(best), sy + pdy(best)),
+                      hkey(n, sx + pdx(c), sy + pdy(c))))
+          best = c;
+      }
+      if (best == u0) {
+        act = false;
+      } else if (m == kQuadStar) {
+        ok = act = false;
+      } else {
+        if (l == 0) sc.star[g][m] = best;
+        ++m;
+        u = best;
+      }
+    }
+    __syncwarp();
+  }
+  // certificate, and where the angular order starts
+  const unsigned gm = 0xffu << (8 * g);
+  bool bad = false;
+  int rot = 0;
+#pragma unroll
+  for (int h = 0; h < kQuadStar / 8; ++h) {
+    const int k = l + 8 * h;
+    bool lead = false;
+    if (ok && k < m) {
+      const int a = sc.star[g][k], p = sc.star[g][k ? k - 1 : m - 1],
+                w = sc.star[g][k + 1 < m ? k + 1 : 0];
+      bad = bad || !disc_surely_in(pdx(a), pdy(a), pdx(w), pdy(w), sx, sy, x0, x1, y0, y1, n);
+      const int ha = half_of(pdx(a), pdy(a)), hq = half_of(pdx(p), pdy(p));
+      lead = ha < hq || (ha == hq && pdx(a) * pdy(p) - pdy(a) * pdx(p) > 0);
+    }
+    const unsigned lm = __ballot_sync(kFull, lead) & gm;
+    if (lm) rot = 8 * h + __ffs(lm >> (8 * g)) - 1;
+  }
+  if (__ballot_sync(kFull, bad) & gm) ok = false;
+  int xm = 0;
+  if (ok && l == 0) xm = site_index(bits, fixed, n, out.coloff, out.colpre, sx, sy);
+  xm = __shfl_sync(kFull, xm, 0, 8);
+  int own = 0;
+#pragma unroll
+  for (int h = 0; h < kQuadStar / 8; ++h) {
+    const int k = l + 8 * h;
+    bool mine = false;
+    if (ok && k < m) {
+      int i = k + rot;
+      if (i >= m) i -= m;
+      const int a = sc.star[g][i], w = sc.star[g][i + 1 < m ? i + 1 : 0];
+      out.stars[(size_t)xm * kStar + k] = a;
+      mine = owns_tri(sx, sy, a, w);
+    }
+    own += __popc(__ballot_sync(kFull, mine) & gm);
+  }
+  if (ok && l == 0) {
+    out.sitepos[xm] = epos;
+    out.degree[xm] = m;
+    out.tcount[xm] = own;
+  }
+  const unsigned left = __ballot_sync(kFull, on && !ok && l == 0);
+  __syncwarp();
+  return (left & 1u) | ((left >> 7) & 2u) | ((left >> 14) & 4u) | ((left >> 21) & 8u);
+}
+
+// The stars of the sites in tile order: a warp per site for the nedge sites
+// of edge tiles (their stars reach far), four sites per warp for the others.
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, MB)
+    k_dt_star(const uint64_t *__restrict__ bits, const uint64_t *__restrict__ fixed, int n,
+              const int *__restrict__ order, int nsites, int nedge, Pyr py,
+              const unsigned *__restrict__ tilecnt, StarOut out) {
+  __shared__ union {
+    unsigned front[kFrontier];
+    QuadScratch quad;
+  } s_warp[kWarpsPerBlock];
+  const int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  auto &sw = s_warp[threadIdx.x >> 5];
+  if (t < nedge) {
+    full_site(bits, fixed, n, order[t], py, tilecnt, sw.front, out);
+    return;
+  }
+  const int t0 = nedge + 4 * (t - nedge);
+  if (t0 >= nsites) return;  // the whole warp
+  unsigned left = quad_stars(bits, fixed, n, order, t0, nsites, py, tilecnt, sw.quad, out);
+  for (; left; left &= left - 1u)
+    full_site(bits, fixed, n, order[t0 + __ffs(left) - 1], py, tilecnt, sw.front, out);
 }
 
 __global__ void k_dt_emit(const uint64_t *__restrict__ bits, const uint64_t *__restrict__ fixed,
@@ -1012,10 +1407,11 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
   DCK(cudaGetLastError());
   int rc = scan_big(cnt2, 2 * ntiles, tileoff, sc, s);
   if (rc) return rc;
-  unsigned nsites_u = 0;
+  unsigned nsites_u = 0, nedge_u = 0;
   DCK(cudaMemcpyAsync(&nsites_u, coloff + n, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+  DCK(cudaMemcpyAsync(&nedge_u, tileoff + ntiles, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   DCK(cudaStreamSynchronize(s));
-  const int nsites = (int)nsites_u;
+  const int nsites = (int)nsites_u, nedge = (int)nedge_u;
   if (nsites < 3) return GCVT_OK;
   int *order = sc.take<int>(nsites), *sitepos = sc.take<int>(nsites),
       *stars = sc.take<int>((size_t)nsites * kStar), *degree = sc.take<int>(nsites);
@@ -1023,9 +1419,10 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
   if (!order || !sitepos || !stars || !degree || !tcnt || !toff) return GCVT_ERR_ALLOC;
   k_dt_order<<<nblk(ntiles, 128), 128, 0, s>>>(bits, fixed, n, nt0, tileoff, cls, order);
   DCK(cudaGetLastError());
-  k_dt_star<<<nblk(32ll * nsites, 32 * kWarpsPerBlock), 32 * kWarpsPerBlock, 0, s>>>(
-      bits, fixed, n, order, nsites, py, coloff, colpre, tilecnt, sitepos, stars, degree, tcnt,
-      err);
+  const StarOut out{coloff, colpre, sitepos, stars, degree, tcnt, err};
+  const long long warps = nedge + (nsites - nedge + 3ll) / 4;
+  k_dt_star<<<nblk(warps, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, s>>>(
+      bits, fixed, n, order, nsites, nedge, py, tilecnt, out);
   DCK(cudaGetLastError());
   if ((rc = scan_big(tcnt, nsites, toff, sc, s))) return rc;
   if (tris && cap) {
