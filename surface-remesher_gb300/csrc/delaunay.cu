@@ -14,13 +14,18 @@
 // triangulation of the sites, and every site that evaluates a predicate
 // gets the same sign, so all stars agree.
 //
-// Each site's Delaunay star (its neighbours in angular order) is computed
-// by one warp from the sites in a window around it: inverted about the
-// site, the star is the part of the candidates' convex hull facing away from
-// the site, so the candidates are inserted one by one into a sorted cyclic
-// list held in the warp's registers (a candidate inside the current hull
-// never becomes a neighbour later; an inserted one removes the neighbours it
-// covers).  Certificate, exact: a triangle of the star is final when no site
+// Each site's Delaunay star (its neighbours in angular order) is wrapped from
+// the sites in a window around it (quad_stars: four sites of a warp in step,
+// eight lanes each; wwrap: a site by the whole warp, where the first does not
+// settle it).  What does not fit is inserted one by one into the star, a sorted
+// cyclic list in the warp's registers: inverted about the site, the star is the
+// part of the candidates' convex hull facing away from the site (a candidate
+// inside the current hull never becomes a neighbour later; an inserted one
+// removes the neighbours it covers).  What bounds the star kernel is issue
+// slots, and at the end the few sites on the hull whose flat triangles take
+// many searches.  4096^2, 262,144 CVT sites: 1.43 ms with one warp per site
+// inserting every candidate (3,913 instructions a site), 0.29 ms now.
+// Certificate, exact: a triangle of the star is final when no site
 // outside the window lies in its circumcircle, an open angular gap (>= pi)
 // when no site lies strictly inside its cone (then the site is on the
 // sites' convex hull); both are searched through a pyramid of tile
@@ -157,6 +162,17 @@ struct Pyr {
   int off[kLevels], nt[kLevels];
   int top;  // the one-node level
 };
+
+// The sites in tile order (k_dt_order): tile i's (brick order) are order[p ..
+// p + count[i]), p = off[cls[i] ntiles + i].
+struct TileSites {
+  const int *order;
+  const unsigned *off, *count;
+  const uint8_t *cls;
+};
+__device__ __forceinline__ unsigned tile_start(const TileSites &ts, int nt0, int i) {
+  return __ldg(ts.off + (size_t)ts.cls[i] * nt0 * nt0 + i);
+}
 
 // Free sites: bits & ~fixed.
 __device__ __forceinline__ uint64_t free_word(const uint64_t *bits, const uint64_t *fixed,
@@ -551,12 +567,22 @@ struct Probe {
   bool cone;
   int ux, uy, wx, wy;
   long long Nx, Ny, D, hp, hu, hw;
+  float cx, cy, r, slack;  // the disc in floats, and the error of a distance to it
 };
 
 // Can the tile [px0, px1] x [qy0, qy1] hold a site the probe looks for?
 __device__ __forceinline__ bool probe_node(const Probe &pr, int sx, int sy, int px0, int px1,
                                            int qy0, int qy1) {
-  if (!pr.cone) return !clear_of(pr.Nx, pr.Ny, pr.D, px0 - sx, px1 - sx, qy0 - sy, qy1 - sy);
+  if (!pr.cone) {
+    // the tile's distance from the centre against the radius, in floats where
+    // their difference is above the error, else exactly
+    const float dx = fmaxf(fmaxf((float)(px0 - sx) - pr.cx, pr.cx - (float)(px1 - sx)), 0.f);
+    const float dy = fmaxf(fmaxf((float)(qy0 - sy) - pr.cy, pr.cy - (float)(qy1 - sy)), 0.f);
+    const float d = sqrtf(dx * dx + dy * dy) - pr.r;
+    if (d > pr.slack) return false;
+    if (d < -pr.slack) return true;
+    return !clear_of(pr.Nx, pr.Ny, pr.D, px0 - sx, px1 - sx, qy0 - sy, qy1 - sy);
+  }
   // the cross products are linear: their largest value is at a corner
   long long cu = LLONG_MIN, cw = LLONG_MIN;
   for (int c = 0; c < 4; ++c) {
@@ -571,6 +597,11 @@ __device__ __forceinline__ bool probe_node(const Probe &pr, int sx, int sy, int 
 __device__ __forceinline__ bool probe_site(const Probe &pr, int n, int sx, int sy, int qx,
                                            int qy) {
   if (pr.cone) return cross(pr.ux, pr.uy, qx, qy) > 0 || cross(qx, qy, pr.wx, pr.wy) > 0;
+  // decided by the float distance where that is safe (probe_node's bound)
+  const float dx = (float)qx - pr.cx, dy = (float)qy - pr.cy;
+  const float d = sqrtf(dx * dx + dy * dy) - pr.r;
+  if (d > pr.slack) return false;
+  if (d < -pr.slack) return true;
   if ((qx == pr.ux && qy == pr.uy) || (qx == pr.wx && qy == pr.wy)) return false;
   return in_circle(pr.ux, pr.uy, pr.wx, pr.wy, qx, qy, pr.hp, pr.hu, pr.hw,
                    hkey(n, sx + qx, sy + qy));
@@ -593,10 +624,9 @@ enum { kFinal = 0, kInserted = 1, kGaveUp = 2 };
 // pops at least one node and pushes only lower levels, so the search ends;
 // a descent adds at most 3 x 32 nodes per level, so 14 levels stay below
 // kFrontier.
-__device__ int wsearch(WStar &st, const Pyr &py, const uint64_t *bits, const uint64_t *fixed,
-                       int n, int sx, int sy, const Probe &pr, int x0, int x1, int y0, int y1,
-                       unsigned *stk, int sp) {
-  const int lane = lane_id();
+__device__ int wsearch(WStar &st, const Pyr &py, const TileSites &ts, int n, int sx, int sy,
+                       const Probe &pr, int x0, int x1, int y0, int y1, unsigned *stk, int sp) {
+  const int lane = lane_id(), nt0 = py.nt[0];
   while (sp > 0) {
     const int k = min(sp, 32);
     unsigned v = 0;
@@ -621,24 +651,16 @@ __device__ int wsearch(WStar &st, const Pyr &py, const uint64_t *bits, const uin
             if (cx < cn && cy < cn)
               ch[nch++] = ((unsigned)(l - 1) << 28) | ((unsigned)cx << 14) | (unsigned)cy;
           }
-        } else {  // a tile: its sites, column by column, until one is found
-          const int b = qy0 / kBand, sh = qy0 % kBand;
-          bool found = false;
-          for (int x = px0; x <= px1 && !found; ++x) {
-            unsigned w = (unsigned)((free_word(bits, fixed, (size_t)b * n + x) >> sh) & 0xffffull);
-            while (w) {
-              const int i = __ffs(w) - 1;
-              w &= w - 1u;
-              if (probe_site(pr, n, sx, sy, x - sx, qy0 + i - sy)) {
-                found = true;
-                hq = pk(x - sx, qy0 + i - sy);
-                break;
-              }
-            }
-          }
-          if (found) {
+        } else {  // a tile: its sites until one is found
+          const int i = brick_of(tx, ty, nt0);
+          const unsigned p = tile_start(ts, nt0, i);
+          for (unsigned j = 0, cnt = ts.count[i]; j < cnt; ++j) {
+            const int q = __ldg(ts.order + p + j), qx = (q & 0xffff) - sx, qy = pdy(q) - sy;
+            if (!probe_site(pr, n, sx, sy, qx, qy)) continue;
+            hq = pk(qx, qy);
             const long long dx = px0 + kTile / 2 - sx, dy = qy0 + kTile / 2 - sy;
             key = (unsigned)min((dx * dx + dy * dy) >> 4, (long long)(1 << 26)) << 5 | lane;
+            break;
           }
         }
       }
@@ -652,28 +674,20 @@ __device__ int wsearch(WStar &st, const Pyr &py, const uint64_t *bits, const uin
         winsert(st, n, sx, sy, pdx(qL), pdy(qL));
         return kInserted;
       }
-      // the disc: every site of that tile inside the circle, a lane per column
-      const int tx = (int)((vL >> 14) & 0x3fff), ty = (int)(vL & 0x3fff);
-      const int px0 = tx * kTile, qy0 = ty * kTile, b = qy0 / kBand, sh = qy0 % kBand;
-      const int x = px0 + lane;
-      unsigned hit = 0;
-      if (lane < kTile && x < n) {
-        unsigned w = (unsigned)((free_word(bits, fixed, (size_t)b * n + x) >> sh) & 0xffffull);
-        while (w) {
-          const int i = __ffs(w) - 1;
-          w &= w - 1u;
-          if (probe_site(pr, n, sx, sy, x - sx, qy0 + i - sy)) hit |= 1u << i;
+      // the disc: every site of that tile inside the circle, a lane per site
+      const int i = brick_of((int)((vL >> 14) & 0x3fff), (int)(vL & 0x3fff), nt0);
+      const unsigned p = tile_start(ts, nt0, i), cnt = ts.count[i];
+      for (unsigned j0 = 0; j0 < cnt; j0 += 32) {
+        int q = 0;
+        bool hit = false;
+        if (j0 + lane < cnt) {
+          const int e = __ldg(ts.order + p + j0 + lane);
+          q = pk((e & 0xffff) - sx, pdy(e) - sy);
+          hit = probe_site(pr, n, sx, sy, pdx(q), pdy(q));
         }
-      }
-      unsigned pend = __ballot_sync(kFull, hit != 0);
-      while (pend) {
-        const int Lc = __ffs(pend) - 1;
-        pend &= pend - 1u;
-        unsigned hl = __shfl_sync(kFull, hit, Lc);
-        while (hl) {
-          const int i = __ffs(hl) - 1;
-          hl &= hl - 1u;
-          winsert(st, n, sx, sy, px0 + Lc - sx, qy0 + i - sy);
+        for (unsigned pend = __ballot_sync(kFull, hit); pend; pend &= pend - 1u) {
+          const int c = __shfl_sync(kFull, q, __ffs(pend) - 1);
+          winsert(st, n, sx, sy, pdx(c), pdy(c));
         }
       }
       return kInserted;
@@ -697,8 +711,7 @@ __device__ int wsearch(WStar &st, const Pyr &py, const uint64_t *bits, const uin
 // Search for the sites in the circumcircle of (site, u, w) outside the
 // window, starting at the pyramid level where the disc's bounding box spans
 // at most 2 x 2 nodes.
-__device__ int wdisc_search(WStar &st, const Pyr &py, const uint64_t *bits, const uint64_t *fixed,
-                            int n, int sx, int sy, int ux, int uy, int wx, int wy, int x0, int x1,
+__device__ int wdisc_search(WStar &st, const Pyr &py, const TileSites &ts, int n, int sx, int sy, int ux, int uy, int wx, int wy, int x0, int x1,
                             int y0, int y1, unsigned *stk) {
   Probe pr;
   pr.cone = false;
@@ -709,6 +722,14 @@ __device__ int wdisc_search(WStar &st, const Pyr &py, const uint64_t *bits, cons
   pr.Nx = wy * u2 - uy * w2;
   pr.Ny = ux * w2 - wx * u2;
   pr.hp = hkey(n, sx, sy), pr.hu = hkey(n, sx + ux, sy + uy), pr.hw = hkey(n, sx + wx, sy + wy);
+  {
+    const double cx = (double)pr.Nx / (double)pr.D, cy = (double)pr.Ny / (double)pr.D;
+    pr.cx = (float)cx, pr.cy = (float)cy;
+    pr.r = (float)sqrt(cx * cx + cy * cy);
+    // centre, radius, squares, root and difference: a few roundings of at most
+    // |c| + r + n each
+    pr.slack = (2.f * pr.r + 16384.f) * 0x1p-20f;
+  }
   int bx0, bx1, by0, by1;
   disc_box(pr.Nx, pr.Ny, pr.D, sx, sy, n, bx0, bx1, by0, by1);
   int l0 = 0;
@@ -722,20 +743,20 @@ __device__ int wdisc_search(WStar &st, const Pyr &py, const uint64_t *bits, cons
     stk[lane] = ((unsigned)l0 << 28) | ((unsigned)(tx0 + lane % ntx) << 14) |
                 (unsigned)(ty0 + lane / ntx);
   __syncwarp();
-  return wsearch(st, py, bits, fixed, n, sx, sy, pr, x0, x1, y0, y1, stk, ntx * nty);
+  return wsearch(st, py, ts, n, sx, sy, pr, x0, x1, y0, y1, stk, ntx * nty);
 }
 
 // Search for the sites strictly inside the open gap's cone, from the root.
-__device__ int wcone_search(WStar &st, const Pyr &py, const uint64_t *bits, const uint64_t *fixed,
-                            int n, int sx, int sy, int ux, int uy, int wx, int wy, int x0, int x1,
+__device__ int wcone_search(WStar &st, const Pyr &py, const TileSites &ts, int n, int sx, int sy, int ux, int uy, int wx, int wy, int x0, int x1,
                             int y0, int y1, unsigned *stk) {
   Probe pr;
   pr.cone = true;
   pr.ux = ux, pr.uy = uy, pr.wx = wx, pr.wy = wy;
   pr.Nx = pr.Ny = pr.D = pr.hp = pr.hu = pr.hw = 0;
+  pr.cx = pr.cy = pr.r = pr.slack = 0.f;
   if (lane_id() == 0) stk[0] = (unsigned)py.top << 28;
   __syncwarp();
-  return wsearch(st, py, bits, fixed, n, sx, sy, pr, x0, x1, y0, y1, stk, 1);
+  return wsearch(st, py, ts, n, sx, sy, pr, x0, x1, y0, y1, stk, 1);
 }
 
 // Neighbour (k + 1) % m for the lane's entry k (lane l: k = l or l + 32).
@@ -749,27 +770,18 @@ __device__ __forceinline__ int wnext(const WStar &s, int k) {
 // is sized from the local site density (the 3 x 3 tiles around the site:
 // half-width kWindow site spacings, which holds a regular site's neighbours
 // and triangles' circles).  When kWiden or more of its triangles reach past
-// it (as around irregular sites), the window doubles once before any search
-// (inserting a ring costs less than searching); then the certificate
-// settles the triangles exactly, and only a star of fewer than two
-// neighbours doubles the window again (each time inserting just the new
-// ring).  kWindow and kWiden are the fastest of a sweep on converged CVT
-// sites and on uniform random ones at 4096^2 and 8192^2.  Returns false
-// when the star overflowed.
-#ifndef KWIN
-#define KWIN 2.0f
-#endif
-#ifndef KWID
-#define KWID 1
-#endif
-#ifndef KGROW
-#define KGROW 1.7f
-#endif
-constexpr float kWindow = KWIN;
-constexpr int kWiden = KWID;
+// it (as around irregular sites), the window grows once before any search
+// (wrapping again costs less than searching); then the certificate settles the
+// triangles exactly, and only a star of fewer than two neighbours doubles the
+// window again.  More than 64 candidates are inserted ring by ring instead of
+// wrapped.  (kWindow 1.6 to 2.3 and kGrow 1.5 to 2 measure within 5 %, kWiden 3 or
+// never 8 % slower on irregular sites.)  Returns false when the star
+// overflowed.
+constexpr float kWindow = 2.0f, kGrow = 1.7f;
+constexpr int kWiden = 1;
 constexpr int kBoxCols = 96, kBoxBands = 3;  // largest disc box scanned directly
 __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixed, int n, int sx,
-                           int sy, const Pyr &py, const unsigned *tilecnt, unsigned *stk) {
+                           int sy, const Pyr &py, const TileSites &ts, unsigned *stk) {
   st.a = st.b = 0;
   st.m = 0;
   st.overflow = false;
@@ -777,7 +789,7 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
   // (a lane per tile)
   const int ti = tx - 1 + lane % 3, tj = ty - 1 + lane / 3;
   const bool tile = lane < 9 && ti >= 0 && ti < nt0 && tj >= 0 && tj < nt0;
-  const unsigned cnt = __reduce_add_sync(kFull, tile ? tilecnt[brick_of(ti, tj, nt0)] : 0u);
+  const unsigned cnt = __reduce_add_sync(kFull, tile ? ts.count[brick_of(ti, tj, nt0)] : 0u);
   const int tiles = __popc(__ballot_sync(kFull, tile));
   int W = (int)ceilf(kWindow * sqrtf((float)(tiles * kTile * kTile) / (float)max(cnt, 1u)));
   W = min(max(W, 4), 2 * n);
@@ -851,7 +863,7 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
         if (__ballot_sync(kFull, lane < nver && vkey == key)) continue;  // known final
         int res;
         if (open_gap(ux, uy, wx, wy)) {
-          res = wcone_search(st, py, bits, fixed, n, sx, sy, ux, uy, wx, wy, x0, x1, y0, y1, stk);
+          res = wcone_search(st, py, ts, n, sx, sy, ux, uy, wx, wy, x0, x1, y0, y1, stk);
         } else {
           // a small disc: its bounding box outside the window, column by
           // column; a large one through the occupancy pyramid
@@ -865,7 +877,7 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
                                  bx1, by0, by1)
                            ? kInserted
                            : kFinal)
-                    : wdisc_search(st, py, bits, fixed, n, sx, sy, ux, uy, wx, wy, x0, x1, y0, y1,
+                    : wdisc_search(st, py, ts, n, sx, sy, ux, uy, wx, wy, x0, x1, y0, y1,
                                    stk);
         }
         if (res == kGaveUp) {  // the search did not fit: a wider window instead
@@ -885,7 +897,7 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
       }
     } while (changed);
     if (ok) return true;
-    W = first ? min((int)ceilf(KGROW * W), 2 * n) : min(2 * W, 2 * n);
+    W = first ? min((int)ceilf(kGrow * W), 2 * n) : min(2 * W, 2 * n);
     first = false;
   }
 }
@@ -993,9 +1005,6 @@ __device__ __forceinline__ int site_index(const uint64_t *bits, const uint64_t *
   return (int)(coloff[x] + colpre[(size_t)b * n + x] + (unsigned)__popcll(below));
 }
 
-#ifndef MB
-#define MB 6
-#endif
 // What a star kernel writes per site (under its index in delaunayInput's
 // order): its pixel, its star, the star's size and the triangles it writes --
 // the ones it comes first in, in (x, y) order.
@@ -1013,13 +1022,13 @@ __device__ __forceinline__ bool owns_tri(int sx, int sy, int u, int w) {
 
 // One site by the whole warp, any case.
 __device__ __noinline__ void full_site(const uint64_t *bits, const uint64_t *fixed, int n, int pos,
-                                       const Pyr &py, const unsigned *tilecnt, unsigned *stk,
+                                       const Pyr &py, const TileSites &ts, unsigned *stk,
                                        const StarOut &out) {
   const int lane = lane_id();
   const int sx = pdx(pos) & 0xffff, sy = pdy(pos);
   const int xm = site_index(bits, fixed, n, out.coloff, out.colpre, sx, sy);
   WStar st;
-  if (!wsite_star(st, bits, fixed, n, sx, sy, py, tilecnt, stk)) {
+  if (!wsite_star(st, bits, fixed, n, sx, sy, py, ts, stk)) {
     if (lane == 0) {
       atomicOr(out.err, 1);
       out.sitepos[xm] = pos;
@@ -1051,8 +1060,8 @@ __device__ __noinline__ void full_site(const uint64_t *bits, const uint64_t *fix
 // The same gift wrapping as wwrap; the four walks go in step, so a step's
 // instructions serve four sites.  Offsets up to 31 pixels keep every cotangent's
 // numerator and denominator exact in floats.  Returns the groups it leaves to
-// full_site.  4096^2, 262,144 CVT sites: a warp per site by wwrap alone took
-// 1,449 instructions a site.
+// full_site (none of 258,177 interior sites at 4096^2).  A warp per site by wwrap
+// alone took 1,449 instructions a site, this 600.
 constexpr float kQuadWindow = 1.8f;
 constexpr int kQuadCand = 32, kQuadStar = 16;
 struct QuadScratch {
@@ -1061,19 +1070,19 @@ struct QuadScratch {
 };
 
 __device__ __forceinline__ unsigned quad_stars(const uint64_t *bits, const uint64_t *fixed, int n,
-                                               const int *order, int t0, int nsites, const Pyr &py,
-                                               const unsigned *tilecnt, QuadScratch &sc,
+                                               int t0, int nsites, const Pyr &py,
+                                               const TileSites &ts, QuadScratch &sc,
                                                const StarOut &out) {
   const int lane = lane_id(), g = lane >> 3, l = lane & 7;
   const bool on = t0 + g < nsites;
-  const int epos = order[min(t0 + g, nsites - 1)];
+  const int epos = ts.order[min(t0 + g, nsites - 1)];
   const int sx = pdx(epos) & 0xffff, sy = pdy(epos);
   // the window from the 3 x 3 tiles' site counts
   const int tx = sx / kTile, ty = sy / kTile, nt0 = py.nt[0];
   unsigned near = 0;
   for (int k = l; k < 9; k += 8) {
     const int i = tx - 1 + k % 3, j = ty - 1 + k / 3;
-    if (i >= 0 && i < nt0 && j >= 0 && j < nt0) near += tilecnt[brick_of(i, j, nt0)];
+    if (i >= 0 && i < nt0 && j >= 0 && j < nt0) near += ts.count[brick_of(i, j, nt0)];
   }
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) near += __shfl_xor_sync(kFull, near, o);
@@ -1234,10 +1243,9 @@ __device__ __forceinline__ unsigned quad_stars(const uint64_t *bits, const uint6
 
 // The stars of the sites in tile order: a warp per site for the nedge sites
 // of edge tiles (their stars reach far), four sites per warp for the others.
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, MB)
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, 5)
     k_dt_star(const uint64_t *__restrict__ bits, const uint64_t *__restrict__ fixed, int n,
-              const int *__restrict__ order, int nsites, int nedge, Pyr py,
-              const unsigned *__restrict__ tilecnt, StarOut out) {
+              int nsites, int nedge, Pyr py, TileSites ts, StarOut out) {
   __shared__ union {
     unsigned front[kFrontier];
     QuadScratch quad;
@@ -1245,14 +1253,14 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MB)
   const int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   auto &sw = s_warp[threadIdx.x >> 5];
   if (t < nedge) {
-    full_site(bits, fixed, n, order[t], py, tilecnt, sw.front, out);
+    full_site(bits, fixed, n, ts.order[t], py, ts, sw.front, out);
     return;
   }
   const int t0 = nedge + 4 * (t - nedge);
   if (t0 >= nsites) return;  // the whole warp
-  unsigned left = quad_stars(bits, fixed, n, order, t0, nsites, py, tilecnt, sw.quad, out);
+  unsigned left = quad_stars(bits, fixed, n, t0, nsites, py, ts, sw.quad, out);
   for (; left; left &= left - 1u)
-    full_site(bits, fixed, n, order[t0 + __ffs(left) - 1], py, tilecnt, sw.front, out);
+    full_site(bits, fixed, n, ts.order[t0 + __ffs(left) - 1], py, ts, sw.front, out);
 }
 
 __global__ void k_dt_emit(const uint64_t *__restrict__ bits, const uint64_t *__restrict__ fixed,
@@ -1411,6 +1419,7 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
   DCK(cudaMemcpyAsync(&nsites_u, coloff + n, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   DCK(cudaMemcpyAsync(&nedge_u, tileoff + ntiles, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   DCK(cudaStreamSynchronize(s));
+  
   const int nsites = (int)nsites_u, nedge = (int)nedge_u;
   if (nsites < 3) return GCVT_OK;
   int *order = sc.take<int>(nsites), *sitepos = sc.take<int>(nsites),
@@ -1419,10 +1428,11 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
   if (!order || !sitepos || !stars || !degree || !tcnt || !toff) return GCVT_ERR_ALLOC;
   k_dt_order<<<nblk(ntiles, 128), 128, 0, s>>>(bits, fixed, n, nt0, tileoff, cls, order);
   DCK(cudaGetLastError());
+  const TileSites ts{order, tileoff, tilecnt, cls};
   const StarOut out{coloff, colpre, sitepos, stars, degree, tcnt, err};
   const long long warps = nedge + (nsites - nedge + 3ll) / 4;
   k_dt_star<<<nblk(warps, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, s>>>(
-      bits, fixed, n, order, nsites, nedge, py, tilecnt, out);
+      bits, fixed, n, nsites, nedge, py, ts, out);
   DCK(cudaGetLastError());
   if ((rc = scan_big(tcnt, nsites, toff, sc, s))) return rc;
   if (tris && cap) {

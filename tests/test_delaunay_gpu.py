@@ -204,3 +204,21 @@ def test_full_size_workloads_pass_the_checks(gcvt_lib, cuda_device, workload):
     ctx.close()
     info = dorc.check_fast(pts, tris)
     assert info["vertices"] == len(pts) and info["triangles"] == len(tris)
+
+
+@pytest.mark.parametrize("n,step,jitter,count", [(256, 2, 0, 4000), (256, 3, 1, 3001),
+                                                 (256, 7, 2, 1102), (512, 13, 4, 1303),
+                                                 (512, 17, 5, 805), (768, 20, 6, 1206),
+                                                 (1024, 40, 18, 607)])
+def test_star_paths_by_spacing(gcvt_lib, cuda_device, n, step, jitter, count):
+    """The star kernels' dispatch: windows up to and past 31 pixels, up to and
+    past 32 and 64 candidates, a last warp of one to four sites, exact ties at
+    every step (no jitter) and none, long stars on the sites' hull."""
+    rng = np.random.default_rng(step)
+    g = np.arange(step, n - step, step)
+    q = np.stack(np.meshgrid(g, g), -1).reshape(-1, 2)
+    q = np.clip(q + rng.integers(-jitter, jitter + 1, q.shape), 0, n - 1)
+    q = np.unique(q[rng.permutation(len(q))[:count]], axis=0)
+    pts, tris = _triangulate(gcvt_lib, _grid(n, q.tolist()))
+    info = dorc.check(pts, tris)
+    assert info["triangles"] == len(tris) > 0
