@@ -505,7 +505,10 @@ __global__ void k_seg_apply(Mesh m, const int *__restrict__ segs, int base, int 
 // triangulations split such segments).  Crossing segments set err.
 __global__ void k_segments(Mesh m, const int *__restrict__ segs, int S, const int *state,
                            int *queue, int *stack, int *err) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
+  // (usually none: the block looks first, one thread walking the list took 70 us)
+  bool any = false;
+  for (int k = threadIdx.x; k < S; k += blockDim.x) any = any || state[k] != kSegDone;
+  if (!__syncthreads_or(any) || threadIdx.x != 0) return;
   for (int k = 0; k < S; ++k) {
     if (state[k] == kSegDone) continue;
     const int a = segs[2 * k], b = segs[2 * k + 1];
@@ -545,19 +548,21 @@ __global__ void k_emit(Mesh m, int T, const int *__restrict__ off, int *out, int
   }
 }
 
-// Start triangles of the constraint points: a site near each (the first
-// found in growing squares around its pixel in the site index grid), or any
-// triangle.
+// Start triangles of the constraint points: a site near each (the first found
+// in growing squares around its pixel in the site index grid), or any triangle.
+// A warp per point, its lanes side by side along a square (a thread per point
+// took 70 us for 832 points).
 __global__ void k_ins_start(const i64 *__restrict__ X, const i64 *__restrict__ Y, int F, int C,
                             const int *__restrict__ site_at, int n, const int *vt, int *start) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= C) return;
+  const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (j >= C) return;  // the whole warp
   const int px = (int)(X[F + j] >> 15), py = (int)(Y[F + j] >> 15);
   int found = -1;
   for (int r = 0; r < 64 && found < 0; ++r) {
-    // the ring at Chebyshev distance r: its 8 r cells (1 for r = 0), side by side
+    // the ring at Chebyshev distance r: its 8 r cells (1 for r = 0)
     const int cells = r ? 8 * r : 1;
-    for (int k = 0; k < cells; ++k) {
+    for (int k0 = 0; k0 < cells && found < 0; k0 += 32) {
+      const int k = k0 + lane;
       int dx, dy;
       if (r == 0) dx = dy = 0;
       else if (k < 2 * r) dx = -r + k, dy = -r;          // top, left to right
@@ -565,15 +570,13 @@ __global__ void k_ins_start(const i64 *__restrict__ X, const i64 *__restrict__ Y
       else if (k < 6 * r) dx = r - (k - 4 * r), dy = r;   // bottom, right to left
       else dx = -r, dy = r - (k - 6 * r);                 // left, bottom to top
       const int x = px + dx, y = py + dy;
-      if (x < 0 || y < 0 || x >= n || y >= n) continue;
-      const int v = site_at[(size_t)y * n + x];
-      if (v >= 0) {
-        found = v;
-        break;
-      }
+      const int v = k < cells && x >= 0 && y >= 0 && x < n && y < n
+                        ? site_at[(size_t)y * n + x] : -1;
+      const unsigned hit = __ballot_sync(0xffffffffu, v >= 0);
+      if (hit) found = __shfl_sync(0xffffffffu, v, __ffs(hit) - 1);
     }
   }
-  start[j] = found >= 0 ? vt[found] : 0;
+  if (lane == 0) start[j] = found >= 0 ? vt[found] : 0;
 }
 
 __global__ void k_site_at(const i64 *__restrict__ X, const i64 *__restrict__ Y, int F, int n,
@@ -727,7 +730,7 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
     if (!site_at || !pend || !pend2 || !start || !start2 || !done || !loc) return GCVT_ERR_ALLOC;
     CCK(cudaMemsetAsync(site_at, 0xff, (size_t)n * n * sizeof(int), s));
     k_site_at<<<nblk(F, 256), 256, 0, s>>>(X, Y, (int)F, n, site_at);
-    k_ins_start<<<nblk(C, 128), 128, 0, s>>>(X, Y, (int)F, C, site_at, n, vt, start);
+    k_ins_start<<<nblk(32ll * C, 128), 128, 0, s>>>(X, Y, (int)F, C, site_at, n, vt, start);
     k_iota<<<nblk(C, 256), 256, 0, s>>>(pend, C, (int)F);  // point indices F + j
     CCK(cudaGetLastError());
     // one round: the points of list a (count *na) locate, claim and insert;
@@ -804,7 +807,7 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
         if (h[5] == 0) break;
       }
     }
-    k_segments<<<1, 32, 0, s>>>(m, segs, S, state, queue, stack, ctr);
+    k_segments<<<1, 1024, 0, s>>>(m, segs, S, state, queue, stack, ctr);
     CCK(cudaGetLastError());
     if ((rc = pull())) return rc;
   }
@@ -814,13 +817,12 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
     return (h[0] & (kErrCoord | kErrDuplicate | kErrSegment)) ? GCVT_ERR_INPUT : GCVT_ERR_CUDA;
   }
   // 6. output in a fixed order
-  int *cnt = sc.take<int>((size_t)V + 1), *off = sc.take<int>((size_t)V + 1),
-      *cur = sc.take<int>((size_t)V + 1);
-  if (!cnt || !off || !cur) return GCVT_ERR_ALLOC;
+  int *cnt = sc.take<int>((size_t)V + 1), *off = sc.take<int>((size_t)V + 1);
+  if (!cnt || !off) return GCVT_ERR_ALLOC;
   CCK(cudaMemsetAsync(cnt, 0, ((size_t)V + 1) * sizeof(int), s));
   k_emit_count<<<nblk(T, 256), 256, 0, s>>>(m, T, cnt);
   CCK(cudaGetLastError());
-  CCK(launch_scan(cnt, (int)V, off, cur, s));
+  if ((rc = scan_counts(cnt, (int)V, off, nullptr, sc, s))) return rc;
   if (out && cap) {
     k_emit<<<nblk(T, 256), 256, 0, s>>>(m, T, off, out, (int)cap, ctr);
     CCK(cudaGetLastError());

@@ -1288,52 +1288,6 @@ __global__ void k_dt_emit(const uint64_t *__restrict__ bits, const uint64_t *__r
   }
 }
 
-// Exclusive scan of large count arrays: blocks of 4096 counts scanned in
-// shared memory, the block totals by launch_scan, then the block offsets
-// added (offset[n] = total).
-constexpr int kScanBlock = 4096;
-__global__ void __launch_bounds__(1024) k_scan_local(const unsigned *__restrict__ count, int n,
-                                                     unsigned *offset, unsigned *total) {
-  __shared__ unsigned v[kScanBlock];
-  __shared__ unsigned wsum[32];
-  const int base = blockIdx.x * kScanBlock, t = threadIdx.x;
-  for (int k = t; k < kScanBlock; k += 1024) v[k] = base + k < n ? count[base + k] : 0u;
-  __syncthreads();
-  const unsigned a0 = v[4 * t], a1 = v[4 * t + 1], a2 = v[4 * t + 2], a3 = v[4 * t + 3];
-  const unsigned sum = a0 + a1 + a2 + a3;
-  unsigned inc = sum;  // inclusive scan over the warp
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
-    if ((t & 31) >= o) inc += y;
-  }
-  if ((t & 31) == 31) wsum[t >> 5] = inc;
-  __syncthreads();
-  if (t < 32) {
-    unsigned w = wsum[t], wi = w;
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned y = __shfl_up_sync(0xffffffffu, wi, o);
-      if (t >= o) wi += y;
-    }
-    wsum[t] = wi - w;
-    if (t == 31) total[blockIdx.x] = wi;
-  }
-  __syncthreads();
-  const unsigned ex = wsum[t >> 5] + inc - sum;
-  v[4 * t] = ex;
-  v[4 * t + 1] = ex + a0;
-  v[4 * t + 2] = ex + a0 + a1;
-  v[4 * t + 3] = ex + a0 + a1 + a2;
-  __syncthreads();
-  for (int k = t; k < kScanBlock; k += 1024)
-    if (base + k < n) offset[base + k] = v[k];
-}
-
-__global__ void k_scan_add(unsigned *offset, int n, const unsigned *__restrict__ boff, int nblock) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) offset[i] += boff[i / kScanBlock];
-  if (i == 0) offset[n] = boff[nblock];
-}
-
 inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 #define DCK(call)                                 \
@@ -1341,19 +1295,9 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
     if ((call) != cudaSuccess) return GCVT_ERR_CUDA; \
   } while (0)
 
-// Exclusive scan of count[0..n) into offset[0..n] (n >= 1).
-int scan_big(const unsigned *count, int n, unsigned *offset, Scratch &sc, cudaStream_t s) {
-  const int nblock = (n + kScanBlock - 1) / kScanBlock;
-  unsigned *tot = sc.take<unsigned>(nblock), *boff = sc.take<unsigned>(nblock + 1),
-           *cur = sc.take<unsigned>(nblock);
-  if (!tot || !boff || !cur) return GCVT_ERR_ALLOC;
-  k_scan_local<<<nblock, 1024, 0, s>>>(count, n, offset, tot);
-  DCK(cudaGetLastError());
-  DCK(launch_scan(reinterpret_cast<const int *>(tot), nblock, reinterpret_cast<int *>(boff),
-                  reinterpret_cast<int *>(cur), s));
-  k_scan_add<<<nblk(n, 256), 256, 0, s>>>(offset, n, boff, nblock);
-  DCK(cudaGetLastError());
-  return GCVT_OK;
+int scan(const unsigned *count, int n, unsigned *offset, Scratch &sc, cudaStream_t s) {
+  return scan_counts(reinterpret_cast<const int *>(count), n, reinterpret_cast<int *>(offset),
+                     nullptr, sc, s);
 }
 
 }  // namespace
@@ -1375,7 +1319,7 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
   const size_t nb = (size_t)(n / kBand) * n;
   const int nt0 = n / kTile, ntiles = nt0 * nt0;
   unsigned *colpre = sc.take<unsigned>(nb), *colcnt = sc.take<unsigned>(n),
-           *coloff = sc.take<unsigned>(n + 1), *cur = sc.take<unsigned>(n),
+           *coloff = sc.take<unsigned>(n + 1),
            *tilecnt = sc.take<unsigned>(ntiles), *cnt2 = sc.take<unsigned>(2 * (size_t)ntiles),
            *tileoff = sc.take<unsigned>(2 * (size_t)ntiles + 1);
   uint8_t *cls = sc.take<uint8_t>(ntiles);
@@ -1394,7 +1338,7 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
   }
   uint8_t *occ = sc.take<uint8_t>(occ_bytes);
   py.occ = occ;
-  if (!colpre || !colcnt || !coloff || !cur || !tilecnt || !cnt2 || !tileoff || !cls || !err ||
+  if (!colpre || !colcnt || !coloff || !tilecnt || !cnt2 || !tileoff || !cls || !err ||
       !occ)
     return GCVT_ERR_ALLOC;
   DCK(cudaMemsetAsync(err, 0, sizeof(int), s));
@@ -1409,12 +1353,11 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
         occ + py.off[l - 1], py.nt[l - 1], occ + py.off[l], py.nt[l]);
     DCK(cudaGetLastError());
   }
-  DCK(launch_scan(reinterpret_cast<const int *>(colcnt), n, reinterpret_cast<int *>(coloff),
-                  reinterpret_cast<int *>(cur), s));
+  int rc = scan(colcnt, n, coloff, sc, s);
+  if (rc) return rc;
   k_dt_class<<<nblk(ntiles, 256), 256, 0, s>>>(occ, nt0, tilecnt, cnt2, cls);
   DCK(cudaGetLastError());
-  int rc = scan_big(cnt2, 2 * ntiles, tileoff, sc, s);
-  if (rc) return rc;
+  if ((rc = scan(cnt2, 2 * ntiles, tileoff, sc, s))) return rc;
   unsigned nsites_u = 0, nedge_u = 0;
   DCK(cudaMemcpyAsync(&nsites_u, coloff + n, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   DCK(cudaMemcpyAsync(&nedge_u, tileoff + ntiles, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
@@ -1434,7 +1377,7 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
   k_dt_star<<<nblk(warps, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, s>>>(
       bits, fixed, n, nsites, nedge, py, ts, out);
   DCK(cudaGetLastError());
-  if ((rc = scan_big(tcnt, nsites, toff, sc, s))) return rc;
+  if ((rc = scan(tcnt, nsites, toff, sc, s))) return rc;
   if (tris && cap) {
     k_dt_emit<<<nblk(nsites, 128), 128, 0, s>>>(bits, fixed, n, sitepos, nsites, coloff, colpre,
                                                 stars, degree, toff, tris, cap);

@@ -216,9 +216,9 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
                 double lower, int *out, unsigned cap, unsigned *ntris, int *detail,
                 cudaStream_t s);
 
-// Exclusive scan of n counts into offset[0..n] (offset[n] = total) and a copy
-// in cursor[0..n-1]; one block, n <= 2^26.
-cudaError_t launch_scan(const int *count, int n, int *offset, int *cursor, cudaStream_t s);
+// Exclusive scan of n <= 2^26 counts into offset[0..n] (offset[n] = total) and,
+// unless null, a copy in cursor[0..n-1]; a GCVT status.
+int scan_counts(const int *count, int n, int *offset, int *cursor, Scratch &sc, cudaStream_t s);
 cudaError_t cells_configure();
 size_t list_blocks(int n);
 size_t cell_groups(int n);

@@ -19,7 +19,10 @@
 // A point scans its grid cell's list (sorted, so the first face that passes
 // ends the scan) and the global list, keeps the smallest face index whose
 // test passes -- the reference's first hit -- and a point with a non-finite
-// coordinate tests every face in order.  The test is the
+// coordinate tests every face in order.  What bounds it is the FP64 pipe: a float
+// pre-test (tri_test.cuh) finds the next candidate, the FP64 test runs once the
+// warp's lanes have one and divides by known reciprocals (69,000 points and 134,000
+// triangles on 93,000 faces: 200 -> 41 us).  The test is the
 // reference's arithmetic with every product, sum and quotient rounded once
 // (the reference's host build has no fused multiply-add), so the weights are
 // bit-identical.  Why the enlarged box cannot drop a match for a local face:
@@ -37,6 +40,7 @@
 // by a prefix maximum; with none (no earlier located point, where the
 // reference reads an uninitialised location) it gets NaN.
 #include "gcvt_internal.cuh"
+#include "tri_test.cuh"
 #include "../../include/gcvt_gb300.h"
 
 #include <climits>
@@ -58,6 +62,7 @@ constexpr int kLocal = 1, kGlobal = 2;
 // (the same expressions, so the same values).
 struct LiftFace {
   double x1, y1, v0x, v0y, v1x, v1y, d00, d01, d11, denom;
+  double rden;  // 1 / denom, rounded
 };
 
 struct __align__(32) Box {
@@ -87,17 +92,9 @@ __device__ __forceinline__ bool face_test(const LiftFace &f, double px, double p
   return !(c < 0 || a < 0 || b < 0);
 }
 
-// RN(num / denom) < 0 for denom > 0, decided without dividing: num < 0 and
-// the quotient too large to round to -0 (|q| >= 2^-1074 when denom <= 1;
-// otherwise |num| >= denom 2^-1000 keeps it far from underflow).  False
-// means "divide to know".
-__device__ __forceinline__ bool quot_negative(double num, double denom) {
-  return num < 0 && (denom <= 1.0 || -num >= __dmul_rn(denom, 0x1p-1000));
-}
-
 // face_test for a face with a finite denominator > 0 and a finite point: the
 // same results, but a weight whose numerator already shows it negative
-// rejects the face before the two divisions (FP64 issue is scarce on GB300).
+// rejects the face before the two divisions.
 __device__ __forceinline__ bool face_test_local(const LiftFace &f, double px, double py,
                                                 double &c, double &a, double &b) {
   const double v2x = __dsub_rn(px, f.x1), v2y = __dsub_rn(py, f.y1);
@@ -107,10 +104,10 @@ __device__ __forceinline__ bool face_test_local(const LiftFace &f, double px, do
   if (quot_negative(na, f.denom)) return false;
   const double nb = __dsub_rn(__dmul_rn(f.d00, d21), __dmul_rn(f.d01, d20));
   if (quot_negative(nb, f.denom)) return false;
-  a = __ddiv_rn(na, f.denom);
-  b = __ddiv_rn(nb, f.denom);
+  a = div_by(na, f.denom, f.rden);
+  b = div_by(nb, f.denom, f.rden);
   c = __dsub_rn(__dsub_rn(1.0, a), b);
-  return !(c < 0 || a < 0 || b < 0);
+  return !(below_zero(c) || below_zero(a) || below_zero(b));
 }
 
 // Order-preserving 64-bit keys of doubles for atomic min / max.
@@ -159,6 +156,7 @@ __device__ __forceinline__ bool classify_face(const double *__restrict__ uv, int
   f.d01 = dot_rn(f.v0x, f.v0y, f.v1x, f.v1y);
   f.d11 = dot_rn(f.v1x, f.v1y, f.v1x, f.v1y);
   f.denom = __dsub_rn(__dmul_rn(f.d00, f.d11), __dmul_rn(f.d01, f.d01));
+  f.rden = __drcp_rn(f.denom);
   faces[i] = f;
   if (f.denom == 0) {
     kind[i] = 0;
@@ -168,7 +166,7 @@ __device__ __forceinline__ bool classify_face(const double *__restrict__ uv, int
   const double ymin = fmin(y1, fmin(y2, y3)), ymax = fmax(y1, fmax(y2, y3));
   const bool finite = isfinite(x1) && isfinite(y1) && isfinite(x2) && isfinite(y2) &&
                       isfinite(x3) && isfinite(y3) && isfinite(f.denom);
-  const double cond = f.d00 * f.d11 / f.denom;
+  const double cond = f.d00 * f.d11 * f.rden;
   if (!finite || !(f.denom > 0) || !(cond <= kMaxCond)) {
     kind[i] = kGlobal;
     ebox[i] = Box{-INFINITY, -INFINITY, INFINITY, INFINITY};
@@ -222,14 +220,15 @@ __global__ void __launch_bounds__(256) k_lift_faces(const double *__restrict__ u
   }
 }
 
-// Local faces: count their cells, or move them to the global list when their
-// box covers more than kMaxCellsPerFace cells; global faces join the list.
-__global__ void k_lift_count(const Box *__restrict__ ebox, unsigned char *kind, int nt, Grid g,
-                             int *cell_count, int *glist, int *gcount,
-                             unsigned long long *entries) {
+// Local faces: count their cells and make their float pre-test (in cells of the
+// grid), or move them to the global list when their box covers more than
+// kMaxCellsPerFace cells; global faces join the list.
+__global__ void k_lift_count(const LiftFace *__restrict__ faces, const Box *__restrict__ ebox,
+                             unsigned char *kind, int nt, Grid g, TriPre *pre, int *cell_count,
+                             int *glist, int *gcount, unsigned long long *entries) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nt) return;
-  int k = kind[i];
+  int k = i < nt ? kind[i] : 0;
+  unsigned cells = 0;
   if (k == kLocal) {
     const Box e = ebox[i];
     const int cx0 = cell_x(g, e.x), cx1 = cell_x(g, e.z);
@@ -237,13 +236,21 @@ __global__ void k_lift_count(const Box *__restrict__ ebox, unsigned char *kind, 
     if ((long long)(cx1 - cx0 + 1) * (cy1 - cy0 + 1) > kMaxCellsPerFace) {
       kind[i] = k = kGlobal;
     } else {
-      atomicAdd(entries, (unsigned long long)((cx1 - cx0 + 1) * (cy1 - cy0 + 1)));
+      cells = (unsigned)((cx1 - cx0 + 1) * (cy1 - cy0 + 1));
       for (int cy = cy0; cy <= cy1; ++cy)
         for (int cx = cx0; cx <= cx1; ++cx) atomicAdd(&cell_count[cy * g.gx + cx], 1);
-      return;
+      const LiftFace &f = faces[i];
+      TriPre p{0, 0, 0, 0, 0, 0, 0, 0};
+      // (cells square within a factor of 4: the pre-test's bound)
+      if (g.ix <= 4.0 * g.iy && g.iy <= 4.0 * g.ix)
+        p = make_pre(f.x1 - g.x0, f.y1 - g.y0, f.v0x, f.v0y, f.v1x, f.v1y, g.ix, g.iy,
+                     (float)max(g.gx, g.gy), f.d00 * f.d11 * f.rden);
+      pre[i] = p;
     }
   }
   if (k == kGlobal) glist[atomicAdd(gcount, 1)] = i;
+  cells = __reduce_add_sync(0xffffffffu, cells);  // (at most 32 kMaxCellsPerFace)
+  if ((threadIdx.x & 31) == 0 && cells) atomicAdd(entries, (unsigned long long)cells);
 }
 
 __global__ void k_lift_scatter(const Box *__restrict__ ebox,
@@ -258,26 +265,44 @@ __global__ void k_lift_scatter(const Box *__restrict__ ebox,
     for (int cx = cx0; cx <= cx1; ++cx) list[atomicAdd(&cursor[cy * g.gx + cx], 1)] = i;
 }
 
-// Each cell's list in ascending face order (one thread per cell; lists are
-// a few faces long).
+// Each cell's list in ascending face order: eight lanes per cell rank lists of up
+// to 32 faces; one lane sorts a longer one in place.
 __global__ void k_lift_sort(const int *__restrict__ offset, int ncell, int *list) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncell) return;
-  const int l0 = offset[c], l1 = offset[c + 1];
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, c = t >> 3, l = t & 7;
+  const int l0 = c < ncell ? offset[c] : 0, len = c < ncell ? offset[c + 1] - l0 : 0;
+  const bool small = len <= 32;
+  int x[4], rank[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) x[j] = small && l + 8 * j < len ? list[l0 + l + 8 * j] : INT_MAX;
+  for (int k = 0; small && k < len; ++k) {
+    const int v = list[l0 + k];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) rank[j] += v < x[j];
+  }
+  __syncwarp();
+  if (small) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (l + 8 * j < len) list[l0 + rank[j]] = x[j];
+    return;
+  }
+  if (l) return;
+  const int l1 = l0 + len;
   for (int k = l0 + 1; k < l1; ++k) {
-    const int x = list[k];
+    const int v = list[k];
     int j = k - 1;
-    while (j >= l0 && list[j] > x) {
+    while (j >= l0 && list[j] > v) {
       list[j + 1] = list[j];
       --j;
     }
-    list[j + 1] = x;
+    list[j + 1] = v;
   }
 }
 
 struct Locator {
   const LiftFace *faces;
   const Box *ebox;
+  const TriPre *pre;
   const int *offset, *list, *glist;
   int ngl, nt;
   Grid g;
@@ -296,14 +321,21 @@ struct Locator {
     }
     int best = INT_MAX;
     if (g.gx > 0 && px >= g.x0 && px <= g.x1 && py >= g.y0 && py <= g.y1) {
-      // the cell's faces in ascending order: the first that passes is the answer
-      const int cell = cell_y(g, py) * g.gx + cell_x(g, px);
+      // the cell's faces in ascending order: the first that passes is the
+      // answer.  The next face the float pre-test leaves, then the FP64 test
+      // (the warp's lanes come to it together).
+      const double ux = __dmul_rn(__dsub_rn(px, g.x0), g.ix),
+                   uy = __dmul_rn(__dsub_rn(py, g.y0), g.iy);
+      const float fx = (float)ux, fy = (float)uy;
+      const int cell = min(g.gy - 1, (int)uy) * g.gx + min(g.gx - 1, (int)ux);
       const int l1 = offset[cell + 1];
-      for (int k = offset[cell]; k < l1; ++k) {
-        const int i = list[k];
-        const Box e = ebox[i];
-        if (px < e.x || px > e.z || py < e.y || py > e.w) continue;
-        if (face_test_local(faces[i], px, py, wc, wa, wb)) {
+      for (int k = offset[cell]; k < l1;) {
+        int i = -1;
+        while (k < l1 && i < 0) {
+          i = list[k++];
+          if (pre_outside(pre[i], fx, fy)) i = -1;
+        }
+        if (i >= 0 && face_test_local(faces[i], px, py, wc, wa, wb)) {
           best = i, c = wc, a = wa, b = wb;
           break;
         }
@@ -363,9 +395,10 @@ __global__ void k_lift_locate(Locator L, const double *__restrict__ xyz, int nv,
       return;
     }
     // CGAL::centroid of three Point_2: ((p + q + r) / 3) per coordinate
-    const double cx = __ddiv_rn(__dadd_rn(__dadd_rn(pts[2 * p0], pts[2 * p1]), pts[2 * p2]), 3.0);
-    const double cy =
-        __ddiv_rn(__dadd_rn(__dadd_rn(pts[2 * p0 + 1], pts[2 * p1 + 1]), pts[2 * p2 + 1]), 3.0);
+    const double cx = div_by(__dadd_rn(__dadd_rn(pts[2 * p0], pts[2 * p1]), pts[2 * p2]), 3.0,
+                             1.0 / 3.0);
+    const double cy = div_by(__dadd_rn(__dadd_rn(pts[2 * p0 + 1], pts[2 * p1 + 1]),
+                                       pts[2 * p2 + 1]), 3.0, 1.0 / 3.0);
     double c, a, b;
     keep[t] = L.find(cx, cy, c, a, b) >= 0 ? 1 : 0;
   }
@@ -531,11 +564,13 @@ int lift_device(Scratch &sc, const double *uv, const double *xyz, int nv, const 
                 int nc, double *out_xyz, int *out_face, unsigned char *keep) {
   LiftFace *faces;
   Box *ebox;
+  TriPre *pre;
   unsigned char *kind;
   int *glist, *scal, *cnt, *off, *cur, *list, *face, *blast;
   long long *keys;
   TAKE(faces, LiftFace, nt);
   TAKE(ebox, Box, nt);
+  TAKE(pre, TriPre, nt);
   TAKE(kind, unsigned char, nt);
   TAKE(glist, int, nt);
   TAKE(keys, long long, 4);
@@ -573,7 +608,8 @@ int lift_device(Scratch &sc, const double *uv, const double *xyz, int nv, const 
   TAKE(cur, int, ncell);
   LCK(cudaMemset(cnt, 0, (size_t)ncell * sizeof(int)));
   if (nt > 0) {
-    k_lift_count<<<blocks(nt, 256), 256>>>(ebox, kind, nt, g, cnt, glist, gcount, entries);
+    k_lift_count<<<blocks(nt, 256), 256>>>(faces, ebox, kind, nt, g, pre, cnt, glist, gcount,
+                                           entries);
     LCK(cudaGetLastError());
   }
   unsigned long long nentries = 0;
@@ -581,18 +617,18 @@ int lift_device(Scratch &sc, const double *uv, const double *xyz, int nv, const 
   if (nentries > (unsigned long long)INT_MAX) return GCVT_ERR_SIZE;
   int total = 0;
   if (ncell > 0) {
-    LCK(launch_scan(cnt, ncell, off, cur, 0));
+    if (const int rc = scan_counts(cnt, ncell, off, cur, sc, 0)) return rc;
     LCK(cudaMemcpy(&total, off + ncell, sizeof(int), cudaMemcpyDeviceToHost));
   }
   TAKE(list, int, total);
   if (nt > 0 && ncell > 0) {
     k_lift_scatter<<<blocks(nt, 256), 256>>>(ebox, kind, nt, g, cur, list);
     LCK(cudaGetLastError());
-    k_lift_sort<<<blocks(ncell, 256), 256>>>(off, ncell, list);
+    k_lift_sort<<<blocks(8ll * ncell, 256), 256>>>(off, ncell, list);
     LCK(cudaGetLastError());
   }
   LCK(cudaMemcpy(hs, scal, sizeof hs, cudaMemcpyDeviceToHost));
-  Locator L{faces, ebox, off, list, glist, hs[2], nt, g};
+  Locator L{faces, ebox, pre, off, list, glist, hs[2], nt, g};
   face = out_face;
   if (!face) TAKE(face, int, np);
   const long long nq = (long long)np + nc;
@@ -634,7 +670,7 @@ int weights_device(Scratch &sc, const double *uv, const double *xyz, int nv, con
     k_face_areas<<<blocks(nt, 256), 256>>>(uv, xyz, nv, tri, nt, area, cnt, err);
     LCK(cudaGetLastError());
   }
-  LCK(launch_scan(cnt, nv, off, cur, 0));
+  if (const int rc = scan_counts(cnt, nv, off, cur, sc, 0)) return rc;
   if (nt > 0) {
     k_vertex_faces<<<blocks(nt, 256), 256>>>(tri, nt, nv, cur, inc);
     LCK(cudaGetLastError());

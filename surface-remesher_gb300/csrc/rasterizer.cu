@@ -23,10 +23,16 @@
 // test can pass: a false hit at distance D needs D < 2^-48 kappa (D + L), L
 // the triangle's size (u = 2^-53), so under 4e-9 L at kappa <= 2^20 and a
 // factor 8 inside the margin up to kappa = 2^40.  A denominator of exactly 0
-// never passes.  Tile lists are sorted, so a pixel stops at its first hit,
-// and a weight whose numerator is already negative rejects a triangle before
-// the FP64 divisions.
+// never passes.
+//
+// What bounds it is the FP64 pipe (84 % busy when each lane ran its own tests and
+// divisions as it came to them: a warp instruction costs the same whatever its
+// active lanes).  So a warp first looks for every pixel's next candidate with
+// the float pre-test (tri_test.cuh), from the tile's triangles sorted and staged
+// in shared memory, and then runs the FP64 test for all its pixels at once,
+// dividing by known reciprocals.  2048^2, 93,000 triangles: 1.27 -> 0.24 ms.
 #include "gcvt_internal.cuh"
+#include "tri_test.cuh"
 #include "../../include/gcvt_gb300.h"
 
 #include <cstdio>
@@ -42,6 +48,7 @@ constexpr int kMaxTilesPerTri = 4096;
 // (discretization.cu:32-55) precomputed as the kernel would compute them.
 struct TriData {
   double x1, y1, v0x, v0y, v1x, v1y, d00, d01, d11, denom;
+  double rden;     // 1 / denom, rounded
   int p1, p2, p3;  // vertex indices (for the weights)
   int global;      // 1: on the global list
 };
@@ -58,6 +65,7 @@ __device__ __forceinline__ void tri_terms(double x1, double y1, double x2, doubl
   t.d01 = __fma_rn(t.v0x, t.v1x, __dmul_rn(t.v0y, t.v1y));
   t.d11 = __fma_rn(t.v1x, t.v1x, __dmul_rn(t.v1y, t.v1y));
   t.denom = __fma_rn(t.d00, t.d11, -__dmul_rn(t.d01, t.d01));
+  t.rden = __drcp_rn(t.denom);
 }
 
 // barycentric_coordinate with the reference's operation order and the fused
@@ -77,15 +85,9 @@ __device__ __forceinline__ bool bary_inside(const TriData &t, double x0, double 
   return !(w1 < 0 || w2 < 0 || w3 < 0);
 }
 
-// RN(num / denom) < 0 for denom > 0, decided without dividing (false: divide
-// to know): num < 0 and the quotient too large to round to -0.
-__device__ __forceinline__ bool quot_negative(double num, double denom) {
-  return num < 0 && (denom <= 1.0 || -num >= __dmul_rn(denom, 0x1p-1000));
-}
-
 // bary_inside for a finite triangle with denom > 0: same results, but a
 // weight whose numerator already shows it negative rejects the triangle
-// before the divisions (FP64 issue is scarce on GB300).
+// before the divisions.
 __device__ __forceinline__ bool bary_inside_local(const TriData &t, double x0, double y0,
                                                   double &w1, double &w2, double &w3) {
   const double v2x = __dsub_rn(x0, t.x1), v2y = __dsub_rn(y0, t.y1);
@@ -95,63 +97,12 @@ __device__ __forceinline__ bool bary_inside_local(const TriData &t, double x0, d
   if (quot_negative(na, t.denom)) return false;
   const double nb = __fma_rn(t.d00, d21, -__dmul_rn(t.d01, d20));
   if (quot_negative(nb, t.denom)) return false;
-  const double a = __ddiv_rn(na, t.denom);
-  const double b = __ddiv_rn(nb, t.denom);
+  const double a = div_by(na, t.denom, t.rden);
+  const double b = div_by(nb, t.denom, t.rden);
   w2 = a;
   w3 = b;
   w1 = __dsub_rn(__dsub_rn(1.0, a), b);
-  return !(w1 < 0 || w2 < 0 || w3 < 0);
-}
-
-// An FP32 pre-test that rejects a pixel clearly outside a triangle before the
-// FP64 test, for triangles with conditioning <= 2^20 (sgn = 0: no pre-test).
-// In pixel units, r = q - P1, edge functions E0 = v0 x r, E1 = (v1 - v0) x
-// (r - v0), E2 = (-v1) x (r - v1), all >= 0 inside a counter-clockwise
-// triangle (sgn folds the orientation).  With M the largest coordinate
-// magnitude, L the longest edge and |r| <= 3 L inside the triangle's box, the
-// FP32 error of each E_k is below L (2^-22 M + 2^-19 L) (rounded coordinates
-// and edge vectors, three roundings in the products); so sgn E_k < -t with
-// t = L (2^-21 M + 2^-16 L) means E_k < -2^-17 L^2 exactly: the pixel lies
-// more than 2^-17 L outside edge k, far beyond the FP64 test's own error
-// there (2^-48 kappa (|r| + L) <= 2^-26 L), so the FP64 weight of the
-// opposite vertex is negative and the reference's test fails too.
-struct TriPre {
-  float p1x, p1y, v0x, v0y, v1x, v1y, t, sgn;
-};
-
-__device__ __forceinline__ bool pre_outside(const TriPre &q, int tx, int ty) {
-  if (q.sgn == 0.f) return false;
-  const float rx = (float)tx - q.p1x, ry = (float)ty - q.p1y;
-  const float e0 = q.v0x * ry - q.v0y * rx;
-  const float e1 = (q.v1x - q.v0x) * (ry - q.v0y) - (q.v1y - q.v0y) * (rx - q.v0x);
-  const float e2 = q.v1y * (rx - q.v1x) - q.v1x * (ry - q.v1y);
-  return q.sgn * e0 < -q.t || q.sgn * e1 < -q.t || q.sgn * e2 < -q.t;
-}
-
-__device__ __forceinline__ TriPre make_pre(const TriData &t, double inv_scale, int n,
-                                           double cond) {
-  TriPre q{0, 0, 0, 0, 0, 0, 0, 0};
-  if (!(cond <= 1048576.0)) return q;
-  const double cr = t.v0x * t.v1y - t.v0y * t.v1x;
-  if (!(cr != 0.0) || !isfinite(cr)) return q;
-  const double p1x = t.x1 * inv_scale, p1y = t.y1 * inv_scale;
-  const double ax = t.v0x * inv_scale, ay = t.v0y * inv_scale;
-  const double bx = t.v1x * inv_scale, by = t.v1y * inv_scale;
-  const double l0 = sqrt(ax * ax + ay * ay), l2 = sqrt(bx * bx + by * by);
-  const double l1 = sqrt((bx - ax) * (bx - ax) + (by - ay) * (by - ay));
-  const double L = fmax(l0, fmax(l1, l2));
-  const double M = fmax((double)n, fmax(fabs(p1x), fabs(p1y)) + 4.0 * L);
-  if (!(L >= 1e-9 && M <= 1e9)) return q;  // keep FP32 away from over/underflow
-  const double thr = L * (0x1p-21 * M + 0x1p-16 * L) * 1.0625;
-  q.p1x = (float)p1x;
-  q.p1y = (float)p1y;
-  q.v0x = (float)ax;
-  q.v0y = (float)ay;
-  q.v1x = (float)bx;
-  q.v1y = (float)by;
-  q.t = (float)thr;
-  q.sgn = cr > 0 ? 1.f : -1.f;
-  return q;
+  return !(below_zero(w1) || below_zero(w2) || below_zero(w3));
 }
 
 __global__ void k_tri_setup(const double *__restrict__ pts, const int *__restrict__ tri, int T,
@@ -188,7 +139,7 @@ __global__ void k_tri_setup(const double *__restrict__ pts, const int *__restric
     tbox[i] = make_int4(1, 1, 0, 0);
     return;
   }
-  const double cond = t.d00 * t.d11 / t.denom;
+  const double cond = t.d00 * t.d11 * t.rden;
   if (!finite || !(t.denom > 0) || !(cond <= kMaxCond)) {
     t.global = 1;
     td[i] = t;
@@ -224,42 +175,81 @@ __global__ void k_tri_setup(const double *__restrict__ pts, const int *__restric
     return;
   }
   td[i] = t;
-  tpre[i] = make_pre(t, inv_scale, n, cond);
+  tpre[i] = make_pre(t.x1, t.y1, t.v0x, t.v0y, t.v1x, t.v1y, inv_scale, inv_scale, (float)n, cond);
   const int nt = n / kTile;
   for (int ty = y0 / kTile; ty <= y1p / kTile; ++ty)
     for (int tx = x0 / kTile; tx <= x1p / kTile; ++tx) atomicAdd(&tile_count[ty * nt + tx], 1);
 }
 
-// Exclusive scan of the tile counts, one block (tiles <= 1024 * 64).
-__global__ void __launch_bounds__(1024) k_tile_scan(const int *count, int ntiles, int *offset,
-                                                   int *cursor) {
-  __shared__ int part[1024];
-  const int t = threadIdx.x;
-  const int per = (ntiles + 1023) / 1024;
-  const int b0 = min(ntiles, t * per), b1 = min(ntiles, b0 + per);
+// Exclusive scan of n counts: blocks of 4096, each adding up the block sums
+// before it (one block needs no sums).  One block striding over everything took
+// 24 us for 16,384 counts and 53 us for 69,000; this takes about 3 + 3 us.
+constexpr int kScanChunk = 4096;
+
+__global__ void __launch_bounds__(256) k_scan_sums(const int *__restrict__ count, int n, int *sums) {
+  __shared__ int ws[8];
   int s = 0;
-  for (int i = b0; i < b1; ++i) s += count[i];
-  part[t] = s;
+  for (int i = blockIdx.x * kScanChunk + threadIdx.x, e = min(n, ((int)blockIdx.x + 1) * kScanChunk);
+       i < e; i += 256)
+    s += count[i];
+  s = __reduce_add_sync(0xffffffffu, s);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
   __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    int add = t >= o ? part[t - o] : 0;
-    __syncthreads();
-    part[t] += add;
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) s += ws[k];
+    sums[blockIdx.x] = s;
   }
-  int run = part[t] - s;
-  for (int i = b0; i < b1; ++i) {
-    offset[i] = run;
-    cursor[i] = run;
-    run += count[i];
-  }
-  if (t == 1023) offset[ntiles] = part[1023];
 }
 
-cudaError_t launch_scan(const int *count, int n, int *offset, int *cursor, cudaStream_t s) {
-  if (n < 0 || n > 1024 * 65536) return cudaErrorInvalidValue;
-  k_tile_scan<<<1, 1024, 0, s>>>(count, n, offset, cursor);
-  return cudaGetLastError();
+__global__ void __launch_bounds__(256) k_scan_write(const int *__restrict__ count, int n,
+                                                   const int *__restrict__ sums, int *offset,
+                                                   int *cursor) {
+  __shared__ int v[kScanChunk];
+  __shared__ int ws[8], wp[8];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5, base = blockIdx.x * kScanChunk;
+  int pre = 0;
+  for (int k = t; k < (int)blockIdx.x; k += 256) pre += sums[k];
+  pre = __reduce_add_sync(0xffffffffu, pre);
+  for (int k = t; k < kScanChunk; k += 256) v[k] = base + k < n ? count[base + k] : 0;
+  __syncthreads();
+  // 16 consecutive counts per thread
+  int x[16], s = 0;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    x[k] = s;
+    s += v[16 * t + k];
+  }
+  int inc = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += y;
+  }
+  if (lane == 31) ws[w] = inc;
+  if (lane == 0) wp[w] = pre;
+  __syncthreads();
+  int add = inc - s;
+  for (int k = 0; k < 8; ++k) add += wp[k] + (k < w ? ws[k] : 0);
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[16 * t + k] = add + x[k];
+  if (base + kScanChunk >= n && t == 255) offset[n] = add + s;
+  __syncthreads();
+  for (int k = t; k < kScanChunk && base + k < n; k += 256) {
+    offset[base + k] = v[k];
+    if (cursor) cursor[base + k] = v[k];
+  }
+}
+
+int scan_counts(const int *count, int n, int *offset, int *cursor, Scratch &sc, cudaStream_t s) {
+  if (n < 0 || n > 1024 * 65536) return GCVT_ERR_SIZE;
+  const int blocks = n > kScanChunk ? (n + kScanChunk - 1) / kScanChunk : 1;
+  int *sums = nullptr;
+  if (blocks > 1) {
+    if (!(sums = sc.take<int>(blocks))) return GCVT_ERR_ALLOC;
+    k_scan_sums<<<blocks, 256, 0, s>>>(count, n, sums);
+  }
+  k_scan_write<<<blocks, 256, 0, s>>>(count, n, sums, offset, cursor);
+  return cudaGetLastError() == cudaSuccess ? GCVT_OK : GCVT_ERR_CUDA;
 }
 
 __global__ void k_tri_scatter(const TriData *__restrict__ td, const int4 *__restrict__ tbox, int T,
@@ -276,24 +266,12 @@ __global__ void k_tri_scatter(const TriData *__restrict__ td, const int4 *__rest
     }
 }
 
-// Each tile's list in ascending triangle order (one thread per tile).
-__global__ void k_tile_sort(const int *__restrict__ offset, int ntiles, int *list) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ntiles) return;
-  const int l0 = offset[c], l1 = offset[c + 1];
-  for (int k = l0 + 1; k < l1; ++k) {
-    const int x = list[k];
-    int j = k - 1;
-    while (j >= l0 && list[j] > x) {
-      list[j + 1] = list[j];
-      --j;
-    }
-    list[j + 1] = x;
-  }
-}
+// One block per tile, one thread per pixel.  The tile's triangles are sorted and
+// staged in shared memory, so a pixel's first hit in list order is its answer; a
+// tile of more than kTileList triangles keeps every pixel's smallest hit of the
+// unsorted list instead.
+constexpr int kTileList = 256;
 
-// One block per tile, one thread per pixel; the tile's list is sorted, so the
-// first triangle that passes is the answer.
 __global__ void __launch_bounds__(kTile *kTile) k_raster(const TriData *__restrict__ td,
                                                         const TriPre *__restrict__ tpre,
                                                         const int4 *__restrict__ tbox,
@@ -303,26 +281,76 @@ __global__ void __launch_bounds__(kTile *kTile) k_raster(const TriData *__restri
                                                         const int *__restrict__ gcount,
                                                         const double *__restrict__ weight,
                                                         double scale, int n, float *density) {
-  const int nt = n / kTile;
+  __shared__ int s_raw[kTileList], s_id[kTileList];
+  __shared__ TriPre s_pre[kTileList];
+  __shared__ ushort4 s_box[kTileList];  // n <= 16384
+  constexpr unsigned kFull = 0xffffffffu;
+  const int nt = n / kTile, tid = threadIdx.x;
   const int tile = blockIdx.x;
-  const int tx = (tile % nt) * kTile + threadIdx.x % kTile;
-  const int ty = (tile / nt) * kTile + threadIdx.x / kTile;
+  const int tx = (tile % nt) * kTile + tid % kTile;
+  const int ty = (tile / nt) * kTile + tid / kTile;
   const double x = tx * scale, y = ty * scale;
-  const int l0 = offset[tile], l1 = offset[tile + 1];
+  const float fx = (float)tx, fy = (float)ty;
+  const int l0 = offset[tile], len = offset[tile + 1] - l0;
   int best = 0x7fffffff;
   double bw1 = 0, bw2 = 0, bw3 = 0;
-  for (int k = l0; k < l1; ++k) {
-    const int i = list[k];
-    const int4 b = __ldg(&tbox[i]);
-    if (tx < b.x || tx > b.z || ty < b.y || ty > b.w) continue;
-    if (pre_outside(tpre[i], tx, ty)) continue;
-    double w1, w2, w3;
-    if (bary_inside_local(td[i], x, y, w1, w2, w3)) {
-      best = i;
-      bw1 = w1;
-      bw2 = w2;
-      bw3 = w3;
-      break;
+  if (len <= kTileList) {
+    for (int e = tid; e < len; e += kTile * kTile) s_raw[e] = list[l0 + e];
+    __syncthreads();
+    for (int e = tid; e < len; e += kTile * kTile) {
+      const int i = s_raw[e];
+      int rank = 0;
+      for (int k = 0; k < len; ++k) rank += s_raw[k] < i;
+      s_id[rank] = i;
+      s_pre[rank] = tpre[i];
+      const int4 b = tbox[i];
+      s_box[rank] = make_ushort4((unsigned short)b.x, (unsigned short)b.y, (unsigned short)b.z,
+                                 (unsigned short)b.w);
+    }
+    __syncthreads();
+    // every pixel's next candidate, then the FP64 test for all of them; a pixel
+    // whose candidate fails (within a hair of an edge) looks on
+    int from = 0;
+    bool open = len > 0;
+    while (__any_sync(kFull, open)) {
+      int cand = -1;
+      for (int k = (int)__reduce_min_sync(kFull, open ? (unsigned)from : (unsigned)len); k < len;
+           ++k) {
+        if (open && cand < 0 && k >= from) {
+          const ushort4 b = s_box[k];
+          if (tx >= b.x && tx <= b.z && ty >= b.y && ty <= b.w && !pre_outside(s_pre[k], fx, fy))
+            cand = k;
+        }
+        if (!__any_sync(kFull, open && cand < 0)) break;
+      }
+      if (cand < 0) open = false;
+      if (open) {
+        from = cand + 1;
+        const int i = s_id[cand];
+        double w1, w2, w3;
+        if (bary_inside_local(td[i], x, y, w1, w2, w3)) {
+          best = i;
+          bw1 = w1;
+          bw2 = w2;
+          bw3 = w3;
+          open = false;
+        }
+      }
+    }
+  } else {
+    for (int k = l0; k < l0 + len; ++k) {
+      const int i = list[k];
+      if (i >= best) continue;
+      const int4 b = __ldg(&tbox[i]);
+      if (tx < b.x || tx > b.z || ty < b.y || ty > b.w) continue;
+      if (pre_outside(tpre[i], fx, fy)) continue;
+      double w1, w2, w3;
+      if (bary_inside_local(td[i], x, y, w1, w2, w3)) {
+        best = i;
+        bw1 = w1;
+        bw2 = w2;
+        bw3 = w3;
+      }
     }
   }
   const int ng = *gcount;
@@ -341,7 +369,7 @@ __global__ void __launch_bounds__(kTile *kTile) k_raster(const TriData *__restri
   }
   float res = 0.0f;
   if (best != 0x7fffffff) {
-    const TriData t = td[best];
+    const TriData &t = td[best];
     // w1*weight[p1] + w2*weight[p2] + w3*weight[p3] as nvcc contracts it
     const double v = __fma_rn(bw3, weight[t.p3],
                               __fma_rn(bw1, weight[t.p1], __dmul_rn(bw2, weight[t.p2])));
@@ -400,16 +428,14 @@ extern "C" int gcvt_rasterize(const double *points, const double *weight, int nu
                                                 d_cnt, d_glist, d_scal, num_point, d_scal + 1);
     RCK(cudaGetLastError());
   }
-  k_tile_scan<<<1, 1024>>>(d_cnt, ntiles, d_off, d_cur);
-  RCK(cudaGetLastError());
+  const int src = scan_counts(d_cnt, ntiles, d_off, d_cur, sc, nullptr);
+  if (src) return src;
   int total = 0;
   RCK(cudaMemcpy(&total, d_off + ntiles, sizeof(int), cudaMemcpyDeviceToHost));
   int *d_list = sc.take<int>(total);
   if (!d_list) return GCVT_ERR_ALLOC;
   if (num_tri > 0) {
     k_tri_scatter<<<(num_tri + 255) / 256, 256>>>(d_td, d_box, num_tri, n, d_cur, d_list);
-    RCK(cudaGetLastError());
-    k_tile_sort<<<(ntiles + 255) / 256, 256>>>(d_off, ntiles, d_list);
     RCK(cudaGetLastError());
   }
   k_raster<<<ntiles, kTile * kTile>>>(d_td, d_pre, d_box, d_off, d_list, d_glist, d_scal, Wt, scale, n,

@@ -109,3 +109,22 @@ def test_raster_slivers_across_conditioning(gcvt_lib, cuda_device):
     got = gcvt_lib.rasterize(pts, w, tris, 1.0, n)
     want = orc.rasterize(pts, w, tris, 1.0, n)
     assert _same_f32(got, want)
+
+
+@pytest.mark.parametrize("n,count,scale", [(64, 255, 1.0), (64, 256, 1.0), (64, 257, 1.0),
+                                           (64, 900, 1.0), (1024, 40, 1.0), (1040, 40, 1.0),
+                                           (64, 60, 1e-70), (64, 60, 1e60), (16, 5, 1.0)])
+def test_raster_lists_and_divisions(gcvt_lib, cuda_device, n, count, scale):
+    """The tile list at and past the shared-memory limit (256), the tile count at
+    and past one scan block (64^2 and 65^2 tiles), overlapping triangles that share
+    edges with pixel samples, and coordinates whose denominators leave the range
+    of the reciprocal division -- bit for bit."""
+    rng = np.random.default_rng(count)
+    c = rng.integers(2, min(n, 60) - 2, (count, 1, 2)).astype(np.float64)
+    q = c + rng.integers(-9, 10, (count, 3, 2)) * rng.choice([0.25, 1.0], (count, 1, 1))
+    pts = np.ascontiguousarray(q.reshape(-1, 2) * scale)
+    w = rng.uniform(0.5, 2.0, len(pts))
+    T = np.arange(3 * count, dtype=np.int32).reshape(-1, 3)
+    got = gcvt_lib.rasterize(pts, w, T, scale, n)
+    want = orc.rasterize(pts, w, T, scale, n)
+    assert np.array_equal(got.view(np.int32), want.view(np.int32))
