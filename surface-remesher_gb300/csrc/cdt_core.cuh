@@ -101,14 +101,17 @@ enum { kLocIn = 0, kLocEdge = 1, kLocOut = 2, kLocVertex = 3, kLocFail = 4 };
 // kLocIn (p inside *ot), kLocEdge (p inside the edge opposite vertex *oi of
 // *ot), kLocOut (p outside the hull beyond the boundary edge opposite *oi of
 // *ot), kLocVertex (p coincides with vertex *oi of *ot), kLocFail (no answer
-// within max_steps).  The edges are tried from a rotating start, which keeps
-// the walk from cycling.
+// within max_steps).  The edges are tried from a hashed start at every
+// step: in a mesh that is not Delaunay yet a walk with a fixed or rotating order can
+// cycle (with the rotation, about one call in 2,500 on a 2048^2 mesh boundary ran
+// out of steps).
 CDT_HD int locate(const Mesh &m, int p, int t, int max_steps, int *ot, int *oi) {
   for (int s = 0; s < max_steps; ++s) {
     const int *v = m.tri + 3 * t;
     int zeros = 0, zi = -1, next = -1;
+    const int first = (int)((prio((unsigned)s) >> 8) % 3u);
     for (int q = 0; q < 3; ++q) {
-      const int i = (q + s) % 3;
+      const int i = (q + first) % 3;
       const int o = orient(m, v[nx3(i)], v[pv3(i)], p);
       if (o < 0) {
         next = i;
