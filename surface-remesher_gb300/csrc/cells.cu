@@ -898,18 +898,6 @@ __device__ __forceinline__ void take_snapshot(DevState *st) {
   st->snap_cover = st->cover;
 }
 
-// Clear the bitmap and counts the next iteration writes (nobody reads them
-// in this one); this thread's grid-stride share.
-__device__ __forceinline__ void clear_ahead(const LevelBufs &a, int cur, size_t t0,
-                                            size_t gthreads) {
-  const size_t nwords = (size_t)(a.n / kBand) * a.n;
-  uint64_t *zro = bits_at(a, cur == 0 ? 2 : cur - 1);
-  unsigned *czro = counts_at(a, cur == 0 ? 2 : cur - 1);
-  for (size_t i = t0; i < nwords; i += gthreads) zro[i] = 0ull;
-  const size_t nlb = (nwords + kListWords - 1) / kListWords;
-  for (size_t i = t0; i < nlb; i += gthreads) czro[i] = 0u;
-}
-
 // Features of listed site idx at (sx, sy) with cell sums cs, for the learned
 // step, all in units of the mean cell radius (DevState::feat_scale): its
 // pending Lloyd displacement (the centroid of its cell minus the site, not
@@ -1485,7 +1473,7 @@ __device__ __forceinline__ void few_groups_tail(const LevelBufs &a, const IterVi
 // alone).  1024^2 / 4096 sites, list included: 43 -> 19 us an iteration (38.8 -> 25 us
 // for the cell kernel with each warp folding its own site).  MODE 0, 4 and 5 as
 // in k_cell (MODE 4 also writes the learned step's features, MODE 5 judges a
-// jump and does not clear ahead).
+// jump).
 template <int MODE>
 __global__ void __launch_bounds__(32 * kBlockSites, 4) k_cell_warp(LevelBufs a) {
   __shared__ WarpScratch scratch[kBlockSites];
@@ -1495,9 +1483,6 @@ __global__ void __launch_bounds__(32 * kBlockSites, 4) k_cell_warp(LevelBufs a) 
   if (st->snap_stopped) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const IterView v = iter_view(a);
-  if (MODE != 5 || !st->gate_active)
-    clear_ahead(a, v.cur, (size_t)blockIdx.x * blockDim.x + threadIdx.x,
-                (size_t)gridDim.x * blockDim.x);
   if (v.ngroups == 0) {  // no sites: the schedule still advances
     if (blockIdx.x == 0 && threadIdx.x == 0) pass_done<MODE>(st, 0.0, 0u, 0u, a.n, v.cur);
     return;
@@ -1584,10 +1569,9 @@ __global__ void __launch_bounds__(32 * kBlockSites, 4) k_cell_warp(LevelBufs a) 
 // MODE 2: the learned step's features of the sites (LevelBufs::feat);
 //         nothing moves.
 // MODE 4: MODE 0 and the features, for a jump from these sites.
-// MODE 5: MODE 0 for the jumped sites without clearing ahead (the bitmap
-//         after next holds the plain step's sites until the gate decides),
-//         and the gate's decision (DevState::gate_accept); when no jump was
-//         proposed (DevState::gate_active 0), exactly MODE 0.
+// MODE 5: MODE 0 for the jumped sites, and the gate's decision
+//         (DevState::gate_accept); when no jump was proposed
+//         (DevState::gate_active 0), exactly MODE 0.
 template <int MODE>
 __global__ void __launch_bounds__(32, 32) k_cell(LevelBufs a, double *out4) {
   DevState *st = a.st;
@@ -1595,10 +1579,6 @@ __global__ void __launch_bounds__(32, 32) k_cell(LevelBufs a, double *out4) {
   if (kMoves && st->snap_stopped) return;
   const int lane = threadIdx.x;
   const IterView v = iter_view(a);
-  // MODE 5 keeps the bitmap after next (the plain step's sites) while a jump
-  // is judged; without a jump it is a plain iteration
-  if (MODE == 0 || MODE == 4 || (MODE == 5 && !st->gate_active))
-    clear_ahead(a, v.cur, (size_t)blockIdx.x * 32 + lane, (size_t)gridDim.x * 32);
   if (MODE != 1 && v.ngroups == 0) {  // no sites: the schedule still advances
     if (blockIdx.x == 0 && lane == 0) pass_done<MODE>(st, 0.0, 0u, 0u, a.n, v.cur);
     return;
@@ -1614,24 +1594,27 @@ __global__ void __launch_bounds__(32, 32) k_cell(LevelBufs a, double *out4) {
 // one sequence (group offsets per chart from k_list_batch, gofs[c] .. gofs[c+1]),
 // handed out by one ticket; each chart keeps its own state, reduction and
 // schedule, so a chart's iteration is the same as in k_cell.  MODE 0, 4, 5 as
-// in k_cell.
+// in k_cell.  A warp keeps its chart's buffer pointers in shared memory (read
+// through the descriptor in global memory, they cost a reload after every store).
 template <int MODE>
 __global__ void __launch_bounds__(32, 32) k_cell_batch(const LevelBufs *__restrict__ charts,
                                                        int nchart,
                                                        const unsigned *__restrict__ gofs,
                                                        unsigned *ticket) {
+  __shared__ LevelBufs a;
+  static_assert(sizeof(LevelBufs) % 8 == 0, "copied in 8-byte words");
   const int lane = threadIdx.x;
-  const size_t t0 = (size_t)blockIdx.x * 32 + lane, gthreads = (size_t)gridDim.x * 32;
-  for (int c = 0; c < nchart; ++c) {
-    const LevelBufs &a = charts[c];
-    DevState *st = a.st;
-    if (st->snap_stopped) continue;
-    const int cur = st->snap_cur;
-    if (MODE != 5 || !st->gate_active) clear_ahead(a, cur, t0, gthreads);
-    if (st->snap_count == 0 && blockIdx.x == 0 && lane == 0)
-      pass_done<MODE>(st, 0.0, 0u, 0u, a.n, cur);
+  if (blockIdx.x == 0) {  // running charts without sites: the schedule still advances
+    for (int c = lane; c < nchart; c += 32) {
+      DevState *st = charts[c].st;
+      if (!st->snap_stopped && st->snap_count == 0)
+        pass_done<MODE>(st, 0.0, 0u, 0u, charts[c].n, st->snap_cur);
+    }
   }
   const unsigned total = gofs[nchart];
+  int chart = -1;
+  IterView v{};
+  unsigned g0 = 0;
   for (bool first = true;; first = false) {
     const unsigned g = next_item(ticket, first, lane);
     if (g >= total) break;
@@ -1641,17 +1624,28 @@ __global__ void __launch_bounds__(32, 32) k_cell_batch(const LevelBufs *__restri
       if (__ldg(gofs + mid) <= g) lo = mid;
       else hi = mid - 1;
     }
-    const LevelBufs &a = charts[lo];
-    const IterView v = iter_view(a);
-    cell_group<MODE>(a, v, g - __ldg(gofs + lo), lane, nullptr);
+    if (lo != chart) {
+      chart = lo;
+      __syncwarp();
+      for (int k = lane; k < (int)(sizeof(LevelBufs) / 8); k += 32)
+        reinterpret_cast<unsigned long long *>(&a)[k] =
+            __ldg(reinterpret_cast<const unsigned long long *>(charts + chart) + k);
+      __syncwarp();
+      v = iter_view(a);
+      g0 = __ldg(gofs + chart);
+    }
+    cell_group<MODE>(a, v, g - g0, lane, nullptr);
   }
 }
 
 // Block `blk` of a chart's site list: the sites of bitmap words
 // [blk kListWords, (blk+1) kListWords) in bitmap order (word by word, bits in
 // row order) with the fixed flag, at the offset the per-block counts give.
-// The chart's last block records the list length.
-__device__ void list_block(const LevelBufs &a, unsigned blk, unsigned nblk) {
+// The chart's last block records the list length.  clear: also zero the block's
+// words (and count) of the bitmap the next iteration writes -- nobody reads them in
+// this one -- unless a jump is being judged (the bitmap then holds the plain step's
+// sites until the gate decides).
+__device__ void list_block(const LevelBufs &a, unsigned blk, unsigned nblk, bool clear) {
   constexpr int kPer = kListWords / 256;
   __shared__ unsigned wsum[8];
   __shared__ unsigned base_s;
@@ -1681,6 +1675,13 @@ __device__ void list_block(const LevelBufs &a, unsigned blk, unsigned nblk) {
   const unsigned base = base_s;
   // this thread's words and their sites
   const size_t w0 = (size_t)blk * kListWords + (size_t)tid * kPer;
+  if (clear && !st->gate_active) {
+    const int z = cur == 0 ? 2 : cur - 1;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      if (w0 + k < nwords) bits_at(a, z)[w0 + k] = 0ull;
+    if (tid == 0) counts_at(a, z)[blk] = 0u;
+  }
   uint64_t w[kPer];
   unsigned cnt = 0;
 #pragma unroll
@@ -1736,47 +1737,84 @@ __global__ void __launch_bounds__(256) k_list(LevelBufs a, int respect_stop) {
     return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) st->ticket = 0u;
-  list_block(a, blockIdx.x, gridDim.x);
+  list_block(a, blockIdx.x, gridDim.x, respect_stop != 0);
   if (!respect_stop && blockIdx.x == 0 && threadIdx.x == 0) st->snap_stopped = 0;
 }
 
-// The site lists of many charts: chart c owns blocks lofs[c] .. lofs[c+1].
-// The block that finishes last lays out the group offsets of the charts that
-// run (gofs) for k_cell_batch and rearms its ticket.
+// The site lists of many charts: chart c owns blocks lofs[c] .. lofs[c+1].  The
+// blocks after those lay out the group offsets of the charts that run (gofs) for
+// k_cell_batch and rearm its ticket, from the charts' block counts alone: a warp per
+// chart adds them up, the last of these blocks scans the charts.  (With every list
+// block counting itself finished and one thread walking the charts at the end, 64
+// charts took 42 us; this way 20.)
+constexpr int kChartsPerBlock = 8;
+
 __global__ void __launch_bounds__(256) k_list_batch(const LevelBufs *__restrict__ charts,
                                                     int nchart,
                                                     const unsigned *__restrict__ lofs,
                                                     unsigned *gofs, unsigned *done,
                                                     unsigned *ticket) {
-  __shared__ bool is_last;
-  int lo = 0, hi = nchart - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (__ldg(lofs + mid) <= blockIdx.x) lo = mid;
-    else hi = mid - 1;
+  const unsigned nlist = __ldg(lofs + nchart);
+  if (blockIdx.x < nlist) {
+    int lo = 0, hi = nchart - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (__ldg(lofs + mid) <= blockIdx.x) lo = mid;
+      else hi = mid - 1;
+    }
+    const LevelBufs &a = charts[lo];
+    const unsigned blk = blockIdx.x - __ldg(lofs + lo);
+    if (!a.st->stopped) list_block(a, blk, __ldg(lofs + lo + 1) - __ldg(lofs + lo), true);
+    else if (blk == 0 && threadIdx.x == 0) a.st->snap_stopped = 1;
+    return;
   }
-  const LevelBufs &a = charts[lo];
-  const unsigned blk = blockIdx.x - __ldg(lofs + lo);
-  if (!a.st->stopped) list_block(a, blk, __ldg(lofs + lo + 1) - __ldg(lofs + lo));
-  else if (blk == 0 && threadIdx.x == 0) a.st->snap_stopped = 1;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    is_last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __shared__ bool is_last;
+  __shared__ unsigned ws[8];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int mc = (int)(blockIdx.x - nlist) * kChartsPerBlock + wib;
+  if (mc < nchart) {
+    const LevelBufs &a = charts[mc];
+    unsigned sum = 0;
+    if (!a.st->stopped) {
+      const unsigned *counts = counts_at(a, a.st->cur);
+      for (unsigned k = lane; k < __ldg(lofs + mc + 1) - __ldg(lofs + mc); k += 32) sum += counts[k];
+    }
+    sum = min(__reduce_add_sync(0xffffffffu, sum), (unsigned)a.n * (unsigned)a.n);
+    if (lane == 0) gofs[mc] = (sum + 31) / 32;
   }
   __syncthreads();
-  if (!is_last || threadIdx.x != 0) return;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    is_last = atomicAdd(done, 1u) == gridDim.x - nlist - 1;
+  }
+  __syncthreads();
+  if (!is_last) return;
   __threadfence();
   unsigned acc = 0;
-  for (int c = 0; c < nchart; ++c) {
-    gofs[c] = acc;
-    const DevState *st = charts[c].st;
-    const int cnt = *((volatile const int *)&st->snap_count);
-    if (!*((volatile const int *)&st->snap_stopped)) acc += (unsigned)(cnt + 31) / 32;
+  for (int c0 = 0; c0 < nchart; c0 += 256) {  // 256 charts at a time
+    const int c = c0 + threadIdx.x;
+    const unsigned mine = c < nchart ? __ldcg(gofs + c) : 0u;
+    unsigned incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    if (lane == 31) ws[wib] = incl;
+    __syncthreads();
+    unsigned before = acc;
+    for (int k = 0; k < 8; ++k) {
+      if (k < wib) before += ws[k];
+      acc += ws[k];
+    }
+    if (c < nchart) gofs[c] = before + incl - mine;
+    __syncthreads();
   }
-  gofs[nchart] = acc;
-  *ticket = 0u;
-  *done = 0u;
-  __threadfence();
+  if (threadIdx.x == 0) {
+    gofs[nchart] = acc;
+    *ticket = 0u;
+    *done = 0u;
+  }
 }
 
 // Per-block site counts of the current bitmap (for the first k_list of a
@@ -1952,7 +1990,8 @@ cudaError_t cells_configure() {
 cudaError_t launch_list_batch(const LevelBufs *charts, int nchart, const unsigned *lofs,
                               unsigned nblocks, unsigned *gofs, unsigned *done, unsigned *ticket,
                               cudaStream_t s) {
-  k_list_batch<<<nblocks, 256, 0, s>>>(charts, nchart, lofs, gofs, done, ticket);
+  const unsigned extra = (unsigned)((nchart + kChartsPerBlock - 1) / kChartsPerBlock);
+  k_list_batch<<<nblocks + extra, 256, 0, s>>>(charts, nchart, lofs, gofs, done, ticket);
   return cudaGetLastError();
 }
 

@@ -80,7 +80,7 @@ struct LevelBufs {
   int n;
   uint64_t *bits[3];       // site bitmaps [band][column], bit i = row 64*band+i;
                            // the Lloyd kernel reads bits[cur], writes
-                           // bits[cur+1] and clears bits[cur+2] (mod 3)
+                           // bits[cur+1]; k_list clears bits[cur+2] (mod 3)
   int16_t *prev;           // [band][column]: nearest site row above the band
   int16_t *next;           // [band][column]: nearest site row below the band
   const float *density;    // n*n

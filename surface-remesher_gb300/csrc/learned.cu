@@ -161,22 +161,37 @@ __global__ void __launch_bounds__(256) k_apply(const LevelBufs *__restrict__ des
   }
 }
 
-// One thread per chart: save the state after the plain iteration, make the
+// A state copied by a warp (one thread took 5 us over its kilobyte).
+__device__ __forceinline__ void copy_state(DevState *dst, const DevState *src) {
+  static_assert(sizeof(DevState) % 8 == 0, "copied in 8-byte words");
+  for (int k = threadIdx.x & 31; k < (int)(sizeof(DevState) / 8); k += 32)
+    reinterpret_cast<unsigned long long *>(dst)[k] =
+        reinterpret_cast<const unsigned long long *>(src)[k];
+  __syncwarp();
+}
+
+// One warp per chart: save the state after the plain iteration, make the
 // jumped sites current.  Every density pixel was within snap_cover of its
 // owner in S, which moved by at most the largest jump, so snap_cover plus
 // that jump bounds L's covering distance.  A chart whose plain iteration
 // stopped its level proposes nothing.
 __global__ void k_gate_switch(const LevelBufs *__restrict__ descs, int nchart) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nchart) return;
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= nchart) return;  // the whole warp
+  const bool lead = (threadIdx.x & 31) == 0;
   const LevelBufs &a = descs[c];
   DevState *st = a.st;
-  if (st->snap_stopped || st->stopped || st->omega < 2.0f) {  // as k_apply decided
-    st->gate_active = 0;
-    st->gate_jump2 = 0;
+  const bool none = st->snap_stopped || st->stopped || st->omega < 2.0f;  // as k_apply decided
+  __syncwarp();
+  if (none) {
+    if (lead) {
+      st->gate_active = 0;
+      st->gate_jump2 = 0;
+    }
     return;
   }
-  *a.gsave = *st;
+  copy_state(a.gsave, st);
+  if (!lead) return;
   const unsigned j2 = st->gate_jump2;
   int j = (int)sqrtf((float)j2);
   while (j * j < (int)j2) ++j;
@@ -206,18 +221,21 @@ __global__ void __launch_bounds__(256) k_gate_clear(const LevelBufs *__restrict_
   for (size_t i = t0; i < nlb; i += gs) cz[i] = 0u;
 }
 
-// One thread per chart: count the jump; a rejected jump restores the state
+// One warp per chart: count the jump; a rejected jump restores the state
 // saved after the plain iteration (the bitmap written by the jumped sites'
 // iteration is cleared ahead by the next iteration, as every third one is).
 __global__ void k_gate_commit(const LevelBufs *__restrict__ descs, int nchart) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nchart) return;
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= nchart) return;  // the whole warp
   const LevelBufs &a = descs[c];
   DevState *st = a.st;
-  if (!st->gate_active) return;
+  const int active = st->gate_active;
   const int acc = st->gate_accept, tried = st->gate_tried + 1, kept = st->gate_kept + acc;
   const double e0 = st->gate_e0, e1 = st->gate_e1;
-  if (!acc) *st = *a.gsave;
+  __syncwarp();
+  if (!active) return;
+  if (!acc) copy_state(st, a.gsave);
+  if (threadIdx.x & 31) return;
   st->gate_tried = tried;
   st->gate_kept = kept;
   st->gate_e0 = e0;
@@ -632,14 +650,14 @@ cudaError_t launch_apply(const LevelBufs *descs, int nchart, cudaStream_t s) {
 }
 
 cudaError_t launch_gate_switch(const LevelBufs *descs, int nchart, cudaStream_t s) {
-  k_gate_switch<<<(nchart + 127) / 128, 128, 0, s>>>(descs, nchart);
+  k_gate_switch<<<(32 * nchart + 127) / 128, 128, 0, s>>>(descs, nchart);
   return cudaGetLastError();
 }
 
 cudaError_t launch_gate_resolve(const LevelBufs *descs, int nchart, cudaStream_t s) {
   const int per = max(8, 1216 / max(nchart, 1));
   k_gate_clear<<<dim3((unsigned)per, (unsigned)nchart), 256, 0, s>>>(descs);
-  k_gate_commit<<<(nchart + 127) / 128, 128, 0, s>>>(descs, nchart);
+  k_gate_commit<<<(32 * nchart + 127) / 128, 128, 0, s>>>(descs, nchart);
   return cudaGetLastError();
 }
 
