@@ -41,6 +41,8 @@ struct gcvt_ctx {
   uint32_t *grid = nullptr;   // staging: labels and site dumps
   uint64_t *bits[3] = {};
   int16_t *prev = nullptr, *next = nullptr;
+  unsigned *occ = nullptr;         // labelling: see LevelBufs
+  unsigned *open_tiles = nullptr;
   DevState *st = nullptr;
   DevState *st_host = nullptr;  // pinned mirror
   uint32_t *list = nullptr;     // site list, n_max^2 entries
@@ -111,6 +113,8 @@ LevelBufs level_bufs(gcvt_ctx *c, int n, int level) {
   for (int k = 0; k < 3; ++k) b.bits[k] = c->bits[k];
   b.prev = c->prev;
   b.next = c->next;
+  b.occ = c->occ;
+  b.open_tiles = c->open_tiles;
   b.density = c->density[level];
   b.support = c->support[level];
   b.sup_range = c->sup_range[level];
@@ -220,8 +224,7 @@ int ensure_cover(gcvt_ctx *c, int n, int level) {
   int rc = pull_state(c);
   if (rc) return rc;
   const LevelBufs b = level_bufs(c, n, level);
-  CK(launch_summary(b, 0, c->stream));
-  CK(launch_rows(b, 0, c->stream));
+  CK(launch_label(b, c->stream));
   CK(cudaMemsetAsync(c->hint, 0, (size_t)n * n, c->stream));
   CK(launch_cover(b, c->stream));  // also each site's first window (hint)
   CK(launch_count(b, c->stream));
@@ -431,6 +434,8 @@ int gcvt_ctx_create(int n_max, gcvt_ctx **out) {
   for (int k = 0; k < 3; ++k) ok = ok && dal(&c->bits[k], words * sizeof(uint64_t));
   ok = ok && dal(&c->prev, words * sizeof(int16_t));
   ok = ok && dal(&c->next, words * sizeof(int16_t));
+  ok = ok && dal(&c->occ, (size_t)(n_max / kBand) * 4 * sizeof(unsigned));
+  ok = ok && dal(&c->open_tiles, label_blocks(n_max) * sizeof(unsigned));
   ok = ok && dal(&c->st, sizeof(DevState));
   ok = ok && dal(&c->list, nn * sizeof(uint32_t));
   for (int k = 0; k < 3; ++k) ok = ok && dal(&c->counts[k], list_blocks(n_max) * sizeof(unsigned));
@@ -475,6 +480,8 @@ int gcvt_ctx_destroy(gcvt_ctx *c) {
   for (int k = 0; k < 3; ++k) cudaFree(c->bits[k]);
   cudaFree(c->prev);
   cudaFree(c->next);
+  cudaFree(c->occ);
+  cudaFree(c->open_tiles);
   cudaFree(c->st);
   cudaFree(c->list);
   for (int k = 0; k < 3; ++k) cudaFree(c->counts[k]);
@@ -534,10 +541,14 @@ int gcvt_ctx_label(gcvt_ctx *c, int16_t *labels, int mem) {
   if (!c->loaded) return GCVT_ERR_STATE;
   if (c->input_err) return GCVT_ERR_INPUT;
   const int n = c->cur_n;
-  const LevelBufs b = level_bufs(c, n, level_of(c, n));
-  CK(launch_summary(b, 0, c->stream));
-  CK(launch_rows(b, 0, c->stream));
-  return copy_out(labels, c->grid, (size_t)n * n * sizeof(uint32_t), mem, c->stream);
+  LevelBufs b = level_bufs(c, n, level_of(c, n));
+  // straight into the caller's device buffer where words can be written there (the
+  // staging grid and a copy of 8 bytes a pixel otherwise: 0.08 ms at 8192^2)
+  const bool direct = mem == GCVT_MEM_DEVICE && reinterpret_cast<uintptr_t>(labels) % 4 == 0;
+  if (direct) b.labels = reinterpret_cast<uint32_t *>(labels);
+  CK(launch_label(b, c->stream));
+  return direct ? GCVT_OK
+                : copy_out(labels, c->grid, (size_t)n * n * sizeof(uint32_t), mem, c->stream);
 }
 
 int gcvt_ctx_iterate(gcvt_ctx *c, int iterations) {
@@ -760,8 +771,7 @@ int gcvt_ctx_jfa_label(gcvt_ctx *c, int16_t *labels, unsigned long long *stats, 
   CK(launch_jfa(a, b, n, c->err, &res, c->stream, c->jfa_halo));
   if (stats) {
     const LevelBufs lb = level_bufs(c, n, level_of(c, n));
-    CK(launch_summary(lb, 0, c->stream));
-    CK(launch_rows(lb, 0, c->stream));  // exact labels into the staging grid
+    CK(launch_label(lb, c->stream));  // exact labels into the staging grid
     CK(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), c->stream));
     CK(launch_jfa_compare(res, c->grid, n, counts, c->stream));
     unsigned long long h[2] = {0, 0};
@@ -1293,8 +1303,7 @@ int gcvt_ctx_time_kernels(gcvt_ctx *c, int iterations, float *ms3) {
         launch_list(b, 1, c->stream) != cudaSuccess ||
         launch_cells(b, 0, nullptr, c->stream, c->cell_grid) != cudaSuccess ||
         cudaEventRecord(ev[1], c->stream) != cudaSuccess ||
-        launch_summary(b, 0, c->stream) != cudaSuccess ||
-        launch_rows(b, 0, c->stream) != cudaSuccess ||
+        launch_label(b, c->stream) != cudaSuccess ||
         cudaEventRecord(ev[2], c->stream) != cudaSuccess ||
         cudaEventSynchronize(ev[2]) != cudaSuccess ||
         cudaEventElapsedTime(&ms0, ev[0], ev[1]) != cudaSuccess ||

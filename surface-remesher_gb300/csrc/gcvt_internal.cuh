@@ -70,6 +70,8 @@ struct DevState {
   int gate_tried, gate_kept;  // jumps proposed / kept
   double gate_e0;      // energy of the sites the jump starts from
   double gate_e1;      // energy of the jumped sites
+  int label_ovf;       // labelling: a tile's lists did not fit (label_tiles.cu)
+  int pad1;
   // Labelling (labeller.cu): rows whose candidate hull did not fit the
   // bounded buffer of k_rows, for k_rows_full (zero between labellings).
   unsigned row_ovf[kMaxN / 32];
@@ -83,6 +85,9 @@ struct LevelBufs {
                            // bits[cur+1]; k_list clears bits[cur+2] (mod 3)
   int16_t *prev;           // [band][column]: nearest site row above the band
   int16_t *next;           // [band][column]: nearest site row below the band
+  unsigned *occ;           // labelling: per row of 64 x 64 pixel blocks, 128 bits: whether
+                           // a block holds a site
+  unsigned *open_tiles;    // labelling: per 64 x 64 pixels, a bit per 16 x 16 tile left open
   const float *density;    // n*n
   const int2 *support;     // per row [first, last+1) of nonzero density
   const int2 *sup_range;   // rows [x, y) containing every nonzero density
@@ -131,9 +136,13 @@ cudaError_t launch_bits_to_grid(const uint64_t *bits, int n, uint32_t *grid, cud
 inline cudaError_t launch_jfa_seed(const uint64_t *bits, int n, uint32_t *grid, cudaStream_t s) {
   return launch_bits_to_grid(bits, n, grid, s, kJfaNone, true);
 }
-cudaError_t launch_summary(const LevelBufs &b, int respect_stop, cudaStream_t s);
+// The exact labels of the current sites into b.labels (label_tiles.cu); the row
+// pass behind it (column summaries, rows) runs where DevState::label_ovf says so.
+cudaError_t launch_label(const LevelBufs &b, cudaStream_t s);
+size_t label_blocks(int n);  // entries of LevelBufs::open_tiles (::occ: 4 per row of blocks)
+cudaError_t launch_summary(const LevelBufs &b, cudaStream_t s);
 cudaError_t launch_fixed_bits(const uint8_t *mask, int n, uint64_t *fixed_bits, cudaStream_t s);
-cudaError_t launch_rows(const LevelBufs &b, int respect_stop, cudaStream_t s);
+cudaError_t launch_rows(const LevelBufs &b, cudaStream_t s);
 cudaError_t launch_list(const LevelBufs &b, int respect_stop, cudaStream_t s);
 cudaError_t launch_count(const LevelBufs &b, cudaStream_t s);
 // MODE 0, 4 and 5 run one site per warp when b.sitev and b.gcnt are set,

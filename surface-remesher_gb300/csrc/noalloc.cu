@@ -35,7 +35,10 @@ constexpr size_t kWords = (size_t)(kNoAllocMaxN / kBand) * kNoAllocMaxN;
 constexpr size_t kOffBits = 0;
 constexpr size_t kOffPrev = align_up(kOffBits + kWords * sizeof(uint64_t));
 constexpr size_t kOffNext = align_up(kOffPrev + kWords * sizeof(int16_t));
-constexpr size_t kOffState = align_up(kOffNext + kWords * sizeof(int16_t));
+constexpr size_t kBlocks = (size_t)(kNoAllocMaxN / kBand) * (kNoAllocMaxN / kBand);
+constexpr size_t kOffOcc = align_up(kOffNext + kWords * sizeof(int16_t));
+constexpr size_t kOffOpen = align_up(kOffOcc + (size_t)(kNoAllocMaxN / kBand) * 4 * sizeof(unsigned));
+constexpr size_t kOffState = align_up(kOffOpen + kBlocks * sizeof(unsigned));
 constexpr size_t kOffErr = align_up(kOffState + sizeof(DevState));
 constexpr size_t kNoAllocBytes = align_up(kOffErr + sizeof(int));
 
@@ -105,8 +108,9 @@ extern "C" int gcvt_label_grid_static(const int16_t *sites, int16_t *labels, int
   b.next = reinterpret_cast<int16_t *>(base + kOffNext);
   b.labels = reinterpret_cast<uint32_t *>(labels);
   b.st = st;
-  if (launch_summary(b, 0, s) != cudaSuccess) return GCVT_ERR_CUDA;
-  if (launch_rows(b, 0, s) != cudaSuccess) return GCVT_ERR_CUDA;
+  b.occ = reinterpret_cast<unsigned *>(base + kOffOcc);
+  b.open_tiles = reinterpret_cast<unsigned *>(base + kOffOpen);
+  if (launch_label(b, s) != cudaSuccess) return GCVT_ERR_CUDA;
   int herr = 0;  // host stack: the only readback, no allocation
   if (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)

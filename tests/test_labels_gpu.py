@@ -82,3 +82,34 @@ def test_context_label_device_buffers(gcvt_lib, oracle, cuda_device):
     torch.cuda.synchronize()
     assert np.array_equal(out.cpu().numpy(), want)
     ctx.close()
+
+
+@pytest.mark.parametrize("n,kind", [(512, "1"), (512, "2"), (768, "3"), (512, "5"), (512, "18"),
+                                    (1024, "mirror"), (768, "far"), (2048, "one"), (256, "one")])
+def test_tile_lists_and_their_overflows(gcvt_lib, oracle, cuda_device, n, kind):
+    """The tile labeller's dispatch: a crowded block of one site per 1 to 18 pixels
+    beside empty space (window, candidate and block lists at and past their ends,
+    tiles far from any site, the row pass behind them), mirror pairs across bands seen
+    from near and far, lone sites."""
+    rng = np.random.default_rng(n)
+    if kind == "mirror":  # pairs of one column about band edges and tile rows, far apart
+        xs, ys = [], []
+        for x in range(40, n, 170):
+            for c in (64, 128, 200, 448, 512, 720):
+                k = int(rng.integers(1, 40))
+                xs += [x, x]
+                ys += [c - k, c + k]
+        pts = set(zip(xs, ys))
+    elif kind == "far":
+        pts = {(3, 5), (3, 765), (760, 2), (384, 384), (385, 384), (384, 386)}
+    elif kind == "one":
+        pts = {(n - 1, n // 3)}
+    else:
+        b = rng.random((160, 200)) < 1.0 / int(kind)
+        ys, xs = np.nonzero(b)
+        pts = set(zip((xs + 37).tolist(), (ys + 61).tolist()))
+        pts |= {tuple(p) for p in rng.integers(0, n, (9, 2)).tolist()}
+    g = grid(n, sorted(pts))
+    got, want = gcvt_lib.label_grid(g), oracle.spec_label(g)
+    bad = np.argwhere((got != want).any(-1))
+    assert bad.size == 0, (len(bad), bad[:3], got[tuple(bad[0])], want[tuple(bad[0])])
