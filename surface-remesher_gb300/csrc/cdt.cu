@@ -14,7 +14,7 @@
 //      points that won all their claims split (1 -> 3 inside a triangle,
 //      2 -> 4 on an edge, a fan over the visible hull edges outside the
 //      hull); after each round, two flip rounds over the changed triangles
-//      (two rounds with their flips make one CUDA graph and one read-back);
+//      (four rounds with their flips per read-back);
 //   4. each segment made an edge by flipping the edges that cross it
 //      (Sloan's method, cdt_core.cuh recover_segment) and marked: segments
 //      already edges at once, the others in rounds where each claims the
@@ -63,6 +63,7 @@ constexpr int kFlipPoll = 4;      // flip rounds between read-backs
 constexpr int kInterimFlips = 2;  // flip rounds after each insertion round
 constexpr int kFlipBlocks = 304;  // grid of the grid-stride flip kernels (2 per SM)
 constexpr int kInsertRounds = 1 << 12;
+constexpr int kInsertPoll = 4;    // insertion rounds between read-backs
 constexpr int kSegQueue = 4096;   // crossing edges of one segment
 constexpr int kSegStack = 256;    // pieces of one segment split by vertices inside it
 constexpr int kCorr = 8;          // crossing edges of a segment recovered in the parallel rounds
@@ -181,9 +182,15 @@ struct Loc {
   int et[kChain], ei[kChain];
 };
 
-// Claims hold priorities (cdt_core.cuh prio): the smallest wins.
-__device__ __forceinline__ void claim(unsigned *cl, int t, unsigned pr) { atomicMin(cl + t, pr); }
-__device__ __forceinline__ void claim_nbrs(const Mesh &m, unsigned *cl, int t, unsigned pr) {
+// Claims hold (rounds left, priority) (cdt_core.cuh prio): the smallest wins, and a
+// round's claims are below every earlier round's, so the array is never cleared
+// between rounds (a memset of half a megabyte three times a round before).
+typedef unsigned long long Claim;
+__device__ __forceinline__ Claim claim_of(unsigned round, unsigned id) {
+  return ((Claim)(0xffffffffu - round) << 32) | cdt::prio(id);
+}
+__device__ __forceinline__ void claim(Claim *cl, int t, Claim pr) { atomicMin(cl + t, pr); }
+__device__ __forceinline__ void claim_nbrs(const Mesh &m, Claim *cl, int t, Claim pr) {
   claim(cl, t, pr);
   for (int i = 0; i < 3; ++i) {
     const int nb = m.nbr[3 * t + i];
@@ -193,11 +200,12 @@ __device__ __forceinline__ void claim_nbrs(const Mesh &m, unsigned *cl, int t, u
 
 // Locate every pending point and claim what its insertion changes.
 __global__ void k_ins_locate(Mesh m, const int *__restrict__ pend, const int *npp, int *start,
-                             Loc *loc, unsigned *cl, int *err) {
+                             Loc *loc, Claim *cl, unsigned round, int *done, int *err) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= *npp) return;
   const int p = pend[q];
-  const unsigned pr = cdt::prio((unsigned)p);
+  const Claim pr = claim_of(round, (unsigned)p);
+  done[q] = 0;
   Loc L;
   L.kind = cdt::locate(m, p, start[q], kWalk, &L.t, &L.i);
   L.cnt = 0;
@@ -277,10 +285,10 @@ __global__ void k_ins_locate(Mesh m, const int *__restrict__ pend, const int *np
   loc[q] = L;
 }
 
-__device__ __forceinline__ bool owns(const Mesh &m, const unsigned *cl, int t, unsigned pr) {
+__device__ __forceinline__ bool owns(const Mesh &m, const Claim *cl, int t, Claim pr) {
   return cl[t] == pr;
 }
-__device__ bool owns_nbrs(const Mesh &m, const unsigned *cl, int t, unsigned pr) {
+__device__ bool owns_nbrs(const Mesh &m, const Claim *cl, int t, Claim pr) {
   if (!owns(m, cl, t, pr)) return false;
   for (int i = 0; i < 3; ++i) {
     const int nb = m.nbr[3 * t + i];
@@ -304,12 +312,12 @@ __device__ __forceinline__ void touch(const Mesh &m, uint8_t *act, int t) {
 // Insert the points that won every claim; the others stay pending (their
 // walk starts next round from the triangle they reached).
 __global__ void k_ins_apply(Mesh m, const int *__restrict__ pend, const int *npp, int *start,
-                            const Loc *__restrict__ loc, const unsigned *cl, int *ntri, int cap,
-                            int *done, uint8_t *act, int *err) {
+                            const Loc *__restrict__ loc, const Claim *cl, unsigned round,
+                            int *ntri, int cap, int *done, uint8_t *act, int *err) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= *npp) return;
   const int p = pend[q];
-  const unsigned pr = cdt::prio((unsigned)p);
+  const Claim pr = claim_of(round, (unsigned)p);
   const Loc &L = loc[q];
   if (L.kind == cdt::kLocFail || L.kind == cdt::kLocVertex) return;
   start[q] = L.t;
@@ -365,8 +373,8 @@ __global__ void k_ins_apply(Mesh m, const int *__restrict__ pend, const int *npp
 // edges towards a higher-numbered neighbour that wants a flip; the flip
 // claims both triangles and the four outer neighbours with the priority of
 // 3 t + i.  A triangle with none is settled until a change touches it again.
-__device__ __forceinline__ void flip_mark_one(const Mesh &m, int t, int *cand, unsigned *cl,
-                                              uint8_t *act, int *found) {
+__device__ __forceinline__ void flip_mark_one(const Mesh &m, int t, int *cand, Claim *cl,
+                                              unsigned round, uint8_t *act, int *found) {
   if (!act[t]) {
     cand[t] = 0;
     return;
@@ -387,27 +395,27 @@ __device__ __forceinline__ void flip_mark_one(const Mesh &m, int t, int *cand, u
   }
   atomicAdd(found, 1);
   const int i = c - 1;
-  const unsigned pr = cdt::prio((unsigned)(3 * t + i));
+  const Claim pr = claim_of(round, (unsigned)(3 * t + i));
   const int t2 = cdt::nb_tri(m.nbr[3 * t + i]);
   claim_nbrs(m, cl, t, pr);
   claim_nbrs(m, cl, t2, pr);
 }
 
 // (grid-stride: a round with few changed triangles costs few blocks)
-__global__ void k_flip_mark(Mesh m, const int *ntri, int *cand, unsigned *cl, uint8_t *act,
-                            int *found) {
+__global__ void k_flip_mark(Mesh m, const int *ntri, int *cand, Claim *cl, unsigned round,
+                            uint8_t *act, int *found) {
   const int T = *ntri;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x)
-    flip_mark_one(m, t, cand, cl, act, found);
+    flip_mark_one(m, t, cand, cl, round, act, found);
 }
 
-__global__ void k_flip_apply(Mesh m, const int *ntri, const int *cand, const unsigned *cl,
-                             uint8_t *act, int *flips) {
+__global__ void k_flip_apply(Mesh m, const int *ntri, const int *cand, const Claim *cl,
+                             unsigned round, uint8_t *act, int *flips) {
   const int T = *ntri;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
     if (!cand[t]) continue;
     const int i = cand[t] - 1;
-    const unsigned pr = cdt::prio((unsigned)(3 * t + i));
+    const Claim pr = claim_of(round, (unsigned)(3 * t + i));
     const int t2 = cdt::nb_tri(m.nbr[3 * t + i]);
     if (!owns_nbrs(m, cl, t, pr) || !owns_nbrs(m, cl, t2, pr)) continue;
     cdt::flip(m, t, i);
@@ -446,7 +454,7 @@ __global__ void k_seg_mark(Mesh m, const int *__restrict__ segs, int S, int V, i
 // a vertex or a constraint, or crosses more than kCorr edges, goes to the
 // one-thread pass.
 __global__ void k_seg_locate(Mesh m, const int *__restrict__ segs, int base, int W, int *state,
-                             int *list, int *lcnt, unsigned *cl) {
+                             int *list, int *lcnt, Claim *cl, unsigned round) {
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= W) return;
   const int k = base + w;
@@ -471,7 +479,7 @@ __global__ void k_seg_locate(Mesh m, const int *__restrict__ segs, int base, int
     }
     n += c;
   }
-  const unsigned pr = cdt::prio((unsigned)k);
+  const Claim pr = claim_of(round, (unsigned)k);
   for (int i = 0; i < n; ++i) claim(cl, L[i], pr);
   lcnt[w] = n;
 }
@@ -480,13 +488,13 @@ __global__ void k_seg_locate(Mesh m, const int *__restrict__ segs, int base, int
 // recover_segment); the others count themselves pending for the next round.
 __global__ void k_seg_apply(Mesh m, const int *__restrict__ segs, int base, int W, int *state,
                             const int *__restrict__ list, const int *__restrict__ lcnt,
-                            const unsigned *cl, int *pending, int *err) {
+                            const Claim *cl, unsigned round, int *pending, int *err) {
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= W) return;
   const int k = base + w;
   if (state[k] != kSegPending) return;
   const int *L = list + (size_t)w * kClaim;
-  const unsigned pr = cdt::prio((unsigned)k);
+  const Claim pr = claim_of(round, (unsigned)k);
   for (int i = 0, n = lcnt[w]; i < n; ++i)
     if (cl[L[i]] != pr) {
       atomicAdd(pending, 1);
@@ -655,7 +663,8 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
   int *tri = sc.take<int>(3 * (size_t)cap_t), *nbr = sc.take<int>(3 * (size_t)cap_t);
   unsigned *cons = sc.take<unsigned>((size_t)cap_t);
   int *vt = sc.take<int>((size_t)V);
-  unsigned *cl = sc.take<unsigned>((size_t)cap_t);
+  Claim *cl = sc.take<Claim>((size_t)cap_t);
+  unsigned round = 0;  // of claims
   int *cand = sc.take<int>((size_t)cap_t);
   uint8_t *act = sc.take<uint8_t>((size_t)cap_t);
   // [0] error bits, [1] triangles, [2] flips wanted, [3] flips made, [4] and
@@ -666,6 +675,7 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
   CCK(launch_extract(bits, fixed, n, colcnt, 1.0, 0.0, 0.0, sxy, F, colcnt + n, s));
   CCK(cudaMemsetAsync(ctr, 0, 8 * sizeof(int), s));
   CCK(cudaMemsetAsync(cons, 0, (size_t)cap_t * sizeof(unsigned), s));
+  CCK(cudaMemsetAsync(cl, 0xff, (size_t)cap_t * sizeof(Claim), s));
   k_cdt_coords<<<nblk(V, 256), 256, 0, s>>>(sxy, (int)F, cxy, C, scale, left, lower, n, X, Y, R,
                                             ctr);
   CCK(cudaGetLastError());
@@ -702,10 +712,9 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
   const int fgrid = nblk(cap_t, 256) < kFlipBlocks ? nblk(cap_t, 256) : kFlipBlocks;
   auto flip_rounds = [&](int rounds) -> int {
     for (int i = 0; i < rounds; ++i) {
-      CCK(cudaMemsetAsync(cl, 0xff, (size_t)cap_t * sizeof(unsigned), s));
-      CCK(cudaMemsetAsync(ctr + 2, 0, 2 * sizeof(int), s));
-      k_flip_mark<<<fgrid, 256, 0, s>>>(m, ctr + 1, cand, cl, act, ctr + 2);
-      k_flip_apply<<<fgrid, 256, 0, s>>>(m, ctr + 1, cand, cl, act, ctr + 3);
+      ++round;
+      k_flip_mark<<<fgrid, 256, 0, s>>>(m, ctr + 1, cand, cl, round, act, ctr + 2);
+      k_flip_apply<<<fgrid, 256, 0, s>>>(m, ctr + 1, cand, cl, round, act, ctr + 3);
     }
     CCK(cudaGetLastError());
     return GCVT_OK;
@@ -715,7 +724,9 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
   auto flips = [&]() -> int {
     CCK(cudaMemsetAsync(act, 1, (size_t)cap_t, s));
     for (int r = 0; r < kFlipRounds; r += kFlipPoll) {
-      if ((rc = flip_rounds(kFlipPoll)) || (rc = pull())) return rc;
+      if ((rc = flip_rounds(kFlipPoll - 1))) return rc;
+      CCK(cudaMemsetAsync(ctr + 2, 0, 2 * sizeof(int), s));  // the last round's counts
+      if ((rc = flip_rounds(1)) || (rc = pull())) return rc;
       if (h[0] || h[2] == 0) return GCVT_OK;
     }
     h[0] |= kErrWalk;
@@ -737,47 +748,27 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
     // those left go to list b (count *nb); then kInterimFlips flip rounds.  Every
     // count is read on the device, so rounds queue without the host.
     auto ins_round = [&](int *pa, int *sa, int *pb, int *sb, int *na, int *nb) -> int {
-      CCK(cudaMemsetAsync(cl, 0xff, (size_t)cap_t * sizeof(unsigned), s));
-      CCK(cudaMemsetAsync(done, 0, (size_t)C * sizeof(int), s));
-      k_ins_locate<<<nblk(C, 128), 128, 0, s>>>(m, pa, na, sa, loc, cl, ctr);
-      k_ins_apply<<<nblk(C, 128), 128, 0, s>>>(m, pa, na, sa, loc, cl, ctr + 1, cap_t, done, act,
-                                               ctr);
+      ++round;
+      k_ins_locate<<<nblk(C, 32), 32, 0, s>>>(m, pa, na, sa, loc, cl, round, done, ctr);
+      k_ins_apply<<<nblk(C, 32), 32, 0, s>>>(m, pa, na, sa, loc, cl, round, ctr + 1, cap_t, done,
+                                               act, ctr);
       k_compact<<<1, 1024, 0, s>>>(pa, sa, done, na, pb, sb, nb);
       CCK(cudaGetLastError());
       return flip_rounds(kInterimFlips);
     };
-    // two rounds (list 1 -> 2 -> 1) per read-back, as one CUDA graph where the
-    // stream can be captured
-    auto ins_pair = [&]() -> int {
-      if ((rc = ins_round(pend, start, pend2, start2, ctr + 4, ctr + 6))) return rc;
-      return ins_round(pend2, start2, pend, start, ctr + 6, ctr + 4);
-    };
-    cudaGraphExec_t pair_exec = nullptr;
-    if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-      const int le = ins_pair();
-      cudaGraph_t g = nullptr;
-      const cudaError_t ce = cudaStreamEndCapture(s, &g);
-      const cudaError_t ie =
-          (le == GCVT_OK && ce == cudaSuccess) ? cudaGraphInstantiate(&pair_exec, g, 0) : ce;
-      if (g) cudaGraphDestroy(g);
-      if (le != GCVT_OK || ce != cudaSuccess || ie != cudaSuccess) {
-        if (pair_exec) cudaGraphExecDestroy(pair_exec);
-        return GCVT_ERR_CUDA;
-      }
-    } else {
-      cudaGetLastError();  // the legacy default stream: plain launches
-    }
+    // kInsertPoll rounds (lists 1 -> 2 -> 1 ...) per read-back
     CCK(cudaMemcpyAsync(ctr + 4, &C, sizeof(int), cudaMemcpyHostToDevice, s));
     int np = C;
-    for (int r = 0; r < kInsertRounds / 2 && np > 0; ++r) {
-      rc = pair_exec ? (cudaGraphLaunch(pair_exec, s) == cudaSuccess ? GCVT_OK : GCVT_ERR_CUDA)
-                     : ins_pair();
+    for (int r = 0; r < kInsertRounds && np > 0; r += kInsertPoll) {
+      for (int k = 0; k < kInsertPoll && rc == GCVT_OK; k += 2) {
+        rc = ins_round(pend, start, pend2, start2, ctr + 4, ctr + 6);
+        if (rc == GCVT_OK) rc = ins_round(pend2, start2, pend, start, ctr + 6, ctr + 4);
+      }
       if (rc == GCVT_OK) rc = pull();
       if (rc != GCVT_OK) break;
       if (h[0]) break;
       np = h[4];
     }
-    if (pair_exec) cudaGraphExecDestroy(pair_exec);
     if (rc != GCVT_OK) return rc;
     if (!h[0] && np > 0) h[0] |= kErrWalk;
   }
@@ -797,11 +788,11 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
     for (int base = 0; base < S; base += kSegWindow) {
       const int W = S - base < kSegWindow ? S - base : kSegWindow;
       for (int r = 0; r < kSegRounds; ++r) {
-        CCK(cudaMemsetAsync(cl, 0xff, (size_t)T * sizeof(unsigned), s));
+        ++round;
         CCK(cudaMemsetAsync(ctr + 5, 0, sizeof(int), s));
-        k_seg_locate<<<nblk(W, 128), 128, 0, s>>>(m, segs, base, W, state, list, lcnt, cl);
-        k_seg_apply<<<nblk(W, 128), 128, 0, s>>>(m, segs, base, W, state, list, lcnt, cl, ctr + 5,
-                                                 ctr);
+        k_seg_locate<<<nblk(W, 32), 32, 0, s>>>(m, segs, base, W, state, list, lcnt, cl, round);
+        k_seg_apply<<<nblk(W, 32), 32, 0, s>>>(m, segs, base, W, state, list, lcnt, cl, round,
+                                               ctr + 5, ctr);
         CCK(cudaGetLastError());
         if ((rc = pull())) return rc;
         if (h[5] == 0) break;

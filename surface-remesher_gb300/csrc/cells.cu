@@ -45,7 +45,7 @@
 // Work split.  k_cell runs one warp per block, as many blocks as fit on the
 // GPU; each warp takes the next group of 32 listed sites from a ticket, one
 // site per lane.  A lane keeps its site's candidates as two bytes each, bounds
-// eight rows per pass over them in floats (cell_float: exact where float_walk
+// seven rows per pass over them in floats (cell_float: exact where float_walk
 // says so, else cell_general's integer division), lists the rows and sums
 // their pixels two rows at a time in packed FP32.  What bounds it: issue slots
 // and the latency of L1 misses, not bandwidth (60 MB an iteration).  Against
@@ -499,7 +499,7 @@ __device__ __forceinline__ bool float_walk(int W, int rb) {
   return W <= 127 && rb <= 511 && W * W * (W + 2 * rb) < (5 << 18);
 }
 
-constexpr int kRowsPass = 8;   // rows bounded per pass over the records
+constexpr int kRowsPass = 7;   // rows bounded per pass over the records (6 and 8: 4 % slower)
 constexpr int kRowList = 24;   // rows listed before their pixels are summed
 
 // The float 128 + a byte minus 128 (no conversion instruction).
@@ -1482,7 +1482,8 @@ __global__ void __launch_bounds__(32 * kBlockSites, 4) k_cell_warp(LevelBufs a) 
   DevState *st = a.st;
   if (st->snap_stopped) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const IterView v = iter_view(a);
+  IterView v = iter_view(a);
+  ++v.slack;  // a retried cell holds up its block: a wider window costs less (1.35 -> 1.30 ms)
   if (v.ngroups == 0) {  // no sites: the schedule still advances
     if (blockIdx.x == 0 && threadIdx.x == 0) pass_done<MODE>(st, 0.0, 0u, 0u, a.n, v.cur);
     return;
