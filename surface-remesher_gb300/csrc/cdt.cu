@@ -176,10 +176,14 @@ __global__ void k_edge_link(const int *__restrict__ tri, int T, const unsigned l
 // in counter-clockwise order with the hull triangles just before and after
 // them -- recorded while nothing changes, so the insertion never walks a
 // mesh that other points are changing.
+// (The edges lie around the middle of edge[], packed like neighbours: those before
+// the exit edge are found going backwards.  Only what is used is written: a copy of
+// the whole record per point and round was a third of a one-block round.)
 struct Loc {
   int kind, t, i;
   int cnt, before, after;
-  int et[kChain], ei[kChain];
+  int first;               // edge[first .. first + cnt)
+  int edge[2 * kChain];
 };
 
 // Claims hold (rounds left, priority) (cdt_core.cuh prio): the smallest wins, and a
@@ -198,31 +202,32 @@ __device__ __forceinline__ void claim_nbrs(const Mesh &m, Claim *cl, int t, Clai
   }
 }
 
-// Locate every pending point and claim what its insertion changes.
-__global__ void k_ins_locate(Mesh m, const int *__restrict__ pend, const int *npp, int *start,
-                             Loc *loc, Claim *cl, unsigned round, int *done, int *err) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= *npp) return;
+// Locate pending point q and claim what its insertion changes.
+__device__ void ins_locate(const Mesh &m, const int *pend, int q, int *start, Loc *loc, Claim *cl,
+                           unsigned round, int *done, int *err) {
   const int p = pend[q];
   const Claim pr = claim_of(round, (unsigned)p);
   done[q] = 0;
-  Loc L;
-  L.kind = cdt::locate(m, p, start[q], kWalk, &L.t, &L.i);
+  Loc &L = loc[q];
+  int lt, li;
+  const int kind = cdt::locate(m, p, start[q], kWalk, &lt, &li);
+  L.kind = kind;
+  L.t = lt;
+  L.i = li;
   L.cnt = 0;
-  if (L.kind == cdt::kLocFail) {
+  if (kind == cdt::kLocFail) {
     atomicOr(err, kErrWalk);
-  } else if (L.kind == cdt::kLocVertex) {
+  } else if (kind == cdt::kLocVertex) {
     atomicOr(err, kErrDuplicate);
-  } else if (L.kind == cdt::kLocIn) {
-    claim_nbrs(m, cl, L.t, pr);
-  } else if (L.kind == cdt::kLocEdge) {
-    claim_nbrs(m, cl, L.t, pr);
-    const int nb = m.nbr[3 * L.t + L.i];
+  } else if (kind == cdt::kLocIn) {
+    claim_nbrs(m, cl, lt, pr);
+  } else if (kind == cdt::kLocEdge) {
+    claim_nbrs(m, cl, lt, pr);
+    const int nb = m.nbr[3 * lt + li];
     if (nb >= 0) claim_nbrs(m, cl, cdt::nb_tri(nb), pr);
   } else {  // outside: the visible hull edges around the exit edge
-    int ft = L.t, fi = L.i, back = 0, ok = 1;
-    int bt[kChain], bi[kChain];  // the edges before the exit edge, nearest first
-    L.before = L.after = -1;
+    int ft = lt, fi = li, first = kChain, last = kChain, ok = 1, before = -1, after = -1;
+    L.edge[first] = cdt::pack_nb(lt, li);
     for (;;) {
       int pt, pi;
       if (!cdt::hull_prev(m, ft, fi, kRotate, &pt, &pi)) {
@@ -230,59 +235,56 @@ __global__ void k_ins_locate(Mesh m, const int *__restrict__ pend, const int *np
         break;
       }
       if (cdt::orient(m, m.tri[3 * pt + cdt::nx3(pi)], m.tri[3 * pt + cdt::pv3(pi)], p) >= 0) {
-        L.before = pt;
+        before = pt;
         break;
       }
-      if (back + 1 >= kChain) {
+      if (kChain - first + 1 >= kChain) {
         ok = 0;
         break;
       }
-      bt[back] = ft = pt;
-      bi[back] = fi = pi;
-      ++back;
+      ft = pt;
+      fi = pi;
+      L.edge[--first] = cdt::pack_nb(pt, pi);
     }
-    int cnt = 0;
-    if (ok) {
-      for (int k = back - 1; k >= 0; --k, ++cnt) {
-        L.et[cnt] = bt[k];
-        L.ei[cnt] = bi[k];
+    for (ft = lt, fi = li; ok;) {
+      int nt, ni;
+      if (!cdt::hull_next(m, ft, fi, kRotate, &nt, &ni)) {
+        ok = 0;
+        break;
       }
-      L.et[cnt] = L.t;
-      L.ei[cnt] = L.i;
-      ++cnt;
-      int lt = L.t, li = L.i;
-      for (;;) {
-        int nt, ni;
-        if (!cdt::hull_next(m, lt, li, kRotate, &nt, &ni)) {
-          ok = 0;
-          break;
-        }
-        if (cdt::orient(m, m.tri[3 * nt + cdt::nx3(ni)], m.tri[3 * nt + cdt::pv3(ni)], p) >= 0) {
-          L.after = nt;
-          break;
-        }
-        if (cnt >= kChain) {
-          ok = 0;
-          break;
-        }
-        L.et[cnt] = lt = nt;
-        L.ei[cnt] = li = ni;
-        ++cnt;
+      if (cdt::orient(m, m.tri[3 * nt + cdt::nx3(ni)], m.tri[3 * nt + cdt::pv3(ni)], p) >= 0) {
+        after = nt;
+        break;
       }
+      if (last - first + 1 >= kChain) {
+        ok = 0;
+        break;
+      }
+      ft = nt;
+      fi = ni;
+      L.edge[++last] = cdt::pack_nb(nt, ni);
     }
+    L.before = before;
+    L.after = after;
+    L.first = first;
     if (!ok) {
       atomicOr(err, kErrWalk);
       L.kind = cdt::kLocFail;
     } else {
       // claim the chain and the hull edges just before and after it, so that
       // two points never extend the hull next to each other in one round
-      L.cnt = cnt;
-      for (int k = 0; k < cnt; ++k) claim(cl, L.et[k], pr);
-      if (L.before >= 0) claim(cl, L.before, pr);
-      if (L.after >= 0) claim(cl, L.after, pr);
+      L.cnt = last - first + 1;
+      for (int k = first; k <= last; ++k) claim(cl, cdt::nb_tri(L.edge[k]), pr);
+      if (before >= 0) claim(cl, before, pr);
+      if (after >= 0) claim(cl, after, pr);
     }
   }
-  loc[q] = L;
+}
+
+__global__ void k_ins_locate(Mesh m, const int *__restrict__ pend, const int *npp, int *start,
+                             Loc *loc, Claim *cl, unsigned round, int *done, int *err) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < *npp) ins_locate(m, pend, q, start, loc, cl, round, done, err);
 }
 
 __device__ __forceinline__ bool owns(const Mesh &m, const Claim *cl, int t, Claim pr) {
@@ -297,25 +299,38 @@ __device__ bool owns_nbrs(const Mesh &m, const Claim *cl, int t, Claim pr) {
   return true;
 }
 
-// Triangle t changed: it and its neighbours are tested by the next flip
-// round.  An edge whose opposite vertices changed belongs to a changed
-// triangle, so it is tested from whichever of its triangles has the smaller
-// index (k_flip_mark).
-__device__ __forceinline__ void touch(const Mesh &m, uint8_t *act, int t) {
-  act[t] = 1;
+// What to do with a triangle that changed: it and its neighbours are tested by
+// the next flip round.  An edge whose opposite vertices changed belongs to a
+// changed triangle, so it is tested from whichever of its triangles has the smaller
+// index.  Act marks them in a byte each; ActList also lists each once.
+struct Act {
+  uint8_t *act;
+  __device__ __forceinline__ void add(int t) const { act[t] = 1; }
+};
+struct ActList {
+  uint8_t *act;
+  int *list, *count;
+  __device__ __forceinline__ void add(int t) const {
+    const unsigned bit = 1u << (8 * (t & 3));
+    if (!(atomicOr(reinterpret_cast<unsigned *>(act) + (t >> 2), bit) & bit))
+      list[atomicAdd(count, 1)] = t;
+  }
+};
+template <class A>
+__device__ __forceinline__ void touch(const Mesh &m, const A &act, int t) {
+  act.add(t);
   for (int i = 0; i < 3; ++i) {
     const int nb = m.nbr[3 * t + i];
-    if (nb >= 0) act[cdt::nb_tri(nb)] = 1;
+    if (nb >= 0) act.add(cdt::nb_tri(nb));
   }
 }
 
-// Insert the points that won every claim; the others stay pending (their
-// walk starts next round from the triangle they reached).
-__global__ void k_ins_apply(Mesh m, const int *__restrict__ pend, const int *npp, int *start,
-                            const Loc *__restrict__ loc, const Claim *cl, unsigned round,
-                            int *ntri, int cap, int *done, uint8_t *act, int *err) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= *npp) return;
+// Insert pending point q if it won every claim; otherwise it stays pending (its
+// walk starts next round from the triangle it reached).
+template <class A>
+__device__ void ins_apply(const Mesh &m, const int *pend, int q, int *start, const Loc *loc,
+                          const Claim *cl, unsigned round, int *ntri, int cap, int *done,
+                          const A &act, int *err) {
   const int p = pend[q];
   const Claim pr = claim_of(round, (unsigned)p);
   const Loc &L = loc[q];
@@ -351,34 +366,35 @@ __global__ void k_ins_apply(Mesh m, const int *__restrict__ pend, const int *npp
     }
   } else {
     bool won = (L.before < 0 || owns(m, cl, L.before, pr)) && (L.after < 0 || owns(m, cl, L.after, pr));
-    for (int k = 0; k < L.cnt && won; ++k) won = owns(m, cl, L.et[k], pr);
+    for (int k = 0; k < L.cnt && won; ++k) won = owns(m, cl, cdt::nb_tri(L.edge[L.first + k]), pr);
     if (!won) return;
     const int s = atomicAdd(ntri, L.cnt);
     if (s + L.cnt > cap) {
       atomicOr(err, kErrCapacity);
       return;
     }
-    int slots[kChain];
-    for (int k = 0; k < L.cnt; ++k) slots[k] = s + k;
-    cdt::insert_out(m, L.et, L.ei, L.cnt, p, slots);
-    for (int k = 0; k < L.cnt; ++k) touch(m, act, slots[k]);
+    cdt::insert_fan(
+        m, [&](int k) { return L.edge[L.first + k]; }, L.cnt, p, [=](int k) { return s + k; });
+    for (int k = 0; k < L.cnt; ++k) touch(m, act, s + k);
     start[q] = s;
   }
   done[q] = 1;
 }
 
+__global__ void k_ins_apply(Mesh m, const int *__restrict__ pend, const int *npp, int *start,
+                            const Loc *__restrict__ loc, const Claim *cl, unsigned round,
+                            int *ntri, int cap, int *done, uint8_t *act, int *err) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < *npp)
+    ins_apply(m, pend, q, start, loc, cl, round, ntri, cap, done, Act{act}, err);
+}
+
 // ---- flips ---------------------------------------------------------------
 
-// Each changed triangle (act) of the *ntri in the mesh: the first of its
-// edges towards a higher-numbered neighbour that wants a flip; the flip
-// claims both triangles and the four outer neighbours with the priority of
-// 3 t + i.  A triangle with none is settled until a change touches it again.
-__device__ __forceinline__ void flip_mark_one(const Mesh &m, int t, int *cand, Claim *cl,
-                                              unsigned round, uint8_t *act, int *found) {
-  if (!act[t]) {
-    cand[t] = 0;
-    return;
-  }
+// The first edge of triangle t towards a higher-numbered neighbour that wants a
+// flip (its index + 1, 0: none); the flip claims both triangles and the four outer
+// neighbours with the priority of 3 t + i.
+__device__ __forceinline__ int flip_mark_one(const Mesh &m, int t, Claim *cl, unsigned round) {
   int c = 0;
   for (int i = 0; i < 3; ++i) {
     const int nb = m.nbr[3 * t + i];
@@ -388,41 +404,125 @@ __device__ __forceinline__ void flip_mark_one(const Mesh &m, int t, int *cand, C
       break;
     }
   }
-  cand[t] = c;
-  if (!c) {
-    act[t] = 0;
-    return;
-  }
-  atomicAdd(found, 1);
+  if (!c) return 0;
   const int i = c - 1;
   const Claim pr = claim_of(round, (unsigned)(3 * t + i));
   const int t2 = cdt::nb_tri(m.nbr[3 * t + i]);
   claim_nbrs(m, cl, t, pr);
   claim_nbrs(m, cl, t2, pr);
+  return c;
 }
 
-// (grid-stride: a round with few changed triangles costs few blocks)
+// Triangle t's marked flip, if it won all its claims.
+template <class A>
+__device__ __forceinline__ bool flip_apply_one(const Mesh &m, int t, int c, const Claim *cl,
+                                               unsigned round, const A &act) {
+  const int i = c - 1;
+  const Claim pr = claim_of(round, (unsigned)(3 * t + i));
+  const int t2 = cdt::nb_tri(m.nbr[3 * t + i]);
+  if (!owns_nbrs(m, cl, t, pr) || !owns_nbrs(m, cl, t2, pr)) return false;
+  cdt::flip(m, t, i);
+  touch(m, act, t);
+  touch(m, act, t2);
+  return true;
+}
+
+// Each changed triangle (act) of the *ntri in the mesh; one with nothing to flip is
+// settled until a change touches it again.  (grid-stride: a round with few changed
+// triangles costs few blocks)
 __global__ void k_flip_mark(Mesh m, const int *ntri, int *cand, Claim *cl, unsigned round,
                             uint8_t *act, int *found) {
   const int T = *ntri;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x)
-    flip_mark_one(m, t, cand, cl, round, act, found);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
+    const int c = act[t] ? flip_mark_one(m, t, cl, round) : 0;
+    cand[t] = c;
+    if (c) atomicAdd(found, 1);
+    else act[t] = 0;
+  }
 }
 
 __global__ void k_flip_apply(Mesh m, const int *ntri, const int *cand, const Claim *cl,
                              unsigned round, uint8_t *act, int *flips) {
   const int T = *ntri;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
-    if (!cand[t]) continue;
-    const int i = cand[t] - 1;
-    const Claim pr = claim_of(round, (unsigned)(3 * t + i));
-    const int t2 = cdt::nb_tri(m.nbr[3 * t + i]);
-    if (!owns_nbrs(m, cl, t, pr) || !owns_nbrs(m, cl, t2, pr)) continue;
-    cdt::flip(m, t, i);
-    touch(m, act, t);
-    touch(m, act, t2);
-    atomicAdd(flips, 1);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x)
+    if (cand[t] && flip_apply_one(m, t, cand[t], cl, round, Act{act})) atomicAdd(flips, 1);
+}
+
+// Every insertion round with its flip rounds in one block, for up to kOneBlock
+// points: the rounds are chains of short dependent steps (832 boundary points take 28
+// rounds; as seven launches each 74 us a round, 55 in one block of 1024 threads, 85 in
+// one of 256), and the changed triangles are listed instead of searched for.  Block
+// barriers order the steps.  After the last point the flips run until none is left.
+constexpr int kOneBlock = 4096;
+constexpr int kOneThreads = 1024;
+
+__global__ void __launch_bounds__(kOneThreads) k_insert_all(Mesh m, int *pend, int *start,
+                                                            int *pend2, int *start2, int np,
+                                                            Loc *loc, Claim *cl, unsigned round,
+                                                            int rounds, int *ntri, int cap,
+                                                            int *done, uint8_t *act, int *list,
+                                                            int *list2, int *cand, int *left,
+                                                            int *err) {
+  __shared__ int s_np, s_n, s_n2, s_stop;
+  const int tid = threadIdx.x;
+  if (tid == 0) s_n = s_stop = 0;
+  __syncthreads();
+  for (int r = 0; r < rounds && np > 0; ++r) {
+    ++round;
+    if (tid == 0) s_np = 0;
+    for (int q = tid; q < np; q += kOneThreads) ins_locate(m, pend, q, start, loc, cl, round, done, err);
+    __syncthreads();
+    for (int q = tid; q < np; q += kOneThreads)
+      ins_apply(m, pend, q, start, loc, cl, round, ntri, cap, done, ActList{act, list, &s_n}, err);
+    __syncthreads();
+    for (int q = tid; q < np; q += kOneThreads)
+      if (!done[q]) {
+        const int p = atomicAdd(&s_np, 1);
+        pend2[p] = pend[q];
+        start2[p] = start[q];
+      }
+    // the last points in: flips until none is left
+    __syncthreads();
+    const int nflips = s_np ? kInterimFlips : kFlipRounds;
+    for (int f = 0; f < nflips; ++f) {
+      ++round;
+      if (tid == 0) s_n2 = 0;
+      __syncthreads();
+      const int n = s_n;
+      if (n == 0) break;
+      for (int k = tid; k < n; k += kOneThreads) {
+        const int t = list[k], c = flip_mark_one(m, t, cl, round);
+        cand[k] = c;
+        if (!c)  // settled
+          atomicAnd(reinterpret_cast<unsigned *>(act) + (t >> 2), ~(1u << (8 * (t & 3))));
+      }
+      __syncthreads();
+      const ActList next{act, list2, &s_n2};
+      for (int k = tid; k < n; k += kOneThreads) {
+        if (!cand[k]) continue;
+        const int t = list[k];
+        list2[atomicAdd(&s_n2, 1)] = t;  // (still marked)
+        flip_apply_one(m, t, cand[k], cl, round, next);
+      }
+      __syncthreads();
+      if (tid == 0) s_n = s_n2;
+      int *u = list;
+      list = list2;
+      list2 = u;
+    }
+    if (tid == 0) s_stop = *reinterpret_cast<volatile int *>(err);
+    __syncthreads();
+    np = s_np;
+    int *u = pend;
+    pend = pend2;
+    pend2 = u;
+    u = start;
+    start = start2;
+    start2 = u;
+    if (s_stop) break;
+    __syncthreads();
   }
+  if (tid == 0) *left = np;
 }
 
 // ---- segments --------------------------------------------------------------
@@ -453,10 +553,8 @@ __global__ void k_seg_mark(Mesh m, const int *__restrict__ segs, int S, int V, i
 // The claimed triangles are listed for the apply pass.  A segment that meets
 // a vertex or a constraint, or crosses more than kCorr edges, goes to the
 // one-thread pass.
-__global__ void k_seg_locate(Mesh m, const int *__restrict__ segs, int base, int W, int *state,
-                             int *list, int *lcnt, Claim *cl, unsigned round) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= W) return;
+__device__ void seg_locate(const Mesh &m, const int *segs, int base, int w, int *state, int *list,
+                           int *lcnt, Claim *cl, unsigned round) {
   const int k = base + w;
   if (state[k] != kSegPending) return;
   const int a = segs[2 * k], b = segs[2 * k + 1];
@@ -483,14 +581,17 @@ __global__ void k_seg_locate(Mesh m, const int *__restrict__ segs, int base, int
   for (int i = 0; i < n; ++i) claim(cl, L[i], pr);
   lcnt[w] = n;
 }
+__global__ void k_seg_locate(Mesh m, const int *__restrict__ segs, int base, int W, int *state,
+                             int *list, int *lcnt, Claim *cl, unsigned round) {
+  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+  if (w < W) seg_locate(m, segs, base, w, state, list, lcnt, cl, round);
+}
 
 // The segments that won every claim are recovered (cdt_core.cuh
 // recover_segment); the others count themselves pending for the next round.
-__global__ void k_seg_apply(Mesh m, const int *__restrict__ segs, int base, int W, int *state,
-                            const int *__restrict__ list, const int *__restrict__ lcnt,
-                            const Claim *cl, unsigned round, int *pending, int *err) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= W) return;
+__device__ void seg_apply(const Mesh &m, const int *segs, int base, int w, int *state,
+                          const int *list, const int *lcnt, const Claim *cl, unsigned round,
+                          int *pending, int *err) {
   const int k = base + w;
   if (state[k] != kSegPending) return;
   const int *L = list + (size_t)w * kClaim;
@@ -505,6 +606,33 @@ __global__ void k_seg_apply(Mesh m, const int *__restrict__ segs, int base, int 
   if (r == cdt::kSegCrosses) atomicOr(err, kErrSegment);
   else if (r != cdt::kSegOk) atomicOr(err, kErrSegLimit);
   state[k] = kSegDone;
+}
+__global__ void k_seg_apply(Mesh m, const int *__restrict__ segs, int base, int W, int *state,
+                            const int *__restrict__ list, const int *__restrict__ lcnt,
+                            const Claim *cl, unsigned round, int *pending, int *err) {
+  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+  if (w < W) seg_apply(m, segs, base, w, state, list, lcnt, cl, round, pending, err);
+}
+
+// Every segment round in one block, for up to kOneBlock segments (7 rounds of two
+// launches and a read-back: 0.42 ms for 832, 0.23 this way).
+__global__ void __launch_bounds__(kOneThreads) k_seg_all(Mesh m, const int *__restrict__ segs,
+                                                         int S, int *state, int *list, int *lcnt,
+                                                         Claim *cl, unsigned round, int rounds,
+                                                         int *err) {
+  __shared__ int s_pending;
+  for (int r = 0; r < rounds; ++r) {
+    ++round;
+    if (threadIdx.x == 0) s_pending = 0;
+    for (int w = threadIdx.x; w < S; w += kOneThreads)
+      seg_locate(m, segs, 0, w, state, list, lcnt, cl, round);
+    __syncthreads();
+    for (int w = threadIdx.x; w < S; w += kOneThreads)
+      seg_apply(m, segs, 0, w, state, list, lcnt, cl, round, &s_pending, err);
+    __syncthreads();
+    if (s_pending == 0) break;
+    __syncthreads();
+  }
 }
 
 // The segments left to one thread, one after the other (they may share
@@ -756,10 +884,22 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
       CCK(cudaGetLastError());
       return flip_rounds(kInterimFlips);
     };
-    // kInsertPoll rounds (lists 1 -> 2 -> 1 ...) per read-back
-    CCK(cudaMemcpyAsync(ctr + 4, &C, sizeof(int), cudaMemcpyHostToDevice, s));
     int np = C;
-    for (int r = 0; r < kInsertRounds && np > 0; r += kInsertPoll) {
+    if (C <= kOneBlock) {
+      int *la = sc.take<int>((size_t)cap_t), *lb = sc.take<int>((size_t)cap_t);
+      if (!la || !lb) return GCVT_ERR_ALLOC;
+      k_insert_all<<<1, kOneThreads, 0, s>>>(m, pend, start, pend2, start2, C, loc, cl, round,
+                                             kInsertRounds, ctr + 1, cap_t, done, act, la, lb, cand,
+                                             ctr + 4, ctr);
+      CCK(cudaGetLastError());
+      round += (1 + kInterimFlips) * kInsertRounds + kFlipRounds;
+      if ((rc = pull())) return rc;
+      np = h[0] ? 0 : h[4];
+    } else {
+      CCK(cudaMemcpyAsync(ctr + 4, &C, sizeof(int), cudaMemcpyHostToDevice, s));
+    }
+    // kInsertPoll rounds (lists 1 -> 2 -> 1 ...) per read-back
+    for (int r = 0; C > kOneBlock && r < kInsertRounds && np > 0; r += kInsertPoll) {
       for (int k = 0; k < kInsertPoll && rc == GCVT_OK; k += 2) {
         rc = ins_round(pend, start, pend2, start2, ctr + 4, ctr + 6);
         if (rc == GCVT_OK) rc = ins_round(pend2, start2, pend, start, ctr + 6, ctr + 4);
@@ -785,7 +925,13 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
     if (!state || !lcnt || !list || !queue || !stack) return GCVT_ERR_ALLOC;
     k_seg_mark<<<nblk(S, 256), 256, 0, s>>>(m, segs, S, (int)V, state, ctr);
     CCK(cudaGetLastError());
-    for (int base = 0; base < S; base += kSegWindow) {
+    if (S <= kOneBlock) {
+      k_seg_all<<<1, kOneThreads, 0, s>>>(m, segs, S, state, list, lcnt, cl, round, kSegRounds,
+                                          ctr);
+      CCK(cudaGetLastError());
+      round += kSegRounds;
+    }
+    for (int base = 0; S > kOneBlock && base < S; base += kSegWindow) {
       const int W = S - base < kSegWindow ? S - base : kSegWindow;
       for (int r = 0; r < kSegRounds; ++r) {
         ++round;

@@ -288,26 +288,32 @@ CDT_HD bool hull_prev(const Mesh &m, int t, int i, int max_steps, int *ot, int *
   return false;
 }
 
-// p outside the hull, seeing the m boundary edges (et[k], ei[k]), k = 0 .. m-1
-// in counter-clockwise hull order (edge k runs u_k -> w_k = u_{k+1}): the
-// new triangles slots[k] = (w_k, u_k, p), each facing its hull edge's
-// triangle and its fan neighbours; their outer edges (u_0, p) and
-// (p, w_{m-1}) are the new hull.
-CDT_HD void insert_out(const Mesh &m, const int *et, const int *ei, int cnt, int p,
-                       const int *slots) {
+// p outside the hull, seeing cnt boundary edges, edge(k) = (t << 2) | i, in
+// counter-clockwise hull order (edge k runs u_k -> w_k = u_{k+1}): the new
+// triangles slot(k) = (w_k, u_k, p), each facing its hull edge's triangle and its fan
+// neighbours; their outer edges (u_0, p) and (p, w_{cnt-1}) are the new hull.
+template <class Edge, class Slot>
+CDT_HD void insert_fan(const Mesh &m, const Edge &edge, int cnt, int p, const Slot &slot) {
   for (int k = 0; k < cnt; ++k) {
-    const int t = et[k], i = ei[k];
+    const int e = edge(k), t = nb_tri(e), i = nb_idx(e);
     const int u = m.tri[3 * t + nx3(i)], w = m.tri[3 * t + pv3(i)];
-    const int s = slots[k];
+    const int s = slot(k);
     set_tri(m, s, w, u, p);
     m.cons[s] = 0;
-    link(m, s, 2, pack_nb(t, i));
-    m.nbr[3 * s] = k == 0 ? kNone : pack_nb(slots[k - 1], 1);
-    m.nbr[3 * s + 1] = k + 1 == cnt ? kNone : pack_nb(slots[k + 1], 0);
+    link(m, s, 2, e);
+    m.nbr[3 * s] = k == 0 ? kNone : pack_nb(slot(k - 1), 1);
+    m.nbr[3 * s + 1] = k + 1 == cnt ? kNone : pack_nb(slot(k + 1), 0);
     m.vt[u] = s;
     m.vt[w] = s;
   }
-  m.vt[p] = slots[0];
+  m.vt[p] = slot(0);
+}
+
+// The same with the edges (et[k], ei[k]) and the triangles slots[k] in arrays.
+CDT_HD void insert_out(const Mesh &m, const int *et, const int *ei, int cnt, int p,
+                       const int *slots) {
+  insert_fan(
+      m, [=](int k) { return pack_nb(et[k], ei[k]); }, cnt, p, [=](int k) { return slots[k]; });
 }
 
 // Flip the edge opposite vertex i of t (a = apex, edge (b, c)) with the

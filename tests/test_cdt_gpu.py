@@ -190,3 +190,23 @@ def test_cdt_of_too_few_points_is_empty(gcvt_lib, cuda_device):
     tri, detail = ctx.cdt(1.0, 0.0, 0.0, np.zeros((0, 2)), np.zeros((0, 2), np.int32))
     assert len(tri) == 0 and detail == 0
     ctx.close()
+
+
+@pytest.mark.parametrize("count", [4096, 4600])
+def test_cdt_round_forms(gcvt_lib, cuda_device, count):
+    """Up to 4096 points (segments) the rounds run in one block, above it as kernels
+    over the grid: points at random, segments from their own triangulation (so none
+    cross), a site here and there on the way of one."""
+    from scipy.spatial import Delaunay
+    ctx, sp = loaded(gcvt_lib, 512, 700, 76)
+    F = len(sp)
+    rng = np.random.default_rng(count)
+    c = rng.uniform(20, 490, (count, 2))
+    t = Delaunay(c).simplices
+    e = np.unique(np.sort(np.concatenate([t[:, [0, 1]], t[:, [1, 2]], t[:, [2, 0]]]), 1), axis=0)
+    segs = F + e[rng.permutation(len(e))[:count]]
+    tri, detail = ctx.cdt(1.0, 0.0, 0.0, c, segs)
+    pts, R, _ = exact_points(ctx, 512, c, 1.0, 0.0, 0.0)
+    info = D.check_cdt(pts, tri, segs, R.tolist())
+    assert detail == 0 and info["vertices"] == F + count and info["constraints"] >= len(segs)
+    ctx.close()
