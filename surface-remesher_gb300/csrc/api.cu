@@ -10,6 +10,7 @@
 #include "gcvt_internal.cuh"
 #include "../../include/gcvt_gb300.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -80,7 +81,8 @@ struct gcvt_ctx {
   cudaGraphExec_t chunk_exec = nullptr;  // kChunk iterations of one level
   int chunk_n = 0;
   int chunk_level = -1;
-  bool chunk_warp = false;  // captured one site per warp
+  bool chunk_warp = false;  // captured one site per warp, for this many sites
+  int chunk_sites = 0;
 };
 
 namespace {
@@ -130,6 +132,7 @@ LevelBufs level_bufs(gcvt_ctx *c, int n, int level) {
   if (warp_cells(c)) {
     b.sitev = c->sitev;
     b.gcnt = c->gcnt;
+    b.few = c->sites <= kFewSites ? std::max(c->sites, 1) : 0;
   }
   if (c->learning && level == 0) {
     for (int k = 0; k < 3; ++k) {
@@ -160,7 +163,8 @@ int push_state(gcvt_ctx *c) {
 // gets plain launches.
 int enqueue_chunk(gcvt_ctx *c, int n, int level) {
   if (c->chunk_exec &&
-      (c->chunk_n != n || c->chunk_level != level || c->chunk_warp != warp_cells(c))) {
+      (c->chunk_n != n || c->chunk_level != level || c->chunk_warp != warp_cells(c) ||
+       (c->chunk_warp && c->chunk_sites != c->sites))) {
     cudaGraphExecDestroy(c->chunk_exec);
     c->chunk_exec = nullptr;
   }
@@ -169,15 +173,13 @@ int enqueue_chunk(gcvt_ctx *c, int n, int level) {
     if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       cudaGetLastError();
       for (int i = 0; i < kChunk; ++i) {
-        CK(launch_list(b, 1, c->stream));
-        CK(launch_cells(b, 0, nullptr, c->stream, c->cell_grid));
+        CK(launch_iteration(b, c->stream, c->cell_grid));
       }
       return GCVT_OK;
     }
     cudaError_t le = cudaSuccess;
     for (int i = 0; i < kChunk && le == cudaSuccess; ++i) {
-      le = launch_list(b, 1, c->stream);
-      if (le == cudaSuccess) le = launch_cells(b, 0, nullptr, c->stream, c->cell_grid);
+      le = launch_iteration(b, c->stream, c->cell_grid);
     }
     cudaGraph_t g = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(c->stream, &g);
@@ -194,6 +196,7 @@ int enqueue_chunk(gcvt_ctx *c, int n, int level) {
     c->chunk_n = n;
     c->chunk_level = level;
     c->chunk_warp = warp_cells(c);
+    c->chunk_sites = c->sites;
   }
   CK(cudaGraphLaunch(c->chunk_exec, c->stream));
   return GCVT_OK;
@@ -861,8 +864,7 @@ int gcvt_ctx_autotune(gcvt_ctx *c, gcvt_tuning *out) {
   if (!rc) {
     const LevelBufs lb = level_bufs(c, n, 0);
     for (int it = 0; it < 16 && !rc; ++it)
-      if (launch_list(lb, 1, c->stream) != cudaSuccess ||
-          launch_cells(lb, 0, nullptr, c->stream) != cudaSuccess)
+      if (launch_iteration(lb, c->stream) != cudaSuccess)
         rc = GCVT_ERR_CUDA;
   }
   if (!rc) rc = pull_state(c);
@@ -895,8 +897,7 @@ int gcvt_ctx_autotune(gcvt_ctx *c, gcvt_tuning *out) {
       float ms = 0.f;
       for (int it = 0; it < 4 && !rc; ++it) {
         if (it == 1 && cudaEventRecord(e0, c->stream) != cudaSuccess) rc = GCVT_ERR_CUDA;
-        if (launch_list(lb, 1, c->stream) != cudaSuccess ||
-            launch_cells(lb, 0, nullptr, c->stream, grid) != cudaSuccess)
+        if (launch_iteration(lb, c->stream, grid) != cudaSuccess)
           rc = GCVT_ERR_CUDA;
       }
       if (!rc && (cudaEventRecord(e1, c->stream) != cudaSuccess ||
@@ -1127,8 +1128,7 @@ int gcvt_ctx_iterate_learned(gcvt_ctx *c, int iterations, int jump_every, int *t
   for (;;) {
     for (int r = 0; r < per_poll; ++r) {
       for (int i = 0; i + 1 < jump_every; ++i) {
-        CK(launch_list(b, 1, c->stream));
-        CK(launch_cells(b, 0, nullptr, c->stream, c->cell_grid));
+        CK(launch_iteration(b, c->stream, c->cell_grid));
       }
       if ((rc = enqueue_jump(c))) return rc;
     }
@@ -1300,8 +1300,7 @@ int gcvt_ctx_time_kernels(gcvt_ctx *c, int iterations, float *ms3) {
   for (int it = 0; it < iterations && status == GCVT_OK; ++it) {
     float ms0 = 0.f, ms1 = 0.f;
     if (cudaEventRecord(ev[0], c->stream) != cudaSuccess ||
-        launch_list(b, 1, c->stream) != cudaSuccess ||
-        launch_cells(b, 0, nullptr, c->stream, c->cell_grid) != cudaSuccess ||
+        launch_iteration(b, c->stream, c->cell_grid) != cudaSuccess ||
         cudaEventRecord(ev[1], c->stream) != cudaSuccess ||
         launch_label(b, c->stream) != cudaSuccess ||
         cudaEventRecord(ev[2], c->stream) != cudaSuccess ||

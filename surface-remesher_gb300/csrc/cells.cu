@@ -1428,6 +1428,33 @@ __device__ void cell_sums_warp(const LevelBufs &a, const uint64_t *__restrict__ 
   if (lane == 0) ws.r2 = r2;
 }
 
+// The end of an iteration of few groups, from the groups' totals gt (visible to this
+// warp): group_tail's reduction of the slots and of their totals.
+template <int MODE>
+__device__ __forceinline__ void few_slots(const LevelBufs &a, const IterView &v, const float4 *gt,
+                                          int lane) {
+  float th = 0.f, tl = 0.f;  // lane k: slot k's total
+  unsigned tr2 = 0, tmv = 0;
+  for (unsigned sb = 0, k = 0; sb < v.ngroups; sb += kGroupsPerSlot, ++k) {
+    float eh = 0.f, el = 0.f;
+    unsigned r2 = 0, mv = 0;
+    for (unsigned i = lane; i < min((unsigned)kGroupsPerSlot, v.ngroups - sb); i += 32) {
+      const float4 q = gt == a.gslot ? __ldcg(gt + sb + i) : gt[sb + i];
+      dfa(eh, el, q.x, q.y);
+      r2 = max(r2, __float_as_uint(q.z));
+      mv = max(mv, __float_as_uint(q.w));
+    }
+    warp_reduce(eh, el, r2, mv);
+    tr2 = max(tr2, r2), tmv = max(tmv, mv);
+    if (lane == (int)k) dfa(th, tl, eh, el);
+  }
+  warp_reduce(th, tl, tr2, tmv);
+  if (lane == 0) {
+    const double E = ((double)th + (double)tl) * a.st->energy_scale;
+    pass_done<MODE>(a.st, E, tr2, tmv, a.n, v.cur);
+  }
+}
+
 // The energy reduction after group g of the block kernel below: group_tail's
 // sums in the same order, but with one counter (the groups are few), so the
 // warp finishing the last group reduces every slot.
@@ -1444,26 +1471,54 @@ __device__ __forceinline__ void few_groups_tail(const LevelBufs &a, const IterVi
   }
   if (!__shfl_sync(0xffffffffu, last, 0)) return;
   __threadfence();
-  float th = 0.f, tl = 0.f;  // lane k: slot k's total
-  unsigned tr2 = 0, tmv = 0;
-  for (unsigned sb = 0, k = 0; sb < v.ngroups; sb += kGroupsPerSlot, ++k) {
-    eh = el = 0.f;
-    r2 = mv = 0;
-    for (unsigned i = lane; i < min((unsigned)kGroupsPerSlot, v.ngroups - sb); i += 32) {
-      const float4 q = __ldcg(a.gslot + sb + i);
-      dfa(eh, el, q.x, q.y);
-      r2 = max(r2, __float_as_uint(q.z));
-      mv = max(mv, __float_as_uint(q.w));
-    }
-    warp_reduce(eh, el, r2, mv);
-    tr2 = max(tr2, r2), tmv = max(tmv, mv);
-    if (lane == (int)k) dfa(th, tl, eh, el);
+  few_slots<MODE>(a, v, a.gslot, lane);
+}
+
+// The sums of the block's sites, folded by one warp: lane 4 s + q takes sum q of
+// site s; lane s (and s + 8 ...) gets site s's.
+__device__ __forceinline__ CellSums fold_block(const WarpScratch *scratch, int count, int lane) {
+  const int s = lane >> 2, q = lane & 3;
+  float ah = 0.f, al = 0.f;
+  if (s < count) {
+    const WarpScratch &ws = scratch[s];
+    const int m = ws.m;
+    if (m < 0) ah = ws.sum[q], al = ws.sum[4 + q];
+#pragma unroll 4
+    for (int k = 0; k < m; ++k) dfa(ah, al, ws.ent[k][q], ws.ent[k][4 + q]);
   }
-  warp_reduce(th, tl, tr2, tmv);
-  if (lane == 0) {
-    const double E = ((double)th + (double)tl) * st->energy_scale;
-    pass_done<MODE>(st, E, tr2, tmv, a.n, v.cur);
+  CellSums cs;
+  const int src = (lane & 7) * 4;
+  constexpr unsigned kFull = 0xffffffffu;
+  cs.wh = __shfl_sync(kFull, ah, src), cs.wl = __shfl_sync(kFull, al, src);
+  cs.xh = __shfl_sync(kFull, ah, src + 1), cs.xl = __shfl_sync(kFull, al, src + 1);
+  cs.yh = __shfl_sync(kFull, ah, src + 2), cs.yl = __shfl_sync(kFull, al, src + 2);
+  cs.eh = __shfl_sync(kFull, ah, src + 3), cs.el = __shfl_sync(kFull, al, src + 3);
+  return cs;
+}
+
+__device__ __forceinline__ void site_values(const LevelBufs &a, const IterView &v, unsigned g,
+                                            int lane, float &eh, float &el, unsigned &r2,
+                                            unsigned &mv) {
+  eh = el = 0.f, r2 = mv = 0;
+  if (g < v.ngroups && g * 32 + lane < (unsigned)v.nsites) {
+    const float4 t = __ldcg(a.sitev + g * 32 + lane);
+    eh = t.x, el = t.y, r2 = __float_as_uint(t.z), mv = __float_as_uint(t.w);
   }
+}
+
+// After a block wrote `count` of group g's site values: if they were the group's
+// last, the group's values, lane l site l's.
+__device__ __forceinline__ bool group_done(const LevelBufs &a, const IterView &v, unsigned g,
+                                           unsigned count, int lane, float &eh, float &el,
+                                           unsigned &r2, unsigned &mv) {
+  const unsigned gsize = min(32u, (unsigned)v.nsites - g * 32);
+  int last = 0;
+  if (lane == 0) last = add_release(a.gcnt + g, count) == gsize - count;
+  if (!__shfl_sync(0xffffffffu, last, 0)) return false;
+  __threadfence();
+  if (lane == 0) a.gcnt[g] = 0u;
+  site_values(a, v, g, lane, eh, el, r2, mv);
+  return true;
 }
 
 // One Lloyd iteration, one listed site per warp, kBlockSites sites per block.
@@ -1511,23 +1566,7 @@ __global__ void __launch_bounds__(32 * kBlockSites, 4) k_cell_warp(LevelBufs a) 
     __syncthreads();
     item = s_item;
     if (warp == 0) {
-      // fold: lane 4 s + q takes sum q of site s
-      const int s = lane >> 2, q = lane & 3;
-      float ah = 0.f, al = 0.f;
-      if (s < count) {
-        const WarpScratch &ws = scratch[s];
-        const int m = ws.m;
-        if (m < 0) ah = ws.sum[q], al = ws.sum[4 + q];
-#pragma unroll 4
-        for (int k = 0; k < m; ++k) dfa(ah, al, ws.ent[k][q], ws.ent[k][4 + q]);
-      }
-      CellSums cs;
-      const int src = (lane & 7) * 4;
-      constexpr unsigned kFull = 0xffffffffu;
-      cs.wh = __shfl_sync(kFull, ah, src), cs.wl = __shfl_sync(kFull, al, src);
-      cs.xh = __shfl_sync(kFull, ah, src + 1), cs.xl = __shfl_sync(kFull, al, src + 1);
-      cs.yh = __shfl_sync(kFull, ah, src + 2), cs.yl = __shfl_sync(kFull, al, src + 2);
-      cs.eh = __shfl_sync(kFull, ah, src + 3), cs.el = __shfl_sync(kFull, al, src + 3);
+      CellSums cs = fold_block(scratch, count, lane);
       const unsigned g = idx0 / 32;  // the block's sites lie in one group
       if (lane < count) {
         cs.r2 = scratch[lane].r2;
@@ -1544,24 +1583,178 @@ __global__ void __launch_bounds__(32 * kBlockSites, 4) k_cell_warp(LevelBufs a) 
             make_float4(eh, el, __uint_as_float((unsigned)cs.r2), __uint_as_float(mv));
       }
       __syncwarp();
-      // the group's last sites: its values in lane order, then the tail
-      const unsigned gsize = min(32u, (unsigned)v.nsites - g * 32);
-      int last = 0;
-      if (lane == 0)
-        last = add_release(a.gcnt + g, (unsigned)count) == gsize - (unsigned)count;
-      if (__shfl_sync(0xffffffffu, last, 0)) {
-        __threadfence();
-        float eh = 0.f, el = 0.f;
-        unsigned r2 = 0, mv = 0;
-        if ((unsigned)lane < gsize) {
-          const float4 t = __ldcg(a.sitev + g * 32 + lane);
-          eh = t.x, el = t.y, r2 = __float_as_uint(t.z), mv = __float_as_uint(t.w);
-        }
-        if (lane == 0) a.gcnt[g] = 0u;
+      float eh, el;
+      unsigned r2, mv;
+      if (group_done(a, v, g, (unsigned)count, lane, eh, el, r2, mv))
         few_groups_tail<MODE>(a, v, g, lane, eh, el, r2, mv);
-      }
     }
     __syncthreads();  // the scratch and s_item are free again
+  }
+}
+
+// The whole iteration of a few sites (up to kFewSites) in one launch, without
+// k_list: a block finds its eight sites from the bitmap and the per-block counts
+// itself (2 to 3 us, every block the same), and the block that arrives last reduces
+// the energy (in the groups' order) and runs the schedule.  Every block arrives
+// exactly once, so none still starts when the state changes.  Such an iteration is
+// latency from end to end (a launch, the list, one cell per warp, the tail), so the
+// launch it saves shows: 50 iterations of 4096 sites of 1024 x 1024 1.30 -> 1.27 ms,
+// with a learned step every fourth 2.15 -> 2.02 ms, a whole 256 x 256 run of about 70
+// 1.47 -> 1.38 ms.
+// Above 8192 sites a block would take several turns at finding its sites; k_list then
+// costs less than they do.
+constexpr int kFewBlocks = 512;  // list blocks at most (grids up to 4096^2)
+
+__global__ void __launch_bounds__(32 * kBlockSites, 4) k_cell_few(LevelBufs a) {
+  __shared__ WarpScratch scratch[kBlockSites];
+  __shared__ unsigned s_pre[kFewBlocks + 1], s_w[kBlockSites];
+  __shared__ uint32_t s_site[kBlockSites];
+  __shared__ bool s_last;
+  constexpr int kThreads = 32 * kBlockSites;
+  static_assert(kListWords == 2 * kThreads && kFewBlocks == 2 * kThreads, "two per thread");
+  static_assert(4 * kBlockSites * sizeof(float4) <= sizeof(scratch), "group totals in scratch");
+  DevState *st = a.st;
+  if (st->stopped) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = a.n;
+  const size_t nwords = (size_t)(n / kBand) * n;
+  const int nlb = (int)((nwords + kListWords - 1) / kListWords);
+  IterView v;
+  v.cur = st->cur;
+  v.nxt_i = v.cur == 2 ? 0 : v.cur + 1;
+  v.bits = bits_at(a, v.cur);
+  v.nxt = bits_at(a, v.nxt_i);
+  v.cnt_nxt = counts_at(a, v.nxt_i);
+  v.omega = st->omega;
+  v.W0 = st->window;
+  v.rb = st->cover;
+  v.slack = st->hint_slack + 1;  // (as in k_cell_warp)
+  if (!st->gate_active) {  // the bitmap and counts the next iteration writes (as k_list)
+    const int z = v.cur == 0 ? 2 : v.cur - 1;
+    uint64_t *zw = bits_at(a, z);
+    unsigned *zc = counts_at(a, z);
+    const size_t t0 = (size_t)blockIdx.x * kThreads + tid, step = (size_t)gridDim.x * kThreads;
+    for (size_t i = t0; i < nwords; i += step) zw[i] = 0ull;
+    for (size_t i = t0; i < (size_t)nlb; i += step) zc[i] = 0u;
+  }
+  // inclusive scan of two values a thread over the block; returns the sum before them
+  auto before = [&](unsigned mine, unsigned &total) {
+    unsigned incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    if (lane == 31) s_w[warp] = incl;
+    __syncthreads();
+    unsigned off = incl - mine;
+    total = 0;
+    for (int k = 0; k < kBlockSites; ++k) {
+      if (k < warp) off += s_w[k];
+      total += s_w[k];
+    }
+    __syncthreads();
+    return off;
+  };
+  {
+    const unsigned *counts = counts_at(a, v.cur);
+    const unsigned c0 = 2 * tid < nlb ? counts[2 * tid] : 0u,
+                   c1 = 2 * tid + 1 < nlb ? counts[2 * tid + 1] : 0u;
+    unsigned total;
+    const unsigned off = before(c0 + c1, total);
+    s_pre[2 * tid] = off;
+    s_pre[2 * tid + 1] = off + c0;
+    if (tid == 0) s_pre[kFewBlocks] = total;
+    __syncthreads();
+  }
+  v.nsites = min((int)s_pre[kFewBlocks], kFewSites);  // (sites are never added)
+  v.ngroups = (unsigned)(v.nsites + 31) / 32;
+  // up to 32 groups: the last block reduces them in one go; more: each group by the
+  // block that completes it (one block alone took 8 us for 128 groups)
+  const bool fold_last = v.ngroups <= 4 * kBlockSites;
+  for (unsigned item = blockIdx.x; item * kBlockSites < (unsigned)v.nsites; item += gridDim.x) {
+    const unsigned idx0 = item * kBlockSites;
+    const int count = min(kBlockSites, v.nsites - (int)idx0);
+    int lb = 0, hi = nlb - 1;  // the list block of site idx0
+    while (lb < hi) {
+      const int mid = (lb + hi + 1) >> 1;
+      if (s_pre[mid] <= idx0) lb = mid;
+      else hi = mid - 1;
+    }
+    for (; lb < nlb && s_pre[lb] < idx0 + count; ++lb) {
+      if (s_pre[lb + 1] == s_pre[lb]) continue;
+      const size_t w0 = (size_t)lb * kListWords + 2 * tid;
+      uint64_t w[2] = {0ull, 0ull};
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (w0 + k < nwords) w[k] = __ldg(v.bits + w0 + k);
+      unsigned total;
+      unsigned idx = s_pre[lb] + before((unsigned)(__popcll(w[0]) + __popcll(w[1])), total) - idx0;
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        for (uint64_t q = w[k]; q; q &= q - 1ull, ++idx)
+          if (idx < (unsigned)count) {  // (idx wraps below idx0)
+            const size_t t = w0 + k;
+            const int b = (int)(t / (unsigned)n);
+            s_site[idx] = (uint32_t)(t % (unsigned)n) |
+                          ((uint32_t)(b * kBand + __ffsll((long long)q) - 1) << 16);
+          }
+    }
+    __syncthreads();
+    if (warp < count) {
+      const uint32_t e = s_site[warp];
+      const int sx = (int)(e & 0x7fffu), sy = (int)(e >> 16);
+      const int h = a.hint[(size_t)sy * n + sx];
+      cell_sums_warp(a, v.bits, n, sx, sy, h ? h : v.W0, v.rb, lane, scratch[warp]);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      CellSums cs = fold_block(scratch, count, lane);
+      if (lane < count) {
+        cs.r2 = scratch[lane].r2;
+        uint32_t e = s_site[lane];
+        const int sx = (int)(e & 0x7fffu), sy = (int)(e >> 16);
+        e |= (uint32_t)((a.fixed_bits[(size_t)(sy / kBand) * n + sx] >> (sy % kBand)) & 1ull) << 15;
+        float eh = 0.f, el = 0.f;
+        dfa(eh, el, cs.eh, cs.el);
+        const unsigned mv = move_site(a, v, e, sx, sy, cs);
+        a.sitev[idx0 + lane] =
+            make_float4(eh, el, __uint_as_float((unsigned)cs.r2), __uint_as_float(mv));
+      }
+      __syncwarp();
+      float eh, el;
+      unsigned r2, mv;
+      const unsigned g = idx0 / 32;
+      if (!fold_last && group_done(a, v, g, (unsigned)count, lane, eh, el, r2, mv)) {
+        warp_reduce(eh, el, r2, mv);
+        if (lane == 0) a.gslot[g] = make_float4(eh, el, __uint_as_float(r2), __uint_as_float(mv));
+      }
+    }
+    __syncthreads();  // the scratch is free again
+  }
+  if (tid == 0) s_last = add_release(&st->done_blocks) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  float4 *gt = reinterpret_cast<float4 *>(scratch);
+  if (fold_last) {  // four groups a warp, their loads in flight together
+    float eh[4], el[4];
+    unsigned r2[4], mv[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      site_values(a, v, warp + k * kBlockSites, lane, eh[k], el[k], r2[k], mv[k]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const unsigned g = warp + k * kBlockSites;
+      if (g >= v.ngroups) break;
+      warp_reduce(eh[k], el[k], r2[k], mv[k]);
+      if (lane == 0)
+        gt[g] = make_float4(eh[k], el[k], __uint_as_float(r2[k]), __uint_as_float(mv[k]));
+    }
+    __syncthreads();
+  }
+  if (warp == 0) {
+    if (lane == 0) st->snap_count = st->list_count = v.nsites;
+    few_slots<0>(a, v, fold_last ? gt : a.gslot, lane);
   }
 }
 
@@ -1983,6 +2176,16 @@ cudaError_t cells_configure() {
       return e;
     perw = perw ? min(perw, per) : per;
   }
+  {
+    int per = 0;
+    if ((e = cudaFuncSetAttribute(k_cell_few, cudaFuncAttributePreferredSharedMemoryCarveout, 70)) !=
+        cudaSuccess)
+      return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cell_few, 32 * kBlockSites, 0)) !=
+        cudaSuccess)
+      return e;
+    perw = min(perw, per);
+  }
   g_warp_grid[dev] = sms * max(1, perw);
   g_cell_grid[dev] = sms * max(1, min(per0, per1));
   return cudaSuccess;
@@ -2015,6 +2218,23 @@ int cells_default_grid() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   return g_cell_grid[dev];
+}
+
+// One plain Lloyd iteration: the site list and the cells, or, for few sites, one
+// launch.
+cudaError_t launch_iteration(const LevelBufs &b, cudaStream_t s, int grid) {
+  if (b.few && b.sitev && list_blocks(b.n) <= (size_t)kFewBlocks) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64 || !g_warp_grid[dev]) return cudaErrorNotReady;
+    int wg = min((b.few + kBlockSites - 1) / kBlockSites, g_warp_grid[dev]);
+    if (grid > 0) wg = min(wg, grid / kBlockSites);
+    k_cell_few<<<max(1, wg), 32 * kBlockSites, 0, s>>>(b);
+    return cudaGetLastError();
+  }
+  const cudaError_t e = launch_list(b, 1, s);
+  return e != cudaSuccess ? e : launch_cells(b, 0, nullptr, s, grid);
 }
 
 // grid: the persistent grid in blocks (0: every block that fits).

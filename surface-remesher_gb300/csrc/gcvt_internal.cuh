@@ -21,6 +21,7 @@ constexpr int kNoneBelow = 32767;   // "no site below"
 constexpr int kBand = 64;           // PBA+ phase-1 band height: n / m1 == 64 for
                                     // every entry of gcvt.cu:842-847
 constexpr int kWarpSites = 32768;  // one site per warp at most for this many sites
+constexpr int kFewSites = 8192;    // one launch per iteration at most for this many sites
 constexpr int kListWords = 512;    // bitmap words per site-list block
 constexpr int kMinN = 256;   // n must be a multiple of 256 (S = n/32 >= 8)
 constexpr int kMaxN = 8192;  // largest grid (the row pass's whole-row buffer: 32 KB)
@@ -118,6 +119,9 @@ struct LevelBufs {
   // done (null: lane-per-site only)
   float4 *sitev;
   unsigned *gcnt;
+  int few;                 // 0, or at least the number of sites, up to kFewSites: a plain
+                           // iteration is one launch (k_cell_few)
+  int pad;
 };
 
 __device__ __forceinline__ const uint64_t *cur_bits(const LevelBufs &a) {
@@ -149,6 +153,7 @@ cudaError_t launch_count(const LevelBufs &b, cudaStream_t s);
 // else one site per lane; MODE 1 and 2 run one site per lane.
 cudaError_t launch_cells(const LevelBufs &b, int moments_only, double *out4, cudaStream_t s,
                          int grid = 0);
+cudaError_t launch_iteration(const LevelBufs &b, cudaStream_t s, int grid = 0);
 int cells_default_grid();
 cudaError_t launch_zoom(const uint64_t *src, int n, uint64_t *dst, cudaStream_t s);
 cudaError_t launch_density_halve(const float *in, float *out, int n_out, cudaStream_t s);

@@ -63,3 +63,28 @@ def test_cells_match_fp64_and_each_other(gcvt_lib, oracle, cuda_device, n, kind)
     assert np.array_equal(runs[0][0], runs[1][0])
     assert runs[0][1] == runs[1][1]
     ctx.close()
+
+
+@pytest.mark.parametrize("n,m", [(256, 0), (256, 1), (256, 7), (256, 9), (512, 1024), (512, 1025),
+                                 (1024, 8185), (1024, 8192), (1024, 8193), (4096, 700),
+                                 (4352, 700)])
+def test_one_launch_iterations(gcvt_lib, cuda_device, n, m):
+    """Few sites' one-launch iterations against the list and the lane-per-site
+    kernel, bit for bit: no site, a part of a block, the group counts around the
+    two ways of folding them, the site and grid limits of the dispatch."""
+    rng = np.random.default_rng(m)
+    rho = gaussian_density(n, 6, 4.0, 0.05, 0.2, 3)
+    p = rng.choice(np.flatnonzero(rho.ravel() > 0), m, replace=False)
+    fixed = np.zeros((n, n), np.uint8)
+    fixed.ravel()[p[::5]] = 1
+    sites = gcvt_lib.sites_from_points(n, p % n, p // n)
+    ctx = gcvt_lib.Context(n)
+    runs = []
+    for mode in (1, 2):
+        ctx.set_tuning(cell_mode=mode)
+        ctx.load(sites, rho, fixed)
+        ctx.iterate(12)
+        runs.append((ctx.sites(), ctx.info()))
+    assert np.array_equal(runs[0][0], runs[1][0])
+    assert runs[0][1] == runs[1][1]
+    ctx.close()
