@@ -22,14 +22,18 @@
 //   e = |c|^2 - 2 c.p + bias  (= |c - p|^2 - |p|^2 + bias),
 // costs one multiply-add per further pixel that uses it; |p|^2 is the same for
 // all nine candidates of p, so (e, x, y) orders them as (distance, x, y) does.
-// A pixel's first candidate initialises its key; the other eight compare.
-// The compare and select of the 64-bit keys (four integer-ALU instructions
-// per candidate) bound the kernels: the integer ALU pipe runs at ~85 %.
+// A pixel's label is the smallest word among the candidates of its smallest e:
+// three-way minima of the nine e, then an equality test and a predicated minimum
+// per candidate.  That is 23 integer-ALU instructions per pixel where comparing and
+// selecting nine 64-bit (e, word) keys took 32.  A step of 4096 x 4096 reads and
+// writes 134 MB (20 us); the ALU pipe (83 % busy) and the issue slots bound it:
+// 52 -> 45 us, the whole labelling 712 -> 618 us.
 //
 //   * k > H/2: k_jfa_step, one launch per step, one unit per thread, every
-//     load and store 128-bit (a warp reads 512 contiguous bytes per row).
+//     load and store 128-bit (a warp reads 512 contiguous bytes per row); k = 2
+//     takes units of 8-byte words, k = 1 k_jfa_step_one.
 //   * H = 0 (the fastest on GB300, as the autotuner finds): every step its
-//     own launch, k_jfa_step down to k = 4, k_jfa_step_small for 2, 1, 1.
+//     own launch.
 //   * H = 8, 16 or 32: k = H/2, ..., 1, 1 in one k_jfa_tail<H> launch.  A
 //     block loads its 64 x 64 tile with an H-pixel halo ((64 + 2H)^2 labels)
 //     into shared memory with one TMA tile copy, runs the steps there on a
@@ -60,17 +64,9 @@ template <int H> constexpr unsigned tail_bytes() {
 __device__ __forceinline__ int lab_x(uint32_t v) { return (int)(int16_t)(v & 0xffffu); }
 __device__ __forceinline__ int lab_y(uint32_t v) { return (int)(int16_t)(v >> 16); }
 
-__device__ __forceinline__ unsigned long long kmin(unsigned long long a, unsigned long long b) {
-  return b < a ? b : a;
-}
-
+__device__ __forceinline__ uint32_t comp(const uint2 &v, int i) { return i == 0 ? v.x : v.y; }
 __device__ __forceinline__ uint32_t comp(const uint4 &v, int i) {
   return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
-}
-
-// the words of four keys, as they are between launches
-__device__ __forceinline__ uint4 words(const unsigned long long (&k)[4]) {
-  return make_uint4((uint32_t)k[0], (uint32_t)k[1], (uint32_t)k[2], (uint32_t)k[3]);
 }
 
 // a word between launches -> the label of the result (MARKER for none)
@@ -85,9 +81,12 @@ __device__ __forceinline__ uint4 final_labels(uint4 v) {
 // The 16 words (r, s) of a unit at column x0 + (s - 1) cs, row y + (r - 1) k;
 // outside the grid kJfaNone.  (A second path without the bounds tests, for
 // units wholly inside the grid, measured slower: it raised the registers.)
+template <typename V>
 __device__ __forceinline__ void unit_load(const uint32_t *__restrict__ in, int n, int x0, int y,
-                                          int k, int cs, uint4 (&w)[4][4]) {
-  const uint4 none = make_uint4(kJfaNone, kJfaNone, kJfaNone, kJfaNone);
+                                          int k, int cs, V (&w)[4][4]) {
+  V none;
+  none.x = none.y = kJfaNone;
+  if constexpr (sizeof(V) == 16) none.z = none.w = kJfaNone;
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int yy = y + (r - 1) * k;
@@ -95,73 +94,139 @@ __device__ __forceinline__ void unit_load(const uint32_t *__restrict__ in, int n
     for (int s = 0; s < 4; ++s) {
       const int xx = x0 + (s - 1) * cs;
       w[r][s] = (yy >= 0 && yy < n && xx >= 0 && xx < n)
-                    ? __ldg(reinterpret_cast<const uint4 *>(in + (size_t)yy * n + xx))
+                    ? __ldg(reinterpret_cast<const V *>(in + (size_t)yy * n + xx))
                     : none;
     }
   }
 }
 
-// The nearest label of each pixel of a unit (see the file comment) among its
-// nine candidates, words (x << 16) | y: best[a][b][i] = (e << 32) | word,
-// smallest first.
-// KS = 0: cs = k, k a multiple of 4 (any value); KS = 1 or 2: k = KS, cs = 4.
-template <int KS>
-__device__ __forceinline__ void unit_best(const uint4 (&w)[4][4], int x0, int y, int k,
-                                          unsigned long long (&best)[2][2][4]) {
-  const unsigned m2x = 0u - 2u * (unsigned)x0, m2y = 0u - 2u * (unsigned)y;
-  const unsigned m2k = 0u - 2u * (unsigned)(KS ? KS : k);
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t c = comp(w[r][s], j);
-        const unsigned cx = c >> 16, cy = c & 0xffffu;
-        // e for the pixel at (x0, y)
-        const unsigned base = cx * cx + cy * cy + kJfaBias + cx * m2x + cy * m2y;
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          if (r - 1 - b < -1 || r - 1 - b > 1) continue;
-          const unsigned eb = b ? base + cy * m2k : base;
-#pragma unroll
-          for (int a = 0; a < 2; ++a)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              unsigned e;
-              bool first;  // the pixel's first candidate in this loop order
-              if (KS == 0) {
-                if (i != j || s - 1 - a < -1 || s - 1 - a > 1) continue;
-                e = eb + cx * (0u - 2u * (unsigned)i) + (a ? cx * m2k : 0u);
-                first = r - 1 - b == -1 && s - 1 - a == -1;
-              } else {
-                const int off = 4 * (s - 1) + j - 4 * a - i;
-                if (off != -KS && off != 0 && off != KS) continue;
-                e = eb + cx * (0u - 2u * (unsigned)(4 * a + i));
-                first = r - 1 - b == -1 && off == -KS;
-              }
-              const unsigned long long key = ((unsigned long long)e << 32) | c;
-              best[a][b][i] = first ? key : kmin(best[a][b][i], key);
-            }
-        }
-      }
+// min of three words below 0x7f800000: as floats they order the same way, and the
+// float minimum has a three-input form.
+__device__ __forceinline__ unsigned min3(unsigned a, unsigned b, unsigned c) {
+  float m;
+  asm("min.f32 %0, %1, %2, %3;"
+      : "=f"(m)
+      : "f"(__uint_as_float(a)), "f"(__uint_as_float(b)), "f"(__uint_as_float(c)));
+  return __float_as_uint(m);
 }
 
-// One step of offset k (a multiple of 4): thread qi of row yi takes the unit
-// with cs = k at x0 = (qi / (k/4)) 2k + 4 (qi % (k/4)), y = (yi / k) 2k + yi % k.
-__global__ void __launch_bounds__(256) k_jfa_step(const uint32_t *__restrict__ in,
-                                                  uint32_t *__restrict__ out, int n, int k) {
-  const int kq = k / 4;
-  const int blocks = (n + 2 * k - 1) / (2 * k);  // k-blocks of even index
-  const int qi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (qi >= blocks * kq) return;
-  const int yi = blockIdx.y;
-  const int x0 = (qi / kq) * 2 * k + (qi % kq) * 4;
-  const int y = (yi / k) * 2 * k + (yi % k);
-  uint4 w[4][4];
+// The smallest word among the candidates of the smallest e (e < 2^30, c <= kJfaNone).
+// Three chains of predicated minima: 618 us a labelling of 4096 x 4096; four chains
+// 627, nine selects and three-way minima of them 641.
+__device__ __forceinline__ uint32_t pick(const unsigned (&e)[9], const uint32_t (&c)[9]) {
+  const unsigned m = min3(min3(e[0], e[1], e[2]), min3(e[3], e[4], e[5]), min3(e[6], e[7], e[8]));
+  uint32_t v[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    v[q] = e[q] == m ? c[q] : 0x7f800000u;
+#pragma unroll
+    for (int r = q + 3; r < 9; r += 3)
+      asm("{ .reg .pred p; setp.eq.u32 p, %1, %2; @p min.u32 %0, %0, %3; }"
+          : "+r"(v[q])
+          : "r"(e[r]), "r"(m), "r"(c[r]));
+  }
+  return min3(v[0], v[1], v[2]);
+}
+
+__device__ __forceinline__ void set_comp(uint2 &v, int i, uint32_t w) {
+  if (i == 0) v.x = w;
+  else v.y = w;
+}
+__device__ __forceinline__ void set_comp(uint4 &v, int i, uint32_t w) {
+  if (i == 0) v.x = w;
+  else if (i == 1) v.y = w;
+  else if (i == 2) v.z = w;
+  else v.w = w;
+}
+
+// The nearest label of each pixel of a unit (see the file comment) among its nine
+// candidates.  V: uint4, or uint2 (KS = 0 only; i < 2).
+// KS = 0: cs = k, a multiple of V's words (any value); KS = 1 or 2: k = KS, cs = 4.
+template <int KS, typename V>
+__device__ __forceinline__ void unit_best(const V (&w)[4][4], int x0, int y, int k,
+                                          V (&best)[2][2]) {
+  const unsigned m2x = 0u - 2u * (unsigned)x0, m2y = 0u - 2u * (unsigned)y;
+  const unsigned m2k = 0u - 2u * (unsigned)(KS ? KS : k), m2yk = m2y + m2k;
+  if constexpr (KS == 0) {
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(V) / 4; ++i) {
+      unsigned u[4][2][3], cy[4][4];
+      const unsigned mx = m2x - 2u * (unsigned)i;
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const uint32_t c = comp(w[r][s], i);
+          const unsigned cx = c >> 16;
+          cy[r][s] = c & 0xffffu;
+          const unsigned e = cx * (cx + mx) + (cy[r][s] * cy[r][s] + kJfaBias);
+          if (s < 3) u[r][0][s] = e;
+          if (s > 0) u[r][1][s - 1] = e + cx * m2k;
+        }
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+          unsigned e[9];
+#pragma unroll
+          for (int q = 0; q < 9; ++q)
+            e[q] = u[b + q / 3][a][q % 3] + cy[b + q / 3][a + q % 3] * (b ? m2yk : m2y);
+          uint32_t c[9];
+#pragma unroll
+          for (int q = 0; q < 9; ++q) c[q] = comp(w[b + q / 3][a + q % 3], i);
+          set_comp(best[b][a], i, pick(e, c));
+        }
+    }
+  } else {
+    // columns x0 - 4 .. x0 + 11: label column l at x0 - 4 + l
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      unsigned e[3][4];
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const int l = 4 + p + (d - 1) * KS;
+          const uint32_t c = comp(w[r][l / 4], l % 4);
+          const unsigned cx = c >> 16, cy = c & 0xffffu;
+          e[d][r] = cx * (cx + m2x - 2u * (unsigned)p) + cy * cy + kJfaBias;
+        }
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        unsigned f[9];
+        uint32_t g[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+          const int l = 4 + p + (q % 3 - 1) * KS;
+          g[q] = comp(w[b + q / 3][l / 4], l % 4);
+          f[q] = e[q % 3][b + q / 3] + (g[q] & 0xffffu) * (b ? m2yk : m2y);
+        }
+        set_comp(best[b][p / 4], p % 4, pick(f, g));
+      }
+    }
+  }
+}
+
+// One step of offset k (a power of two, a multiple of W's words: 16-byte units for
+// k >= 4, 8-byte ones for k = 2): thread qi of row yi takes the unit with cs = k at
+// x0 = (qi / (k/kW)) 2k + kW (qi % (k/kW)), y = (yi / k) 2k + yi % k.  The loads all
+// come first, so the resident warps are what hides them: 96 registers and five blocks
+// of 128 (four: 642 us for the labelling, five: 618); 8-byte units for every step, with
+// 72 registers: 656.
+constexpr int kStepThreads = 128;
+template <typename W>
+__global__ void __launch_bounds__(kStepThreads, sizeof(W) == 16 ? 5 : 7)
+    k_jfa_step(const uint32_t *__restrict__ in, uint32_t *__restrict__ out, int n, int k) {
+  constexpr int kW = (int)sizeof(W) / 4;
+  const int lk = 31 - __clz(k), lq = lk - (kW == 4 ? 2 : 1);  // k is a power of two
+  const int qi = blockIdx.x * blockDim.x + threadIdx.x, yi = blockIdx.y;
+  const int x0 = (qi >> lq << (lk + 1)) + (qi & ((1 << lq) - 1)) * kW;
+  if (x0 >= n) return;
+  const int y = (yi >> lk << (lk + 1)) + (yi & (k - 1));
+  W w[4][4];
   unit_load(in, n, x0, y, k, k, w);
-  unsigned long long best[2][2][4];
-  unit_best<0>(w, x0, y, k, best);
+  W best[2][2];
+  unit_best<0, W>(w, x0, y, k, best);
 #pragma unroll
   for (int b = 0; b < 2; ++b) {
     const int py = y + b * k;
@@ -170,31 +235,29 @@ __global__ void __launch_bounds__(256) k_jfa_step(const uint32_t *__restrict__ i
     for (int a = 0; a < 2; ++a) {
       const int px = x0 + a * k;
       if (px >= n) continue;
-      *reinterpret_cast<uint4 *>(out + (size_t)py * n + px) = words(best[a][b]);
+      *reinterpret_cast<W *>(out + (size_t)py * n + px) = best[b][a];
     }
   }
 }
 
-// A step of offset KS = 2 or 1 (on the last step, "no label" becomes MARKER):
-// thread qi of row pair yi takes the unit with cs = 4 at x0 = 8 qi,
-// y = (yi / KS) 2 KS + yi % KS.
-template <int KS, bool LAST>
-__global__ void __launch_bounds__(256) k_jfa_step_small(const uint32_t *__restrict__ in,
-                                                        uint32_t *__restrict__ out, int n) {
+// A step of offset 1 (on the last step, "no label" becomes MARKER): thread qi of row
+// pair yi takes the unit with cs = 4 at x0 = 8 qi, y = 2 yi.
+template <bool LAST>
+__global__ void __launch_bounds__(kStepThreads, 4)
+    k_jfa_step_one(const uint32_t *__restrict__ in, uint32_t *__restrict__ out, int n) {
   const int qi = blockIdx.x * blockDim.x + threadIdx.x;
   if (qi >= n / 8) return;
-  const int yi = blockIdx.y;
-  const int x0 = 8 * qi, y = (yi / KS) * 2 * KS + yi % KS;
+  const int x0 = 8 * qi, y = 2 * blockIdx.y;
   uint4 w[4][4];
-  unit_load(in, n, x0, y, KS, 4, w);
-  unsigned long long best[2][2][4];
-  unit_best<KS>(w, x0, y, KS, best);
+  unit_load(in, n, x0, y, 1, 4, w);
+  uint4 best[2][2];
+  unit_best<1, uint4>(w, x0, y, 1, best);
 #pragma unroll
   for (int b = 0; b < 2; ++b)
 #pragma unroll
     for (int a = 0; a < 2; ++a) {
-      const uint4 v = words(best[a][b]);
-      *reinterpret_cast<uint4 *>(out + (size_t)(y + b * KS) * n + x0 + 4 * a) =
+      const uint4 v = best[b][a];
+      *reinterpret_cast<uint4 *>(out + (size_t)(y + b) * n + x0 + 4 * a) =
           LAST ? final_labels(v) : v;
     }
 }
@@ -233,14 +296,14 @@ __device__ __forceinline__ void tail_step(const uint32_t *__restrict__ cur,
 #pragma unroll
       for (int s = 0; s < 4; ++s)
         w[r][s] = *reinterpret_cast<const uint4 *>(cur + (y + (r - 1) * K) * R + x0 + (s - 1) * CS);
-    unsigned long long best[2][2][4];
-    unit_best<KS>(w, ox + x0, oy + y, K, best);
+    uint4 best[2][2];
+    unit_best<KS, uint4>(w, ox + x0, oy + y, K, best);
 #pragma unroll
     for (int b = 0; b < 2; ++b)
 #pragma unroll
       for (int a = 0; a < 2; ++a) {
         const int row = y + b * K, col = x0 + a * CS;
-        uint4 v = words(best[a][b]);
+        uint4 v = best[b][a];
         if (!inner) {
           const int gy = oy + row, gx = ox + col;
           const bool rin = gy >= 0 && gy < n;
@@ -420,20 +483,21 @@ cudaError_t launch_jfa(uint32_t *a, uint32_t *b, int n, int *err, uint32_t **res
   uint32_t *in = a, *out = b;
   int k = 1;
   while (2 * k <= n / 2) k *= 2;  // the largest power of two <= n/2
-  for (; k > (tail_halo ? tail_halo / 2 : 2); k /= 2) {
-    const int blocks = (n + 2 * k - 1) / (2 * k);
-    const dim3 grid((unsigned)((blocks * (k / 4) + 255) / 256), (unsigned)(blocks * k));
-    k_jfa_step<<<grid, 256, 0, s>>>(in, out, n, k);
+  for (; k > (tail_halo ? tail_halo / 2 : 1); k /= 2) {
+    const int blocks = (n + 2 * k - 1) / (2 * k), per = k >= 4 ? 4 : 2;
+    const dim3 grid((unsigned)((blocks * (k / per) + kStepThreads - 1) / kStepThreads),
+                    (unsigned)(blocks * k));
+    if (per == 4) k_jfa_step<uint4><<<grid, kStepThreads, 0, s>>>(in, out, n, k);
+    else k_jfa_step<uint2><<<grid, kStepThreads, 0, s>>>(in, out, n, k);
     uint32_t *t = in;
     in = out;
     out = t;
   }
-  if (!tail_halo) {  // k = 2, 1 and the extra 1
-    const dim3 grid((unsigned)((n / 8 + 255) / 256), (unsigned)(n / 2));
-    k_jfa_step_small<2, false><<<grid, 256, 0, s>>>(in, out, n);
-    k_jfa_step_small<1, false><<<grid, 256, 0, s>>>(out, in, n);
-    k_jfa_step_small<1, true><<<grid, 256, 0, s>>>(in, out, n);
-    *result = out;
+  if (!tail_halo) {  // k = 1 and the extra 1
+    const dim3 grid((unsigned)((n / 8 + kStepThreads - 1) / kStepThreads), (unsigned)(n / 2));
+    k_jfa_step_one<false><<<grid, kStepThreads, 0, s>>>(in, out, n);
+    k_jfa_step_one<true><<<grid, kStepThreads, 0, s>>>(out, in, n);
+    *result = in;
     return cudaGetLastError();
   }
   if (tail_halo == 8) e = launch_tail<8>(in, out, n, err, s);

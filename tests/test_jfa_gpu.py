@@ -100,3 +100,22 @@ def test_jfa_error_on_clustered_sites(gcvt_lib, cuda_device):
     assert np.array_equal(got, jfa_numpy(sites))
     assert far < 0.01 * px
     ctx.close()
+
+
+@pytest.mark.parametrize("halo", [0, 16])
+@pytest.mark.parametrize("n,kind", [(256, "lattice"), (512, "diagonal"), (768, "lattice"),
+                                    (2048, "corner"), (512, "full")])
+def test_ties_and_distances(gcvt_lib, cuda_device, halo, n, kind):
+    # several candidates at the smallest distance (lattices: up to four sites), a
+    # single site far from almost every pixel, a site on every pixel
+    ys, xs = np.mgrid[0:n, 0:n]
+    put = {"lattice": (xs % 8 == 3) & (ys % 8 == 5), "diagonal": (xs + ys) % 16 == 0,
+           "corner": (xs == n - 1) & (ys == n - 1), "full": xs >= 0}[kind]
+    sites = np.full((n, n, 2), MARKER, np.int16)
+    sites[put, 0], sites[put, 1] = xs[put], ys[put]
+    ctx = gcvt_lib.Context(n)
+    ctx.load(sites, np.ones((n, n), np.float32), np.zeros((n, n), np.uint8))
+    ctx.set_tuning(jfa_tail_halo=halo)
+    got, _ = ctx.jfa_label()
+    assert np.array_equal(got, jfa_numpy(sites))
+    ctx.close()
