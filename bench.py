@@ -18,8 +18,8 @@ Metric: Gpix-pass/s = n^2 x labelling passes / second, 101 passes per step
   e2e   : the same through the C ABI with pinned host buffers: host->device
           copies of sites, density and mask and the device->host copy of the
           label grid inside every timed step.
-  roofline: one Lloyd iteration, the launch pair k_list + k_cell<0> (89.5 % +
-          3.9 % of the run's device time): algorithmic bytes per iteration /
+  roofline: one Lloyd iteration, the launch pair k_list + k_cell<0> (most of
+          the run's device time): algorithmic bytes per iteration /
           its mean duration over iterations 2-100 of the timed steps (CUDA
           events on the launching stream around them) against the measured
           HBM copy bandwidth.
@@ -64,8 +64,8 @@ def metric_of(workload, n, nsites, iters=ITERS):
 UNIT = "Gpix-pass/s"
 # Algorithmic bytes of one Lloyd iteration (k_list + k_cell<0>): the density
 # once over its row support (4 B per support pixel: every such pixel belongs
-# to exactly one cell); the current site bitmap read by k_list and the bitmap
-# two iterations ahead cleared by k_cell (1/8 B per pixel each); per site its
+# to exactly one cell); the current site bitmap read and the bitmap
+# two iterations ahead cleared by k_list (1/8 B per pixel each); per site its
 # list entry written and read (4 + 4 B), its word of the fixed-site bitmap
 # read and its bit OR-ed into the next bitmap (8 + 8 B).
 ALG_BYTES_PER_SUPPORT_PX = 4.0
@@ -74,12 +74,12 @@ ALG_BYTES_PER_SITE = 24.0
 # dram__bytes_read.sum + dram__bytes_write.sum of k_list + k_cell<0> for one
 # iteration of this workload (iteration 31 of a graph-replayed run, warm L2),
 # from the ncu capture summarised in profiles/cell_kernel_plain_4096.md:
-# k_list 789,248 + 264,448, k_cell 13,910,784 + 6,594,304 bytes.
-NCU_TRAFFIC_BYTES = 21558784
+# k_list 983,040 + 647,424, k_cell 23,058,176 + 14,166,784 bytes.
+NCU_TRAFFIC_BYTES = 38855424
 # the same capture on the 8192^2 / 1,048,576-site workload (iteration 31,
-# profiles/cell_kernel_plain_8192.md): k_list 13,138,176 + 3,403,520, k_cell
-# 265,760,256 + 77,200,896 bytes
-NCU_TRAFFIC = {"plain_4096": NCU_TRAFFIC_BYTES, "plain_8192": 359502848, "plain_1024": None}
+# profiles/cell_kernel_plain_8192.md): k_list 13,178,112 + 4,192,768, k_cell
+# 260,119,552 + 60,122,624 bytes
+NCU_TRAFFIC = {"plain_4096": NCU_TRAFFIC_BYTES, "plain_8192": 337613056, "plain_1024": None}
 
 
 def support_pixels(rho):
@@ -452,6 +452,7 @@ def run_ours(args):
         ctx.load(d_sites, d_rho, d_mask)
         ctx.iterate(3)
         tuning = ctx.autotune()
+        one_launch = nsites <= 8192 and n <= 4096 and tuning["cell_mode"] != 1  # k_cell_few
         for _ in range(args.warmup):
             step_device()
         with ClockSampler(local) as clk:
@@ -506,18 +507,21 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": NCU_TRAFFIC.get(workload),
                      "peak_source": peak_kind,
-                     "kernel": "k_list + k_cell<0> (one Lloyd iteration, iterations 2-100)",
+                     "kernel": "%s (one Lloyd iteration, iterations 2-%d)" % (
+                         "k_cell_few" if one_launch else "k_list + k_cell<0>", iters),
                      "algorithmic_bytes": alg},
         "e2e": {"value": e2e, "unit": UNIT,
                 "h2d_bytes_per_step": int(h_sites.numel() * 2 + h_rho.numel() * 4 + h_mask.numel()),
                 "d2h_bytes_per_step": int(h_out.numel() * 2),
                 "ms_per_step": t_e2e / args.steps * 1e3},
         # per step: load (row support, fixed bitmap, site bitmap); level
-        # start (column summaries, rows, k_cover, k_cover_finish, k_count);
-        # iterate(1) and iterate(ITERS - 1) as graphs of ten (k_list, k_cell)
-        # pairs, launches past the last iteration returning at once; final
-        # labelling (column summaries, rows)
-        "gpu_launches": args.steps * (3 + 5 + 2 * 10 * (1 + (iters - 1 + 9) // 10) + 2),
+        # start (six label launches, k_cover, k_cover_finish, k_count);
+        # iterate(1) and iterate(ITERS - 1) as graphs of ten iterations (k_list
+        # and k_cell, or k_cell_few alone), launches past the last iteration
+        # returning at once; final labelling (tile summaries, tiles, far blocks,
+        # and the row pass's three kernels, which return at once)
+        "gpu_launches": args.steps * (3 + 9 + (1 if one_launch else 2) * 10 *
+                                      (1 + (iters - 1 + 9) // 10) + 6),
         "clocks": clk.summary(),
         "final_energy": info["energy"],
     }

@@ -50,8 +50,8 @@
 // their pixels two rows at a time in packed FP32.  What bounds it: issue slots
 // and the latency of L1 misses, not bandwidth (60 MB an iteration).  Against
 // integer bounds row pair by row pair and scalar sums: 118 -> 81 us an
-// iteration at 4096^2 / 262,144 sites (75.5 -> 46.2 M warp instructions), 0.42
-// -> 0.28 ms at 8192^2.  Records of 8 bytes in shared memory (4 KB a warp) took
+// iteration at 4096^2 / 262,144 sites (75.5 -> 45.1 M warp instructions), 0.42
+// -> 0.26 ms at 8192^2.  Records of 8 bytes in shared memory (4 KB a warp) took
 // 120 us: they leave the density rows too little L1.  The energy is reduced in a fixed order
 // whatever warp takes which group: the sites of a group by a butterfly, 64
 // groups by the warp finishing the last of them, the 64-group totals by the
@@ -1598,9 +1598,9 @@ __global__ void __launch_bounds__(32 * kBlockSites, 4) k_cell_warp(LevelBufs a) 
 // the energy (in the groups' order) and runs the schedule.  Every block arrives
 // exactly once, so none still starts when the state changes.  Such an iteration is
 // latency from end to end (a launch, the list, one cell per warp, the tail), so the
-// launch it saves shows: 50 iterations of 4096 sites of 1024 x 1024 1.30 -> 1.27 ms,
-// with a learned step every fourth 2.15 -> 2.02 ms, a whole 256 x 256 run of about 70
-// 1.47 -> 1.38 ms.
+// launch it saves shows: 50 iterations of 4096 sites of 1024 x 1024 1.31 -> 1.25 ms,
+// with a learned step every fourth 2.11 -> 2.00 ms, a whole 256 x 256 run of about 70
+// 1.65 -> 1.46 ms.
 // Above 8192 sites a block would take several turns at finding its sites; k_list then
 // costs less than they do.
 constexpr int kFewBlocks = 512;  // list blocks at most (grids up to 4096^2)
