@@ -141,12 +141,13 @@ inline cudaError_t launch_jfa_seed(const uint64_t *bits, int n, uint32_t *grid, 
   return launch_bits_to_grid(bits, n, grid, s, kJfaNone, true);
 }
 // The exact labels of the current sites into b.labels (label_tiles.cu); the row
-// pass behind it (column summaries, rows) runs where DevState::label_ovf says so.
+// pass (column summaries, rows) does small grids (always) and those where
+// DevState::label_ovf says so.
 cudaError_t launch_label(const LevelBufs &b, cudaStream_t s);
 size_t label_blocks(int n);  // entries of LevelBufs::open_tiles (::occ: 4 per row of blocks)
-cudaError_t launch_summary(const LevelBufs &b, cudaStream_t s);
+cudaError_t launch_summary(const LevelBufs &b, bool always, cudaStream_t s);
 cudaError_t launch_fixed_bits(const uint8_t *mask, int n, uint64_t *fixed_bits, cudaStream_t s);
-cudaError_t launch_rows(const LevelBufs &b, cudaStream_t s);
+cudaError_t launch_rows(const LevelBufs &b, bool always, cudaStream_t s);
 cudaError_t launch_list(const LevelBufs &b, int respect_stop, cudaStream_t s);
 cudaError_t launch_count(const LevelBufs &b, cudaStream_t s);
 // MODE 0, 4 and 5 run one site per warp when b.sitev and b.gcnt are set,

@@ -22,7 +22,8 @@
 //     over the occupied 64 x 64 blocks, gathers the sites that can own any of its
 //     pixels by the same test, and prunes that list for each of its open tiles.
 //   * what does not fit its lists (a block crowded with sites) sets
-//     DevState::label_ovf, and the row pass (labeller.cu) does the whole grid.
+//     DevState::label_ovf, and the row pass (labeller.cu) does the whole grid, as it
+//     does for grids up to 512 x 512.
 //
 // What bounds it is issue slots: half of a CVT tile's warp instructions are its 15
 // candidates x 256 pixels.  The row pass this replaces spent 330 per row and 32
@@ -395,15 +396,24 @@ __global__ void __launch_bounds__(kFarThreads) k_label_far(LevelBufs a) {
 
 size_t label_blocks(int n) { return (size_t)(n / kBand) * (n / kBand); }
 
+// Up to 512 x 512 the row pass labels: three launches instead of six (the tiles' three
+// and the row pass's, which then look at label_ovf), and both are latency there.  A
+// labelling call took, rows / tiles: 37 / 51 us at 256 x 256, 50 / 57 at 512 x 512, 92 /
+// 75 at 1024 x 1024.
+constexpr int kRowLabels = 512;
+
 cudaError_t launch_label(const LevelBufs &b, cudaStream_t s) {
   const unsigned M = (unsigned)(b.n / kBand);
-  k_label_occ<<<M, 1024, 0, s>>>(b);
-  k_label_tiles<<<dim3((unsigned)b.n / (kT * kTileWarps), (unsigned)b.n / kT), 32 * kTileWarps, 0,
-                  s>>>(b);
-  k_label_far<<<dim3(M, M), kFarThreads, 0, s>>>(b);
-  // the row pass, where the lists overflowed
-  cudaError_t e = launch_summary(b, s);
-  if (e == cudaSuccess) e = launch_rows(b, s);
+  const bool rows = b.n <= kRowLabels;
+  if (!rows) {
+    k_label_occ<<<M, 1024, 0, s>>>(b);
+    k_label_tiles<<<dim3((unsigned)b.n / (kT * kTileWarps), (unsigned)b.n / kT), 32 * kTileWarps,
+                    0, s>>>(b);
+    k_label_far<<<dim3(M, M), kFarThreads, 0, s>>>(b);
+  }
+  // the row pass, always or where the lists overflowed
+  cudaError_t e = launch_summary(b, rows, s);
+  if (e == cudaSuccess) e = launch_rows(b, rows, s);
   return e == cudaSuccess ? cudaGetLastError() : e;
 }
 

@@ -30,8 +30,8 @@
 //     lanes write the row's label words from the hull's breakpoints.  A row
 //     whose survivors do not fit the buffer is flagged and redone by
 //     k_rows_full with a whole-row buffer: the smaller buffer lets 2.5 times
-//     the rows share an SM.  label_tiles.cu labels ahead of this pass, which does the
-//     whole grid when that one's lists overflow (DevState::label_ovf).
+//     the rows share an SM.  Above 512 x 512 label_tiles.cu labels, and this pass
+//     does the whole grid only when that one's lists overflow (DevState::label_ovf).
 #include "gcvt_internal.cuh"
 
 namespace cvtgb {
@@ -104,8 +104,8 @@ cudaError_t launch_bits_to_grid(const uint64_t *bits, int n, uint32_t *grid, cud
 // One block per 32-column group: 32 columns x 32 band groups, each thread
 // owning ceil(nb/32) consecutive bands.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_summary(LevelBufs a) {
-  if (!a.st->label_ovf) return;
+__global__ void __launch_bounds__(1024) k_summary(LevelBufs a, bool always) {
+  if (!always && !a.st->label_ovf) return;
   __shared__ int sLast[32][33];
   __shared__ int sFirst[32][33];
   const int n = a.n, nb = n / kBand;
@@ -141,9 +141,9 @@ __global__ void __launch_bounds__(1024) k_summary(LevelBufs a) {
   }
 }
 
-cudaError_t launch_summary(const LevelBufs &b, cudaStream_t s) {
+cudaError_t launch_summary(const LevelBufs &b, bool always, cudaStream_t s) {
   dim3 blk(32, 32), grd(b.n / 32);
-  k_summary<<<grd, blk, 0, s>>>(b);
+  k_summary<<<grd, blk, 0, s>>>(b, always);
   return cudaGetLastError();
 }
 
@@ -350,9 +350,9 @@ __device__ void write_row(uint32_t *out, int n, int r, const int *C, int K) {
 // whole-row buffer.
 constexpr int row_cap(int n) { return n * 2 / 5; }
 
-__global__ void __launch_bounds__(32) k_rows(LevelBufs a) {
+__global__ void __launch_bounds__(32) k_rows(LevelBufs a, bool always) {
   extern __shared__ __align__(16) int smem[];
-  if (!a.st->label_ovf) return;
+  if (!always && !a.st->label_ovf) return;
   const int n = a.n, r = blockIdx.x;
   if (r >= n) return;
   const int K = row_hull(a, r, smem, row_cap(n));
@@ -365,9 +365,9 @@ __global__ void __launch_bounds__(32) k_rows(LevelBufs a) {
 
 // The flagged rows, with a whole-row buffer (a grid of a few blocks per SM
 // striding over the rows); clears their flags.
-__global__ void __launch_bounds__(32) k_rows_full(LevelBufs a) {
+__global__ void __launch_bounds__(32) k_rows_full(LevelBufs a, bool always) {
   extern __shared__ __align__(16) int smem[];
-  if (!a.st->label_ovf) return;
+  if (!always && !a.st->label_ovf) return;
   const int n = a.n;
   for (int r = blockIdx.x; r < n; r += gridDim.x) {
     if (!((a.st->row_ovf[r >> 5] >> (r & 31)) & 1u)) continue;
@@ -385,9 +385,9 @@ cudaError_t rows_configure() {
                               (int)rows_smem_bytes(kMaxN));
 }
 
-cudaError_t launch_rows(const LevelBufs &b, cudaStream_t s) {
-  k_rows<<<b.n, 32, rows_smem_bytes(row_cap(b.n)), s>>>(b);
-  k_rows_full<<<b.n < 304 ? b.n : 304, 32, rows_smem_bytes(b.n), s>>>(b);
+cudaError_t launch_rows(const LevelBufs &b, bool always, cudaStream_t s) {
+  k_rows<<<b.n, 32, rows_smem_bytes(row_cap(b.n)), s>>>(b, always);
+  k_rows_full<<<b.n < 304 ? b.n : 304, 32, rows_smem_bytes(b.n), s>>>(b, always);
   return cudaGetLastError();
 }
 

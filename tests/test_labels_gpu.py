@@ -85,11 +85,12 @@ def test_context_label_device_buffers(gcvt_lib, oracle, cuda_device):
 
 
 @pytest.mark.parametrize("n,kind", [(512, "1"), (512, "2"), (768, "3"), (512, "5"), (512, "18"),
-                                    (1024, "mirror"), (768, "far"), (2048, "one"), (256, "one")])
+                                    (1024, "mirror"), (768, "far"), (2048, "one"), (256, "one"),
+                                    (768, "1"), (768, "2"), (768, "5"), (768, "18")])
 def test_tile_lists_and_their_overflows(gcvt_lib, oracle, cuda_device, n, kind):
     """The tile labeller's dispatch: a crowded block of one site per 1 to 18 pixels
     beside empty space (window, candidate and block lists at and past their ends,
-    tiles far from any site, the row pass behind them), mirror pairs across bands seen
+    tiles far from any site, the row pass behind them and on grids up to 512), mirror pairs across bands seen
     from near and far, lone sites."""
     rng = np.random.default_rng(n)
     if kind == "mirror":  # pairs of one column about band edges and tile rows, far apart
