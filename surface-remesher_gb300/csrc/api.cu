@@ -126,6 +126,7 @@ LevelBufs level_bufs(gcvt_ctx *c, int n, int level) {
   b.list = c->list;
   for (int k = 0; k < 3; ++k) b.counts[k] = c->counts[k];
   b.hint = c->hint;
+  b.sites = c->sites;
   b.gslot = c->gslot;
   b.sslot = c->sslot;
   b.scnt = c->scnt;

@@ -121,7 +121,7 @@ struct LevelBufs {
   unsigned *gcnt;
   int few;                 // 0, or at least the number of sites, up to kFewSites: a plain
                            // iteration is one launch (k_cell_few)
-  int pad;
+  int sites;               // the sites, 0: not known (the labeller's choice of path)
 };
 
 __device__ __forceinline__ const uint64_t *cur_bits(const LevelBufs &a) {

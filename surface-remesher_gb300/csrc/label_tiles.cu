@@ -23,7 +23,7 @@
 //     pixels by the same test, and prunes that list for each of its open tiles.
 //   * what does not fit its lists (a block crowded with sites) sets
 //     DevState::label_ovf, and the row pass (labeller.cu) does the whole grid, as it
-//     does for grids up to 512 x 512.
+//     does for grids up to 512 x 512 and for crowded ones.
 //
 // What bounds it is issue slots: half of a CVT tile's warp instructions are its 15
 // candidates x 256 pixels.  The row pass this replaces spent 330 per row and 32
@@ -399,12 +399,15 @@ size_t label_blocks(int n) { return (size_t)(n / kBand) * (n / kBand); }
 // Up to 512 x 512 the row pass labels: three launches instead of six (the tiles' three
 // and the row pass's, which then look at label_ovf), and both are latency there.  A
 // labelling call took, rows / tiles: 37 / 51 us at 256 x 256, 50 / 57 at 512 x 512, 92 /
-// 75 at 1024 x 1024.
+// 75 at 1024 x 1024.  So it does where the sites crowd the tiles' lists (fewer than 16
+// pixels a site): 2048 x 2048 of 16 pixels a site 190 / 104 us, of 11 595 / 706, the row
+// pass having to follow the tiles.
 constexpr int kRowLabels = 512;
+constexpr long long kRowCrowd = 16;
 
 cudaError_t launch_label(const LevelBufs &b, cudaStream_t s) {
   const unsigned M = (unsigned)(b.n / kBand);
-  const bool rows = b.n <= kRowLabels;
+  const bool rows = b.n <= kRowLabels || kRowCrowd * b.sites > (long long)b.n * b.n;
   if (!rows) {
     k_label_occ<<<M, 1024, 0, s>>>(b);
     k_label_tiles<<<dim3((unsigned)b.n / (kT * kTileWarps), (unsigned)b.n / kT), 32 * kTileWarps,
