@@ -395,15 +395,18 @@ __global__ void k_ins_apply(Mesh m, const int *__restrict__ pend, const int *npp
 // flip (its index + 1, 0: none); the flip claims both triangles and the four outer
 // neighbours with the priority of 3 t + i.
 __device__ __forceinline__ int flip_mark_one(const Mesh &m, int t, Claim *cl, unsigned round) {
-  int c = 0;
-  for (int i = 0; i < 3; ++i) {
+  int c = 0, d[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {  // (the three apexes' loads together)
     const int nb = m.nbr[3 * t + i];
-    if (nb < 0 || cdt::nb_tri(nb) < t) continue;
-    if (cdt::wants_flip(m, t, i)) {
-      c = i + 1;
-      break;
-    }
+    d[i] = nb < 0 || cdt::nb_tri(nb) < t || ((m.cons[t] >> i) & 1)
+               ? -1
+               : m.tri[3 * cdt::nb_tri(nb) + cdt::nb_idx(nb)];
   }
+#pragma unroll
+  for (int i = 2; i >= 0; --i)  // the first that wants a flip
+    if (d[i] >= 0 && cdt::incircle(m, m.tri[3 * t], m.tri[3 * t + 1], m.tri[3 * t + 2], d[i]))
+      c = i + 1;
   if (!c) return 0;
   const int i = c - 1;
   const Claim pr = claim_of(round, (unsigned)(3 * t + i));
@@ -451,7 +454,7 @@ __global__ void k_flip_apply(Mesh m, const int *ntri, const int *cand, const Cla
 // Every insertion round with its flip rounds in one block, for up to kOneBlock
 // points: the rounds are chains of short dependent steps (832 boundary points take 28
 // rounds; as seven launches each 74 us a round, 55 in one block of 1024 threads, 85 in
-// one of 256), and the changed triangles are listed instead of searched for.  Block
+// one of 256; 46 since the predicates are short), and the changed triangles are listed instead of searched for.  Block
 // barriers order the steps.  After the last point the flips run until none is left.
 constexpr int kOneBlock = 4096;
 constexpr int kOneThreads = 1024;

