@@ -290,39 +290,51 @@ __global__ void k_ins_locate(Mesh m, const int *__restrict__ pend, const int *np
 __device__ __forceinline__ bool owns(const Mesh &m, const Claim *cl, int t, Claim pr) {
   return cl[t] == pr;
 }
-__device__ bool owns_nbrs(const Mesh &m, const Claim *cl, int t, Claim pr) {
-  if (!owns(m, cl, t, pr)) return false;
+// (every claim is read whatever the others say: the loads are in flight together)
+__device__ __forceinline__ bool owns_nbrs(const Mesh &m, const Claim *cl, int t, Claim pr) {
+  bool ok = owns(m, cl, t, pr);
+#pragma unroll
   for (int i = 0; i < 3; ++i) {
     const int nb = m.nbr[3 * t + i];
-    if (nb >= 0 && !owns(m, cl, cdt::nb_tri(nb), pr)) return false;
+    ok &= owns(m, cl, nb >= 0 ? cdt::nb_tri(nb) : t, pr);
   }
-  return true;
+  return ok;
 }
 
 // What to do with a triangle that changed: it and its neighbours are tested by
 // the next flip round.  An edge whose opposite vertices changed belongs to a
 // changed triangle, so it is tested from whichever of its triangles has the smaller
-// index.  Act marks them in a byte each; ActList also lists each once.
+// index.  Act marks them in a byte each; ActList also lists each once (the four
+// marks of a triangle and its neighbours are set before the first answer is needed).
 struct Act {
   uint8_t *act;
-  __device__ __forceinline__ void add(int t) const { act[t] = 1; }
+  __device__ __forceinline__ void add(const int (&t)[4]) const {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) act[t[k]] = 1;
+  }
 };
 struct ActList {
   uint8_t *act;
   int *list, *count;
-  __device__ __forceinline__ void add(int t) const {
-    const unsigned bit = 1u << (8 * (t & 3));
-    if (!(atomicOr(reinterpret_cast<unsigned *>(act) + (t >> 2), bit) & bit))
-      list[atomicAdd(count, 1)] = t;
+  __device__ __forceinline__ void add(const int (&t)[4]) const {
+    unsigned was[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      was[k] = atomicOr(reinterpret_cast<unsigned *>(act) + (t[k] >> 2), 1u << (8 * (t[k] & 3)));
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (!((was[k] >> (8 * (t[k] & 3))) & 1u)) list[atomicAdd(count, 1)] = t[k];
   }
 };
 template <class A>
 __device__ __forceinline__ void touch(const Mesh &m, const A &act, int t) {
-  act.add(t);
+  int id[4] = {t, t, t, t};
+#pragma unroll
   for (int i = 0; i < 3; ++i) {
     const int nb = m.nbr[3 * t + i];
-    if (nb >= 0) act.add(cdt::nb_tri(nb));
+    if (nb >= 0) id[i + 1] = cdt::nb_tri(nb);
   }
+  act.add(id);
 }
 
 // Insert pending point q if it won every claim; otherwise it stays pending (its
@@ -423,7 +435,8 @@ __device__ __forceinline__ bool flip_apply_one(const Mesh &m, int t, int c, cons
   const int i = c - 1;
   const Claim pr = claim_of(round, (unsigned)(3 * t + i));
   const int t2 = cdt::nb_tri(m.nbr[3 * t + i]);
-  if (!owns_nbrs(m, cl, t, pr) || !owns_nbrs(m, cl, t2, pr)) return false;
+  const bool first = owns_nbrs(m, cl, t, pr), second = owns_nbrs(m, cl, t2, pr);
+  if (!first || !second) return false;
   cdt::flip(m, t, i);
   touch(m, act, t);
   touch(m, act, t2);
@@ -454,7 +467,8 @@ __global__ void k_flip_apply(Mesh m, const int *ntri, const int *cand, const Cla
 // Every insertion round with its flip rounds in one block, for up to kOneBlock
 // points: the rounds are chains of short dependent steps (832 boundary points take 28
 // rounds; as seven launches each 74 us a round, 55 in one block of 1024 threads, 85 in
-// one of 256; 46 since the predicates are short), and the changed triangles are listed instead of searched for.  Block
+// one of 256; 36 with short predicates and the loads and marks of a triangle's
+// neighbours in flight together), and the changed triangles are listed instead of searched for.  Block
 // barriers order the steps.  After the last point the flips run until none is left.
 constexpr int kOneBlock = 4096;
 constexpr int kOneThreads = 1024;
