@@ -468,8 +468,9 @@ __global__ void k_flip_apply(Mesh m, const int *ntri, const int *cand, const Cla
 // points: the rounds are chains of short dependent steps (832 boundary points take 28
 // rounds; as seven launches each 74 us a round, 55 in one block of 1024 threads, 85 in
 // one of 256; 36 with short predicates and the loads and marks of a triangle's
-// neighbours in flight together), and the changed triangles are listed instead of searched for.  Block
-// barriers order the steps.  After the last point the flips run until none is left.
+// neighbours in flight together), and the changed triangles are listed instead of
+// searched for.  Block barriers order the steps.  After the last point the flips run
+// until none is left.
 constexpr int kOneBlock = 4096;
 constexpr int kOneThreads = 1024;
 
@@ -658,16 +659,24 @@ __global__ void __launch_bounds__(kOneThreads) k_seg_all(Mesh m, const int *__re
 // triangulations split such segments).  Crossing segments set err.
 __global__ void k_segments(Mesh m, const int *__restrict__ segs, int S, const int *state,
                            int *queue, int *stack, int *err) {
-  // (usually none: the block looks first, one thread walking the list took 70 us)
-  bool any = false;
-  for (int k = threadIdx.x; k < S; k += blockDim.x) any = any || state[k] != kSegDone;
-  if (!__syncthreads_or(any) || threadIdx.x != 0) return;
-  for (int k = 0; k < S; ++k) {
-    if (state[k] == kSegDone) continue;
-    const int a = segs[2 * k], b = segs[2 * k + 1];
-    const int r = cdt::recover_chain(m, a, b, queue, kSegQueue, stack, kSegStack, kWalk);
-    if (r == cdt::kSegCrosses) atomicOr(err, kErrSegment);
-    else if (r != cdt::kSegOk) atomicOr(err, kErrSegLimit);
+  // (usually few or none: the block finds them; one thread walking the list took 50 us
+  // more of 832 segments)
+  __shared__ unsigned s_left[32];
+  for (int base = 0; base < S; base += blockDim.x) {
+    const int j = base + threadIdx.x;
+    const unsigned left = __ballot_sync(0xffffffffu, j < S && state[j] != kSegDone);
+    if ((threadIdx.x & 31) == 0) s_left[threadIdx.x >> 5] = left;
+    if (!__syncthreads_or(left != 0)) continue;
+    if (threadIdx.x == 0)
+      for (int g = 0; g < (int)blockDim.x / 32; ++g)
+        for (unsigned q = s_left[g]; q; q &= q - 1u) {
+          const int k = base + 32 * g + __ffs((int)q) - 1;
+          const int a = segs[2 * k], b = segs[2 * k + 1];
+          const int r = cdt::recover_chain(m, a, b, queue, kSegQueue, stack, kSegStack, kWalk);
+          if (r == cdt::kSegCrosses) atomicOr(err, kErrSegment);
+          else if (r != cdt::kSegOk) atomicOr(err, kErrSegLimit);
+        }
+    __syncthreads();
   }
 }
 
