@@ -210,3 +210,22 @@ def test_cdt_round_forms(gcvt_lib, cuda_device, count):
     info = D.check_cdt(pts, tri, segs, R.tolist())
     assert detail == 0 and info["vertices"] == F + count and info["constraints"] >= len(segs)
     ctx.close()
+
+
+@pytest.mark.parametrize("n,m,seed", [(256, 40, 78), (512, 300, 79)])
+def test_cdt_of_points_at_the_coordinate_limit(gcvt_lib, cuda_device, n, m, seed):
+    """Constraint points up to 2^14 pixels from the origin on every side (differences of
+    2^30 units: the widest operands of the 64-bit and 128-bit predicates), exactly
+    co-circular ones among them."""
+    ctx, sp = loaded(gcvt_lib, n, m, seed)
+    rng = np.random.default_rng(seed)
+    lim = 16384.0 - 2.0 ** -15
+    ring = [(s * lim * x, t * lim * y) for s in (1, -1) for t in (1, -1)
+            for x, y in ((1.0, 1.0), (0.5, 0.25), (0.25, 0.5))]
+    c = np.concatenate([np.array(ring), rng.uniform(-lim, lim, (24, 2)),
+                        rng.uniform(5, n - 5, (12, 2)) // 1 + 0.5])
+    tri, detail = ctx.cdt(1.0, 0.0, 0.0, c, np.zeros((0, 2), np.int32))
+    pts, R, F = exact_points(ctx, n, c, 1.0, 0.0, 0.0)
+    info = D.check_cdt(pts, tri, np.zeros((0, 2), np.int64), R.tolist())
+    assert detail == 0 and info["vertices"] == F + len(c)
+    ctx.close()
