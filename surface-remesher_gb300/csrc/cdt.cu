@@ -614,11 +614,13 @@ __device__ void seg_apply(const Mesh &m, const int *segs, int base, int w, int *
   if (state[k] != kSegPending) return;
   const int *L = list + (size_t)w * kClaim;
   const Claim pr = claim_of(round, (unsigned)k);
-  for (int i = 0, n = lcnt[w]; i < n; ++i)
-    if (cl[L[i]] != pr) {
-      atomicAdd(pending, 1);
-      return;
-    }
+  bool own = true;  // (no early exit: the loads are in flight together)
+#pragma unroll 8
+  for (int i = 0, n = lcnt[w]; i < n; ++i) own &= cl[L[i]] == pr;
+  if (!own) {
+    atomicAdd(pending, 1);
+    return;
+  }
   int q[2 * kCorr], on = -1;
   const int r = cdt::recover_segment(m, segs[2 * k], segs[2 * k + 1], q, kCorr, kWalk, &on);
   if (r == cdt::kSegCrosses) atomicOr(err, kErrSegment);
@@ -633,7 +635,7 @@ __global__ void k_seg_apply(Mesh m, const int *__restrict__ segs, int base, int 
 }
 
 // Every segment round in one block, for up to kOneBlock segments (7 rounds of two
-// launches and a read-back: 0.42 ms for 832, 0.23 this way).
+// launches and a read-back: 0.42 ms for 832, 0.19 this way).
 __global__ void __launch_bounds__(kOneThreads) k_seg_all(Mesh m, const int *__restrict__ segs,
                                                          int S, int *state, int *list, int *lcnt,
                                                          Claim *cl, unsigned round, int rounds,
