@@ -422,9 +422,10 @@ __device__ __forceinline__ int flip_mark_one(const Mesh &m, int t, Claim *cl, un
   if (!c) return 0;
   const int i = c - 1;
   const Claim pr = claim_of(round, (unsigned)(3 * t + i));
-  const int t2 = cdt::nb_tri(m.nbr[3 * t + i]);
-  claim_nbrs(m, cl, t, pr);
-  claim_nbrs(m, cl, t2, pr);
+  int id[8];
+  cdt::flip_claims(m, t, i, id);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) claim(cl, id[k], pr);
   return c;
 }
 
@@ -434,12 +435,15 @@ __device__ __forceinline__ bool flip_apply_one(const Mesh &m, int t, int c, cons
                                                unsigned round, const A &act) {
   const int i = c - 1;
   const Claim pr = claim_of(round, (unsigned)(3 * t + i));
-  const int t2 = cdt::nb_tri(m.nbr[3 * t + i]);
-  const bool first = owns_nbrs(m, cl, t, pr), second = owns_nbrs(m, cl, t2, pr);
-  if (!first || !second) return false;
+  int id[8];
+  cdt::flip_claims(m, t, i, id);
+  bool own = true;  // (no early exit: the loads are in flight together)
+#pragma unroll
+  for (int k = 0; k < 8; ++k) own &= owns(m, cl, id[k], pr);
+  if (!own) return false;
   cdt::flip(m, t, i);
   touch(m, act, t);
-  touch(m, act, t2);
+  touch(m, act, id[4]);
   return true;
 }
 

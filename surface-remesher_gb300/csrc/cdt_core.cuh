@@ -362,6 +362,23 @@ CDT_HD void flip(const Mesh &m, int t, int i) {
   m.vt[c] = t2;
 }
 
+// The triangles a flip of the edge opposite vertex i of t claims: t, the triangle
+// across that edge and the neighbours of both (t again where there is none).  A flip
+// that has lost t reads them while the winner rewrites t: the edge may be a hull edge
+// by then, so a missing neighbour counts here too.  It has lost whatever it reads; one
+// that owns t reads what it claimed, since nobody else writes t's links.
+CDT_HD void flip_claims(const Mesh &m, int t, int i, int (&id)[8]) {
+  const int opp = m.nbr[3 * t + i], t2 = opp >= 0 ? nb_tri(opp) : t;
+  for (int h = 0; h < 2; ++h) {
+    const int c = h ? t2 : t;
+    id[4 * h] = c;
+    for (int k = 0; k < 3; ++k) {
+      const int nb = m.nbr[3 * c + k];
+      id[4 * h + 1 + k] = nb >= 0 ? nb_tri(nb) : c;
+    }
+  }
+}
+
 // Should the edge opposite vertex i of t be flipped for the Delaunay
 // property (it has a neighbour, is not a constraint, and the neighbour's
 // apex is inside t's circle)?
