@@ -440,6 +440,19 @@ __device__ bool wwrap(WStar &st, const uint64_t *bits, const uint64_t *fixed, in
       }
       wins(st, 0, u);
     }
+    if (st.m == 1) {
+      // nothing on either side: every candidate lies on one line through the site,
+      // and the nearest one beyond the site is its other neighbour
+      const int ux = pdx(u0), uy = pdy(u0);
+      const unsigned oa = ax * ux + ay * uy < 0 ? (unsigned)a2 : 0xffffffffu,
+                     ob = bx * ux + by * uy < 0 ? (unsigned)b2 : 0xffffffffu;
+      const unsigned o = __reduce_min_sync(kFull, min(oa, ob));
+      const unsigned ma = __ballot_sync(kFull, oa == o), mb = __ballot_sync(kFull, ob == o);
+      if (o != 0xffffffffu) {
+        wset(st, 1, ma ? __shfl_sync(kFull, qa, __ffs(ma) - 1) : __shfl_sync(kFull, qb, __ffs(mb) - 1));
+        st.m = 2;
+      }
+    }
   }
   // the list starts with the smallest angle from the +x axis
   m = st.m;

@@ -229,3 +229,20 @@ def test_cdt_of_points_at_the_coordinate_limit(gcvt_lib, cuda_device, n, m, seed
     info = D.check_cdt(pts, tri, np.zeros((0, 2), np.int64), R.tolist())
     assert detail == 0 and info["vertices"] == F + len(c)
     ctx.close()
+
+
+@pytest.mark.parametrize("dx,dy", [(2, 32), (32, 2)])
+def test_cdt_on_a_lattice_of_lines(gcvt_lib, cuda_device, dx, dy):
+    """Sites whose first windows hold one line through the site only."""
+    n = 256
+    q = np.stack(np.meshgrid(np.arange(0, n, dx), np.arange(0, n, dy)), -1).reshape(-1, 2)
+    ctx = gcvt_lib.Context(n)
+    ctx.load(gcvt_lib.sites_from_points(n, q[:, 0], q[:, 1]), np.ones((n, n), np.float32),
+             np.zeros((n, n), np.uint8))
+    c = np.array([(40.25, 60.5), (210.75, 190.125), (100.5, 33.0), (280.0, 120.5)])
+    segs = np.array([(len(q), len(q) + 1), (len(q) + 1, len(q) + 3)])
+    tri, detail = ctx.cdt(1.0, 0.0, 0.0, c, segs)
+    pts, R, F = exact_points(ctx, n, c, 1.0, 0.0, 0.0)
+    info = D.check_cdt(pts, tri, segs, R.tolist())
+    assert detail == 0 and info["vertices"] == F + len(c)
+    ctx.close()

@@ -222,3 +222,48 @@ def test_star_paths_by_spacing(gcvt_lib, cuda_device, n, step, jitter, count):
     pts, tris = _triangulate(gcvt_lib, _grid(n, q.tolist()))
     info = dorc.check(pts, tris)
     assert info["triangles"] == len(tris) > 0
+
+
+def _lattice(n, dx, dy):
+    return np.stack(np.meshgrid(np.arange(0, n, dx), np.arange(0, n, dy)), -1).reshape(-1, 2)
+
+
+def _collinear_set(kind, n):
+    if kind == "row":
+        return np.stack([np.arange(n), np.full(n, n // 3)], 1)
+    if kind.startswith("diagonal"):  # diagonals `step` rows apart, a site every `every` columns
+        every, step = (int(v) for v in kind[8:].split(","))
+        x = np.arange(0, n, every)
+        q = np.concatenate([np.stack([x, x + k * step], 1) for k in range(-n // step, n // step + 1)])
+        return q[(q[:, 1] >= 0) & (q[:, 1] < n)]
+    dx, dy = (int(v) for v in kind.split(","))
+    return _lattice(n, dx, dy)
+
+
+@pytest.mark.parametrize("kind,n", [("1,16", 256), ("16,1", 256), ("2,32", 256), ("32,2", 256),
+                                    ("3,40", 256), ("40,3", 256), ("2,24", 256), ("4,64", 512),
+                                    ("5,60", 512), ("8,128", 1024), ("128,8", 1024),
+                                    ("diagonal1,24", 256), ("diagonal2,40", 256),
+                                    ("diagonal3,66", 512),
+                                    ("row", 256), ("row", 1024)])
+def test_collinear_windows(gcvt_lib, cuda_device, kind, n):
+    """Sites whose first windows hold one line through the site only: structured
+    lattices, diagonals, a single row."""
+    q = _collinear_set(kind, n)
+    pts, tris = _triangulate(gcvt_lib, _grid(n, q.tolist()))
+    if kind == "row":
+        assert len(tris) == 0
+        return
+    info = dorc.check(pts, tris)
+    assert info["triangles"] == len(tris) > 0 and info["vertices"] == len(q)
+
+
+@pytest.mark.parametrize("dx,dy,cols,rows", [(1, 16, 26, 3), (2, 32, 24, 3), (32, 2, 3, 24),
+                                             (3, 40, 25, 3)])
+def test_collinear_windows_perturbed(gcvt_lib, cuda_device, dx, dy, cols, rows):
+    """A few rows of such a lattice: the very triangles of the perturbation."""
+    q = _lattice(256, dx, dy)
+    q = q[(q[:, 0] < cols * dx) & (q[:, 1] < rows * dy)]
+    got_pts, tris = _triangulate(gcvt_lib, _grid(256, q.tolist()))
+    want = dorc.sos_triangulation(got_pts, 256)
+    assert dorc.canonical(tris) == [tuple(r) for r in want.tolist()]
