@@ -789,12 +789,14 @@ __device__ __forceinline__ int wnext(const WStar &s, int k) {
 // window again.  More than 64 candidates are inserted ring by ring instead of
 // wrapped.  (kWindow 1.6 to 2.3 and kGrow 1.5 to 2 measure within 5 %, kWiden 3 or
 // never 8 % slower on irregular sites.)  Returns false when the star
-// overflowed.
-constexpr float kWindow = 2.0f, kGrow = 1.7f;
+// overflowed, which depends on the order of the insertions too: `rings` inserts the
+// windows of 1.4, 2.8, 5.6 ... spacings ring by ring, nearer sites first.
+constexpr float kWindow = 2.0f, kGrow = 1.7f, kRing = 1.4f;
 constexpr int kWiden = 1;
 constexpr int kBoxCols = 96, kBoxBands = 3;  // largest disc box scanned directly
 __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixed, int n, int sx,
-                           int sy, const Pyr &py, const TileSites &ts, unsigned *stk) {
+                           int sy, const Pyr &py, const TileSites &ts, unsigned *stk,
+                           bool rings) {
   st.a = st.b = 0;
   st.m = 0;
   st.overflow = false;
@@ -804,10 +806,11 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
   const bool tile = lane < 9 && ti >= 0 && ti < nt0 && tj >= 0 && tj < nt0;
   const unsigned cnt = __reduce_add_sync(kFull, tile ? ts.count[brick_of(ti, tj, nt0)] : 0u);
   const int tiles = __popc(__ballot_sync(kFull, tile));
-  int W = (int)ceilf(kWindow * sqrtf((float)(tiles * kTile * kTile) / (float)max(cnt, 1u)));
+  int W = (int)ceilf((rings ? kRing : kWindow) *
+                     sqrtf((float)(tiles * kTile * kTile) / (float)max(cnt, 1u)));
   W = min(max(W, 4), 2 * n);
   int x0 = sx, x1 = sx, y0 = sy, y1 = sy;  // the window so far: the site
-  bool first = true, wrap = true;
+  bool first = true, wrap = !rings;
   for (;;) {
     const int nx0 = max(0, sx - W), nx1 = min(n - 1, sx + W);
     const int ny0 = max(0, sy - W), ny1 = min(n - 1, sy + W);
@@ -910,7 +913,7 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
       }
     } while (changed);
     if (ok) return true;
-    W = first ? min((int)ceilf(kGrow * W), 2 * n) : min(2 * W, 2 * n);
+    W = first && !rings ? min((int)ceilf(kGrow * W), 2 * n) : min(2 * W, 2 * n);
     first = false;
   }
 }
@@ -1041,7 +1044,10 @@ __device__ __noinline__ void full_site(const uint64_t *bits, const uint64_t *fix
   const int sx = pdx(pos) & 0xffff, sy = pdy(pos);
   const int xm = site_index(bits, fixed, n, out.coloff, out.colpre, sx, sy);
   WStar st;
-  if (!wsite_star(st, bits, fixed, n, sx, sy, py, ts, stk)) {
+  bool fits = false;
+  for (int k = 0; k < 2 && !fits; ++k)
+    fits = wsite_star(st, bits, fixed, n, sx, sy, py, ts, stk, k != 0);
+  if (!fits) {
     if (lane == 0) {
       atomicOr(out.err, 1);
       out.sitepos[xm] = pos;

@@ -229,6 +229,11 @@ def _lattice(n, dx, dy):
 
 
 def _collinear_set(kind, n):
+    if kind == "border":  # a site on every pixel of the border, an interior far from it
+        t, i = np.arange(n), _lattice(n, 20, 20) + 4
+        q = [np.stack([t, 0 * t], 1), np.stack([t, 0 * t + n - 1], 1), np.stack([0 * t, t], 1),
+             np.stack([0 * t + n - 1, t], 1), i[((i > 20) & (i < n - 20)).all(1)]]
+        return np.unique(np.concatenate(q), axis=0)
     if kind == "row":
         return np.stack([np.arange(n), np.full(n, n // 3)], 1)
     if kind.startswith("diagonal"):  # diagonals `step` rows apart, a site every `every` columns
@@ -244,11 +249,11 @@ def _collinear_set(kind, n):
                                     ("3,40", 256), ("40,3", 256), ("2,24", 256), ("4,64", 512),
                                     ("5,60", 512), ("8,128", 1024), ("128,8", 1024),
                                     ("diagonal1,24", 256), ("diagonal2,40", 256),
-                                    ("diagonal3,66", 512),
+                                    ("diagonal3,66", 512), ("border", 256), ("border", 512),
                                     ("row", 256), ("row", 1024)])
 def test_collinear_windows(gcvt_lib, cuda_device, kind, n):
     """Sites whose first windows hold one line through the site only: structured
-    lattices, diagonals, a single row."""
+    lattices, diagonals, a densely sampled border, a single row."""
     q = _collinear_set(kind, n)
     pts, tris = _triangulate(gcvt_lib, _grid(n, q.tolist()))
     if kind == "row":
