@@ -794,9 +794,9 @@ __device__ __forceinline__ int wnext(const WStar &s, int k) {
 constexpr float kWindow = 2.0f, kGrow = 1.7f, kRing = 1.4f;
 constexpr int kWiden = 1;
 constexpr int kBoxCols = 96, kBoxBands = 3;  // largest disc box scanned directly
+template <bool rings>
 __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixed, int n, int sx,
-                           int sy, const Pyr &py, const TileSites &ts, unsigned *stk,
-                           bool rings) {
+                           int sy, const Pyr &py, const TileSites &ts, unsigned *stk) {
   st.a = st.b = 0;
   st.m = 0;
   st.overflow = false;
@@ -1037,6 +1037,7 @@ __device__ __forceinline__ bool owns_tri(int sx, int sy, int u, int w) {
 }
 
 // One site by the whole warp, any case.
+template <bool rings>
 __device__ __noinline__ void full_site(const uint64_t *bits, const uint64_t *fixed, int n, int pos,
                                        const Pyr &py, const TileSites &ts, unsigned *stk,
                                        const StarOut &out) {
@@ -1044,10 +1045,7 @@ __device__ __noinline__ void full_site(const uint64_t *bits, const uint64_t *fix
   const int sx = pdx(pos) & 0xffff, sy = pdy(pos);
   const int xm = site_index(bits, fixed, n, out.coloff, out.colpre, sx, sy);
   WStar st;
-  bool fits = false;
-  for (int k = 0; k < 2 && !fits; ++k)
-    fits = wsite_star(st, bits, fixed, n, sx, sy, py, ts, stk, k != 0);
-  if (!fits) {
+  if (!wsite_star<rings>(st, bits, fixed, n, sx, sy, py, ts, stk)) {
     if (lane == 0) {
       atomicOr(out.err, 1);
       out.sitepos[xm] = pos;
@@ -1272,14 +1270,25 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 5)
   const int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   auto &sw = s_warp[threadIdx.x >> 5];
   if (t < nedge) {
-    full_site(bits, fixed, n, ts.order[t], py, ts, sw.front, out);
+    full_site<false>(bits, fixed, n, ts.order[t], py, ts, sw.front, out);
     return;
   }
   const int t0 = nedge + 4 * (t - nedge);
   if (t0 >= nsites) return;  // the whole warp
   unsigned left = quad_stars(bits, fixed, n, t0, nsites, py, ts, sw.quad, out);
   for (; left; left &= left - 1u)
-    full_site(bits, fixed, n, ts.order[t0 + __ffs(left) - 1], py, ts, sw.front, out);
+    full_site<false>(bits, fixed, n, ts.order[t0 + __ffs(left) - 1], py, ts, sw.front, out);
+}
+
+// The sites whose star overflowed (no neighbours), ring by ring.  (In k_dt_star this
+// path would cost every launch 2 %: registers spilled.)
+__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+    k_dt_rings(const uint64_t *__restrict__ bits, const uint64_t *__restrict__ fixed, int n,
+               int nsites, Pyr py, TileSites ts, StarOut out) {
+  __shared__ unsigned s_front[kWarpsPerBlock][kFrontier];
+  const int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (t >= nsites || out.degree[t]) return;  // the whole warp
+  full_site<true>(bits, fixed, n, out.sitepos[t], py, ts, s_front[threadIdx.x >> 5], out);
 }
 
 __global__ void k_dt_emit(const uint64_t *__restrict__ bits, const uint64_t *__restrict__ fixed,
@@ -1396,16 +1405,25 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
   k_dt_star<<<nblk(warps, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, s>>>(
       bits, fixed, n, nsites, nedge, py, ts, out);
   DCK(cudaGetLastError());
-  if ((rc = scan(tcnt, nsites, toff, sc, s))) return rc;
-  if (tris && cap) {
-    k_dt_emit<<<nblk(nsites, 128), 128, 0, s>>>(bits, fixed, n, sitepos, nsites, coloff, colpre,
-                                                stars, degree, toff, tris, cap);
-    DCK(cudaGetLastError());
-  }
   unsigned h[2] = {0, 0};
-  DCK(cudaMemcpyAsync(&h[0], toff + nsites, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-  DCK(cudaMemcpyAsync(&h[1], err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-  DCK(cudaStreamSynchronize(s));
+  for (int k = 0; k < 2; ++k) {
+    if (k) {
+      DCK(cudaMemsetAsync(err, 0, sizeof(int), s));
+      k_dt_rings<<<nblk(nsites, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, s>>>(
+          bits, fixed, n, nsites, py, ts, out);
+      DCK(cudaGetLastError());
+    }
+    if ((rc = scan(tcnt, nsites, toff, sc, s))) return rc;
+    if (tris && cap) {
+      k_dt_emit<<<nblk(nsites, 128), 128, 0, s>>>(bits, fixed, n, sitepos, nsites, coloff, colpre,
+                                                  stars, degree, toff, tris, cap);
+      DCK(cudaGetLastError());
+    }
+    DCK(cudaMemcpyAsync(&h[0], toff + nsites, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    DCK(cudaMemcpyAsync(&h[1], err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    DCK(cudaStreamSynchronize(s));
+    if (!h[1]) break;  // else the stars that overflowed once more
+  }
   if (h[1]) return GCVT_ERR_INPUT;
   *ntris = h[0];
   return GCVT_OK;

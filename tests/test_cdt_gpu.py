@@ -231,16 +231,23 @@ def test_cdt_of_points_at_the_coordinate_limit(gcvt_lib, cuda_device, n, m, seed
     ctx.close()
 
 
-@pytest.mark.parametrize("dx,dy", [(2, 32), (32, 2)])
-def test_cdt_on_a_lattice_of_lines(gcvt_lib, cuda_device, dx, dy):
-    """Sites whose first windows hold one line through the site only."""
+@pytest.mark.parametrize("dx,dy,count", [(2, 32, 4), (32, 2, 4), (2, 32, 3), (32, 2, 3)])
+def test_cdt_on_a_lattice_of_lines(gcvt_lib, cuda_device, dx, dy, count):
+    """Sites whose first windows hold one line through the site only.  The fourth
+    constraint point lies to the right of them all and sees the last column's edges: seven,
+    or 127, over the 64 a point may see."""
     n = 256
     q = np.stack(np.meshgrid(np.arange(0, n, dx), np.arange(0, n, dy)), -1).reshape(-1, 2)
     ctx = gcvt_lib.Context(n)
     ctx.load(gcvt_lib.sites_from_points(n, q[:, 0], q[:, 1]), np.ones((n, n), np.float32),
              np.zeros((n, n), np.uint8))
     c = np.array([(40.25, 60.5), (210.75, 190.125), (100.5, 33.0), (280.0, 120.5)])
-    segs = np.array([(len(q), len(q) + 1), (len(q) + 1, len(q) + 3)])
+    c, segs = c[:count], np.array([(len(q), len(q) + 1), (len(q) + 1, len(q) + count - 1)])
+    if dx == 32 and count == 4:
+        with pytest.raises(gcvt_lib.GcvtError, match="detail 4"):
+            ctx.cdt(1.0, 0.0, 0.0, c, segs)
+        ctx.close()
+        return
     tri, detail = ctx.cdt(1.0, 0.0, 0.0, c, segs)
     pts, R, F = exact_points(ctx, n, c, 1.0, 0.0, 0.0)
     info = D.check_cdt(pts, tri, segs, R.tolist())
