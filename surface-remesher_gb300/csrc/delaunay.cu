@@ -485,14 +485,31 @@ __device__ bool wwrap(WStar &st, const uint64_t *bits, const uint64_t *fixed, in
 
 // Insert the free sites of the window [nx0, nx1] x [ny0, ny1] that are not
 // in the window [x0, x1] x [y0, y1] inserted before; the lanes take 32
-// columns at a time, then insert the sites they found one by one.
+// columns at a time, then insert the sites they found one by one.  A tall window
+// (few sites, or one at the end of a row, whose windows grow to the grid) looks at
+// the occupancy of 64 x 64 pixels first, a lane per band: a load and a vote per 32
+// columns of every band of an empty 8192 x 8192 took one warp 10 ms.
 __device__ void wwindow(WStar &st, const uint64_t *bits, const uint64_t *fixed, int n, int sx,
-                        int sy, int nx0, int nx1, int ny0, int ny1, int x0, int x1, int y0,
-                        int y1) {
-  const int l = lane_id();
+                        int sy, const Pyr &py, int nx0, int nx1, int ny0, int ny1, int x0, int x1,
+                        int y0, int y1) {
+  const int l = lane_id(), b1 = ny1 / kBand;
+  const bool tall = b1 - ny0 / kBand >= 4;
+  const uint8_t *occ = py.occ + py.off[2];  // (tiles of 64 pixels)
   for (int cx = nx0; cx <= nx1; cx += 32) {
     const int x = cx + l;
-    for (int b = ny0 / kBand; b <= ny1 / kBand; ++b) {
+    unsigned used = 0;
+    for (int b = ny0 / kBand; b <= b1; ++b) {
+      if (tall) {
+        const int i = (b - ny0 / kBand) & 31;
+        if (i == 0) {
+          const uint8_t *o = occ + (size_t)min(b + l, n / kBand - 1) * py.nt[2];
+          used = __ballot_sync(kFull, o[cx / kBand] | o[min(cx + 31, n - 1) / kBand]);
+        }
+        if (!((used >> i) & 1u)) {  // on to the next occupied band
+          b += ((used >> i) ? __ffs((int)(used >> i)) - 1 : 32 - i) - 1;
+          continue;
+        }
+      }
       uint64_t w = 0;
       if (x <= nx1) {
         w = free_word(bits, fixed, (size_t)b * n + x) & band_rows(b, ny0, ny1);
@@ -788,11 +805,14 @@ __device__ __forceinline__ int wnext(const WStar &s, int k) {
 // triangles exactly, and only a star of fewer than two neighbours doubles the
 // window again.  More than 64 candidates are inserted ring by ring instead of
 // wrapped.  (kWindow 1.6 to 2.3 and kGrow 1.5 to 2 measure within 5 %, kWiden 3 or
-// never 8 % slower on irregular sites.)  Returns false when the star
+// never 8 % slower on irregular sites.)  A star whose sites all lie on one line
+// widens up to kLine first: the next row of a lattice is nearer than what a search of
+// the gap's half plane finds.  Returns false when the star
 // overflowed, which depends on the order of the insertions too: `rings` inserts the
 // windows of 1.4, 2.8, 5.6 ... spacings ring by ring, nearer sites first.
 constexpr float kWindow = 2.0f, kGrow = 1.7f, kRing = 1.4f;
 constexpr int kWiden = 1;
+constexpr int kLine = 128;
 constexpr int kBoxCols = 96, kBoxBands = 3;  // largest disc box scanned directly
 template <bool rings>
 __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixed, int n, int sx,
@@ -814,9 +834,10 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
   for (;;) {
     const int nx0 = max(0, sx - W), nx1 = min(n - 1, sx + W);
     const int ny0 = max(0, sy - W), ny1 = min(n - 1, sy + W);
-    // wrapped while the candidates are few, then ring by ring
+    // wrapped in the first two windows while the candidates are few, then ring by ring
+    // (the star so far is the one of every site of the window before)
     wrap = wrap && wwrap(st, bits, fixed, n, sx, sy, nx0, nx1, ny0, ny1, reinterpret_cast<int *>(stk));
-    if (!wrap) wwindow(st, bits, fixed, n, sx, sy, nx0, nx1, ny0, ny1, x0, x1, y0, y1);
+    if (!wrap) wwindow(st, bits, fixed, n, sx, sy, py, nx0, nx1, ny0, ny1, x0, x1, y0, y1);
     x0 = nx0;
     x1 = nx1;
     y0 = ny0;
@@ -840,6 +861,10 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
       changed = false;
       const int m = st.m;
       ok = m >= 2;  // fewer than two neighbours: a wider window
+      if (m == 2 && !rings && W < kLine) {
+        const int u = wget(st, 0), w = wget(st, 1);
+        ok = cross(pdx(u), pdy(u), pdx(w), pdy(w)) != 0;
+      }
       if (!ok) break;
       // each lane checks its two triangles against the window; the ones
       // that the window does not settle are searched one by one
@@ -913,6 +938,7 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
       }
     } while (changed);
     if (ok) return true;
+    wrap = wrap && first;
     W = first && !rings ? min((int)ceilf(kGrow * W), 2 * n) : min(2 * W, 2 * n);
     first = false;
   }
