@@ -71,8 +71,8 @@ struct DevState {
   int gate_tried, gate_kept;  // jumps proposed / kept
   double gate_e0;      // energy of the sites the jump starts from
   double gate_e1;      // energy of the jumped sites
-  int label_ovf;       // labelling: a tile's lists did not fit (label_tiles.cu)
-  int pad1;
+  // Labelling (label_tiles.cu): per 64 rows, 1 where the row pass labels them.
+  uint8_t band_rows[kMaxN / kBand];
   // Labelling (labeller.cu): rows whose candidate hull did not fit the
   // bounded buffer of k_rows, for k_rows_full (zero between labellings).
   unsigned row_ovf[kMaxN / 32];
@@ -129,6 +129,16 @@ __device__ __forceinline__ const uint64_t *cur_bits(const LevelBufs &a) {
   return c == 0 ? a.bits[0] : (c == 1 ? a.bits[1] : a.bits[2]);
 }
 
+// Does the row pass label band b?  On small grids it labels all bands when there is
+// one: its time there is one row's, and the tiles would be on top of it.  (The whole
+// warp asks.)
+constexpr int kAllBands = 2048;
+__device__ __forceinline__ bool by_rows(const LevelBufs &a, int b) {
+  if (a.n > kAllBands) return a.st->band_rows[b] != 0;
+  const int l = threadIdx.x & 31;  // n / kBand <= 32 bands
+  return __any_sync(0xffffffffu, l < a.n / kBand && a.st->band_rows[l]);
+}
+
 // Kernels (launch helpers in labeller.cu / lloyd.cu / cells.cu).
 cudaError_t launch_grid_to_bits(const uint32_t *grid, int n, uint64_t *bits, int *err,
                                 int *count, cudaStream_t s);
@@ -141,8 +151,8 @@ inline cudaError_t launch_jfa_seed(const uint64_t *bits, int n, uint32_t *grid, 
   return launch_bits_to_grid(bits, n, grid, s, kJfaNone, true);
 }
 // The exact labels of the current sites into b.labels (label_tiles.cu); the row
-// pass (column summaries, rows) does small grids (always) and those where
-// DevState::label_ovf says so.
+// pass (column summaries, rows) does small grids (always) and the rows that
+// DevState::band_rows says.
 cudaError_t launch_label(const LevelBufs &b, cudaStream_t s);
 size_t label_blocks(int n);  // entries of LevelBufs::open_tiles (::occ: 4 per row of blocks)
 cudaError_t launch_summary(const LevelBufs &b, bool always, cudaStream_t s);

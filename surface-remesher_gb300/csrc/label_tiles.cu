@@ -21,9 +21,9 @@
 //     from any site, or crowded).  It finds the nearest site to the block's centre
 //     over the occupied 64 x 64 blocks, gathers the sites that can own any of its
 //     pixels by the same test, and prunes that list for each of its open tiles.
-//   * what does not fit its lists (a block crowded with sites) sets
-//     DevState::label_ovf, and the row pass (labeller.cu) does the whole grid, as it
-//     does for grids up to 512 x 512 and for crowded ones.
+//   * the row pass (labeller.cu) does grids up to 512 x 512 and crowded ones, and of
+//     the others the rows of a band (64 rows) that holds a crowded 64 x 64 block, which
+//     the tiles skip, or one that does not fit its lists (by_rows).
 //
 // What bounds it is issue slots: half of a CVT tile's warp instructions are its 15
 // candidates x 256 pixels.  The row pass this replaces spent 330 per row and 32
@@ -42,9 +42,9 @@ constexpr int kWin = kT + 2 * kMargin;
 constexpr int kTileWarps = 4;       // tiles per block
 constexpr int kGather = 512;        // sites of a window
 constexpr int kCand = 128;          // candidates of a tile (below 256: the key's low byte)
-constexpr int kFarThreads = 128;
 constexpr int kFarMacros = 1024;    // 64 x 64 blocks looked at
 constexpr int kFarSites = 2048;     // sites gathered for one
+constexpr int kCrowdBlock = 380;    // sites of a 64 x 64 block: above it the row pass
 
 // A candidate t relative to a reference site r: |p - t|^2 - |p - r|^2 = c + p.x ax +
 // p.y ay for the pixel p of the tile, and t's label.
@@ -89,20 +89,22 @@ __device__ __forceinline__ bool corner_in(int x, int y, int s, const int4 &r2) {
 }
 
 // Occupied 64 x 64 blocks (a bitmap word per column) as a bit mask per row of
-// them, no open tiles, no overflow.  One block per row.
+// them, whether one is crowded, no open tiles.  One block per row.
 __global__ void __launch_bounds__(1024) k_label_occ(LevelBufs a) {
-  __shared__ unsigned mask[4];
+  __shared__ unsigned mask[4], crowded;
   const int M = a.n / kBand, row = blockIdx.x, lane = threadIdx.x & 31;
-  if (row == 0 && threadIdx.x == 0) a.st->label_ovf = 0;
   if (threadIdx.x < 4) mask[threadIdx.x] = 0u;
+  if (threadIdx.x == 0) crowded = 0u;
   if ((int)threadIdx.x < M) a.open_tiles[row * M + threadIdx.x] = 0u;
   __syncthreads();
   for (int m = threadIdx.x >> 5; m < M; m += 32) {
     const uint64_t *w = cur_bits(a) + (size_t)row * a.n + m * kBand;
-    if (__any_sync(kFull, (w[lane] | w[lane + 32]) != 0ull) && lane == 0)
-      atomicOr(mask + (m >> 5), 1u << (m & 31));
+    const int sites = __reduce_add_sync(kFull, __popcll(w[lane]) + __popcll(w[lane + 32]));
+    if (lane == 0 && sites) atomicOr(mask + (m >> 5), 1u << (m & 31));
+    if (lane == 0 && sites > kCrowdBlock) crowded = 1u;
   }
   __syncthreads();
+  if (threadIdx.x == 0) a.st->band_rows[row] = (uint8_t)crowded;
   if (threadIdx.x < 4) a.occ[4 * row + threadIdx.x] = mask[threadIdx.x];
 }
 
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_label_tiles(LevelBufs a) {
     }
     col[h] = w & ((1ull << kWin) - 1ull);
   }
+  if (by_rows(a, y0 / kBand)) return;  // (beside the loads above)
   int cnt = 0;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -202,6 +205,7 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_label_tiles(LevelBufs a) {
 
 __device__ __forceinline__ int box_gap(int p, int lo, int hi) { return max(max(lo - p, p - hi), 0); }
 
+template <int kFarThreads>
 __global__ void __launch_bounds__(kFarThreads) k_label_far(LevelBufs a) {
   __shared__ uint32_t s_site[kFarSites];      // x | y << 16
   __shared__ unsigned short s_macro[kFarMacros];
@@ -212,7 +216,7 @@ __global__ void __launch_bounds__(kFarThreads) k_label_far(LevelBufs a) {
   const int n = a.n, M = n / kBand, tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
   const int mx = blockIdx.x, my = blockIdx.y;
   const unsigned open = a.open_tiles[my * M + mx];
-  if (!open) return;
+  if (!open || by_rows(a, my)) return;
   const int x0 = mx * kBand, y0 = my * kBand;
   const uint64_t *bits = cur_bits(a);
   if (tid == 0) {
@@ -338,7 +342,7 @@ __global__ void __launch_bounds__(kFarThreads) k_label_far(LevelBufs a) {
     }
   }
   if (!ok) {
-    if (tid == 0) a.st->label_ovf = 1;
+    if (tid == 0) a.st->band_rows[my] = 1;
     return;
   }
   // the open tiles, a warp each: nearest site to the centre, corner test, tie order
@@ -375,7 +379,7 @@ __global__ void __launch_bounds__(kFarThreads) k_label_far(LevelBufs a) {
       m += __popc(km);
     }
     if (m > kCand) {
-      if (lane == 0) a.st->label_ovf = 1;
+      if (lane == 0) a.st->band_rows[my] = 1;
       continue;
     }
     __syncwarp();
@@ -397,24 +401,31 @@ __global__ void __launch_bounds__(kFarThreads) k_label_far(LevelBufs a) {
 size_t label_blocks(int n) { return (size_t)(n / kBand) * (n / kBand); }
 
 // Up to 512 x 512 the row pass labels: three launches instead of six (the tiles' three
-// and the row pass's, which then look at label_ovf), and both are latency there.  A
+// and the row pass's, which then look at band_rows), and both are latency there.  A
 // labelling call took, rows / tiles: 37 / 51 us at 256 x 256, 50 / 57 at 512 x 512, 92 /
-// 75 at 1024 x 1024.  So it does where the sites crowd the tiles' lists (fewer than 16
-// pixels a site): 2048 x 2048 of 16 pixels a site 190 / 104 us, of 11 595 / 706, the row
-// pass having to follow the tiles.
+// 75 at 1024 x 1024.  So it does where the sites crowd the tiles' lists, which are too
+// short from about 12 pixels a site on, the row pass then following the tiles: 2048 x 2048
+// of 16 pixels a site 189 / 106 us, of 13 600 / 95, of 12 595 / 556, of 11 596 / 707; 8192
+// x 8192 of 13 8.35 / 3.23 ms, of 12 8.99 / 9.62.  A 64 x 64 block of more than kCrowdBlock
+// (10.8 pixels a site) sends its band there before the tiles look at it: the quarter of
+// 2048 x 2048 at 4 pixels a site 487 by rows alone, 576 by tiles and all rows, 494 us now;
+// a crowded 128 x 128 corner of 8192 x 8192 1.17, 1.39 and 0.55 ms.
 constexpr int kRowLabels = 512;
-constexpr long long kRowCrowd = 16;
+constexpr long long kRowCrowd = 13;
 
 cudaError_t launch_label(const LevelBufs &b, cudaStream_t s) {
   const unsigned M = (unsigned)(b.n / kBand);
-  const bool rows = b.n <= kRowLabels || kRowCrowd * b.sites > (long long)b.n * b.n;
+  const bool rows = b.n <= kRowLabels || kRowCrowd * b.sites >= (long long)b.n * b.n;
   if (!rows) {
     k_label_occ<<<M, 1024, 0, s>>>(b);
     k_label_tiles<<<dim3((unsigned)b.n / (kT * kTileWarps), (unsigned)b.n / kT), 32 * kTileWarps,
                     0, s>>>(b);
-    k_label_far<<<dim3(M, M), kFarThreads, 0, s>>>(b);
+    // (wider blocks where a few of them are the kernel's time: 1024 x 1024 with a 64-pixel
+    // cluster 50 -> 45 us; 8192 x 8192 with ten sites 205 -> 223)
+    if (b.n <= 1536) k_label_far<256><<<dim3(M, M), 256, 0, s>>>(b);
+    else k_label_far<128><<<dim3(M, M), 128, 0, s>>>(b);
   }
-  // the row pass, always or where the lists overflowed
+  // the row pass, always or for its bands
   cudaError_t e = launch_summary(b, rows, s);
   if (e == cudaSuccess) e = launch_rows(b, rows, s);
   return e == cudaSuccess ? cudaGetLastError() : e;

@@ -31,7 +31,8 @@
 //     whose survivors do not fit the buffer is flagged and redone by
 //     k_rows_full with a whole-row buffer: the smaller buffer lets 2.5 times
 //     the rows share an SM.  Above 512 x 512 label_tiles.cu labels, and this pass
-//     does the whole grid only when that one's lists overflow (DevState::label_ovf).
+//     does crowded grids, and of others the 64-row bands that hold a crowded part
+//     (by_rows).
 #include "gcvt_internal.cuh"
 
 namespace cvtgb {
@@ -105,7 +106,8 @@ cudaError_t launch_bits_to_grid(const uint64_t *bits, int n, uint32_t *grid, cud
 // owning ceil(nb/32) consecutive bands.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_summary(LevelBufs a, bool always) {
-  if (!always && !a.st->label_ovf) return;
+  const int tid = threadIdx.y * 32 + threadIdx.x;
+  if (!always && !__syncthreads_or(tid < a.n / kBand && a.st->band_rows[tid])) return;
   __shared__ int sLast[32][33];
   __shared__ int sFirst[32][33];
   const int n = a.n, nb = n / kBand;
@@ -352,8 +354,8 @@ constexpr int row_cap(int n) { return n * 2 / 5; }
 
 __global__ void __launch_bounds__(32) k_rows(LevelBufs a, bool always) {
   extern __shared__ __align__(16) int smem[];
-  if (!always && !a.st->label_ovf) return;
   const int n = a.n, r = blockIdx.x;
+  if (!always && !by_rows(a, r / kBand)) return;
   if (r >= n) return;
   const int K = row_hull(a, r, smem, row_cap(n));
   if (K < 0) {
@@ -367,8 +369,10 @@ __global__ void __launch_bounds__(32) k_rows(LevelBufs a, bool always) {
 // striding over the rows); clears their flags.
 __global__ void __launch_bounds__(32) k_rows_full(LevelBufs a, bool always) {
   extern __shared__ __align__(16) int smem[];
-  if (!always && !a.st->label_ovf) return;
   const int n = a.n;
+  bool any = always;
+  for (int k = threadIdx.x; k < n / kBand; k += 32) any |= a.st->band_rows[k] != 0;
+  if (!__any_sync(0xffffffffu, any)) return;
   for (int r = blockIdx.x; r < n; r += gridDim.x) {
     if (!((a.st->row_ovf[r >> 5] >> (r & 31)) & 1u)) continue;
     const int K = row_hull(a, r, smem, n);

@@ -114,3 +114,46 @@ def test_tile_lists_and_their_overflows(gcvt_lib, oracle, cuda_device, n, kind):
     got, want = gcvt_lib.label_grid(g), oracle.spec_label(g)
     bad = np.argwhere((got != want).any(-1))
     assert bad.size == 0, (len(bad), bad[:3], got[tuple(bad[0])], want[tuple(bad[0])])
+
+
+@pytest.mark.parametrize("n,kind", [(768, "block380"), (768, "block381"), (1024, "band"),
+                                    (2048, "late"), (2304, "late"), (2304, "block380"),
+                                    (2304, "block381"), (2304, "band"), (2048, "quarter"),
+                                    (2304, "quarter"), (2304, "stripe"), (1024, "uniform13"),
+                                    (1024, "uniform12")])
+def test_crowded_bands(gcvt_lib, oracle, cuda_device, n, kind):
+    """Bands labelled by rows beside bands labelled by tiles: a 64 x 64 block at and past
+    the count that sends its band to the rows, a crowded band, tiles whose lists overflow
+    in a block below that count, crowded parts of the grid, the count that sends all of
+    it there; grids up to and past the size where one such band takes the others along."""
+    import torch
+    rng = np.random.default_rng(n)
+    b = np.zeros((n, n), bool)
+    b.ravel()[rng.choice(n * n, n * n // 300, replace=False)] = True
+    if kind.startswith("block"):
+        q = np.zeros(64 * 64, bool)
+        q[rng.choice(64 * 64, int(kind[5:]), replace=False)] = True
+        b[128:192, 320:384] = q.reshape(64, 64)
+    elif kind == "band":
+        b[256:320] = rng.random((64, n)) < 0.3
+    elif kind == "late":  # 196 sites of one tile, a lone block far from any other site
+        b[300:314, 420:434] = True
+        b[n // 2:] = False
+        b[n - 70, n - 70] = True
+    elif kind == "quarter":
+        b[:n // 2, :n // 2] = rng.random((n // 2, n // 2)) < 0.25
+    elif kind == "stripe":
+        b[:, 700:800] = rng.random((n, 100)) < 0.25
+    else:
+        b[:] = False
+        b.ravel()[rng.choice(n * n, n * n // int(kind[7:]), replace=False)] = True
+    ys, xs = np.nonzero(b)
+    g = grid(n, list(zip(xs.tolist(), ys.tolist())))
+    want = oracle.spec_label(g)
+    assert np.array_equal(gcvt_lib.label_grid(g), want)
+    d = torch.from_numpy(g).cuda()
+    o = torch.empty_like(d)
+    if n <= 2048:
+        lib = gcvt_lib.load_library()
+        assert lib.gcvt_label_grid_static(d.data_ptr(), o.data_ptr(), n, None) == 0
+        assert np.array_equal(o.cpu().numpy(), want)
