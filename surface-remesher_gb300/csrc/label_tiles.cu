@@ -216,7 +216,8 @@ __global__ void __launch_bounds__(kFarThreads) k_label_far(LevelBufs a) {
   const int n = a.n, M = n / kBand, tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
   const int mx = blockIdx.x, my = blockIdx.y;
   const unsigned open = a.open_tiles[my * M + mx];
-  if (!open || by_rows(a, my)) return;
+  // (another block may be flagging the band: one answer for the whole block)
+  if (!open || __syncthreads_or(by_rows(a, my))) return;
   const int x0 = mx * kBand, y0 = my * kBand;
   const uint64_t *bits = cur_bits(a);
   if (tid == 0) {
