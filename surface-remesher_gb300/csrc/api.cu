@@ -10,7 +10,6 @@
 #include "gcvt_internal.cuh"
 #include "../../include/gcvt_gb300.h"
 
-#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -20,6 +19,12 @@
 #include <vector>
 
 using namespace cvtgb;
+
+// The forms of a plain iteration's launches (cell_form): 0 one site per lane, 1 one
+// per warp, 2 + k one launch with blocks for kFewClass << k sites.
+constexpr int kFewClass = 256;
+constexpr int kCellForms = 8;
+static_assert(kFewClass << (kCellForms - 3) == cvtgb::kFewSites, "the largest class");
 
 struct gcvt_ctx {
   int device = 0;
@@ -78,11 +83,9 @@ struct gcvt_ctx {
   double *moments = nullptr;    // 4*n_max^2 doubles, allocated on first use
   int *err = nullptr;           // [0] malformed-grid flag, [1] site count
   int last_levels = 0;
-  cudaGraphExec_t chunk_exec = nullptr;  // kChunk iterations of one level
+  cudaGraphExec_t chunk_exec[kCellForms] = {};  // kChunk iterations of one level
   int chunk_n = 0;
   int chunk_level = -1;
-  bool chunk_warp = false;  // captured one site per warp, for this many sites
-  int chunk_sites = 0;
 };
 
 namespace {
@@ -109,6 +112,25 @@ bool warp_cells(const gcvt_ctx *c) {
   return c->sites <= 8192 || (c->sites <= kWarpSites && c->per_site > c->sites / 96.0 - 55.0);
 }
 
+// The form of an iteration at size n.  The kernels read the number of sites on the
+// device; only the grid of the one-launch form depends on it, by size class, so that
+// contexts fed with ever other counts replay the graphs they have (a capture and an
+// instantiation cost 20 us of a 256 x 256 call's 440).
+int cell_form(const gcvt_ctx *c, int n) {
+  if (!warp_cells(c)) return 0;
+  if (c->sites > kFewSites || list_blocks(n) > (size_t)kFewBlocks) return 1;
+  int k = 0;
+  while (kFewClass << k < c->sites) ++k;
+  return 2 + k;
+}
+
+void drop_chunks(gcvt_ctx *c) {
+  for (auto &e : c->chunk_exec) {
+    if (e) cudaGraphExecDestroy(e);
+    e = nullptr;
+  }
+}
+
 LevelBufs level_bufs(gcvt_ctx *c, int n, int level) {
   LevelBufs b = {};
   b.n = n;
@@ -130,10 +152,10 @@ LevelBufs level_bufs(gcvt_ctx *c, int n, int level) {
   b.gslot = c->gslot;
   b.sslot = c->sslot;
   b.scnt = c->scnt;
-  if (warp_cells(c)) {
+  if (const int form = cell_form(c, n)) {
     b.sitev = c->sitev;
     b.gcnt = c->gcnt;
-    b.few = c->sites <= kFewSites ? std::max(c->sites, 1) : 0;
+    b.few = form >= 2 ? kFewClass << (form - 2) : 0;
   }
   if (c->learning && level == 0) {
     for (int k = 0; k < 3; ++k) {
@@ -160,17 +182,15 @@ int push_state(gcvt_ctx *c) {
 }
 
 // Enqueue kChunk Lloyd iterations through a CUDA graph captured once per
-// (size, level); a stream that cannot be captured (the legacy default stream)
-// gets plain launches.
+// (size, level) and form; a stream that cannot be captured (the legacy default
+// stream) gets plain launches.
 int enqueue_chunk(gcvt_ctx *c, int n, int level) {
-  if (c->chunk_exec &&
-      (c->chunk_n != n || c->chunk_level != level || c->chunk_warp != warp_cells(c) ||
-       (c->chunk_warp && c->chunk_sites != c->sites))) {
-    cudaGraphExecDestroy(c->chunk_exec);
-    c->chunk_exec = nullptr;
-  }
+  if (c->chunk_n != n || c->chunk_level != level) drop_chunks(c);
+  c->chunk_n = n;
+  c->chunk_level = level;
   const LevelBufs b = level_bufs(c, n, level);
-  if (!c->chunk_exec) {
+  cudaGraphExec_t &exec = c->chunk_exec[cell_form(c, n)];
+  if (!exec) {
     if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       cudaGetLastError();
       for (int i = 0; i < kChunk; ++i) {
@@ -188,18 +208,14 @@ int enqueue_chunk(gcvt_ctx *c, int n, int level) {
       if (g) cudaGraphDestroy(g);
       return GCVT_ERR_CUDA;
     }
-    const cudaError_t ie = cudaGraphInstantiate(&c->chunk_exec, g, 0);
+    const cudaError_t ie = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     if (ie != cudaSuccess) {
-      c->chunk_exec = nullptr;
+      exec = nullptr;
       return GCVT_ERR_CUDA;
     }
-    c->chunk_n = n;
-    c->chunk_level = level;
-    c->chunk_warp = warp_cells(c);
-    c->chunk_sites = c->sites;
   }
-  CK(cudaGraphLaunch(c->chunk_exec, c->stream));
+  CK(cudaGraphLaunch(exec, c->stream));
   return GCVT_OK;
 }
 
@@ -470,7 +486,7 @@ int gcvt_ctx_create(int n_max, gcvt_ctx **out) {
 int gcvt_ctx_destroy(gcvt_ctx *c) {
   if (!c) return GCVT_ERR_ARGUMENT;
   if (c->stream) cudaStreamSynchronize(c->stream);
-  if (c->chunk_exec) cudaGraphExecDestroy(c->chunk_exec);
+  drop_chunks(c);
   for (int l = 0; l < 8; ++l) {
     cudaFree(c->density[l]);
     cudaFree(c->support[l]);
@@ -804,10 +820,7 @@ int gcvt_ctx_set_tuning(gcvt_ctx *c, const gcvt_tuning *t) {
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess)
     return GCVT_ERR_CUDA;
   const int grid = t->cell_blocks_per_sm * sms;
-  if ((grid != c->cell_grid || t->cell_mode != c->cell_mode) && c->chunk_exec) {
-    cudaGraphExecDestroy(c->chunk_exec);  // the captured launches change
-    c->chunk_exec = nullptr;
-  }
+  if (grid != c->cell_grid) drop_chunks(c);  // the captured launches change
   c->cell_grid = grid;
   c->cell_mode = t->cell_mode;
   c->hint_slack = t->hint_slack;
@@ -974,10 +987,7 @@ int gcvt_ctx_learning(gcvt_ctx *c, int enable, int track_ids) {
     c->ids[k] = nullptr;
   }
   c->learning = c->track_ids = 0;
-  if (c->chunk_exec) {  // captured launches hold the old buffer pointers
-    cudaGraphExecDestroy(c->chunk_exec);
-    c->chunk_exec = nullptr;
-  }
+  drop_chunks(c);  // captured launches hold the old buffer pointers
   c->cover_valid = 0;  // the next level start sets histories (and ids) up
   if (!enable) return GCVT_OK;
   const size_t nn = (size_t)c->n_max * c->n_max;
@@ -1015,10 +1025,7 @@ int ensure_feat(gcvt_ctx *c) {
   c->feat = c->pred = nullptr;
   c->jaux = nullptr;
   c->feat_cap = 0;
-  if (c->chunk_exec) {
-    cudaGraphExecDestroy(c->chunk_exec);
-    c->chunk_exec = nullptr;
-  }
+  drop_chunks(c);
   if (cudaMalloc(reinterpret_cast<void **>(&c->feat), need * 10 * sizeof(float)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void **>(&c->pred), need * 2 * sizeof(float)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void **>(&c->jaux), need * sizeof(uint32_t)) != cudaSuccess)

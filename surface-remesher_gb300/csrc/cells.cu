@@ -1603,8 +1603,6 @@ __global__ void __launch_bounds__(32 * kBlockSites, 4) k_cell_warp(LevelBufs a) 
 // 1.65 -> 1.46 ms.
 // Above 8192 sites a block would take several turns at finding its sites; k_list then
 // costs less than they do.
-constexpr int kFewBlocks = 512;  // list blocks at most (grids up to 4096^2)
-
 __global__ void __launch_bounds__(32 * kBlockSites, 4) k_cell_few(LevelBufs a) {
   __shared__ WarpScratch scratch[kBlockSites];
   __shared__ unsigned s_pre[kFewBlocks + 1], s_w[kBlockSites];
@@ -2223,7 +2221,7 @@ int cells_default_grid() {
 // One plain Lloyd iteration: the site list and the cells, or, for few sites, one
 // launch.
 cudaError_t launch_iteration(const LevelBufs &b, cudaStream_t s, int grid) {
-  if (b.few && b.sitev && list_blocks(b.n) <= (size_t)kFewBlocks) {
+  if (b.few && b.sitev) {
     int dev = 0;
     const cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;

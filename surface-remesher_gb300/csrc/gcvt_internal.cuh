@@ -22,6 +22,7 @@ constexpr int kBand = 64;           // PBA+ phase-1 band height: n / m1 == 64 fo
                                     // every entry of gcvt.cu:842-847
 constexpr int kWarpSites = 32768;  // one site per warp at most for this many sites
 constexpr int kFewSites = 8192;    // one launch per iteration at most for this many sites
+constexpr int kFewBlocks = 512;    // and site-list blocks (grids up to 4096^2)
 constexpr int kListWords = 512;    // bitmap words per site-list block
 constexpr int kMinN = 256;   // n must be a multiple of 256 (S = n/32 >= 8)
 constexpr int kMaxN = 8192;  // largest grid (the row pass's whole-row buffer: 32 KB)
@@ -119,8 +120,8 @@ struct LevelBufs {
   // done (null: lane-per-site only)
   float4 *sitev;
   unsigned *gcnt;
-  int few;                 // 0, or at least the number of sites, up to kFewSites: a plain
-                           // iteration is one launch (k_cell_few)
+  int few;                 // 0, or the sites a plain iteration's one launch (k_cell_few) has
+                           // blocks for, up to kFewSites (its blocks take turns at more)
   int sites;               // the sites, 0: not known (the labeller's choice of path)
 };
 

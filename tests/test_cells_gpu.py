@@ -88,3 +88,28 @@ def test_one_launch_iterations(gcvt_lib, cuda_device, n, m):
     assert np.array_equal(runs[0][0], runs[1][0])
     assert runs[0][1] == runs[1][1]
     ctx.close()
+
+
+@pytest.mark.parametrize("n,gaussians", [(1024, 2), (1024, 9), (512, 6)])
+def test_one_context_with_changing_counts(gcvt_lib, cuda_device, n, gaussians):
+    """The form of an iteration and its recorded launches follow the loaded sites: one
+    context by its own rule against fresh ones with a site per lane, bit for bit, over the
+    one-launch form's size classes and the limits between the forms, up and down."""
+    rng = np.random.default_rng(n + gaussians)
+    rho = gaussian_density(n, gaussians, 4.0, 0.05, 0.2, 3)
+    inside = np.flatnonzero(rho.ravel() > 0)
+    fixed = np.zeros((n, n), np.uint8)
+    ctx = gcvt_lib.Context(n)
+    for m in (700, 9000, 20000, 300, 40000, 8192, 8193, 700, 32768, 32769, 256, 257, 9000, 20):
+        p = rng.choice(inside, m, replace=False)
+        sites = gcvt_lib.sites_from_points(n, p % n, p // n)
+        ctx.load(sites, rho, fixed)
+        ctx.iterate(21)
+        one = gcvt_lib.Context(n)
+        one.set_tuning(cell_mode=1)
+        one.load(sites, rho, fixed)
+        one.iterate(21)
+        assert np.array_equal(ctx.sites(), one.sites()), m
+        assert ctx.info() == one.info(), m
+        one.close()
+    ctx.close()
