@@ -13,9 +13,10 @@
 //               kappa = d00*d11/denom <= 2^40: binned by its bounding box
 //               enlarged by max(1e-6, kappa 2^-45) of its width + height into
 //               a uniform grid over the faces;
-//   * global -- everything else (non-finite coordinates, negative
-//               denominator, kappa above 2^40, boxes over more than 1024
-//               cells): tested by every point.
+//   * global -- everything else (non-finite coordinates, edges so long that
+//               a weight's products overflow, negative denominator, kappa
+//               above 2^40, boxes over more than 1024 cells): tested by
+//               every point.
 // A point scans its grid cell's list (sorted, so the first face that passes
 // ends the scan) and the global list, keeps the smallest face index whose
 // test passes -- the reference's first hit -- and a point with a non-finite
@@ -167,7 +168,7 @@ __device__ __forceinline__ bool classify_face(const double *__restrict__ uv, int
   const bool finite = isfinite(x1) && isfinite(y1) && isfinite(x2) && isfinite(y2) &&
                       isfinite(x3) && isfinite(y3) && isfinite(f.denom);
   const double cond = f.d00 * f.d11 * f.rden;
-  if (!finite || !(f.denom > 0) || !(cond <= kMaxCond)) {
+  if (!finite || !(f.denom > 0) || !(cond <= kMaxCond) || !(fmax(f.d00, f.d11) < kMaxLen2)) {
     kind[i] = kGlobal;
     ebox[i] = Box{-INFINITY, -INFINITY, INFINITY, INFINITY};
     return false;

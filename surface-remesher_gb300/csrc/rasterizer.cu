@@ -15,10 +15,10 @@
 // forms from them written out explicitly -- on the rest, and keeps the
 // smallest index that passes, which is the reference's first hit.  Triangles
 // the boxes cannot place go to a global list every pixel tests: non-finite
-// coordinates (their weights are NaN and pass the test), a negative
-// denominator, a conditioning kappa = d00*d11/denom above 2^40 (near-flat
-// slivers, whose rounded weights can pass far outside the triangle), or a box
-// over more than 4096 tiles.  For the rest the box, enlarged by
+// coordinates (their weights are NaN and pass the test), edges so long that a
+// weight's products overflow (NaN again), a negative denominator, a conditioning
+// kappa = d00*d11/denom above 2^40 (near-flat slivers, whose rounded weights can
+// pass far outside the triangle), or a box over more than 4096 tiles.  For the rest the box, enlarged by
 // max(1e-6, kappa 2^-45) of its width + height, keeps every pixel whose FP64
 // test can pass: a false hit at distance D needs D < 2^-48 kappa (D + L), L
 // the triangle's size (u = 2^-53), so under 4e-9 L at kappa <= 2^20 and a
@@ -140,7 +140,7 @@ __global__ void k_tri_setup(const double *__restrict__ pts, const int *__restric
     return;
   }
   const double cond = t.d00 * t.d11 * t.rden;
-  if (!finite || !(t.denom > 0) || !(cond <= kMaxCond)) {
+  if (!finite || !(t.denom > 0) || !(cond <= kMaxCond) || !(fmax(t.d00, t.d11) < kMaxLen2)) {
     t.global = 1;
     td[i] = t;
     tbox[i] = make_int4(0, 0, n - 1, n - 1);

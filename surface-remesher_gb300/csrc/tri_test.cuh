@@ -11,6 +11,11 @@
 
 namespace cvtgb {
 
+// Squared edge lengths up to which a weight's products stay finite (below 2^1000), so
+// that no numerator is NaN: what quot_negative and below_zero need, and what lets a box
+// bound where a test passes.  Longer triangles take the plain test everywhere.
+constexpr double kMaxLen2 = 0x1p499;
+
 __device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 
 // RN(num / den), y = RN(1 / den): Markstein's theorem (IBM J. Res. Dev. 34, 1990):

@@ -196,3 +196,26 @@ def test_gpu_lift_slivers_equal_oracle(gcvt_lib, oracle):
     got, face, _ = gcvt_lib.lift(uv, xyz, tris, pts)
     assert np.array_equal(face, wface)
     assert same_f64(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("s,t,u", [(150.0, 350.0, 1.0), (150.0, 350.0, 0.0), (0.0, 511.0, 0.0),
+                                   (100.0, 400.0, 1.0), (-200.0, 500.0, 0.5), (249.0, 249.0, 1.0),
+                                   (250.0, 250.0, 1.0), (20.0, 20.0, 1.0)])
+def test_gpu_lift_near_overflow(gcvt_lib, oracle, cuda_device, s, t, u):
+    """Faces with legs of 2^s and 2^t (u: their slant), whose products of lengths overflow
+    in the weights: infinities and NaN fall as in the oracle's arithmetic."""
+    a, b = np.array([2.0 ** s, 0.0]), np.array([u * 2.0 ** t, 2.0 ** t])
+    k = np.arange(-3, 4)
+    uv = np.concatenate([np.stack([k * 0.0, k * 0.0], 1) + o for o in (0 * a, a, b)]) + \
+        np.tile(k[:, None] * (a + b)[None, :], (3, 1))
+    T = np.array([[i, 7 + i, 14 + i] for i in range(7)] +
+                 [[7 + i, (7 + i + 1) if i < 6 else i, 14 + i] for i in range(7)], np.int32)
+    rng = np.random.default_rng(int(s + t))
+    xyz = rng.uniform(-1, 1, (len(uv), 3))
+    lo, hi = uv.min(0), uv.max(0)
+    q = np.concatenate([lo / 2 + rng.uniform(0, 1, (300, 2)) * (hi / 2 - lo / 2),
+                        uv[:7] + rng.uniform(0, 1, (7, 1)) * a, uv[7:14], uv[14:]])
+    got, face, _ = gcvt_lib.lift(uv, xyz, T, q)
+    want, wface, _ = oracle.lift(uv, xyz, T, q)
+    assert np.array_equal(face, wface) and same_f64(got, want)

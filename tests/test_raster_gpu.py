@@ -128,3 +128,25 @@ def test_raster_lists_and_divisions(gcvt_lib, cuda_device, n, count, scale):
     got = gcvt_lib.rasterize(pts, w, T, scale, n)
     want = orc.rasterize(pts, w, T, scale, n)
     assert np.array_equal(got.view(np.int32), want.view(np.int32))
+
+
+@pytest.mark.parametrize("s,t,u", [(0.0, 0.0, 0.5), (150.0, 350.0, 0.0), (150.0, 350.0, 1.0),
+                                   (0.0, 511.0, 0.0), (100.0, 400.0, 1.0), (-200.0, 500.0, 0.5),
+                                   (249.0, 249.0, 1.0), (250.0, 250.0, 1.0)])
+def test_raster_near_overflow(gcvt_lib, cuda_device, s, t, u):
+    """Legs of 2^s and 2^t (u: their slant), whose products of lengths overflow in the
+    weights: infinities and NaN fall as in the reference's arithmetic.  The first case
+    has a leg of almost sqrt of the largest double, and pixels just past its end."""
+    n = 16
+    if t == 0.0:
+        leg = np.sqrt(np.finfo(np.float64).max) * (1 - 1e-9)
+        a, b, scale = np.array([u, 0.0]), np.array([0.0, leg]), leg * (1 + 5e-7) / 13
+    else:
+        a, b = np.array([2.0 ** s, 0.0]), np.array([u * 2.0 ** t, 2.0 ** t])
+        scale = 2.0 ** t / 11
+    pts = np.array([[0.0, 0.0], a, b, [0.0, 0.0], b, -a])
+    T = np.array([[0, 1, 2], [3, 4, 5]], np.int32)
+    w = np.array([1.0, 2.0, 3.0, 4.0, 5.0, 6.0])
+    got = gcvt_lib.rasterize(pts, w, T, scale, n)
+    want = orc.rasterize(pts, w, T, scale, n)
+    assert _same_f32(got, want)
