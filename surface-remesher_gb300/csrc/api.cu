@@ -10,6 +10,9 @@
 #include "gcvt_internal.cuh"
 #include "../../include/gcvt_gb300.h"
 
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -337,6 +340,30 @@ int copy_out(void *dst, const void *src, size_t bytes, int mem, cudaStream_t s) 
   return GCVT_OK;
 }
 
+// Is p device memory of `device` with `bytes` bytes left in its allocation?  Kernels
+// write a caller's buffer only then: any other pointer goes to a copy, which takes what
+// it can and refuses the rest with an error, where a kernel would fault.
+bool device_range(const void *p, size_t bytes, int device) {
+  cudaPointerAttributes at = {};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (at.type != cudaMemoryTypeDevice || at.device != device) return false;
+  static const PFN_cuMemGetAddressRange_v3020 range = [] {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &fn, 3020,
+                                                           cudaEnableDefault, &q);
+    if (e != cudaSuccess || q != cudaDriverEntryPointSuccess) fn = nullptr;
+    return reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(fn);
+  }();
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const CUdeviceptr at_p = reinterpret_cast<CUdeviceptr>(p);
+  return range && range(&base, &size, at_p) == CUDA_SUCCESS && at_p - base + bytes <= size;
+}
+
 int reset_schedule(gcvt_ctx *c) {
   DevState &h = *c->st_host;
   std::memset(&h, 0, sizeof(DevState));
@@ -564,11 +591,12 @@ int gcvt_ctx_label(gcvt_ctx *c, int16_t *labels, int mem) {
   LevelBufs b = level_bufs(c, n, level_of(c, n));
   // straight into the caller's device buffer where words can be written there (the
   // staging grid and a copy of 8 bytes a pixel otherwise: 0.08 ms at 8192^2)
-  const bool direct = mem == GCVT_MEM_DEVICE && reinterpret_cast<uintptr_t>(labels) % 4 == 0;
+  const size_t bytes = (size_t)n * n * sizeof(uint32_t);
+  const bool direct = mem == GCVT_MEM_DEVICE && reinterpret_cast<uintptr_t>(labels) % 4 == 0 &&
+                      device_range(labels, bytes, c->device);
   if (direct) b.labels = reinterpret_cast<uint32_t *>(labels);
   CK(launch_label(b, c->stream));
-  return direct ? GCVT_OK
-                : copy_out(labels, c->grid, (size_t)n * n * sizeof(uint32_t), mem, c->stream);
+  return direct ? GCVT_OK : copy_out(labels, c->grid, bytes, mem, c->stream);
 }
 
 int gcvt_ctx_iterate(gcvt_ctx *c, int iterations) {

@@ -157,3 +157,33 @@ def test_crowded_bands(gcvt_lib, oracle, cuda_device, n, kind):
         lib = gcvt_lib.load_library()
         assert lib.gcvt_label_grid_static(d.data_ptr(), o.data_ptr(), n, None) == 0
         assert np.array_equal(o.cpu().numpy(), want)
+
+
+def test_label_into_other_buffers(gcvt_lib, oracle, cuda_device):
+    """Kernels write a device buffer of the context's device that holds the labels; any
+    other pointer goes through a copy, which refuses what it cannot write.  At odd
+    offsets, in pinned host memory passed as device memory, in host memory so passed."""
+    import torch
+    n = 768
+    rng = np.random.default_rng(5)
+    p = rng.choice(n * n, 4000, replace=False)
+    g = gcvt_lib.sites_from_points(n, p % n, p // n)
+    want = oracle.spec_label(g)
+    ctx, lib = gcvt_lib.Context(n), gcvt_lib.load_library()
+    ctx.load(g, np.ones((n, n), np.float32), np.zeros((n, n), np.uint8))
+    raw = torch.zeros(n * n * 2 + 64, dtype=torch.int16, device="cuda")
+    for off in (0, 1, 2, 7, 64):
+        raw.zero_()
+        torch.cuda.synchronize()
+        assert lib.gcvt_ctx_label(ctx.h, raw.data_ptr() + 2 * off, 1) == 0
+        torch.cuda.synchronize()
+        assert np.array_equal(raw.cpu().numpy()[off:off + 2 * n * n].reshape(n, n, 2), want)
+        assert not raw[:off].any() and not raw[off + 2 * n * n:].any()
+    pinned = torch.zeros((n, n, 2), dtype=torch.int16).pin_memory()
+    host = np.zeros((n, n, 2), np.int16)
+    for ptr, out in ((pinned.data_ptr(), pinned.numpy()), (host.ctypes.data, host)):
+        rc = lib.gcvt_ctx_label(ctx.h, ptr, 1)
+        torch.cuda.synchronize()
+        assert rc == 3 or (rc == 0 and np.array_equal(out, want))  # GCVT_ERR_CUDA
+    assert np.array_equal(ctx.label(), want)  # the context goes on
+    ctx.close()
