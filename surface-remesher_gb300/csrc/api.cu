@@ -344,24 +344,25 @@ int copy_out(void *dst, const void *src, size_t bytes, int mem, cudaStream_t s) 
 // write a caller's buffer only then: any other pointer goes to a copy, which takes what
 // it can and refuses the rest with an error, where a kernel would fault.
 bool device_range(const void *p, size_t bytes, int device) {
-  cudaPointerAttributes at = {};
-  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  if (at.type != cudaMemoryTypeDevice || at.device != device) return false;
-  static const PFN_cuMemGetAddressRange_v3020 range = [] {
+  static const PFN_cuPointerGetAttributes_v7000 query = [] {
     void *fn = nullptr;
     cudaDriverEntryPointQueryResult q;
-    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &fn, 3020,
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &fn, 7000,
                                                            cudaEnableDefault, &q);
     if (e != cudaSuccess || q != cudaDriverEntryPointSuccess) fn = nullptr;
-    return reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(fn);
+    return reinterpret_cast<PFN_cuPointerGetAttributes_v7000>(fn);
   }();
-  CUdeviceptr base = 0;
+  CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  unsigned type = 0;
+  int ordinal = -1;
+  CUdeviceptr base = 0, at = reinterpret_cast<CUdeviceptr>(p);
   size_t size = 0;
-  const CUdeviceptr at_p = reinterpret_cast<CUdeviceptr>(p);
-  return range && range(&base, &size, at_p) == CUDA_SUCCESS && at_p - base + bytes <= size;
+  void *data[] = {&type, &ordinal, &base, &size};
+  // (an unknown pointer is no error: its attributes are zero)
+  return query && query(4, what, data, at) == CUDA_SUCCESS && type == CU_MEMORYTYPE_DEVICE &&
+         ordinal == device && at - base + bytes <= size;
 }
 
 int reset_schedule(gcvt_ctx *c) {
@@ -592,10 +593,11 @@ int gcvt_ctx_label(gcvt_ctx *c, int16_t *labels, int mem) {
   // straight into the caller's device buffer where words can be written there (the
   // staging grid and a copy of 8 bytes a pixel otherwise: 0.08 ms at 8192^2)
   const size_t bytes = (size_t)n * n * sizeof(uint32_t);
+  CK(launch_label_sites(b, c->stream));  // (the query's 2 us beside it)
   const bool direct = mem == GCVT_MEM_DEVICE && reinterpret_cast<uintptr_t>(labels) % 4 == 0 &&
                       device_range(labels, bytes, c->device);
   if (direct) b.labels = reinterpret_cast<uint32_t *>(labels);
-  CK(launch_label(b, c->stream));
+  CK(launch_label_write(b, c->stream));
   return direct ? GCVT_OK : copy_out(labels, c->grid, bytes, mem, c->stream);
 }
 

@@ -73,7 +73,7 @@ struct DevState {
   double gate_e0;      // energy of the sites the jump starts from
   double gate_e1;      // energy of the jumped sites
   // Labelling (label_tiles.cu): per 64 rows, 1 where the row pass labels them.
-  uint8_t band_rows[kMaxN / kBand];
+  alignas(4) uint8_t band_rows[kMaxN / kBand];
   // Labelling (labeller.cu): rows whose candidate hull did not fit the
   // bounded buffer of k_rows, for k_rows_full (zero between labellings).
   unsigned row_ovf[kMaxN / 32];
@@ -155,6 +155,9 @@ inline cudaError_t launch_jfa_seed(const uint64_t *bits, int n, uint32_t *grid, 
 // pass (column summaries, rows) does small grids (always) and the rows that
 // DevState::band_rows says.
 cudaError_t launch_label(const LevelBufs &b, cudaStream_t s);
+// launch_label in two parts: what reads the sites alone, and what writes b.labels
+cudaError_t launch_label_sites(const LevelBufs &b, cudaStream_t s);
+cudaError_t launch_label_write(const LevelBufs &b, cudaStream_t s);
 size_t label_blocks(int n);  // entries of LevelBufs::open_tiles (::occ: 4 per row of blocks)
 cudaError_t launch_summary(const LevelBufs &b, bool always, cudaStream_t s);
 cudaError_t launch_fixed_bits(const uint8_t *mask, int n, uint64_t *fixed_bits, cudaStream_t s);

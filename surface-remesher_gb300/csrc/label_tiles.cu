@@ -414,22 +414,33 @@ size_t label_blocks(int n) { return (size_t)(n / kBand) * (n / kBand); }
 constexpr int kRowLabels = 512;
 constexpr long long kRowCrowd = 13;
 
-cudaError_t launch_label(const LevelBufs &b, cudaStream_t s) {
+static bool rows_alone(const LevelBufs &b) {
+  return b.n <= kRowLabels || kRowCrowd * b.sites >= (long long)b.n * b.n;
+}
+
+cudaError_t launch_label_sites(const LevelBufs &b, cudaStream_t s) {
+  if (rows_alone(b)) return launch_summary(b, true, s);
+  k_label_occ<<<(unsigned)(b.n / kBand), 1024, 0, s>>>(b);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_label_write(const LevelBufs &b, cudaStream_t s) {
   const unsigned M = (unsigned)(b.n / kBand);
-  const bool rows = b.n <= kRowLabels || kRowCrowd * b.sites >= (long long)b.n * b.n;
-  if (!rows) {
-    k_label_occ<<<M, 1024, 0, s>>>(b);
-    k_label_tiles<<<dim3((unsigned)b.n / (kT * kTileWarps), (unsigned)b.n / kT), 32 * kTileWarps,
-                    0, s>>>(b);
-    // (wider blocks where a few of them are the kernel's time: 1024 x 1024 with a 64-pixel
-    // cluster 50 -> 45 us; 8192 x 8192 with ten sites 205 -> 223)
-    if (b.n <= 1536) k_label_far<256><<<dim3(M, M), 256, 0, s>>>(b);
-    else k_label_far<128><<<dim3(M, M), 128, 0, s>>>(b);
-  }
-  // the row pass, always or for its bands
-  cudaError_t e = launch_summary(b, rows, s);
-  if (e == cudaSuccess) e = launch_rows(b, rows, s);
-  return e == cudaSuccess ? cudaGetLastError() : e;
+  if (rows_alone(b)) return launch_rows(b, true, s);
+  k_label_tiles<<<dim3((unsigned)b.n / (kT * kTileWarps), (unsigned)b.n / kT), 32 * kTileWarps,
+                  0, s>>>(b);
+  // (wider blocks where a few of them are the kernel's time: 1024 x 1024 with a 64-pixel
+  // cluster 50 -> 45 us; 8192 x 8192 with ten sites 205 -> 223)
+  if (b.n <= 1536) k_label_far<256><<<dim3(M, M), 256, 0, s>>>(b);
+  else k_label_far<128><<<dim3(M, M), 128, 0, s>>>(b);
+  // the row pass for its bands
+  const cudaError_t e = launch_summary(b, false, s);
+  return e == cudaSuccess ? launch_rows(b, false, s) : e;
+}
+
+cudaError_t launch_label(const LevelBufs &b, cudaStream_t s) {
+  const cudaError_t e = launch_label_sites(b, s);
+  return e == cudaSuccess ? launch_label_write(b, s) : e;
 }
 
 }  // namespace cvtgb

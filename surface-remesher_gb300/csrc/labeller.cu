@@ -370,9 +370,10 @@ __global__ void __launch_bounds__(32) k_rows(LevelBufs a, bool always) {
 __global__ void __launch_bounds__(32) k_rows_full(LevelBufs a, bool always) {
   extern __shared__ __align__(16) int smem[];
   const int n = a.n;
-  bool any = always;
-  for (int k = threadIdx.x; k < n / kBand; k += 32) any |= a.st->band_rows[k] != 0;
-  if (!__any_sync(0xffffffffu, any)) return;
+  static_assert(kMinN % (4 * kBand) == 0 && kMaxN / kBand <= 4 * 32, "four bands a lane");
+  const unsigned *rows4 = reinterpret_cast<const unsigned *>(a.st->band_rows);
+  const int l = threadIdx.x;
+  if (!always && !__any_sync(0xffffffffu, l < n / (4 * kBand) && rows4[l])) return;
   for (int r = blockIdx.x; r < n; r += gridDim.x) {
     if (!((a.st->row_ovf[r >> 5] >> (r & 31)) & 1u)) continue;
     const int K = row_hull(a, r, smem, n);
