@@ -468,14 +468,21 @@ __global__ void k_flip_apply(Mesh m, const int *ntri, const int *cand, const Cla
     if (cand[t] && flip_apply_one(m, t, cand[t], cl, round, Act{act})) atomicAdd(flips, 1);
 }
 
-// Every insertion round with its flip rounds in one block, for up to kOneBlock
-// points: the rounds are chains of short dependent steps (832 boundary points take 28
+// Every insertion round with its flip rounds in one block: the rounds are chains of short dependent steps (832 boundary points take 28
 // rounds; as seven launches each 74 us a round, 55 in one block of 1024 threads, 85 in
 // one of 256; 36 with short predicates and the loads and marks of a triangle's
 // neighbours in flight together), and the changed triangles are listed instead of
 // searched for.  Block barriers order the steps.  After the last point the flips run
 // until none is left.
-constexpr int kOneBlock = 4096;
+//   Up to kOneBlock points it does them all.  Above, points inside the sites go in
+// fastest over the grid, nearly all in the first rounds, while of a chain of boundary
+// points few win a round and each round's latency counts.  So up to kOneChain the first
+// kInsertPoll rounds run over the grid, and the block goes on if they left more than half.  A
+// call on 1024 x 1024 / 4369 sites took, block / grid / this: 2000 inside 1.43 / 1.11 /
+// 1.43 ms, 3000 inside 1.82 / 1.24 / 1.25, 2000 in a ring outside 3.35 / 4.26 / 3.35, 3000
+// 4.76 / 5.19 / 4.57, 4000 5.81 / 5.42 / 5.47.
+constexpr int kOneBlock = 2048, kOneChain = 4096;
+constexpr int kOneSegs = 4096;  // segments whose rounds one block does
 constexpr int kOneThreads = 1024;
 
 __global__ void __launch_bounds__(kOneThreads) k_insert_all(Mesh m, int *pend, int *start,
@@ -488,6 +495,13 @@ __global__ void __launch_bounds__(kOneThreads) k_insert_all(Mesh m, int *pend, i
   __shared__ int s_np, s_n, s_n2, s_stop;
   const int tid = threadIdx.x;
   if (tid == 0) s_n = s_stop = 0;
+  __syncthreads();
+  // the triangles that rounds over the grid left marked
+  for (int w = tid, T = *ntri; 4 * w < T; w += kOneThreads)
+    for (unsigned q = reinterpret_cast<const unsigned *>(act)[w] & 0x01010101u; q; q &= q - 1u) {
+      const int t = 4 * w + (__ffs((int)q) - 1) / 8;
+      if (t < T) list[atomicAdd(&s_n, 1)] = t;
+    }
   __syncthreads();
   for (int r = 0; r < rounds && np > 0; ++r) {
     ++round;
@@ -638,7 +652,7 @@ __global__ void k_seg_apply(Mesh m, const int *__restrict__ segs, int base, int 
   if (w < W) seg_apply(m, segs, base, w, state, list, lcnt, cl, round, pending, err);
 }
 
-// Every segment round in one block, for up to kOneBlock segments (7 rounds of two
+// Every segment round in one block, for up to kOneSegs segments (7 rounds of two
 // launches and a read-back: 0.42 ms for 832, 0.19 this way).
 __global__ void __launch_bounds__(kOneThreads) k_seg_all(Mesh m, const int *__restrict__ segs,
                                                          int S, int *state, int *list, int *lcnt,
@@ -917,29 +931,30 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
       return flip_rounds(kInterimFlips);
     };
     int np = C;
-    if (C <= kOneBlock) {
+    bool block = C <= kOneBlock;
+    if (!block) CCK(cudaMemcpyAsync(ctr + 4, &C, sizeof(int), cudaMemcpyHostToDevice, s));
+    // kInsertPoll rounds (lists 1 -> 2 -> 1 ...) per read-back
+    for (int r = 0; !block && r < kInsertRounds && np > 0; r += kInsertPoll) {
+      for (int k = 0; k < kInsertPoll && rc == GCVT_OK; k += 2) {
+        rc = ins_round(pend, start, pend2, start2, ctr + 4, ctr + 6);
+        if (rc == GCVT_OK) rc = ins_round(pend2, start2, pend, start, ctr + 6, ctr + 4);
+      }
+      if (rc == GCVT_OK) rc = pull();
+      if (rc != GCVT_OK) return rc;
+      if (h[0]) break;
+      np = h[4];
+      block = r == 0 && C <= kOneChain && 2 * np > C;
+    }
+    if (block) {
       int *la = sc.take<int>((size_t)cap_t), *lb = sc.take<int>((size_t)cap_t);
       if (!la || !lb) return GCVT_ERR_ALLOC;
-      k_insert_all<<<1, kOneThreads, 0, s>>>(m, pend, start, pend2, start2, C, loc, cl, round,
+      k_insert_all<<<1, kOneThreads, 0, s>>>(m, pend, start, pend2, start2, np, loc, cl, round,
                                              kInsertRounds, ctr + 1, cap_t, done, act, la, lb, cand,
                                              ctr + 4, ctr);
       CCK(cudaGetLastError());
       round += (1 + kInterimFlips) * kInsertRounds + kFlipRounds;
       if ((rc = pull())) return rc;
       np = h[0] ? 0 : h[4];
-    } else {
-      CCK(cudaMemcpyAsync(ctr + 4, &C, sizeof(int), cudaMemcpyHostToDevice, s));
-    }
-    // kInsertPoll rounds (lists 1 -> 2 -> 1 ...) per read-back
-    for (int r = 0; C > kOneBlock && r < kInsertRounds && np > 0; r += kInsertPoll) {
-      for (int k = 0; k < kInsertPoll && rc == GCVT_OK; k += 2) {
-        rc = ins_round(pend, start, pend2, start2, ctr + 4, ctr + 6);
-        if (rc == GCVT_OK) rc = ins_round(pend2, start2, pend, start, ctr + 6, ctr + 4);
-      }
-      if (rc == GCVT_OK) rc = pull();
-      if (rc != GCVT_OK) break;
-      if (h[0]) break;
-      np = h[4];
     }
     if (rc != GCVT_OK) return rc;
     if (!h[0] && np > 0) h[0] |= kErrWalk;
@@ -957,13 +972,13 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
     if (!state || !lcnt || !list || !queue || !stack) return GCVT_ERR_ALLOC;
     k_seg_mark<<<nblk(S, 256), 256, 0, s>>>(m, segs, S, (int)V, state, ctr);
     CCK(cudaGetLastError());
-    if (S <= kOneBlock) {
+    if (S <= kOneSegs) {
       k_seg_all<<<1, kOneThreads, 0, s>>>(m, segs, S, state, list, lcnt, cl, round, kSegRounds,
                                           ctr);
       CCK(cudaGetLastError());
       round += kSegRounds;
     }
-    for (int base = 0; S > kOneBlock && base < S; base += kSegWindow) {
+    for (int base = 0; S > kOneSegs && base < S; base += kSegWindow) {
       const int W = S - base < kSegWindow ? S - base : kSegWindow;
       for (int r = 0; r < kSegRounds; ++r) {
         ++round;

@@ -253,3 +253,67 @@ def test_cdt_on_a_lattice_of_lines(gcvt_lib, cuda_device, dx, dy, count):
     info = D.check_cdt(pts, tri, segs, R.tolist())
     assert detail == 0 and info["vertices"] == F + len(c)
     ctx.close()
+
+
+@pytest.mark.parametrize("count", [2048, 2049, 4096, 4097])
+@pytest.mark.parametrize("kind", ["inside", "chain"])
+def test_cdt_insertion_forms(gcvt_lib, cuda_device, kind, count):
+    """Up to 2048 points one block inserts them; above, rounds over the grid, and up to
+    4096 the block what they leave of points that go in few a round (a chain outside the
+    sites' hull, and its segments), not of points inside."""
+    ctx, sp = loaded(gcvt_lib, 512, 700, 81)
+    F = len(sp)
+    rng = np.random.default_rng(count)
+    if kind == "inside":
+        c, segs = rng.uniform(20, 490, (count, 2)), np.zeros((0, 2), np.int64)
+    else:
+        t, r, i = np.sort(rng.uniform(0, 2 * np.pi, count)), 262 + rng.uniform(0, 0.05, count), \
+            np.arange(count)
+        c = np.stack([256 + r * np.cos(t), 256 + r * np.sin(t)], 1)
+        segs = np.stack([F + i, F + (i + 1) % count], 1)
+    tri, detail = ctx.cdt(1.0, 0.0, 0.0, c, segs)
+    pts, R, _ = exact_points(ctx, 512, c, 1.0, 0.0, 0.0)
+    info = D.check_cdt(pts, tri, segs, R.tolist())
+    assert detail == 0 and info["vertices"] == F + count and info["constraints"] >= len(segs)
+    ctx.close()
+
+
+@pytest.mark.parametrize("case,want", [("outside", 0), ("through", 0), ("long", 0), ("twice", 2),
+                                       ("on_site", 2), ("far", 1), ("crossing", 16),
+                                       ("bad_pair", 16), ("same_pair", 16)])
+def test_cdt_cases_among_many_points(gcvt_lib, cuda_device, case, want):
+    """The small cases above with 4200 more points and segments beside them, so that the
+    rounds run over the grid: points outside the hull, a segment through a site, one that
+    crosses many edges, and every reason to refuse."""
+    from scipy.spatial import Delaunay
+    ctx, sp = loaded(gcvt_lib, 512, 900, 82)
+    F, more = len(sp), 4200
+    rng = np.random.default_rng(82)
+    c = rng.uniform((20, 20), (230, 490), (more, 2))
+    t = Delaunay(c).simplices
+    e = np.unique(np.sort(np.concatenate([t[:, [0, 1]], t[:, [1, 2]], t[:, [2, 0]]]), 1), axis=0)
+    segs = e[rng.permutation(len(e))[:more]]
+    site = sp[np.argmin(np.hypot(sp[:, 0] - 380.0, sp[:, 1] - 256.0))].astype(float)
+    q = {"outside": [(540.2, 250.1), (525.3, 300.4), (533.1, 210.7)],
+         "through": [site - (10.5, 0), site + (10.5, 0)],
+         "long": [(300.3, 120.2), (470.6, 330.9)],
+         "twice": [(400.3, 220.7), (400.3, 220.7)], "on_site": [site, (400.3, 220.7)],
+         "far": [(400.3, 220.7), (40000.0, 128.0)],
+         "crossing": [(320.5, 250.3), (480.5, 249.7), (400.4, 180.2), (399.6, 330.1)],
+         "bad_pair": [(400.3, 220.7), (420.1, 230.9)],
+         "same_pair": [(400.3, 220.7), (420.1, 230.9)]}[case]
+    s = {"outside": [(0, 1), (0, 2)], "crossing": [(0, 1), (2, 3)], "bad_pair": [(0, 2)],
+         "same_pair": [(1, 1)]}.get(case, [(0, 1)])
+    c = np.concatenate([c, np.array(q)])
+    segs = F + np.concatenate([segs, more + np.array(s)])
+    if want:
+        with pytest.raises(gcvt_lib.GcvtError) as err:
+            ctx.cdt(1.0, 0.0, 0.0, c, segs)
+        assert err.value.code == 4 and detail_of(err.value) == want
+    else:
+        tri, detail = ctx.cdt(1.0, 0.0, 0.0, c, segs)
+        pts, R, _ = exact_points(ctx, 512, c, 1.0, 0.0, 0.0)
+        info = D.check_cdt(pts, tri, segs, R.tolist())
+        assert detail == 0 and info["vertices"] == F + len(c)
+        assert info["constraints"] >= len(segs) + (case == "through")
+    ctx.close()
