@@ -59,6 +59,8 @@
 // the first to set a bit also counts it for the next k_list.
 #include "gcvt_internal.cuh"
 
+#include <cstddef>
+
 namespace cvtgb {
 
 constexpr int kMaxCand = 64;  // candidate records per site; more: streamed
@@ -1100,7 +1102,7 @@ constexpr int kWarpEnts = 96;  // chunk sums of a site kept in shared memory
 constexpr int kWarpRec = 128;  // candidates of a site kept in shared memory
 constexpr int kBlockSites = 8;  // sites (warps) per block
 
-struct WarpScratch {
+struct alignas(16) WarpScratch {  // (ent and, reused, the whole are read as float4)
   int2 rec[kWarpRec];  // left of s first: float lines {k, s}, or make_rec's records
   // per 16-pixel chunk of the rows, in fold order: the terms of (W, SX, SY, E),
   // high then low parts (the padding spreads the block's sites over the banks)
@@ -1111,6 +1113,7 @@ struct WarpScratch {
   int pad[26];
 };
 static_assert(sizeof(WarpScratch) % 128 == 16, "sites 4 banks apart (fold: lane 4 s + q)");
+static_assert(offsetof(WarpScratch, ent) % 16 == 0, "float4 entries");
 
 // Sums of the pixels [u0, u1] (at most 16, relative to the site) of a row, all
 // its aligned 16-byte loads in flight together.
