@@ -677,8 +677,10 @@ __global__ void __launch_bounds__(kOneThreads) k_seg_all(Mesh m, const int *__re
 // crossing edges): long ones, and those with vertices inside them, which
 // become the chain of edges between those vertices (as constrained Delaunay
 // triangulations split such segments).  Crossing segments set err.
-__global__ void k_segments(Mesh m, const int *__restrict__ segs, int S, const int *state,
-                           int *queue, int *stack, int *err) {
+constexpr int kSegThreads = 1024;
+__global__ void __launch_bounds__(kSegThreads) k_segments(Mesh m, const int *__restrict__ segs,
+                                                          int S, const int *state, int *queue,
+                                                          int *stack, int *err) {
   // (usually few or none: the block finds them; one thread walking the list took 50 us
   // more of 832 segments)
   __shared__ unsigned s_left[32];
@@ -991,7 +993,7 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
         if (h[5] == 0) break;
       }
     }
-    k_segments<<<1, 1024, 0, s>>>(m, segs, S, state, queue, stack, ctr);
+    k_segments<<<1, kSegThreads, 0, s>>>(m, segs, S, state, queue, stack, ctr);
     CCK(cudaGetLastError());
     if ((rc = pull())) return rc;
   }
