@@ -28,7 +28,7 @@
 //      the next one), so the output does not depend on scheduling.
 //
 // A flip round: every changed triangle tests its edges towards
-// higher-numbered neighbours (cdt_core.cuh wants_flip); a flip claims its two
+// higher-numbered neighbours (cdt_core.cuh first_flip); a flip claims its two
 // triangles and their four outer neighbours (whose back links it rewrites);
 // the flips that won all six claims are applied.  Lawson's flips end (each
 // one lowers the lifted surface), so the rounds end; a round limit turns a
@@ -403,22 +403,10 @@ __global__ void k_ins_apply(Mesh m, const int *__restrict__ pend, const int *npp
 
 // ---- flips ---------------------------------------------------------------
 
-// The first edge of triangle t towards a higher-numbered neighbour that wants a
-// flip (its index + 1, 0: none); the flip claims both triangles and the four outer
-// neighbours with the priority of 3 t + i.
+// The edge that triangle t flips this round (first_flip); the flip claims both triangles
+// and the four outer neighbours with the priority of 3 t + i.
 __device__ __forceinline__ int flip_mark_one(const Mesh &m, int t, Claim *cl, unsigned round) {
-  int c = 0, d[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {  // (the three apexes' loads together)
-    const int nb = m.nbr[3 * t + i];
-    d[i] = nb < 0 || cdt::nb_tri(nb) < t || ((m.cons[t] >> i) & 1)
-               ? -1
-               : m.tri[3 * cdt::nb_tri(nb) + cdt::nb_idx(nb)];
-  }
-#pragma unroll
-  for (int i = 2; i >= 0; --i)  // the first that wants a flip
-    if (d[i] >= 0 && cdt::incircle(m, m.tri[3 * t], m.tri[3 * t + 1], m.tri[3 * t + 2], d[i]))
-      c = i + 1;
+  const int c = cdt::first_flip(m, t);
   if (!c) return 0;
   const int i = c - 1;
   const Claim pr = claim_of(round, (unsigned)(3 * t + i));

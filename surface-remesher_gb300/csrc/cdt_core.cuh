@@ -327,7 +327,8 @@ CDT_HD void insert_fan(const Mesh &m, const Edge &edge, int cnt, int p, const Sl
   m.vt[p] = slot(0);
 }
 
-// The same with the edges (et[k], ei[k]) and the triangles slots[k] in arrays.
+// The same with the edges (et[k], ei[k]) and the triangles slots[k] in arrays (the
+// replay on the CPU; the kernels keep them as insert_fan takes them).
 CDT_HD void insert_out(const Mesh &m, const int *et, const int *ei, int cnt, int p,
                        const int *slots) {
   insert_fan(
@@ -379,14 +380,30 @@ CDT_HD void flip_claims(const Mesh &m, int t, int i, int (&id)[8]) {
   }
 }
 
-// Should the edge opposite vertex i of t be flipped for the Delaunay
-// property (it has a neighbour, is not a constraint, and the neighbour's
-// apex is inside t's circle)?
-CDT_HD bool wants_flip(const Mesh &m, int t, int i) {
+// The neighbour's apex across the edge opposite vertex i of t; none if the edge cannot
+// flip (a hull edge, a constraint) or the neighbour is below `from`.
+CDT_HD int flip_apex(const Mesh &m, int t, int i, int from) {
   const int opp = m.nbr[3 * t + i];
-  if (opp < 0 || ((m.cons[t] >> i) & 1)) return false;
-  const int d = m.tri[3 * nb_tri(opp) + nb_idx(opp)];
-  return incircle(m, m.tri[3 * t], m.tri[3 * t + 1], m.tri[3 * t + 2], d);
+  if (opp < 0 || nb_tri(opp) < from || ((m.cons[t] >> i) & 1)) return kNone;
+  return m.tri[3 * nb_tri(opp) + nb_idx(opp)];
+}
+// Should an edge with the apex d across it be flipped for the Delaunay property (d
+// inside t's circle)?
+CDT_HD bool flips_apex(const Mesh &m, int t, int d) {
+  return d != kNone && incircle(m, m.tri[3 * t], m.tri[3 * t + 1], m.tri[3 * t + 2], d);
+}
+CDT_HD bool wants_flip(const Mesh &m, int t, int i) {
+  return flips_apex(m, t, flip_apex(m, t, i, 0));
+}
+// The first edge of t towards a higher-numbered neighbour that wants a flip (its index
+// + 1, 0: none; each edge is tested from one side).  The three apexes first: their loads
+// are in flight together.
+CDT_HD int first_flip(const Mesh &m, int t) {
+  const int d[3] = {flip_apex(m, t, 0, t), flip_apex(m, t, 1, t), flip_apex(m, t, 2, t)};
+  int c = 0;
+  for (int i = 2; i >= 0; --i)
+    if (flips_apex(m, t, d[i])) c = i + 1;
+  return c;
 }
 
 // The triangle with the directed edge (u, w) (u at index *oi, w next), found

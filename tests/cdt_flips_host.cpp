@@ -43,15 +43,19 @@ int main(int argc, char **argv) {
     std::vector<unsigned> cl(T, 0xffffffffu);
     bool any = false;
     int id[8];
-    for (int t = 0; t < T; ++t)
-      for (int i = 0; i < 3 && edge[t] < 0; ++i) {
-        if (nbr[3 * t + i] < 0 || nb_tri(nbr[3 * t + i]) < t || !wants_flip(m, t, i)) continue;
-        edge[t] = i;
-        any = true;
-        flip_claims(m, t, i, id);
-        for (int k : id) cl[k] = std::min(cl[k], prio((unsigned)(3 * t + i)));
-      }
-    if (!any) return printf("ok %d %ld\n", round, hull), 0;
+    for (int t = 0; t < T; ++t) {
+      const int i = edge[t] = first_flip(m, t) - 1;
+      if (i < 0) continue;
+      any = true;
+      flip_claims(m, t, i, id);
+      for (int k : id) cl[k] = std::min(cl[k], prio((unsigned)(3 * t + i)));
+    }
+    if (!any) {  // Delaunay: no edge of any triangle wants a flip
+      for (int t = 0; t < T; ++t)
+        for (int i = 0; i < 3; ++i)
+          if (wants_flip(m, t, i)) return printf("error left\n"), 0;
+      return printf("ok %d %ld\n", round, hull), 0;
+    }
     std::vector<int> won, lost;
     // (-1: an index out of range)
     auto owns = [&](int t) -> int {
