@@ -479,13 +479,13 @@ __global__ void __launch_bounds__(kOneThreads) k_insert_all(Mesh m, int *pend, i
                                                             int rounds, int *ntri, int cap,
                                                             int *done, uint8_t *act, int *list,
                                                             int *list2, int *cand, int *left,
-                                                            int *err) {
+                                                            bool marked, int *err) {
   __shared__ int s_np, s_n, s_n2, s_stop;
   const int tid = threadIdx.x;
   if (tid == 0) s_n = s_stop = 0;
   __syncthreads();
   // the triangles that rounds over the grid left marked
-  for (int w = tid, T = *ntri; 4 * w < T; w += kOneThreads)
+  for (int w = tid, T = marked ? *ntri : 0; 4 * w < T; w += kOneThreads)
     for (unsigned q = reinterpret_cast<const unsigned *>(act)[w] & 0x01010101u; q; q &= q - 1u) {
       const int t = 4 * w + (__ffs((int)q) - 1) / 8;
       if (t < T) list[atomicAdd(&s_n, 1)] = t;
@@ -940,7 +940,7 @@ int cdt_compute(const uint64_t *bits, const uint64_t *fixed, int n, unsigned *co
       if (!la || !lb) return GCVT_ERR_ALLOC;
       k_insert_all<<<1, kOneThreads, 0, s>>>(m, pend, start, pend2, start2, np, loc, cl, round,
                                              kInsertRounds, ctr + 1, cap_t, done, act, la, lb, cand,
-                                             ctr + 4, ctr);
+                                             ctr + 4, C > kOneBlock, ctr);
       CCK(cudaGetLastError());
       round += (1 + kInterimFlips) * kInsertRounds + kFlipRounds;
       if ((rc = pull())) return rc;
