@@ -158,15 +158,8 @@ __device__ __forceinline__ int isqrt_ceil(int v) {
   return h * h == v ? h : h + 1;
 }
 
-// floor(N / D) for D > 0, exact: from a float estimate when |N| < 2^24 (then
-// the estimate is within 1 of it), else by integer division.
-__device__ __forceinline__ int floordiv_est(int N, int D, float inv, bool fast) {
-  if (fast) {
-    int q = __float2int_rd(__fmul_rn((float)N, inv));
-    const int r = N - q * D;
-    q += (r >= D) - (r < 0);
-    return q;
-  }
+// floor(N / D) for D > 0, exact, by integer division.
+__device__ __forceinline__ int floordiv(int N, int D) {
   int q = N / D;
   if ((N % D != 0) && (N < 0)) --q;
   return q;
@@ -177,8 +170,8 @@ __device__ __forceinline__ int floordiv_est(int N, int D, float inv, bool fast) 
 __device__ __forceinline__ void constrain_rel(int A, int B, int v, int &lo, int &hi) {
   if (A == 0) return;
   const int N = A * A + B * B - 2 * B * v;
-  if (A > 0) hi = min(hi, floordiv_est(N, 2 * A, 0.f, false));
-  else lo = max(lo, floordiv_est(-N, -2 * A, 0.f, false) + 1);
+  if (A > 0) hi = min(hi, floordiv(N, 2 * A));
+  else lo = max(lo, floordiv(-N, -2 * A) + 1);
 }
 
 __device__ __forceinline__ uint64_t row_mask(int lo_i, int hi_i) {  // bits lo_i..hi_i
@@ -233,8 +226,8 @@ __device__ __forceinline__ RowPair row_bounds2(const int2 *rec, int cnt, bool ov
         q0 = floordiv_r(N0, aD, rr);
         q1 = floordiv_r(N1, aD, rr);
       } else {
-        q0 = floordiv_est(N0, aD, 0.f, false);
-        q1 = floordiv_est(N1, aD, 0.f, false);
+        q0 = floordiv(N0, aD);
+        q1 = floordiv(N1, aD);
       }
       if (D > 0) {
         p.hi0 = min(p.hi0, q0);
@@ -1166,7 +1159,7 @@ __device__ __forceinline__ bool warp_row(const int2 *__restrict__ support, const
       const int D = (int)(int16_t)((unsigned)r.y >> 16);
       const int aD = abs(D), N = r.x - S * v;
       const int q = fast ? floordiv_r(N, aD, rcp_approx((float)aD))
-                         : floordiv_est(N, aD, 0.f, false);
+                         : floordiv(N, aD);
       if (D > 0) h = min(h, q);
       else l = max(l, q + 1);
     }
