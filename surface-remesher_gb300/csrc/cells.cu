@@ -1,6 +1,7 @@
-// cells.cu -- one Lloyd iteration as two launches: k_list lays the current
-// sites out in bitmap order, then k_cell lets every site compute its own
-// Voronoi cell exactly, sum the density moments over it, and move.
+// cells.cu -- one Lloyd iteration: k_list lays the current sites out in bitmap
+// order, then k_cell (k_cell_warp for fewer sites) lets every site compute its own
+// Voronoi cell exactly, sum the density moments over it, and move; up to 8192
+// sites both in one launch (k_cell_few).
 //
 // In a Lloyd iteration the labels themselves are never needed, only each
 // site's sums over its cell (gcvt.cu:1008-1023) and the energy

@@ -23,15 +23,15 @@
 // inside the current hull never becomes a neighbour later; an inserted one
 // removes the neighbours it covers).  What bounds the star kernel is issue
 // slots, and at the end the few sites on the hull whose flat triangles take
-// many searches.  4096^2, 262,144 CVT sites: 1.43 ms with one warp per site
+// many searches, one after the other in their warp.  4096^2, 262,144 CVT sites: 1.43 ms with one warp per site
 // inserting every candidate (3,913 instructions a site), 0.29 ms now.
 // Certificate, exact: a triangle of the star is final when no site
 // outside the window lies in its circumcircle, an open angular gap (>= pi)
 // when no site lies strictly inside its cone (then the site is on the
 // sites' convex hull); both are searched through a pyramid of tile
-// occupancy, and a site found is inserted and the star checked again.  Only
-// a star of fewer than two neighbours widens the window (a window covering
-// the grid is exact).  Warps take the sites in tile order; a triangle is
+// occupancy, and a site found is inserted and the star checked again.  After
+// the second window only a star of fewer than two neighbours, or on one line,
+// widens it (a window covering the grid is exact).  Warps take the sites in tile order; a triangle is
 // written by its vertex that comes first in delaunayInput's order (x, then
 // y), counter-clockwise, so the output does not depend on the scheduling.
 #include "gcvt_internal.cuh"
