@@ -113,3 +113,51 @@ def test_one_context_with_changing_counts(gcvt_lib, cuda_device, n, gaussians):
         assert ctx.info() == one.info(), m
         one.close()
     ctx.close()
+
+
+def crowded(kind, n, rng):
+    if kind == "circle":  # cells reach across the empty inside
+        t = rng.uniform(0, 2 * np.pi, 700)
+        return np.rint(n / 2 + (n * 0.4) * np.stack([np.cos(t), np.sin(t)], 1)).astype(int)
+    if kind == "cluster":
+        return np.clip(np.rint(n / 3 + rng.normal(0, 9, (800, 2))), 0, n - 1).astype(int)
+    if kind == "border":  # every second pixel of the border, two sites inside
+        t = np.arange(0, n, 2)
+        q = [np.stack([t, 0 * t], 1), np.stack([t, 0 * t + n - 1], 1), np.stack([0 * t, t], 1),
+             np.stack([0 * t + n - 1, t], 1)]
+        return np.concatenate(q + [np.array([(n // 2, n // 3), (n // 2, n // 3 + 9)])])
+    if kind == "line":  # a full column and its neighbours
+        t = np.arange(0, n)
+        return np.concatenate([np.stack([0 * t + n // 2 + d, t], 1)[d & 1::1 + d % 3] for d in range(5)])
+    b = int(kind)  # that many sites around a lone one, so that its window holds them all
+    a = np.stack(np.meshgrid(np.arange(12), np.arange(12)), -1).reshape(-1, 2)[:b]
+    return np.concatenate([a + n // 2, [(n // 2 + 60, n // 2 + 6)]])
+
+
+@pytest.mark.parametrize("n,kind", [(512, "circle"), (768, "circle"), (512, "cluster"),
+                                    (768, "cluster"), (512, "border"), (512, "line"),
+                                    (256, "127"), (256, "128"), (256, "129"), (256, "144")])
+def test_crowded_windows_by_warps(gcvt_lib, oracle, cuda_device, n, kind):
+    """Windows of more candidates than a warp's list holds (128): a site per warp, with
+    and without the list launch, against a site per lane, bit for bit, and the first
+    iteration's energy against FP64."""
+    rng = np.random.default_rng(n)
+    q = np.unique(crowded(kind, n, rng), axis=0)
+    sites = gcvt_lib.sites_from_points(n, q[:, 0], q[:, 1])
+    rho = gaussian_density(n, 6, 4.0, 0.05, 0.2, 3)
+    fixed = np.zeros((n, n), np.uint8)
+    fixed[q[::7, 1], q[::7, 0]] = 1
+    _, _, energy, _ = oracle.lloyd_step(sites, rho, fixed, 2.0)
+    ctx = gcvt_lib.Context(n)
+    runs = []
+    for mode in (1, 2, 0):
+        ctx.set_tuning(cell_mode=mode)
+        ctx.load(sites, rho, fixed)
+        ctx.iterate(1)
+        first = ctx.info()["energy"]
+        assert abs(first - energy) <= 1e-5 * energy
+        ctx.iterate(3)
+        runs.append((ctx.sites(), ctx.info()))
+    for r in runs[1:]:
+        assert np.array_equal(r[0], runs[0][0]) and r[1] == runs[0][1]
+    ctx.close()
