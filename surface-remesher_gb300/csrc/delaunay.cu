@@ -803,8 +803,9 @@ __device__ __forceinline__ int wnext(const WStar &s, int k) {
 // it (as around irregular sites), the window grows once before any search
 // (wrapping again costs less than searching); then the certificate settles the
 // triangles exactly, and only a star of fewer than two neighbours doubles the
-// window again.  More than 64 candidates are inserted ring by ring instead of
-// wrapped.  (kWindow 1.6 to 2.3 and kGrow 1.5 to 2 measure within 5 %, kWiden 3 or
+// window again.  More than 64 candidates (a crowded or uneven neighbourhood) take windows
+// of kRing spacings, doubled, wrapped if that leaves few enough, else inserted ring by
+// ring: what is inserted one by one counts there.  (kWindow 1.6 to 2.3 and kGrow 1.5 to 2 measure within 5 %, kWiden 3 or
 // never 8 % slower on irregular sites.)  A star whose sites all lie on one line
 // widens up to kLine first: the next row of a lattice is nearer than what a search of
 // the gap's half plane finds.  Returns false when the star
@@ -830,13 +831,20 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
                      sqrtf((float)(tiles * kTile * kTile) / (float)max(cnt, 1u)));
   W = min(max(W, 4), 2 * n);
   int x0 = sx, x1 = sx, y0 = sy, y1 = sy;  // the window so far: the site
-  bool first = true, wrap = !rings;
+  bool first = true, wrap = !rings, small = rings;
   for (;;) {
     const int nx0 = max(0, sx - W), nx1 = min(n - 1, sx + W);
     const int ny0 = max(0, sy - W), ny1 = min(n - 1, sy + W);
     // wrapped in the first two windows while the candidates are few, then ring by ring
     // (the star so far is the one of every site of the window before)
-    wrap = wrap && wwrap(st, bits, fixed, n, sx, sy, nx0, nx1, ny0, ny1, reinterpret_cast<int *>(stk));
+    const bool few = wrap && wwrap(st, bits, fixed, n, sx, sy, nx0, nx1, ny0, ny1,
+                                   reinterpret_cast<int *>(stk));
+    if (wrap && !few && !small) {  // crowded: the smaller windows
+      small = true;
+      W = max(4, (int)ceilf(kRing / kWindow * W));
+      continue;
+    }
+    wrap = few;
     if (!wrap) wwindow(st, bits, fixed, n, sx, sy, py, nx0, nx1, ny0, ny1, x0, x1, y0, y1);
     x0 = nx0;
     x1 = nx1;
@@ -939,7 +947,7 @@ __device__ bool wsite_star(WStar &st, const uint64_t *bits, const uint64_t *fixe
     } while (changed);
     if (ok) return true;
     wrap = wrap && first;
-    W = first && !rings ? min((int)ceilf(kGrow * W), 2 * n) : min(2 * W, 2 * n);
+    W = first && !small ? min((int)ceilf(kGrow * W), 2 * n) : min(2 * W, 2 * n);
     first = false;
   }
 }
