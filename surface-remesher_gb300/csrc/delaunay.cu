@@ -984,14 +984,21 @@ __global__ void k_dt_up(const uint8_t *__restrict__ lo, int nlo, uint8_t *hi, in
   hi[i] = v;
 }
 
+// The four-site form's lists (quad_stars): candidates, neighbours.  In a tile of which
+// more than half is sites its smallest window (9 x 9 pixels) holds about 40: that form
+// would try and leave its four sites to one warp, one after the other, so they take a
+// warp each (a block of 121 x 121 sites 812 -> 691 us).
+constexpr int kQuadCand = 32, kQuadStar = 16;
+constexpr unsigned kTileCrowd = kTile * kTile / 2;
+
 // Edge tiles first: an occupied tile with an empty tile (or the grid's edge)
 // among its eight neighbours holds the sites whose stars reach far (flat
 // triangles along the sites' boundary, convex-hull gaps).  Their sites are
 // listed before the interior ones so the long stars start first instead of
-// finishing last.  cnt2[c * ntiles + i]: the sites of brick-order tile i in
-// class c (0 edge, 1 interior).
+// finishing last.  ccnt[c * ntiles + i]: the sites of brick-order tile i in
+// class c (0 edge, 1 crowded, 2 interior).
 __global__ void k_dt_class(const uint8_t *__restrict__ occ0, int nt0,
-                           const unsigned *__restrict__ tilecnt, unsigned *cnt2, uint8_t *cls) {
+                           const unsigned *__restrict__ tilecnt, unsigned *ccnt, uint8_t *cls) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nt0 * nt0) return;
   const int brick = i / (kBrick * kBrick), in = i % (kBrick * kBrick);
@@ -1004,9 +1011,9 @@ __global__ void k_dt_class(const uint8_t *__restrict__ occ0, int nt0,
       edge |= x < 0 || y < 0 || x >= nt0 || y >= nt0 || !occ0[y * nt0 + x];
     }
   const unsigned c = tilecnt[i];
-  cnt2[i] = edge ? c : 0u;
-  cnt2[nt0 * nt0 + i] = edge ? 0u : c;
-  cls[i] = edge ? 0 : 1;
+  const int k = edge ? 0 : (c > kTileCrowd ? 1 : 2);
+  for (int j = 0; j < 3; ++j) ccnt[(size_t)j * nt0 * nt0 + i] = j == k ? c : 0u;
+  cls[i] = (uint8_t)k;
 }
 
 // Per column: free sites in the bands before each band, and in the column.
@@ -1114,7 +1121,6 @@ __device__ __noinline__ void full_site(const uint64_t *bits, const uint64_t *fix
 // full_site (none of 258,177 interior sites at 4096^2).  A warp per site by wwrap
 // alone took 1,449 instructions a site, this 600.
 constexpr float kQuadWindow = 1.8f;
-constexpr int kQuadCand = 32, kQuadStar = 16;
 struct QuadScratch {
   int cand[4][kQuadCand];
   int star[4][kQuadStar];
@@ -1293,7 +1299,8 @@ __device__ __forceinline__ unsigned quad_stars(const uint64_t *bits, const uint6
 }
 
 // The stars of the sites in tile order: a warp per site for the nedge sites
-// of edge tiles (their stars reach far), four sites per warp for the others.
+// of edge tiles (their stars reach far) and crowded ones, four sites per warp for the
+// others.
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, 5)
     k_dt_star(const uint64_t *__restrict__ bits, const uint64_t *__restrict__ fixed, int n,
               int nsites, int nedge, Pyr py, TileSites ts, StarOut out) {
@@ -1382,8 +1389,8 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
   const int nt0 = n / kTile, ntiles = nt0 * nt0;
   unsigned *colpre = sc.take<unsigned>(nb), *colcnt = sc.take<unsigned>(n),
            *coloff = sc.take<unsigned>(n + 1),
-           *tilecnt = sc.take<unsigned>(ntiles), *cnt2 = sc.take<unsigned>(2 * (size_t)ntiles),
-           *tileoff = sc.take<unsigned>(2 * (size_t)ntiles + 1);
+           *tilecnt = sc.take<unsigned>(ntiles), *ccnt = sc.take<unsigned>(3 * (size_t)ntiles),
+           *tileoff = sc.take<unsigned>(3 * (size_t)ntiles + 1);
   uint8_t *cls = sc.take<uint8_t>(ntiles);
   int *err = sc.take<int>(1);
   Pyr py{};
@@ -1400,7 +1407,7 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
   }
   uint8_t *occ = sc.take<uint8_t>(occ_bytes);
   py.occ = occ;
-  if (!colpre || !colcnt || !coloff || !tilecnt || !cnt2 || !tileoff || !cls || !err ||
+  if (!colpre || !colcnt || !coloff || !tilecnt || !ccnt || !tileoff || !cls || !err ||
       !occ)
     return GCVT_ERR_ALLOC;
   DCK(cudaMemsetAsync(err, 0, sizeof(int), s));
@@ -1417,12 +1424,12 @@ int delaunay_sites_in(const uint64_t *bits, const uint64_t *fixed, int n, int *t
   }
   int rc = scan(colcnt, n, coloff, sc, s);
   if (rc) return rc;
-  k_dt_class<<<nblk(ntiles, 256), 256, 0, s>>>(occ, nt0, tilecnt, cnt2, cls);
+  k_dt_class<<<nblk(ntiles, 256), 256, 0, s>>>(occ, nt0, tilecnt, ccnt, cls);
   DCK(cudaGetLastError());
-  if ((rc = scan(cnt2, 2 * ntiles, tileoff, sc, s))) return rc;
+  if ((rc = scan(ccnt, 3 * ntiles, tileoff, sc, s))) return rc;
   unsigned nsites_u = 0, nedge_u = 0;
   DCK(cudaMemcpyAsync(&nsites_u, coloff + n, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-  DCK(cudaMemcpyAsync(&nedge_u, tileoff + ntiles, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+  DCK(cudaMemcpyAsync(&nedge_u, tileoff + 2 * ntiles, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   DCK(cudaStreamSynchronize(s));
   
   const int nsites = (int)nsites_u, nedge = (int)nedge_u;
