@@ -187,3 +187,25 @@ def test_label_into_other_buffers(gcvt_lib, oracle, cuda_device):
         assert rc == 3 or (rc == 0 and np.array_equal(out, want))  # GCVT_ERR_CUDA
     assert np.array_equal(ctx.label(), want)  # the context goes on
     ctx.close()
+
+
+@pytest.mark.parametrize("n,kind", [(768, "circle"), (1024, "circle"), (2304, "circle"),
+                                    (1024, "column"), (768, "diagonal"), (2304, "diagonal"),
+                                    (2304, "solid"), (1024, "rings"), (768, "late")])
+def test_many_candidates(gcvt_lib, oracle, cuda_device, n, kind):
+    """Tiles of more candidates than their list holds: the middle of a
+    circle of sites (all at one distance, mirror pairs across bands among them), a full
+    column or diagonal, concentric circles; and a solid block, whose sites do not fit the
+    far blocks' lists either."""
+    t = np.arange(6 * n) * (2 * np.pi / (6 * n))
+    cs = np.stack([np.cos(t), np.sin(t)], 1)
+    q = {"circle": lambda: np.rint(n / 2 + 0.45 * n * cs),
+         "rings": lambda: np.concatenate([np.rint(n / 2 + r * n * cs) for r in (0.2, 0.35, 0.48)]),
+         "column": lambda: np.stack([np.full(n, n // 2), np.arange(n)], 1),
+         "diagonal": lambda: np.stack([np.arange(n), n - 1 - np.arange(n)], 1),
+         "solid": lambda: np.stack(np.meshgrid(np.arange(300, 560), np.arange(310, 540)), -1).reshape(-1, 2),
+         "late": lambda: np.concatenate([np.stack(np.meshgrid(np.arange(14), np.arange(14)), -1)
+                                         .reshape(-1, 2) + (420, 300), [(700, 60)]])}[kind]()
+    q = np.unique(q.astype(int), axis=0)
+    g = gcvt_lib.sites_from_points(n, q[:, 0], q[:, 1])
+    assert np.array_equal(gcvt_lib.label_grid(g), oracle.spec_label(g))
