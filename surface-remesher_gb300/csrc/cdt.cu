@@ -456,12 +456,12 @@ __global__ void k_flip_apply(Mesh m, const int *ntri, const int *cand, const Cla
     if (cand[t] && flip_apply_one(m, t, cand[t], cl, round, Act{act})) atomicAdd(flips, 1);
 }
 
-// Every insertion round with its flip rounds in one block: the rounds are chains of short dependent steps (832 boundary points take 28
-// rounds; as seven launches each 74 us a round, 55 in one block of 1024 threads, 85 in
-// one of 256; 36 with short predicates and the loads and marks of a triangle's
-// neighbours in flight together), and the changed triangles are listed instead of
-// searched for.  Block barriers order the steps.  After the last point the flips run
-// until none is left.
+// Every insertion round with its flip rounds in one block: the rounds are chains of short
+// dependent steps (832 boundary points take 28 rounds; as seven launches each 74 us a
+// round, 55 in one block of 1024 threads, 85 in one of 256; 36 with short predicates and
+// the loads and marks of a triangle's neighbours in flight together), and the changed
+// triangles are listed instead of searched for.  Block barriers order the steps.  After the
+// last point the flips run until none is left.
 //   Up to kOneBlock points it does them all.  Above, points inside the sites go in
 // fastest over the grid, nearly all in the first rounds, while of a chain of boundary
 // points few win a round and each round's latency counts.  So up to kOneChain the first
